@@ -248,6 +248,50 @@ __device__ __forceinline__ void soap_fma2(float &x, float &y, float a, float b, 
         : "f"(a), "f"(b), "f"(c), "f"(d));
 }
 
+// Correctly rounded quotients by one divisor (the bits of __ddiv_rn) for one FP64
+// instruction each: q0 = y * rn(1 / n) lies within 1.5 ulp of y / n, so the quotient's
+// significand is that of q0 or a neighbour, and the remainder y - q0 n, an exact integer in
+// units of ulp(q0) ulp(n) below 2^56, says which: its low 64 bits come from three integer
+// multiplications (a quotient of two doubles never lies half way between two others).  The
+// FP64 pipe issues 2 lanes per cycle and SM against 64 on the integer pipes, so the integer
+// work costs less than the two FP64 FMAs of the usual correction.  Needs n > 0, and n, y and
+// q0 normal (the callers check exponents).  A quotient whose low word is 0 (zeros, powers of
+// two, where the neighbours are unevenly spaced) takes the division itself.
+struct QuotBy {
+    double n, r;        // divisor, rn(1 / n)
+    unsigned nlo, nhi;  // its significand
+    int c;              // 1043 - its biased exponent
+};
+__device__ __forceinline__ QuotBy soap_quot_by(double n) {
+    QuotBy d;
+    d.n = n;
+    d.r = __drcp_rn(n);
+    const unsigned hi = (unsigned)__double2hiint(n);
+    d.nlo = (unsigned)__double2loint(n);
+    d.nhi = (hi & 0xfffffu) | 0x100000u;
+    d.c = 1075 - 32 - (int)(hi >> 20);
+    return d;
+}
+__device__ __forceinline__ double soap_quot(double y, const QuotBy &d) {
+    const double q0 = __dmul_rn(y, d.r);
+    const unsigned ql = (unsigned)__double2loint(q0), qh = (unsigned)__double2hiint(q0);
+    if (ql == 0u) return __ddiv_rn(y, d.n);
+    const unsigned yl = (unsigned)__double2loint(y), yh = (unsigned)__double2hiint(y);
+    const unsigned long long p = (unsigned long long)ql * d.nlo;
+    const unsigned ph = (unsigned)(p >> 32) + ql * d.nhi + ((qh & 0xfffffu) | 0x100000u) * d.nlo;
+    const int sh = (int)((yh >> 20) - (qh >> 20)) + d.c;
+    const unsigned long long rem =
+        ((unsigned long long)(yl << sh) << 32) - (((unsigned long long)ph << 32) | (unsigned)p);
+    const long long two = (long long)(rem << 1), N = (long long)(((unsigned long long)d.nhi << 32) | d.nlo);
+    const int adj = (two > N ? 1 : 0) - (two < -N ? 1 : 0);
+    return __longlong_as_double(__double_as_longlong(q0) + adj);
+}
+// biased exponent of |v| within [1023 - span, 1023 + span]: a normal number of moderate size
+__device__ __forceinline__ bool soap_moderate(double v, int span) {
+    const int e = (int)(((unsigned)__double2hiint(v) >> 20) & 0x7ffu);
+    return e >= 1023 - span && e <= 1023 + span;
+}
+
 // Delta_lambda, SOAP_initialize.cu:55-66
 __device__ __forceinline__ double soap_delta_lambda(double line_width, double lambda_line0) {
     double beta = line_width / SOAP_C_LIGHT;
