@@ -11,6 +11,7 @@
 
 #include "internal.cuh"
 #include "fir.cuh"
+#include "plain64.cuh"
 
 using namespace soapgb;
 
@@ -107,14 +108,10 @@ int compact_cells(soapgb_ctx *ctx, int n_lists, int cells_per_list, const double
 }  // namespace soapgb
 
 // --------------------------------------------------------------------------
-// a4-a7 plain FP64: per-pixel gather over all visible cells, in map order.
-// The arithmetic of one (cell, pixel) term is the reference's:
-//   (S[i] + (S[i+1]-S[i]) / (l'_{i+1} - l'_i) * (l_j - l'_i)) * limb
-// with one IEEE rounding per operation (no contraction), so the sum is bit-equal
-// to a sequential CPU loop over cells.
+// a4-a7 plain FP64: per-pixel gather over all visible cells, in map order (plain64.cuh:
+// the reference's expression with one IEEE rounding per operation, so the sum is bit-equal
+// to a sequential CPU loop over cells).
 // --------------------------------------------------------------------------
-constexpr int QUIET_CHUNK = 512;
-
 __device__ __forceinline__ double soap_cell_value(long long j, int n_eff, const double *__restrict__ lam,
                                                   const double *__restrict__ row, double delta,
                                                   double limb, const CellShift &c) {
@@ -131,54 +128,115 @@ __device__ __forceinline__ double soap_cell_value(long long j, int n_eff, const 
     return __dmul_rn(__dadd_rn(s0, t), limb);
 }
 
-__global__ void __launch_bounds__(256) k_quiet_plain64(int n, int n_eff, const double *__restrict__ lam,
-                                                       const double *__restrict__ cube,
-                                                       const int *__restrict__ n_cells_ptr,
-                                                       const int *__restrict__ cells,
-                                                       const double *__restrict__ delta_m,
-                                                       const double *__restrict__ limb_m,
-                                                       const int *__restrict__ region_m, double step, int n_mu,
-                                                       double *__restrict__ out, int *status) {
-    __shared__ double s_delta[QUIET_CHUNK], s_limb[QUIET_CHUNK], s_fb[QUIET_CHUNK], s_sq[QUIET_CHUNK],
-        s_off[QUIET_CHUNK];
-    __shared__ int s_row[QUIET_CHUNK];
-    long long j = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    double lambda0 = lam[0];
+__global__ void __launch_bounds__(64) k_plain_cells(long long gm, int n_eff, const double *__restrict__ lam,
+                                                   const double *__restrict__ delta_m, double step,
+                                                   PlainGeo *__restrict__ geo) {
+    const long long k = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    if (k >= gm) return;
+    const double l0 = lam[0], l1 = lam[n_eff - 1], d = (l1 - l0) / (double)(n_eff - 1);
+    const CellShift c = soap_cell_shift(delta_m[k], l0, step);
+    PlainGeo &g = geo[k];
+    const double u = __dsub_rn(1.0, c.sq), F = 1.0 + c.fbeta;
+    g.sq = c.sq;
+    g.fbeta = c.fbeta;
+    g.off = c.off;
+    g.u = u;
+    g.iF = 1.0 / F;
+    // the reference's x_i carry an error below 2^-51 (3 n + |off|), the tile's z below
+    // 2^-50 (n + |off|); a cell near the speed of light searches per pixel
+    g.eps = F > 0.5 ? 1.8e-15 * (4.0 * (double)n_eff + 2.0 * fabs(c.off) + 4.0) : 2.0;
+    // exact: u is a multiple of 2^-53 (without a table it is not used)
+    const double au = fabs(u);
+    g.w = au < 0x1p-10 ? (unsigned long long)__double2ll_rn(au * 0x1p+53) << PL_FRAC : 0ULL;
+    g.zone = (long long)(g.w >> 53) + 2;
+    pl_table(l0, d, c.sq, u, g.tab[0]);
+    if (pl_exp(l1 - l1 * u) == g.tab[0].ex) g.tab[1].ex = -1;
+    else pl_table(l1, d, c.sq, u, g.tab[1]);
+}
+
+namespace soapgb {
+int plain_cells(soapgb_ctx *ctx, long long gm, int n_eff, const double *d_wave, const double *d_delta, double step,
+                PlainGeo *geo) {
+    SOAP_TRACED(ctx, "plain_cells", k_plain_cells<<<(unsigned)((gm + 63) / 64), 64, 0, ctx->stream>>>(
+                                        gm, n_eff, d_wave, d_delta, step, geo));
+    SOAP_LAUNCHED(ctx);
+    return SOAPGB_OK;
+}
+}  // namespace soapgb
+
+// A block takes PL_TILE pixels, a thread one, all cells in order.  Small blocks: 100,000 px
+// are 10.6 blocks per SM.
+__global__ void __launch_bounds__(PL_THREADS) k_quiet_plain64(int n, int n_eff, const double *__restrict__ lam,
+                                                              const double *__restrict__ cube,
+                                                              const int *__restrict__ n_cells_ptr,
+                                                              const int *__restrict__ cells,
+                                                              const PlainGeo *__restrict__ geo,
+                                                              const double *__restrict__ delta_m,
+                                                              const double *__restrict__ limb_m,
+                                                              const int *__restrict__ region_m, int n_mu,
+                                                              double *__restrict__ out, int *status) {
+    __shared__ PlainRec s_rec[PL_CHUNK];
+    __shared__ unsigned long long s_tab[PL_CHUNK][PL_TAB];
+    __shared__ int s_cell[PL_CHUNK];
+    const int lane = threadIdx.x & 31;
+    const int j0 = blockIdx.x * PL_TILE, j = j0 + (threadIdx.x >> 5) * 31 + lane;
+    const int cnt = max(1, min(PL_TILE, n_eff - j0));
+    const double lmid = lam[min(j0 + cnt / 2, n_eff - 1)];
+    const bool mine = j < n_eff && lane != 31;
+    const double lj = lam[min(j, n_eff - 1)];
     double sum = 0.0;
-    int n_cells = *n_cells_ptr;
-    for (int c0 = 0; c0 < n_cells; c0 += QUIET_CHUNK) {
-        int nc = min(QUIET_CHUNK, n_cells - c0);
+    PlainPix px;
+    PlainVal va;
+    int row_now = -1, m_now = 0;
+    const int n_cells = *n_cells_ptr;
+    for (int c0 = 0; c0 < n_cells; c0 += PL_CHUNK) {
+        const int nc = min(PL_CHUNK, n_cells - c0);
         __syncthreads();
-        for (int t = threadIdx.x; t < nc; t += blockDim.x) {
-            int k = cells[c0 + t];
-            double d = delta_m[k];
-            CellShift cs = soap_cell_shift(d, lambda0, step);
-            s_delta[t] = d;
-            s_limb[t] = limb_m[k];
-            s_fb[t] = cs.fbeta;
-            s_sq[t] = cs.sq;
-            s_off[t] = cs.off;
+        if (threadIdx.x < nc) {
+            const int k = cells[c0 + threadIdx.x];
             int row = region_m[k];
             if ((unsigned)row >= (unsigned)n_mu) {   // mu bin outside the cube: report, use bin 0
                 atomicExch(status, 21);
                 row = 0;
             }
-            s_row[t] = row;
+            s_cell[threadIdx.x] = k;
+            pl_stage(geo + k, delta_m[k], limb_m[k], row, j0, cnt, lmid, s_rec[threadIdx.x], s_tab[threadIdx.x]);
         }
         __syncthreads();
-        if (j < n_eff) {
-            for (int t = 0; t < nc; ++t) {
-                CellShift cs;
-                cs.fbeta = s_fb[t];
-                cs.sq = s_sq[t];
-                cs.off = s_off[t];
-                const double *row = cube + (long long)s_row[t] * n;
-                sum = __dadd_rn(sum, soap_cell_value(j, n_eff, lam, row, s_delta[t], s_limb[t], cs));
+        for (int t = 0; t < nc; ++t) {
+            const PlainRec c = s_rec[t];
+            const double *row = cube + (long long)c.row * n;
+            if (c.flags != PL_CONST) {
+                if (mine) {
+                    const PlainGeo &g = geo[s_cell[t]];
+                    CellShift cs;
+                    cs.sq = g.sq;
+                    cs.fbeta = g.fbeta;
+                    cs.off = g.off;
+                    sum = __dadd_rn(sum, soap_cell_value(j, n_eff, lam, row, c.flags == PL_STILL ? 0.0 : 1.0, c.limb, cs));
+                }
+                continue;
             }
+            if (c.row != row_now || c.m != m_now) {
+                row_now = c.row;
+                m_now = c.m;
+                const int i = min(max(j + c.m, 0), n_eff - 1);
+                px.li = lam[i];
+                px.lm = pl_sig(px.li);
+                px.ok = pl_load(va, row, i, min(i + 1, n_eff - 1));
+            }
+            const double ls = pl_shifted(c, px), ls1 = __shfl_down_sync(0xffffffffu, ls, 1);
+            // lanes without a pixel here must not send their warp the other way
+            const bool in = mine && (unsigned)(j + c.m) <= (unsigned)(n_eff - 2);
+            int k;
+            double X, rise;
+            if ((pl_interval(c, lj, ls, ls1, k, X) && px.ok) || !in) rise = pl_rise(c, va, s_tab[t][k], k, X);
+            else rise = pl_rise_plain(va.g, lj, ls, ls1);
+            const double r = __dadd_rn(sum, __dmul_rn(__dadd_rn(va.s0, rise), c.limb));
+            if (in) sum = r;
         }
     }
-    if (j < n_eff) out[j] = sum;
-    else if (j < n) out[j] = 0.0;
+    if (lane != 31 && j < n) out[j] = mine ? sum : 0.0;
 }
 
 // --------------------------------------------------------------------------
@@ -321,9 +379,11 @@ extern "C" int soapgb_quiet_disk(soapgb_ctx *ctx, int form, int n, int n_eff, co
         // visible cells in map order (limb map is -999 elsewhere)
         rc = compact_cells(ctx, 1, (int)gm, d_limb, -998.0, 1e300, (int)gm, d_cells, d_count);
         if (rc) return rc;
-        SOAP_TRACED(ctx, "quiet_plain64", k_quiet_plain64<<<grid_for(ctx, n, 256), 256, 0, ctx->stream>>>(n, n_eff, d_wave, d_cube, d_count, d_cells,
-                                                                         d_delta, d_limb, d_region, step, n_mu, d_out,
-                                                                         ctx->d_status));
+        PlainGeo *geo = ws.get<PlainGeo>(s_fir);
+        rc = plain_cells(ctx, gm, n_eff, d_wave, d_delta, step, geo);
+        if (rc) return rc;
+        SOAP_TRACED(ctx, "quiet_plain64", k_quiet_plain64<<<(n + PL_TILE - 1) / PL_TILE, PL_THREADS, 0, ctx->stream>>>(
+            n, n_eff, d_wave, d_cube, d_count, d_cells, geo, d_delta, d_limb, d_region, n_mu, d_out, ctx->d_status));
         SOAP_LAUNCHED(ctx);
     } else {
         FirQuietArgs qa;

@@ -30,6 +30,7 @@
 #include <type_traits>
 
 #include "fir.cuh"
+#include "plain64.cuh"
 #include "regions.cuh"
 
 using namespace soapgb;
@@ -2475,7 +2476,10 @@ FirLayout fir_layout(int form, int n, int n_mu, long long gm, int ncube, int n_l
 
 FirPlanSizes fir_plan_sizes(int form, int n, int n_mu, long long gm, bool phase, int n_lists, bool typed_external) {
     FirPlanSizes p;
-    if (form == SOAPGB_PLAIN64) return p;
+    if (form == SOAPGB_PLAIN64) {   // the cells' Doppler constants
+        p.bytes = sizeof(PlainGeo) * (size_t)gm;
+        return p;
+    }
     p.bytes = fir_layout(form, n, n_mu, gm, phase ? 6 : 1, n_lists > 0 ? n_lists : 1, typed_external).total;
     return p;
 }

@@ -10,6 +10,7 @@
 
 #include "internal.cuh"
 #include "fir.cuh"
+#include "plain64.cuh"
 
 using namespace soapgb;
 
@@ -56,100 +57,149 @@ __device__ __forceinline__ double soap_lerp_at(const CellAt &a, long long j, con
     return __dmul_rn(__dadd_rn(s0, t), limb);
 }
 
-__global__ void __launch_bounds__(256) k_phase_plain64(
+// one active cell's three rows and intensity
+struct PhaseCell {
+    int k;          // map index
+    int type;       // 0 spot, 1 facula
+    int unit;       // 1: the intensity is the continuum row itself, 0: scale x the row, -1: a Planck ratio
+    double scale;   // 1 + LB
+};
+
+// cell intensity I at pixel j (fast_intensity / fast_intensity_fac / the solar form)
+__device__ __forceinline__ double soap_intensity(int type, double T, double lbk, double lj, double ssed, double fsed,
+                                                 int solar, int t_norm_fac) {
+    if (type == 0) {
+        // fast_intensity with T_norm = (int)T: the Planck ratio is exactly 1 for whole temperatures
+        const int tn = (int)T;
+        const double ratio = ((double)tn == T) ? 1.0 : soap_planck(lj, T) / soap_planck(lj, (double)tn);
+        return __dmul_rn(ratio, ssed);
+    }
+    if (solar) {
+        const double ratio = ((double)t_norm_fac == T) ? 1.0 : soap_planck(lj, T) / soap_planck(lj, (double)t_norm_fac);
+        return __dmul_rn(ratio, fsed);
+    }
+    return __dmul_rn(__dadd_rn(1.0, lbk), fsed);
+}
+
+// The plain form: block (x, p) sums phase p's active cells, in map order, over a tile of
+// pixels (plain64.cuh); three rows per cell.
+__global__ void __launch_bounds__(PL_THREADS) k_phase_plain64(
     int n, int n_eff, const double *__restrict__ lam, const double *__restrict__ q_norm,
     const double *__restrict__ q_sed, const double *__restrict__ spot_norm, const double *__restrict__ fac_norm,
     const double *__restrict__ spot_sed, const double *__restrict__ fac_sed, int max_cells,
     const int *__restrict__ cells, const int *__restrict__ counts, const double *__restrict__ temp,
-    const double *__restrict__ bi, const double *__restrict__ delta_m, const double *__restrict__ limb_m,
-    const double *__restrict__ lb_m, const int *__restrict__ region_m, long long gm, double step, int solar,
-    int t_star, int t_diff_fac, double *__restrict__ flux, double *__restrict__ bconv, double *__restrict__ tot,
-    long long out_stride, int n_mu, int *status) {
-    __shared__ double s_delta[PHASE_CHUNK], s_limb[PHASE_CHUNK], s_fb[PHASE_CHUNK], s_sq[PHASE_CHUNK],
-        s_off[PHASE_CHUNK], s_lb[PHASE_CHUNK], s_temp[PHASE_CHUNK];
-    __shared__ int s_row[PHASE_CHUNK], s_type[PHASE_CHUNK];
-    int p = blockIdx.y;
-    long long j = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    double lambda0 = lam[0];
+    const double *__restrict__ bi, const PlainGeo *__restrict__ geo, const double *__restrict__ delta_m,
+    const double *__restrict__ limb_m, const double *__restrict__ lb_m, const int *__restrict__ region_m,
+    long long gm, int solar, int t_star, int t_diff_fac, double *__restrict__ flux, double *__restrict__ bconv,
+    double *__restrict__ tot, long long out_stride, int n_mu, int *status) {
+    __shared__ PlainRec s_rec[PL_CHUNK];
+    __shared__ unsigned long long s_tab[PL_CHUNK][PL_TAB];
+    __shared__ PhaseCell s_cell[PL_CHUNK];
+    const int p = blockIdx.y, lane = threadIdx.x & 31;
+    const int j0 = blockIdx.x * PL_TILE, j = j0 + (threadIdx.x >> 5) * 31 + lane;
+    const int cnt = max(1, min(PL_TILE, n_eff - j0));
     const int *pc = cells + (long long)p * max_cells;
-    int nc_all = counts[p];
+    const int nc_all = counts[p];
     const double *pt = temp + (long long)p * gm;
     const double *pb = bi + (long long)p * gm;
+    const double lmid = lam[min(j0 + cnt / 2, n_eff - 1)];
+    const int t_norm_fac = (int)(t_star + t_diff_fac + 0.9 - 216.8);
+    const bool mine = j < n_eff && lane != 31;
+    const int jc = min(j, n_eff - 1);
+    const double lj = lam[jc], ssed = spot_sed[jc], fsed = fac_sed[jc];
     double fx = 0.0, bc = 0.0, tt = 0.0;
-    double lj = (j < n_eff) ? lam[j] : 0.0;
-    double ssed = (j < n_eff) ? spot_sed[j] : 0.0;
-    double fsed = (j < n_eff) ? fac_sed[j] : 0.0;
-    int t_norm_fac = (int)(t_star + t_diff_fac + 0.9 - 216.8);
-    for (int c0 = 0; c0 < nc_all; c0 += PHASE_CHUNK) {
-        int nc = min(PHASE_CHUNK, nc_all - c0);
+    PlainPix px;
+    PlainVal va[3];
+    int row_now = -1, m_now = 0, type_now = 0;
+    for (int c0 = 0; c0 < nc_all; c0 += PL_CHUNK) {
+        const int nc = min(PL_CHUNK, nc_all - c0);
         __syncthreads();
-        for (int t = threadIdx.x; t < nc; t += blockDim.x) {
-            int k = pc[c0 + t];
-            double d = delta_m[k];
-            CellShift cs = soap_cell_shift(d, lambda0, step);
-            s_delta[t] = d;
-            s_limb[t] = limb_m[k];
-            s_fb[t] = cs.fbeta;
-            s_sq[t] = cs.sq;
-            s_off[t] = cs.off;
+        if (threadIdx.x < nc) {
+            const int k = pc[c0 + threadIdx.x];
             int row = region_m[k];
             if ((unsigned)row >= (unsigned)n_mu) {   // mu bin outside the cube: report, use bin 0
                 atomicExch(status, 21);
                 row = 0;
             }
-            s_row[t] = row;
-            s_lb[t] = lb_m[k];
-            s_temp[t] = pt[k];
-            s_type[t] = (pb[k] == 0.0) ? 0 : 1;
+            PhaseCell a;
+            const double T = pt[k];
+            a.k = k;
+            a.type = (pb[k] == 0.0) ? 0 : 1;
+            a.scale = 1.0;
+            if (a.type == 0) {
+                a.unit = ((double)(int)T == T) ? 1 : -1;
+            } else if (solar) {
+                a.unit = ((double)t_norm_fac == T) ? 1 : -1;
+            } else {
+                a.unit = 0;
+                a.scale = __dadd_rn(1.0, lb_m[k]);
+            }
+            s_cell[threadIdx.x] = a;
+            pl_stage(geo + k, delta_m[k], limb_m[k], row, j0, cnt, lmid, s_rec[threadIdx.x], s_tab[threadIdx.x]);
         }
         __syncthreads();
-        if (j < n_eff) {
-            for (int t = 0; t < nc; ++t) {
+        for (int t = 0; t < nc; ++t) {
+            const PlainRec c = s_rec[t];
+            const PhaseCell a = s_cell[t];
+            const long long off = (long long)c.row * n;
+            const double *an = (a.type == 0 ? spot_norm : fac_norm) + off;
+            double q, s, v;
+            if (c.flags != PL_CONST) {   // the pixel itself, or an owner search per pixel
+                const PlainGeo &g = geo[a.k];
                 CellShift cs;
-                cs.fbeta = s_fb[t];
-                cs.sq = s_sq[t];
-                cs.off = s_off[t];
-                double d = s_delta[t], L = s_limb[t];
-                long long off = (long long)s_row[t] * n;
+                cs.sq = g.sq;
+                cs.fbeta = g.fbeta;
+                cs.off = g.off;
+                const double d = c.flags == PL_STILL ? 0.0 : 1.0;
                 CellAt at;
-                if (d != 0.0) at = soap_cell_at(j, n_eff, lam, cs);
-                double q = soap_lerp_at(at, j, q_norm + off, d, L);
-                double s = soap_lerp_at(at, j, q_sed + off, d, L);
-                double a, inten;
-                if (s_type[t] == 0) {
-                    // fast_intensity with T_norm = (int)T: the Planck ratio is exactly 1
-                    double T = s_temp[t];
-                    int tn = (int)T;
-                    double ratio = ((double)tn == T) ? 1.0 : soap_planck(lj, T) / soap_planck(lj, (double)tn);
-                    inten = __dmul_rn(ratio, ssed);
-                    a = soap_lerp_at(at, j, spot_norm + off, d, L);
-                } else {
-                    if (solar) {
-                        double T = s_temp[t];
-                        double ratio = ((double)t_norm_fac == T) ? 1.0
-                                                                  : soap_planck(lj, T) / soap_planck(lj, (double)t_norm_fac);
-                        inten = __dmul_rn(ratio, fsed);
-                    } else {
-                        inten = __dmul_rn(__dadd_rn(1.0, s_lb[t]), fsed);
-                    }
-                    a = soap_lerp_at(at, j, fac_norm + off, d, L);
+                at.i = -1;
+                if (d != 0.0) at = soap_cell_at(jc, n_eff, lam, cs);
+                q = soap_lerp_at(at, jc, q_norm + off, d, c.limb);
+                s = soap_lerp_at(at, jc, q_sed + off, d, c.limb);
+                v = soap_lerp_at(at, jc, an, d, c.limb);
+            } else {
+                if (c.row != row_now || c.m != m_now || a.type != type_now) {
+                    row_now = c.row;
+                    m_now = c.m;
+                    type_now = a.type;
+                    const int i = min(max(j + c.m, 0), n_eff - 1), i1 = min(i + 1, n_eff - 1);
+                    px.li = lam[i];
+                    px.lm = pl_sig(px.li);
+                    const bool ok0 = pl_load(va[0], q_norm + off, i, i1), ok1 = pl_load(va[1], q_sed + off, i, i1);
+                    px.ok = pl_load(va[2], an, i, i1) && ok0 && ok1;
                 }
-                fx = __dsub_rn(__dadd_rn(fx, s), __dmul_rn(inten, q));
-                bc = __dsub_rn(__dadd_rn(bc, q), a);
-                tt = __dsub_rn(__dadd_rn(tt, s), __dmul_rn(a, inten));
+                const double ls = pl_shifted(c, px), ls1 = __shfl_down_sync(0xffffffffu, ls, 1);
+                // lanes without a pixel here must not send their warp the other way
+                const bool in = mine && (unsigned)(j + c.m) <= (unsigned)(n_eff - 2);
+                int k;
+                double X, x[3];
+                if ((pl_interval(c, lj, ls, ls1, k, X) && px.ok) || !in) {
+                    const unsigned long long rec = s_tab[t][k];
+#pragma unroll
+                    for (int r = 0; r < 3; ++r) x[r] = pl_rise(c, va[r], rec, k, X);
+                } else {
+#pragma unroll
+                    for (int r = 0; r < 3; ++r) x[r] = pl_rise_plain(va[r].g, lj, ls, ls1);
+                }
+#pragma unroll
+                for (int r = 0; r < 3; ++r) x[r] = __dmul_rn(__dadd_rn(va[r].s0, x[r]), c.limb);
+                q = in ? x[0] : 0.0;
+                s = in ? x[1] : 0.0;
+                v = in ? x[2] : 0.0;
             }
+            double I = a.type == 0 ? ssed : fsed;
+            if (a.unit == 0) I = __dmul_rn(a.scale, I);
+            else if (a.unit < 0) I = soap_intensity(a.type, pt[a.k], lb_m[a.k], lj, ssed, fsed, solar, t_norm_fac);
+            fx = __dsub_rn(__dadd_rn(fx, s), __dmul_rn(I, q));
+            bc = __dsub_rn(__dadd_rn(bc, q), v);
+            tt = __dsub_rn(__dadd_rn(tt, s), __dmul_rn(v, I));
         }
     }
-    long long o = (long long)p * out_stride + j;
-    if (j < n_eff) {
-        flux[o] = fx;
-        bconv[o] = bc;
-        tot[o] = tt;
-    } else if (j < n) {
-        flux[o] = 0.0;
-        bconv[o] = 0.0;
-        tot[o] = 0.0;
-    }
+    if (lane == 31 || j >= n) return;
+    const long long o = (long long)p * out_stride + j;
+    flux[o] = mine ? fx : 0.0;
+    bconv[o] = mine ? bc : 0.0;
+    tot[o] = mine ? tt : 0.0;
 }
 
 // ---------------------------------------------------------------------------
@@ -202,21 +252,6 @@ __global__ void k_adj_bucket(int n_mu, long long gm, const int *__restrict__ cel
         if ((unsigned)row >= (unsigned)n_mu) row = 0;
         pr[cur[row]++] = pc[c];
     }
-}
-
-// cell intensity I at pixel j (fast_intensity / fast_intensity_fac / the solar form)
-__device__ __forceinline__ double soap_intensity(int type, double T, double lbk, double lj, double ssed, double fsed,
-                                                 int solar, int t_norm_fac) {
-    if (type == 0) {
-        const int tn = (int)T;
-        const double ratio = ((double)tn == T) ? 1.0 : soap_planck(lj, T) / soap_planck(lj, (double)tn);
-        return __dmul_rn(ratio, ssed);
-    }
-    if (solar) {
-        const double ratio = ((double)t_norm_fac == T) ? 1.0 : soap_planck(lj, T) / soap_planck(lj, (double)t_norm_fac);
-        return __dmul_rn(ratio, fsed);
-    }
-    return __dmul_rn(__dadd_rn(1.0, lbk), fsed);
 }
 
 // Per-cell constants of the adjoint weights.  In exact arithmetic the shifted grid is
@@ -567,10 +602,12 @@ int integrate_device(soapgb_ctx *ctx, int form, int n, int n_eff, const double *
     if (form == SOAPGB_PLAIN64) {
         int rc = compact_cells(ctx, n_phase, (int)gm, d_bi, -0.5, 1.5, (int)gm, d_cells, d_counts);
         if (rc) return rc;
-        dim3 g(grid_for(ctx, n, 256), n_phase);
-        SOAP_TRACED(ctx, "integrate_plain64", k_phase_plain64<<<g, 256, 0, ctx->stream>>>(
+        PlainGeo *geo = (PlainGeo *)fir_scratch;   // PLAIN64 has no plans: its cells' constants stand there
+        rc = plain_cells(ctx, gm, n_eff, d_wave, dm.delta, step, geo);
+        if (rc) return rc;
+        SOAP_TRACED(ctx, "integrate_plain64", k_phase_plain64<<<dim3((n + PL_TILE - 1) / PL_TILE, n_phase), PL_THREADS, 0, ctx->stream>>>(
             n, n_eff, d_wave, dc.q_norm, dc.q_sed, dc.spot_norm, dc.fac_norm, dc.spot_sed, dc.fac_sed, (int)gm,
-            d_cells, d_counts, d_temp, d_bi, dm.delta, dm.limb, dm.lb, dm.region, gm, step, act->solar,
+            d_cells, d_counts, d_temp, d_bi, geo, dm.delta, dm.limb, dm.lb, dm.region, gm, act->solar,
             act->t_star, act->t_diff_fac, (double *)d_flux, (double *)d_bconv, (double *)d_tot, out_stride, dc.n_mu,
             ctx->d_status));
         SOAP_LAUNCHED(ctx);

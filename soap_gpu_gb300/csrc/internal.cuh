@@ -255,7 +255,7 @@ __device__ __forceinline__ void soap_fma2(float &x, float &y, float a, float b, 
 // multiplications (a quotient of two doubles never lies half way between two others).  The
 // FP64 pipe issues 2 lanes per cycle and SM against 64 on the integer pipes, so the integer
 // work costs less than the two FP64 FMAs of the usual correction.  Needs n > 0, and n, y and
-// q0 normal (the callers check exponents).  A quotient whose low word is 0 (zeros, powers of
+// q0 normal or y zero (the callers check exponents).  A quotient whose low word is 0 (zeros, powers of
 // two, where the neighbours are unevenly spaced) takes the division itself.
 struct QuotBy {
     double n, r;        // divisor, rn(1 / n)

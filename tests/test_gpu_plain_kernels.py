@@ -60,3 +60,59 @@ def test_plain_convolution(ctx, kind, n, n_spec, reso):
             continue
         assert np.allclose(mm[s], ext, rtol=1e-12, atol=0)
         assert np.max(np.abs(got[s] - ref)) <= 1e-12 * np.max(np.abs(ref))
+
+
+def _disk(grid, vsini, lambda0, n_mu):
+    lb = (0.2, -0.4, 0.3, -0.1)
+    period = 2 * np.pi * 696000.0 / (vsini * 86400.0)
+    return oracle.disk_maps(grid, period, -0.18, 80.0, 696000.0, 0.3, 0.3, np.linspace(0.95, 0.15, n_mu - 1), lb)
+
+
+def _cube(n, n_mu, rng, kind):
+    x = np.arange(n)
+    y = 1.0 - 0.5 * np.exp(-((x % 61) - 30.0) ** 2 / 20.0)
+    y = y[None, :] * (1 + 1e-3 * rng.uniform(-1, 1, (n_mu, n)))
+    if kind == "flat":        # stretches of equal values, negative and positive zeros
+        y[:, n // 4:n // 2] = 1.0
+        y[:, n // 2:n // 2 + 40] = np.where(x[:40] % 3 == 0, -0.0, 0.0)
+    if kind == "wild":        # infinities, NaN, tiny and huge neighbours
+        for k, v in enumerate((np.inf, np.nan, -np.inf, 1e-310, 1e300, 2.0 ** -1000)):
+            y[k % n_mu, n // 3 + 60 * k] = v
+    return y
+
+
+# grids inside a binade and across one (4096 A), an uneven one, ends of tiles of 62 pixels, one
+# pixel count below a tile, slow and fast rotators (above 290 km/s the integer form has no range)
+@pytest.mark.parametrize("lambda0,step,n,vsini,uneven,kind", [
+    (5000.0, 0.01, 62 * 9 + 1, 4.0, False, "lines"), (5000.0, 0.005, 1300, 4.0, False, "flat"),
+    (4092.0, 0.01, 1024, 10.0, False, "lines"), (3800.0, 0.01, 2050, 40.0, False, "wild"),
+    (5000.0, 0.01, 1100, 400.0, False, "lines"), (5000.0, 0.01, 1100, 5.0, True, "lines"),
+    (6000.0, 0.02, 41, 0.5, False, "lines"), (5000.0, 0.0078125, 700, 3.0, False, "lines")])
+def test_plain_sums_are_the_sequential_ones(ctx, lambda0, step, n, vsini, uneven, kind):
+    """Quiet disk and per-phase integration equal the oracle's loops bit for bit."""
+    rng = np.random.default_rng(n)
+    grid, n_mu = 14, 4
+    n_eff = n if n < 62 else n - 7
+    wave = lambda0 + step * np.arange(n)
+    if uneven:
+        wave = wave + step * 0.2 * np.sin(np.arange(n) / 50.0)
+    maps = _disk(grid, vsini, lambda0, n_mu)
+    vis = np.nonzero(maps["limb"] > -998)[0]
+    cube = [_cube(n, n_mu, rng, kind) for _ in range(4)]
+    with np.errstate(all="ignore"):
+        ref = oracle.quiet_disk(wave, cube[0], n_eff, maps, grid, step)
+        got = ctx.quiet_disk("plain64", wave, cube[0], n_eff, maps, grid, step)
+        assert np.array_equal(got, ref, equal_nan=True)
+        bi = np.full(grid * grid, -9999.0)
+        bi[vis[::3]], bi[vis[1::3]] = 0.0, 1.0
+        temp = np.where(bi == 0.0, 5115.0, np.where(bi == 1.0, 5900.0, -9999.0))
+        sed = 0.3 + 0.1 * np.arange(n) / n, 1.0 + 0.1 * np.arange(n) / n
+        from soap_gpu_gb300._lib import Activity
+        names = ("q_norm", "q_sed", "spot_norm", "fac_norm")
+        out = ctx.phase_integrate("plain64", wave, n_eff, grid, np.stack([temp, temp]), np.stack([bi, -9999.0 + 0 * bi]),
+                                  maps, dict(zip(names, cube), spot_sed=sed[0], fac_sed=sed[1]), step,
+                                  Activity(5778, 663, 250, 20, 0))
+        want = oracle.phase_integrate(wave, n_eff, grid, temp, bi, maps, *cube, sed[0], sed[1], step)
+    for o, r in zip(out, want):
+        assert np.array_equal(o[0], r, equal_nan=True)
+        assert not o[1].any()
