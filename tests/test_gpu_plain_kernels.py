@@ -116,3 +116,50 @@ def test_plain_sums_are_the_sequential_ones(ctx, lambda0, step, n, vsini, uneven
     for o, r in zip(out, want):
         assert np.array_equal(o[0], r, equal_nan=True)
         assert not o[1].any()
+
+
+# the adjoint's ranges of equal offsets: tiles of 31 and 256 pixels and their ends, cells at rest
+# (even grids have a column of them), more than 64 offsets in a row, Planck ratios, uneven grids
+@pytest.mark.parametrize("lambda0,step,n,vsini,grid,uneven,solar", [
+    (5000.0, 0.01, 1300, 4.0, 14, False, False), (5000.0, 0.005, 249, 9.0, 13, False, False),
+    (4092.0, 0.01, 1030, 10.0, 14, False, True), (6000.0, 0.01, 900, 60.0, 21, False, False),
+    (5000.0, 0.01, 700, 5.0, 14, True, False), (5000.0, 0.01, 20, 2.0, 8, False, False)])
+def test_adjoint_is_the_transpose(ctx, lambda0, step, n, vsini, grid, uneven, solar):
+    """<W, J V> = <J^T W, V> over the cubes, the continuum rows and the limb map, in which the
+    integration is linear.  Bound: the forward rounds its interpolation weights to 2 ulp(lambda) /
+    step, at most 4e-10 here, so 1e-9 |W| |J V|.  The velocity gradient against a central difference
+    in a common factor of the velocities, 1e-4 (relative step 1e-6, as in the parity of vsini)."""
+    from soap_gpu_gb300._lib import Activity
+    rng = np.random.default_rng(n)
+    n_mu, n_eff = 4, n if n < 256 else n - 5
+    wave = lambda0 + step * np.arange(n)
+    if uneven:
+        wave = wave + step * 0.2 * np.sin(np.arange(n) / 50.0)
+    maps = _disk(grid, vsini, lambda0, n_mu)
+    vis = np.nonzero(maps["limb"] > -998)[0]
+    gm = grid * grid
+    bi = np.full((2, gm), -9999.0)
+    bi[0, vis[::2]], bi[0, vis[1::4]], bi[1, vis[::5]] = 0.0, 1.0, 1.0
+    temp = np.where(bi == 0.0, 5115.0, np.where(bi == 1.0, 5900.0 + np.arange(gm) % 40, -9999.0))
+    temp[0, vis[0]] = 5115.5                      # a spot whose Planck ratio is not 1
+    act = Activity(5778, 663, 250, 20, int(solar))
+    names = ("q_norm", "q_sed", "spot_norm", "fac_norm", "spot_sed", "fac_sed")
+    x = dict(zip(names, [_cube(n, n_mu, rng, "lines") for _ in range(4)] +
+                 [0.3 + 0.1 * np.arange(n) / n, 1.0 + 0.1 * np.arange(n) / n]))
+    W = rng.standard_normal((3, 2, n))
+    fwd = lambda m, c: np.stack(ctx.phase_integrate("plain64", wave, n_eff, grid, temp, bi, m, c, step, act))
+    g = ctx.phase_integrate_adjoint(wave, n_eff, grid, temp, bi, maps, x, step, act, *W)
+    close = lambda jv, rhs: abs((W * jv).sum() - rhs) <= 1e-9 * np.linalg.norm(W) * np.linalg.norm(jv)
+    V = {k: rng.standard_normal(x[k].shape) for k in names[:4]}
+    assert close(fwd(maps, dict(V, spot_sed=x["spot_sed"], fac_sed=x["fac_sed"])),
+                 sum((g[k] * V[k]).sum() for k in V))
+    S = {k: rng.standard_normal(n) for k in names[4:]}
+    zero = {k: np.zeros(n) for k in S}
+    assert close(fwd(maps, dict(x, **S)) - fwd(maps, dict(x, **zero)), sum((g[k] * S[k]).sum() for k in S))
+    dl = rng.standard_normal(gm)
+    assert close(fwd(dict(maps, limb=dl), x), (g["limb"] * dl).sum())
+    h = 1e-6
+    scaled = [fwd(dict(maps, delta=np.where(maps["limb"] > -998, maps["delta"] * (1 + s), -999.0)), x) for s in (h, -h)]
+    jv = (scaled[0] - scaled[1]) / (2 * h)
+    rhs = (g["delta"] * np.where(maps["limb"] > -998, maps["delta"], 0.0)).sum()
+    assert abs((W * jv).sum() - rhs) <= 1e-4 * np.linalg.norm(W) * np.linalg.norm(jv)
