@@ -222,7 +222,7 @@ __global__ void __launch_bounds__(PL_THREADS) k_quiet_plain64(int n, int n_eff, 
                 m_now = c.m;
                 const int i = min(max(j + c.m, 0), n_eff - 1);
                 px.li = lam[i];
-                px.lm = pl_sig(px.li);
+                px.lm = soap_sig(px.li);
                 px.ok = pl_load(va, row, i, min(i + 1, n_eff - 1));
             }
             const double ls = pl_shifted(c, px), ls1 = __shfl_down_sync(0xffffffffu, ls, 1);

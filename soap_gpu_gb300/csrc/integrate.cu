@@ -138,7 +138,7 @@ __global__ void __launch_bounds__(PL_THREADS) k_phase_plain64(
                     type_now = a.type;
                     const int i = min(max(j + c.m, 0), n_eff - 1), i1 = min(i + 1, n_eff - 1);
                     px.li = lam[i];
-                    px.lm = pl_sig(px.li);
+                    px.lm = soap_sig(px.li);
                     const bool ok0 = pl_load(va[0], q_norm + off, i, i1), ok1 = pl_load(va[1], q_sed + off, i, i1);
                     px.ok = pl_load(va[2], an, i, i1) && ok0 && ok1;
                 }

@@ -248,43 +248,62 @@ __device__ __forceinline__ void soap_fma2(float &x, float &y, float a, float b, 
         : "f"(a), "f"(b), "f"(c), "f"(d));
 }
 
-// Correctly rounded quotients by one divisor (the bits of __ddiv_rn) for one FP64
-// instruction each: q0 = y * rn(1 / n) lies within 1.5 ulp of y / n, so the quotient's
-// significand is that of q0 or a neighbour, and the remainder y - q0 n, an exact integer in
-// units of ulp(q0) ulp(n) below 2^56, says which: its low 64 bits come from three integer
-// multiplications (a quotient of two doubles never lies half way between two others).  The
-// FP64 pipe issues 2 lanes per cycle and SM against 64 on the integer pipes, so the integer
-// work costs less than the two FP64 FMAs of the usual correction.  Needs n > 0, and n, y and
-// q0 normal or y zero (the callers check exponents).  A quotient whose low word is 0 (zeros, powers of
-// two, where the neighbours are unevenly spaced) takes the division itself.
+// Correctly rounded quotients (the bits of __ddiv_rn) on the integer pipes: with the divisor's
+// 64-bit reciprocal at hand, a 64-bit product gives the quotient's significand with 10 bits to
+// spare, which decide the rounding; only a quotient within their error of a rounding boundary (a
+// half is never met: a quotient of two doubles does not lie half way between two others) needs the
+// sign of its exact remainder, whose low 64 bits three more multiplications give.  The FP64 pipe
+// issues 2 lanes per cycle and SM against 64 on the integer pipes, and a division is about ten FP64
+// instructions.
+//
+// |v|'s significand with its leading bit at bit 63 (v normal)
+__device__ __forceinline__ unsigned long long soap_sig(double v) {
+    return (((unsigned long long)__double_as_longlong(v)) << 11) | 0x8000000000000000ULL;
+}
+// floor(2^127 / n) to within 1: n's leading bit at bit 63, r = 2^63 / n in FP64
+__device__ __forceinline__ unsigned long long soap_recip64(unsigned long long n, double r) {
+    unsigned long long r0 = r >= 1.0 ? ~0ULL : soap_sig(r);
+    // one Newton step in integers: r0 += r0 (2^127 - n r0) / 2^127
+    const unsigned long long hi = __umul64hi(n, r0), lo = n * r0;
+    const long long d = (long long)(((0x8000000000000000ULL - hi - (lo != 0ULL ? 1ULL : 0ULL)) << 32) |
+                                    ((0ULL - lo) >> 32));   // (2^127 - n r0) / 2^32
+    const long long c = (d >> 12) * (long long)(r0 >> 32) >> 51;
+    const unsigned long long s = r0 + (unsigned long long)c;
+    return (c > 0 && s < r0) ? ~0ULL : s;
+}
+// The bits of y / d: y and the quotient normal, sig = soap_sig(y); d = n 2^x > 0 with the integer n
+// (leading zeros lz), rec its reciprocal, qe = 1023 - (d's biased exponent)
+__device__ __forceinline__ unsigned long long soap_quot_bits(double y, unsigned long long sig, unsigned long long rec,
+                                                             unsigned long long n, int lz, int qe) {
+    unsigned long long q = __umul64hi(sig, rec);   // the quotient's leading 63 or 64 bits: within (-1, +2)
+    const int top = (int)(q >> 63);
+    q <<= 1 - top;
+    unsigned long long s = q >> 11;
+    const unsigned low = (unsigned)q & 0x7ffu;
+    unsigned up = low >> 10;
+    if (low - 1019u <= 10u)   // near a boundary: the remainder against s + 1/2
+        up = (long long)(((sig >> 11) << (65 - lz - top)) - (2ULL * s + 1ULL) * n) > 0 ? 1u : 0u;
+    s += up;
+    // exponent - 1: the significand's leading bit adds the one
+    const unsigned hi = (unsigned)__double2hiint(y);
+    const unsigned e = ((hi >> 20) & 0x7ffu) + (unsigned)(qe + top - 2);
+    return s + ((unsigned long long)((e << 20) + (hi & 0x80000000u)) << 32);
+}
+// a divisor used many times: positive and normal
 struct QuotBy {
-    double n, r;        // divisor, rn(1 / n)
-    unsigned nlo, nhi;  // its significand
-    int c;              // 1043 - its biased exponent
+    unsigned long long rec, n;
+    int qe;
 };
-__device__ __forceinline__ QuotBy soap_quot_by(double n) {
-    QuotBy d;
-    d.n = n;
-    d.r = __drcp_rn(n);
-    const unsigned hi = (unsigned)__double2hiint(n);
-    d.nlo = (unsigned)__double2loint(n);
-    d.nhi = (hi & 0xfffffu) | 0x100000u;
-    d.c = 1075 - 32 - (int)(hi >> 20);
-    return d;
+__device__ __forceinline__ QuotBy soap_quot_by(double d) {
+    QuotBy q;
+    const int hi = __double2hiint(d);
+    q.n = soap_sig(d) >> 11;
+    q.rec = soap_recip64(q.n << 11, 1.0 / __hiloint2double((hi & 0xfffff) | 0x3ff00000, __double2loint(d)));
+    q.qe = 1023 - (hi >> 20);
+    return q;
 }
 __device__ __forceinline__ double soap_quot(double y, const QuotBy &d) {
-    const double q0 = __dmul_rn(y, d.r);
-    const unsigned ql = (unsigned)__double2loint(q0), qh = (unsigned)__double2hiint(q0);
-    if (ql == 0u) return __ddiv_rn(y, d.n);
-    const unsigned yl = (unsigned)__double2loint(y), yh = (unsigned)__double2hiint(y);
-    const unsigned long long p = (unsigned long long)ql * d.nlo;
-    const unsigned ph = (unsigned)(p >> 32) + ql * d.nhi + ((qh & 0xfffffu) | 0x100000u) * d.nlo;
-    const int sh = (int)((yh >> 20) - (qh >> 20)) + d.c;
-    const unsigned long long rem =
-        ((unsigned long long)(yl << sh) << 32) - (((unsigned long long)ph << 32) | (unsigned)p);
-    const long long two = (long long)(rem << 1), N = (long long)(((unsigned long long)d.nhi << 32) | d.nlo);
-    const int adj = (two > N ? 1 : 0) - (two < -N ? 1 : 0);
-    return __longlong_as_double(__double_as_longlong(q0) + adj);
+    return __longlong_as_double((long long)soap_quot_bits(y, soap_sig(y), d.rec, d.n, 11, d.qe));
 }
 // biased exponent of |v| within [1023 - span, 1023 + span]: a normal number of moderate size
 __device__ __forceinline__ bool soap_moderate(double v, int span) {

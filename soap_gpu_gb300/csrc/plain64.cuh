@@ -19,9 +19,8 @@
 //    to one half that the reference's two roundings could go the other way (FP64 then).  l'_{i+1}
 //    is the next lane's l'_i (a shuffle), a warp's last one serving only for this;
 //  - the division.  On a grid of constant step l'_{i+1} - l'_i is one of a few neighbouring
-//    integers in units of ulp: the cell's table holds the 64-bit reciprocals of eight of them,
-//    and a 64-bit product gives the quotient with 10 bits to spare.  A quotient within those
-//    bits' error of a rounding boundary is decided by its exact remainder;
+//    integers in units of ulp: the cell's table holds the 64-bit reciprocals of eight of them for
+//    soap_quot_bits;
 //  - l_j - l'_i.  With X = 2^e + (l_j - l'_i), whose bits are an integer sum, slope x difference is
 //    fma(slope, X, -slope 2^e), rounded once.
 // A cell and pixel takes 4.4 FP64 instructions in the quiet sum (about 60 when every pixel
@@ -75,23 +74,6 @@ struct PlainRec {
 
 __device__ __forceinline__ int pl_exp(double v) { return (int)((unsigned)__double2hiint(v) >> 20); }
 
-// |v|'s significand with its leading bit at bit 63 (v normal)
-__device__ __forceinline__ unsigned long long pl_sig(double v) {
-    return (((unsigned long long)__double_as_longlong(v)) << 11) | 0x8000000000000000ULL;
-}
-
-// floor(2^127 / n) to within 1: n's leading bit at bit 63, r = 2^63 / n in FP64
-__device__ __forceinline__ unsigned long long pl_recip(unsigned long long n, double r) {
-    unsigned long long r0 = r >= 1.0 ? ~0ULL : pl_sig(r);
-    // one Newton step in integers: r0 += r0 (2^127 - n r0) / 2^127
-    const unsigned long long hi = __umul64hi(n, r0), lo = n * r0;
-    const long long d = (long long)(((0x8000000000000000ULL - hi - (lo != 0ULL ? 1ULL : 0ULL)) << 32) |
-                                    ((0ULL - lo) >> 32));   // (2^127 - n r0) / 2^32
-    const long long c = (d >> 12) * (long long)(r0 >> 32) >> 51;
-    const unsigned long long s = r0 + (unsigned long long)c;
-    return (c > 0 && s < r0) ? ~0ULL : s;
-}
-
 // The table of the binade of l (1 - u) around spacings d sq
 __device__ __forceinline__ void pl_table(double l, double d, double sq, double u, PlainTab &t) {
     t.ex = -1;
@@ -112,7 +94,7 @@ __device__ __forceinline__ void pl_table(double l, double d, double sq, double u
         const double nd = nm + (double)(k - PL_TAB / 2) * scale;
         // a Newton step from the middle one's reciprocal leaves (4 / n0)^2
         const double r = n0 >= (1LL << 27) ? fma(rm, fma(-nd, rm, 1.0), rm) : 1.0 / nd;
-        t.rec[k] = pl_recip((unsigned long long)(n0 + k) << lz, r);
+        t.rec[k] = soap_recip64((unsigned long long)(n0 + k) << lz, r);
     }
     t.base = n0;
     t.ex = ex;
@@ -166,7 +148,7 @@ __device__ __forceinline__ bool pl_zero(double g) {
 __device__ __forceinline__ bool pl_load(PlainVal &v, const double *__restrict__ row, int i, int i1) {
     v.s0 = row[i];
     v.g = __dsub_rn(row[i1], v.s0);
-    v.gm = pl_sig(v.g);
+    v.gm = soap_sig(v.g);
     return pl_zero(v.g) || soap_moderate(v.g, 700);
 }
 
@@ -201,23 +183,8 @@ __device__ __forceinline__ bool pl_interval(const PlainRec &c, double lj, double
 // slope x (l_j - l'_i) in integers: rec = floor(2^127 / n) of the interval n
 __device__ __forceinline__ double pl_rise(const PlainRec &c, const PlainVal &v, unsigned long long rec, int k,
                                           double X) {
-    unsigned long long q = __umul64hi(v.gm, rec);   // the quotient's leading 63 or 64 bits: within (-1, +2)
-    const int top = (int)(q >> 63);
-    q <<= 1 - top;
-    unsigned long long s = q >> 11;
-    const unsigned low = (unsigned)q & 0x7ffu;
-    unsigned up = low >> 10;
-    if (low - 1019u <= 10u) {   // near a boundary: the sign of the remainder against s + 1/2
-        const unsigned long long n = (unsigned long long)(c.base + k);
-        const int sh = 64 - (c.qe - 1012 + c.ex) + (1 - top);   // 64 - leading zeros of n, + 1 - top
-        up = (long long)(((v.gm >> 11) << sh) - (2ULL * s + 1ULL) * n) > 0 ? 1u : 0u;
-    }
-    const int hi = __double2hiint(v.g);
-    s += up;
-    // exponent - 1: the significand's leading bit adds the one
-    const unsigned e = ((unsigned)hi >> 20 & 0x7ffu) + (unsigned)(c.qe + top - 2);
     const unsigned long long bits =
-        s + ((unsigned long long)((e << 20) + ((unsigned)hi & 0x80000000u)) << 32);
+        soap_quot_bits(v.g, v.gm, rec, (unsigned long long)(c.base + k), c.qe - 1012 + c.ex, c.qe);
     const double slope = __longlong_as_double((long long)bits);
     const double scaled = __longlong_as_double((long long)((bits + ((unsigned long long)(long long)(c.ex - 1023) << 52)) ^
                                                            0x8000000000000000ULL));   // -slope 2^e

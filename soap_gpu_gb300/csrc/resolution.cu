@@ -114,17 +114,17 @@ __global__ void __launch_bounds__(256) k_conv_plain64(int n, int n_eff, const do
 // spectra [blockIdx.y per, + per).  The weights e^{-d^2 step^2 / (2 s_i^2)} do not depend on the
 // spectrum and are even in d: each thread keeps those of its pixel, d = 0 .. reach, in shared
 // memory for all its spectra.  The spectra's terms step_mult (1 - A) are staged once per block,
-// and the division by s_i sqrt(2 pi) is a soap_quot, so a tap costs three FP64 instructions
-// (quotient, product, sum) instead of about 55.
+// and the division by s_i sqrt(2 pi) is a soap_quot, so a tap costs two FP64 instructions
+// (product, sum) instead of about 55.
 // Taps with a weight below e^-90 are left out: to the right of the centre they cannot change
 // the rounded sum (below a quarter of its ulp), to the left they change its last bit with a
 // probability of about 1e-17 per pixel (the early partial sums' error is rounded away as the
 // weights grow).  That holds for a block's spectrum whose terms in the whole reference window
 // are finite and within a factor 2^20 of one another (continuum and lines of a disk sum are);
 // another one (NaN, infinities, zeros next to large values) goes through conv_plain64_pixel.
-// Bound by the FP64 pipe: (2 reach + 1) x 3 instructions per pixel and spectrum and
+// Bound by the FP64 pipe: (2 reach + 1) x 2 instructions per pixel and spectrum and
 // (reach + 1) x 20 for the weights per pixel and block.  One spectrum of 310,000 px:
-// 3.28 -> 0.78 ms per call; 10 of 100,000 px, forward and adjoint: 36.2 -> 9.9 ms.
+// 3.28 -> 0.71 ms per call; 10 of 100,000 px: 13.9 -> 0.45 ms.
 constexpr int CP_PIX = 128;
 constexpr double CP_CUT = 90.0;
 constexpr int CP_SMEM_MAX = 200 * 1024;
@@ -158,7 +158,8 @@ __global__ void __launch_bounds__(CP_PIX) k_conv_plain64t(int n, int n_eff, cons
     QuotBy by = soap_quot_by(1.0);
     if (!odd_block && live) {
         by = soap_quot_by(den);
-        for (int d = 0; d <= reach; ++d)
+        wt[t] = 1.0;   // exp(0)
+        for (int d = 1; d <= reach; ++d)
             wt[d * CP_PIX + t] = exp(soap_quot(__dmul_rn(__dmul_rn((double)(-d * d), step_exp), step_exp), by));
         by = soap_quot_by(norm);
     }
@@ -211,6 +212,32 @@ __global__ void __launch_bounds__(CP_PIX) k_conv_plain64t(int n, int n_eff, cons
     }
 }
 
+// reach in pixels of the widest Gaussian's weights above e^-CP_CUT (sigma grows with wavelength);
+// pixels that it does not cover take the general form in the kernels
+static int conv_reach(double sigma_v, double wave0, double wave_last, double step_exp, int wid) {
+    const double sig = soap_sigma_per_lambda(sigma_v) * std::max(std::fabs(wave0), std::fabs(wave_last));
+    const double r = std::floor(sqrt(2.0 * CP_CUT) * sig / step_exp * 1.0001) + 1.0;
+    return (r > 0.0 && r < (double)wid) ? (int)r : wid;
+}
+
+// Spectra per block when every block computes its weights (`once` FP64 instructions per pixel) and then
+// its spectra (`each`): the split of the spectra over the blocks that leaves the fullest SM the least.
+static int conv_per_block(soapgb_ctx *ctx, int bx, int n_spec, long long once, long long each) {
+    const long long sms = std::max(ctx->num_sms, 1);
+    long long best = -1;
+    int per = n_spec;
+    for (int groups = 1; groups <= std::min(n_spec, 64); ++groups) {
+        const int q = (n_spec + groups - 1) / groups;
+        const long long blocks = (long long)bx * ((n_spec + q - 1) / q);
+        const long long cost = ((blocks + sms - 1) / sms) * (once + each * q);
+        if (best < 0 || cost < best) {
+            best = cost;
+            per = q;
+        }
+    }
+    return per;
+}
+
 namespace soapgb {
 // the plain convolution of n_spec spectra: the tiled form unless its weights do not fit in
 // shared memory (an instrument of a few hundred pixels' reach)
@@ -218,11 +245,7 @@ static int conv_plain64_launch(soapgb_ctx *ctx, int n, int n_eff, int n_spec, co
                                double wave_last, const double *d_spec, long long spec_stride, const double *base_a,
                                const double *base_b, int b_every, double sigma_v, int wid, double step_mult,
                                double step_exp, double *conv) {
-    // reach in pixels of the widest Gaussian (sigma grows with wavelength); pixels it does not
-    // cover take the general form in the kernel
-    const double sig = soap_sigma_per_lambda(sigma_v) * std::max(std::fabs(wave0), std::fabs(wave_last));
-    const double r = std::floor(sqrt(2.0 * CP_CUT) * sig / step_exp * 1.0001) + 1.0;
-    const int reach = (r > 0.0 && r < (double)wid) ? (int)r : wid;
+    const int reach = conv_reach(sigma_v, wave0, wave_last, step_exp, wid);
     const size_t smem = sizeof(double) * ((size_t)(reach + 1) * CP_PIX + CP_PIX + 2 * (size_t)wid);
     if (smem > (size_t)CP_SMEM_MAX) {
         dim3 g(grid_for(ctx, n_eff, 256), n_spec);
@@ -233,13 +256,9 @@ static int conv_plain64_launch(soapgb_ctx *ctx, int n, int n_eff, int n_spec, co
         return SOAPGB_OK;
     }
     SOAP_CUDA(ctx, cudaFuncSetAttribute(k_conv_plain64t, cudaFuncAttributeMaxDynamicSharedMemorySize, CP_SMEM_MAX));
-    // spectra per block: as many as leave six blocks per SM (the weights, worth about four
-    // spectra's sums, are then shared most)
     const int bx = (n_eff + CP_PIX - 1) / CP_PIX;
-    const long long want = 6LL * std::max(ctx->num_sms, 1);
-    int per = (int)std::max(1LL, std::min<long long>(n_spec, (long long)bx * n_spec / want));
+    const int per = conv_per_block(ctx, bx, n_spec, 20LL * (reach + 1), 2LL * (2 * reach + 1));
     const int groups = (n_spec + per - 1) / per;
-    per = (n_spec + groups - 1) / groups;
     SOAP_TRACED(ctx, "conv_plain64", k_conv_plain64t<<<dim3(bx, groups), CP_PIX, smem, ctx->stream>>>(
         n, n_eff, d_wave, d_spec, spec_stride, base_a, base_b, b_every, n_spec, per, sigma_v, wid, reach, step_mult,
         step_exp, conv, n_eff));
@@ -1786,22 +1805,24 @@ __global__ void k_radj_taps(int n, int n_eff, const double *__restrict__ lam, do
     cq[i] = c;
 }
 
-constexpr int RADJ_THREADS = 512;
+constexpr int RADJ_THREADS = 256;
+constexpr int RADJ_PARTS = 64;   // most shares of a spectrum's pixels
 
-// one block per spectrum: S in a fixed tree order, the first extremum pixels by min
+// one block per share of a spectrum's pixels: its part of S in a fixed tree order, its first extremum pixels
 __global__ void __launch_bounds__(RADJ_THREADS) k_radj_reduce(int n, int n_eff, const double *__restrict__ spec,
                                                                const double *__restrict__ base,
                                                                const double *__restrict__ conv,
                                                                const unsigned long long *__restrict__ mm,
-                                                               const double *__restrict__ g, double *par, int *idx) {
-    const int s = blockIdx.x, t = threadIdx.x;
+                                                               const double *__restrict__ g, double *part, int2 *pidx) {
+    const int s = blockIdx.y, t = threadIdx.x;
     const double *sp = spec + (long long)s * n;
     const double *cp = conv + (long long)s * n_eff;
     const double *gp = g + (long long)s * n_eff;
     const double mn = soap_ord_dec(mm[2 * s]), mx = soap_ord_dec(mm[2 * s + 1]);
+    const int i0 = (int)((long long)n * blockIdx.x / gridDim.x), i1 = (int)((long long)n * (blockIdx.x + 1) / gridDim.x);
     double acc = 0.0;
     int im = INT_MAX, ix = INT_MAX;
-    for (int i = t; i < n; i += RADJ_THREADS) {
+    for (int i = i0 + t; i < i1; i += RADJ_THREADS) {
         const double a = base ? __dsub_rn(base[i], sp[i]) : sp[i];
         if (a == mn && im == INT_MAX) im = i;
         if (i < n_eff) {
@@ -1810,41 +1831,51 @@ __global__ void __launch_bounds__(RADJ_THREADS) k_radj_reduce(int n, int n_eff, 
             if (c != 0.0 && c == mx && ix == INT_MAX) ix = i;
         }
     }
-    __shared__ double sh[RADJ_THREADS];
-    __shared__ int si[RADJ_THREADS], sx[RADJ_THREADS];
-    sh[t] = acc;
-    si[t] = im;
-    sx[t] = ix;
-    __syncthreads();
-    for (int o = RADJ_THREADS / 2; o > 0; o >>= 1) {
-        if (t < o) {
-            sh[t] += sh[t + o];
-            si[t] = min(si[t], si[t + o]);
-            sx[t] = min(sx[t], sx[t + o]);
-        }
-        __syncthreads();
+    __shared__ double sh[RADJ_THREADS / 32];
+    __shared__ int si[RADJ_THREADS / 32], sx[RADJ_THREADS / 32];
+    for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
+    im = __reduce_min_sync(0xffffffffu, im);
+    ix = __reduce_min_sync(0xffffffffu, ix);
+    if ((t & 31) == 0) {
+        sh[t >> 5] = acc;
+        si[t >> 5] = im;
+        sx[t >> 5] = ix;
     }
+    __syncthreads();
     if (t == 0) {
-        const double S = sh[0];
-        par[3 * s] = (1.0 - mn) / mx;
-        par[3 * s + 1] = S / mx;
-        par[3 * s + 2] = S * (1.0 - mn) / (mx * mx);
-        idx[2 * s] = si[0] == INT_MAX ? -1 : si[0];
-        idx[2 * s + 1] = sx[0] == INT_MAX ? -1 : sx[0];
+        for (int w = 1; w < RADJ_THREADS / 32; ++w) {
+            acc += sh[w];
+            im = min(im, si[w]);
+            ix = min(ix, sx[w]);
+        }
+        part[s * RADJ_PARTS + blockIdx.x] = acc;
+        pidx[s * RADJ_PARTS + blockIdx.x] = make_int2(im, ix);
     }
 }
 
-// the transposed tap gather, one thread per (pixel m, spectrum)
-__global__ void __launch_bounds__(256) k_radj_spec(int n, int n_eff, int wid, const double *__restrict__ kq,
-                                                   const double *__restrict__ cq, const double *__restrict__ g,
-                                                   const double *__restrict__ par, const int *__restrict__ idx,
-                                                   int has_base, double *__restrict__ grad_spec) {
-    const int s = blockIdx.y;
-    const int m = blockIdx.x * blockDim.x + threadIdx.x;
-    if (m >= n) return;
-    const double f = par[3 * s], dmn = par[3 * s + 1], dmx = par[3 * s + 2];
-    const int imin = idx[2 * s], imax = idx[2 * s + 1];
-    const double *gp = g + (long long)s * n_eff;
+// the shares in order, one thread per spectrum
+__global__ void k_radj_par(int n_spec, int parts, const unsigned long long *__restrict__ mm,
+                           const double *__restrict__ part, const int2 *__restrict__ pidx, double *par, int *idx) {
+    const int s = blockIdx.x * blockDim.x + threadIdx.x;
+    if (s >= n_spec) return;
+    const double mn = soap_ord_dec(mm[2 * s]), mx = soap_ord_dec(mm[2 * s + 1]);
+    double S = 0.0;
+    int im = INT_MAX, ix = INT_MAX;
+    for (int q = 0; q < parts; ++q) {
+        S += part[s * RADJ_PARTS + q];
+        im = min(im, pidx[s * RADJ_PARTS + q].x);
+        ix = min(ix, pidx[s * RADJ_PARTS + q].y);
+    }
+    par[3 * s] = (1.0 - mn) / mx;
+    par[3 * s + 1] = S / mx;
+    par[3 * s + 2] = S * (1.0 - mn) / (mx * mx);
+    idx[2 * s] = im == INT_MAX ? -1 : im;
+    idx[2 * s + 1] = ix == INT_MAX ? -1 : ix;
+}
+
+// the transposed tap gather of one (pixel m, spectrum) over the whole reference window
+__device__ double radj_pixel(int m, int n_eff, int wid, const double *__restrict__ kq, const double *__restrict__ cq,
+                             const double *__restrict__ gp, double f, double dmx, int imax) {
     const int lo = max(m - wid + 2, 0), hi = min(m + wid, n_eff - 1);
     double acc = 0.0;
     for (int i = lo; i <= hi; ++i) {
@@ -1855,8 +1886,79 @@ __global__ void __launch_bounds__(256) k_radj_spec(int n, int n_eff, int wid, co
         if (i == imax) gc += dmx;
         acc = fma(k * exp(-d * d * cq[i]), gc, acc);
     }
-    const double ga = (m == imin ? dmn : 0.0) - acc;
+    return acc;
+}
+
+// the general form, one thread per (pixel m, spectrum)
+__global__ void __launch_bounds__(256) k_radj_spec(int n, int n_eff, int wid, const double *__restrict__ kq,
+                                                   const double *__restrict__ cq, const double *__restrict__ g,
+                                                   const double *__restrict__ par, const int *__restrict__ idx,
+                                                   int has_base, double *__restrict__ grad_spec) {
+    const int s = blockIdx.y;
+    const int m = blockIdx.x * blockDim.x + threadIdx.x;
+    if (m >= n) return;
+    const double acc = radj_pixel(m, n_eff, wid, kq, cq, g + (long long)s * n_eff, par[3 * s], par[3 * s + 2], idx[2 * s + 1]);
+    const double ga = (m == idx[2 * s] ? par[3 * s + 1] : 0.0) - acc;
     grad_spec[(long long)s * n + m] = has_base ? -ga : ga;
+}
+
+// A block takes blockDim.x pixels m and the spectra [blockIdx.y per, + per).  The weights K(i, m)
+// depend on the pixel pair only and, but for i's own constants, on |m - i|: the block keeps those of
+// every i in reach, |m - i| = 0 .. reach, in shared memory for all its spectra, and a tap costs one
+// FP64 FMA instead of the 28 instructions of an exp of its own.  Pixels beyond the reach have weights
+// below e^-90 of the central one and are left out (an error below 1e-39 of the largest gradient in
+// the window); a spectrum with a non-finite gradient in the reference's window goes through
+// radj_pixel.  Bound by the FP64 pipe.  10 spectra of 100,000 px: 8.2 -> 0.39 ms.
+__global__ void __launch_bounds__(256) k_radj_spect(int n, int n_eff, int n_spec, int per, int wid, int reach,
+                                                    const double *__restrict__ kq, const double *__restrict__ cq,
+                                                    const double *__restrict__ g, const double *__restrict__ par,
+                                                    const int *__restrict__ idx, int has_base,
+                                                    double *__restrict__ grad_spec) {
+    extern __shared__ __align__(16) double sm_radj[];
+    const int t = threadIdx.x, T = blockDim.x, m0 = blockIdx.x * T, m = m0 + t, win = T + 2 * reach, ib = m0 - reach;
+    double *wt = sm_radj;                               // [reach + 1][win], column x: i = ib + x
+    double *gs = sm_radj + (size_t)(reach + 1) * win;   // [win]
+    bool odd = false;
+    for (int x = t; x < win; x += T) {
+        const int i = ib + x;
+        const double k = i >= 0 && i < n_eff ? kq[i] : 0.0, c = k != 0.0 ? cq[i] : 0.0;
+        // the first weight beyond the table must be below the cut
+        if (k != 0.0 && reach < wid) odd |= !((double)(reach + 1) * (double)(reach + 1) * c > CP_CUT);
+        for (int d = 0; d <= reach; ++d) wt[d * win + x] = k != 0.0 ? k * exp(-(double)(d * d) * c) : 0.0;
+    }
+    const bool odd_block = __syncthreads_or(odd ? 1 : 0) != 0;
+    const int s1 = min(n_spec, (int)(blockIdx.y + 1) * per);
+    const int down = min(reach, wid - 2), up = min(reach, wid);   // i = m - down .. m + up
+    for (int s = blockIdx.y * per; s < s1; ++s) {
+        const double f = par[3 * s], dmx = par[3 * s + 2];
+        const int imax = idx[2 * s + 1];
+        const double *gp = g + (long long)s * n_eff;
+        bool wild = odd_block;
+        __syncthreads();   // the previous spectrum's gradients are read
+        for (int x = t - (wid - reach); x < win + wid - reach; x += T) {
+            const int i = ib + x;
+            double gc = 0.0;
+            if (i >= 0 && i < n_eff && kq[i] != 0.0) {
+                gc = -f * gp[i];
+                if (i == imax) gc += dmx;
+                wild |= (((unsigned)__double2hiint(gc) >> 20) & 0x7ffu) == 0x7ffu;
+            }
+            if (x >= 0 && x < win) gs[x] = gc;
+        }
+        wild = __syncthreads_or(wild ? 1 : 0) != 0;
+        if (m < n) {
+            double acc = 0.0;
+            if (wild) {
+                acc = radj_pixel(m, n_eff, wid, kq, cq, gp, f, dmx, imax);
+            } else {
+                const int x = t + reach;
+                for (int d = down; d > 0; --d) acc = fma(wt[d * win + x - d], gs[x - d], acc);
+                for (int d = 0; d <= up; ++d) acc = fma(wt[d * win + x + d], gs[x + d], acc);
+            }
+            const double ga = (m == idx[2 * s] ? par[3 * s + 1] : 0.0) - acc;
+            grad_spec[(long long)s * n + m] = has_base ? -ga : ga;
+        }
+    }
 }
 
 // dL/dbase[m] = sum_s dL/dA_s[m] = -sum_s grad_spec[s][m] (with a base), spectra in order
@@ -1913,6 +2015,7 @@ extern "C" int soapgb_lower_resolution_adjoint(soapgb_ctx *ctx, int n, int n_eff
     int s_mm = ws.add(sizeof(unsigned long long) * 2 * n_spec);
     int s_kq = ws.add(sizeof(double) * n_eff), s_cq = ws.add(sizeof(double) * n_eff);
     int s_par = ws.add(sizeof(double) * 3 * n_spec), s_idx = ws.add(sizeof(int) * 2 * n_spec);
+    int s_part = ws.add(sizeof(double) * RADJ_PARTS * n_spec), s_pidx = ws.add(sizeof(int2) * RADJ_PARTS * n_spec);
     int rc = ws.commit();
     if (rc) return rc;
     const double *d_wave = (const double *)stage_in(ctx, mem, wave, row_b, ws.get<void>(s_wave), &rc);
@@ -1928,6 +2031,8 @@ extern "C" int soapgb_lower_resolution_adjoint(soapgb_ctx *ctx, int n, int n_eff
     double *conv = ws.get<double>(s_conv);
     unsigned long long *mm = ws.get<unsigned long long>(s_mm);
     double *kq = ws.get<double>(s_kq), *cq = ws.get<double>(s_cq), *par = ws.get<double>(s_par);
+    double *part = ws.get<double>(s_part);
+    int2 *pidx = ws.get<int2>(s_pidx);
     int *idx = ws.get<int>(s_idx);
     // the forward's C and extrema, in the reference's operation order
     rc = conv_plain64_launch(ctx, n, n_eff, n_spec, d_wave, w01[0], w01[2], d_spec, n, d_base, nullptr, 0, sigma_v, wid,
@@ -1942,13 +2047,31 @@ extern "C" int soapgb_lower_resolution_adjoint(soapgb_ctx *ctx, int n, int n_eff
     k_radj_taps<<<grid_for(ctx, n_eff, 256), 256, 0, ctx->stream>>>(n, n_eff, d_wave, sigma_v, wid, step_mult,
                                                                      step_exp, kq, cq);
     SOAP_LAUNCHED(ctx);
+    const int parts = std::max(1, std::min({RADJ_PARTS, (n + 2047) / 2048, 8 * std::max(ctx->num_sms, 1) / n_spec}));
     SOAP_TRACED(ctx, "resolution_adjoint_reduce",
-                k_radj_reduce<<<n_spec, RADJ_THREADS, 0, ctx->stream>>>(n, n_eff, d_spec, d_base, conv, mm, d_g, par,
-                                                                        idx));
+                k_radj_reduce<<<dim3(parts, n_spec), RADJ_THREADS, 0, ctx->stream>>>(n, n_eff, d_spec, d_base, conv, mm,
+                                                                                      d_g, part, pidx));
     SOAP_LAUNCHED(ctx);
-    SOAP_TRACED(ctx, "resolution_adjoint",
-                k_radj_spec<<<dim3(grid_for(ctx, n, 256), n_spec), 256, 0, ctx->stream>>>(
-                    n, n_eff, wid, kq, cq, d_g, par, idx, d_base ? 1 : 0, d_gs));
+    k_radj_par<<<(n_spec + 31) / 32, 32, 0, ctx->stream>>>(n_spec, parts, mm, part, pidx, par, idx);
+    SOAP_LAUNCHED(ctx);
+    // the weights' table: 256 pixels per block (fewer weights of neighbouring tiles computed
+    // twice), 128 where the reach is long, the general form where neither fits
+    const int reach = conv_reach(sigma_v, w01[0], w01[2], step_exp, wid);
+    auto smem_of = [&](int T) { return sizeof(double) * (size_t)(reach + 2) * (T + 2 * (size_t)reach); };
+    const int T = smem_of(256) <= (size_t)CP_SMEM_MAX / 2 ? 256 : smem_of(128) <= (size_t)CP_SMEM_MAX ? 128 : 0;
+    if (T) {
+        SOAP_CUDA(ctx, cudaFuncSetAttribute(k_radj_spect, cudaFuncAttributeMaxDynamicSharedMemorySize, CP_SMEM_MAX));
+        const int bx = (n + T - 1) / T;
+        const int per = conv_per_block(ctx, bx, n_spec, 20LL * (reach + 1) * (T + 2 * reach) / T, 2LL * reach + 1);
+        const int groups = (n_spec + per - 1) / per;
+        SOAP_TRACED(ctx, "resolution_adjoint",
+                    k_radj_spect<<<dim3(bx, groups), T, smem_of(T), ctx->stream>>>(
+                        n, n_eff, n_spec, per, wid, reach, kq, cq, d_g, par, idx, d_base ? 1 : 0, d_gs));
+    } else {
+        SOAP_TRACED(ctx, "resolution_adjoint",
+                    k_radj_spec<<<dim3(grid_for(ctx, n, 256), n_spec), 256, 0, ctx->stream>>>(
+                        n, n_eff, wid, kq, cq, d_g, par, idx, d_base ? 1 : 0, d_gs));
+    }
     SOAP_LAUNCHED(ctx);
     if (d_gb) {
         k_radj_base<<<grid_for(ctx, n, 256), 256, 0, ctx->stream>>>(n, n_spec, d_gs, d_gb);

@@ -163,3 +163,47 @@ def test_adjoint_is_the_transpose(ctx, lambda0, step, n, vsini, grid, uneven, so
     jv = (scaled[0] - scaled[1]) / (2 * h)
     rhs = (g["delta"] * np.where(maps["limb"] > -998, maps["delta"], 0.0)).sum()
     assert abs((W * jv).sum() - rhs) <= 1e-4 * np.linalg.norm(W) * np.linalg.norm(jv)
+
+
+@pytest.mark.parametrize("n,n_spec,reso", [(900, 1, 115000.0), (1537, 30, 60000.0), (9000, 2, 9000.0), (9000, 1, 7000.0)])
+def test_resolution_adjoint_is_the_transposed_window(ctx, n, n_spec, reso):
+    """The gradient against the transposed taps of the whole reference window in numpy.  Tolerance: at
+    most 2 wid = 3000 terms, each with a few roundings, so 3000 x 4 x 1.1e-16 = 1.3e-12 of the sum of
+    their magnitudes, which is below f max |g| x 1.01; 1e-11 of that leaves room for the shared factors.
+    A NaN gradient reaches the whole window and no other spectrum."""
+    rng = np.random.default_rng(n)
+    step = 0.01
+    wave = 5000.0 + step * np.arange(n)
+    n_eff = n // 512 * 512
+    sv = _sigma_v(reso)
+    wid = oracle.conv_halfwidth(wave, sv, 50.0)
+    a = _spectra("disk", n, n_eff, n_spec, rng)
+    base = a[0] * 1.5
+    spec = base[None, :] - a
+    kw = dict(base=base, step_mult=step, step_exp=step)
+    g = rng.standard_normal((n_spec, n_eff))
+    gs, gb = ctx.lower_resolution_adjoint(wave, spec, n_eff, sv, g, **kw)
+    b = sv / C
+    sig = -1 * wave[:n_eff] * (1 - np.sqrt((1 + b) / (1 - b)))
+    i = np.arange(n_eff)
+    inside = (i > wid) & (i + wid < n - 1)
+    for s in range(0, n_spec, 13):
+        A = base - spec[s]
+        _, conv, (mn, mx) = oracle.lower_resolution(wave, A, n_eff, sv, step_mult=step, step_exp=step)
+        S = (g[s] * conv).sum()
+        gc = -(1 - mn) / mx * g[s]
+        gc[np.argmax(np.where(conv != 0, conv, -np.inf))] += S * (1 - mn) / mx ** 2
+        ref = np.zeros(n)
+        ref[np.argmin(A)] -= S / mx
+        for d in range(-wid, wid - 1):
+            k = np.where(inside, step * np.exp(-d * d * step * step / (2 * sig * sig)) / (sig * np.sqrt(2 * np.pi)), 0)
+            lo, hi = max(0, -d), min(n_eff, n - d)
+            ref[lo + d:hi + d] += (k * gc)[lo:hi]
+        assert np.max(np.abs(gs[s] - ref)) <= 1e-11 * max(np.abs(gc).max(), abs(S / mx))
+    assert np.allclose(gb, -gs.sum(0), rtol=1e-12, atol=1e-12 * np.abs(gs).max())
+    mid = n_eff // 2
+    g[-1, mid] = np.nan
+    m = np.arange(n)
+    gs = ctx.lower_resolution_adjoint(wave, spec, n_eff, sv, g, **kw)[0]
+    assert np.isnan(gs[-1][(m >= mid - wid) & (m <= mid + wid - 2)]).all()
+    assert not np.isnan(gs[:-1]).any()
