@@ -4,10 +4,17 @@
 // multifit_nlinear trust region with default parameters: Levenberg-Marquardt,
 // More scaling, xtol = gtol = 1e-8, ftol = 0, max_iter = 10000) and :214-317
 // (bisector on 91 depths, span).  The reference spawns one BIS_FIT2 process per
-// spectrum and exchanges text files with it.  Here one warp fits one spectrum:
-// the lanes evaluate residuals and Jacobian rows, warp shuffles reduce J^T J and
-// J^T f, and every lane solves the 4x4 damped normal equations redundantly (no
-// divergence, no shared state).  Damping follows Nielsen's rule as in GSL
+// spectrum and exchanges text files with it.  Here one block of two warps fits one
+// spectrum: the threads evaluate residuals and Jacobian rows, shuffles and shared
+// memory reduce J^T J and J^T f, and every thread solves the 4x4 damped normal
+// equations redundantly (no divergence).
+// What bounds it is the FP64 pipe's latency and rate (half a lane per cycle in each
+// of an SM's four partitions): a few hundred spectra put about one warp on each
+// partition, so an iteration costs its FP64 instructions in a row.  Hence two warps
+// per spectrum, reciprocals instead of divisions inside an iteration, sixteen sums
+// reduced together (16 additions per warp instead of 5 each), and index searches by
+// integer images instead of serial loops of FP64 compares: 303 CCFs of 161 velocities
+// 478 -> 150 us.  Damping follows Nielsen's rule as in GSL
 // (mu *= max(1/3, 1-(2 rho-1)^3) on acceptance, mu *= nu, nu *= 2 on rejection).
 // All iteration loops are bounded.
 #include <cmath>
@@ -16,82 +23,129 @@
 
 using namespace soapgb;
 
-#define FIT_WARPS 4
+constexpr int FIT_THREADS = 64;    // the fit's threads per spectrum
+constexpr int ADJ_THREADS = 128;   // its adjoint's
 #define FIT_DEPTHS 91
+constexpr size_t FIT_SMEM_MAX = 48 * 1024;   // bisector arrays kept in shared memory up to here
 
-// butterfly sum; the final broadcast makes every lane hold lane 0's bits, so all
-// lanes take identical branches in the iteration below
-__device__ __forceinline__ double warp_sum(double v) {
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-    return __shfl_sync(0xffffffffu, v, 0);
+// Sums of v[0 .. 15] over the block in a fixed order, the same bits in every thread's tot[]: a
+// warp's lanes halve the values they hold as they halve the lanes that hold them.
+struct BlockSums {
+    double part[ADJ_THREADS / 32][16], tot[16];
+};
+__device__ __forceinline__ void block_sum16(double (&v)[16], BlockSums &s) {
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, nw = blockDim.x >> 5;
+#pragma unroll
+    for (int o = 16, h = 8; o > 1; o >>= 1, h >>= 1) {
+        const bool up = lane & o;
+#pragma unroll
+        for (int q = 0; q < h; ++q) {
+            const double give = up ? v[q] : v[q + h], keep = up ? v[q + h] : v[q];
+            v[q] = keep + __shfl_xor_sync(0xffffffffu, give, o);
+        }
+    }
+    v[0] += __shfl_xor_sync(0xffffffffu, v[0], 1);
+    __syncthreads();
+    if (!(lane & 1)) s.part[w][lane >> 1] = v[0];
+    __syncthreads();
+    if (threadIdx.x < 16) {
+        double t = s.part[0][threadIdx.x];
+        for (int k = 1; k < nw; ++k) t += s.part[k][threadIdx.x];
+        s.tot[threadIdx.x] = t;
+    }
+    __syncthreads();
+}
+
+// index of the block's largest key, the first at ties (every thread; s: two words)
+__device__ __forceinline__ int block_argmax(unsigned long long key, int i, unsigned long long *s_key, int *s_idx) {
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        *s_key = 0ULL;
+        *s_idx = 0x7fffffff;
+    }
+    __syncthreads();
+    if (key) atomicMax(s_key, key);
+    __syncthreads();
+    if (key && key == *s_key) atomicMin(s_idx, i);
+    __syncthreads();
+    return *s_idx;
 }
 
 __device__ __forceinline__ double gauss_sigma(double fwhm) { return fwhm / 2 / sqrt(2 * log(2.0)); }
 
-// solve (A) x = b (4x4 SPD) by Cholesky; returns false if not positive definite
-__device__ bool chol4(const double *A, const double *b, double *x) {
-    double L[16];
+// solve (A) x = b (4x4 SPD) by Cholesky, the diagonal as reciprocals; false if not positive definite
+__device__ __forceinline__ bool chol4(const double *A, const double *b, double *x) {
+    double L[16], r[4], y[4];
 #pragma unroll
-    for (int q = 0; q < 16; ++q) L[q] = 0.0;
     for (int i = 0; i < 4; i++) {
+#pragma unroll
         for (int j = 0; j <= i; j++) {
             double s = A[i * 4 + j];
+#pragma unroll
             for (int k = 0; k < j; k++) s -= L[i * 4 + k] * L[j * 4 + k];
             if (i == j) {
                 if (!(s > 0)) return false;
-                L[i * 4 + i] = sqrt(s);
+                r[i] = rsqrt(s);
             } else {
-                L[i * 4 + j] = s / L[j * 4 + j];
+                L[i * 4 + j] = s * r[j];
             }
         }
     }
-    double y[4];
+#pragma unroll
     for (int i = 0; i < 4; i++) {
         double s = b[i];
+#pragma unroll
         for (int k = 0; k < i; k++) s -= L[i * 4 + k] * y[k];
-        y[i] = s / L[i * 4 + i];
+        y[i] = s * r[i];
     }
+#pragma unroll
     for (int i = 3; i >= 0; i--) {
         double s = y[i];
+#pragma unroll
         for (int k = i + 1; k < 4; k++) s -= L[k * 4 + i] * x[k];
-        x[i] = s / L[i * 4 + i];
+        x[i] = s * r[i];
     }
     return true;
 }
 
-// residual sum of squares at parameters p (lane-partial sums reduced)
-__device__ double lane_phi(int n, const double *__restrict__ x, const double *__restrict__ y,
-                           const double *__restrict__ err, const double *p, int lane) {
-    double sigma = gauss_sigma(p[3]);
-    double acc = 0.0;
-    for (int i = lane; i < n; i += 32) {
-        double d = x[i] - p[2];
-        double fit = p[0] + p[1] * exp(-d * d / 2 / sigma / sigma);
-        double f = (fit - y[i]) / (err ? err[i] : 1.0);
-        acc += f * f;
-    }
-    return warp_sum(acc);
-}
-
-__global__ void __launch_bounds__(32 * FIT_WARPS) k_gauss_bis(int n_spec, int n, const double *__restrict__ xin,
-                                                              const double *__restrict__ yall,
-                                                              const double *__restrict__ errall,
-                                                              double *__restrict__ xr_scr, double *__restrict__ model,
-                                                              double *__restrict__ par, double *__restrict__ depth_out,
-                                                              double *__restrict__ bis_out, int *__restrict__ iters,
-                                                              double *__restrict__ scratch) {
-    int lane = threadIdx.x & 31;
-    int s = blockIdx.x * FIT_WARPS + (threadIdx.x >> 5);
-    if (s >= n_spec) return;
+__global__ void __launch_bounds__(FIT_THREADS) k_gauss_bis(int n_spec, int n, const double *__restrict__ xin,
+                                                           const double *__restrict__ yall,
+                                                           const double *__restrict__ errall,
+                                                           double *__restrict__ model, double *__restrict__ par,
+                                                           double *__restrict__ depth_out,
+                                                           double *__restrict__ bis_out, int *__restrict__ iters,
+                                                           double *__restrict__ scratch) {
+    extern __shared__ __align__(16) double sm_fit[];
+    __shared__ BlockSums sums;
+    __shared__ unsigned long long s_key;
+    __shared__ int s_idx;
+    __shared__ double s_bis[FIT_DEPTHS];
+    const int s = blockIdx.x, t = threadIdx.x;
     const double *y = yall + (long long)s * n;
     const double *err = errall ? errall + (long long)s * n : nullptr;
-    const double *x = xr_scr;   // rebased velocities x - x[0] (shared by all spectra)
-    // initial guess, BIS_FIT2.cpp:155-160 (done by every lane, identical)
+    const double x00 = xin[0];
+    auto x = [&](int i) { return xin[i] - x00; };   // rebased velocities
+    const double s2l = 2 * sqrt(2 * log(2.0));
+    // initial guess, BIS_FIT2.cpp:155-160: the first largest |y - c|
     double c = (y[0] + y[n - 1]) / 2;
-    double fwhm = (x[n - 1] - x[0]) / 5.;
-    double k = 0., x0 = x[n / 2];
-    for (int i = 0; i < n; i++)
-        if (fabs(y[i] - c) > fabs(k)) { k = y[i] - c; x0 = x[i]; }
+    double fwhm = (x(n - 1) - x(0)) / 5.;
+    double k = 0., x0 = x(n / 2);
+    {
+        unsigned long long key = 0ULL;
+        int at = 0;
+        for (int i = t; i < n; i += FIT_THREADS) {
+            const unsigned long long v = (unsigned long long)__double_as_longlong(fabs(y[i] - c));
+            if (v > key && v <= 0x7ff0000000000000ULL) {   // (a NaN is not larger than anything)
+                key = v;
+                at = i;
+            }
+        }
+        const int best = block_argmax(key, at, &s_key, &s_idx);
+        if (best < n) {
+            k = y[best] - c;
+            x0 = x(best);
+        }
+    }
     double p[4] = {c, k, x0, fwhm};
     double D[4] = {0, 0, 0, 0};
     double mu = 0.0, nu = 2.0;
@@ -100,46 +154,47 @@ __global__ void __launch_bounds__(32 * FIT_WARPS) k_gauss_bis(int n_spec, int n,
     const double xtol = 1e-8, gtol = 1e-8;
     for (int iter = 0; iter <= 10000; ++iter) {
         // J^T J, J^T f, phi at p
-        double sigma = gauss_sigma(p[3]);
-        double jtj[10], g[4], phi = 0.0;
+        const double is = s2l / p[3], is2 = is * is, h = 0.5 * is2;   // 1 / sigma, 1 / sigma^2
+        const double f2 = p[1] * is2, f3 = f2 * is / s2l;             // of J[2], J[3]
+        double v[16];
 #pragma unroll
-        for (int q = 0; q < 10; ++q) jtj[q] = 0.0;
-#pragma unroll
-        for (int q = 0; q < 4; ++q) g[q] = 0.0;
-        for (int i = lane; i < n; i += 32) {
-            double inv = 1.0 / (err ? err[i] : 1.0);
-            double d = x[i] - p[2];
-            double e = exp(-d * d / 2 / sigma / sigma);
-            double f = (p[0] + p[1] * e - y[i]) * inv;
-            double J[4];
-            J[0] = inv;
-            J[1] = e * inv;
-            J[2] = p[1] * inv * e * d / sigma / sigma;
-            J[3] = p[1] * inv * e * d * d / sigma / sigma / sigma / 2 / sqrt(2 * log(2.0));
-            int t = 0;
+        for (int q = 0; q < 16; ++q) v[q] = 0.0;
+        for (int i = t; i < n; i += FIT_THREADS) {
+            const double inv = err ? 1.0 / err[i] : 1.0;
+            const double d = x(i) - p[2];
+            const double e = exp(-d * d * h);
+            const double f = (p[0] + p[1] * e - y[i]) * inv;
+            const double ed = e * inv * d;
+            const double J[4] = {inv, e * inv, f2 * ed, f3 * ed * d};
+            int q = 0;
 #pragma unroll
             for (int a = 0; a < 4; ++a) {
-                g[a] += J[a] * f;
+                v[10 + a] += J[a] * f;
 #pragma unroll
-                for (int b = a; b < 4; ++b) jtj[t++] += J[a] * J[b];
+                for (int b = a; b < 4; ++b) v[q++] += J[a] * J[b];
             }
-            phi += f * f;
+            v[14] += f * f;
         }
-#pragma unroll
-        for (int q = 0; q < 10; ++q) jtj[q] = warp_sum(jtj[q]);
-#pragma unroll
-        for (int q = 0; q < 4; ++q) g[q] = warp_sum(g[q]);
-        phi = warp_sum(phi);
-        double A[16];
+        block_sum16(v, sums);
+        double A[16], g[4];
         {
-            int t = 0;
-            for (int a = 0; a < 4; ++a)
-                for (int b = a; b < 4; ++b) { A[a * 4 + b] = jtj[t]; A[b * 4 + a] = jtj[t]; ++t; }
+            int q = 0;
+#pragma unroll
+            for (int a = 0; a < 4; ++a) {
+                g[a] = sums.tot[10 + a];
+#pragma unroll
+                for (int b = a; b < 4; ++b) { A[a * 4 + b] = A[b * 4 + a] = sums.tot[q]; ++q; }
+            }
         }
+        const double phi = sums.tot[14];
         if (iter == 0) {
-            for (int a = 0; a < 4; ++a) { D[a] = sqrt(A[a * 5]); if (D[a] == 0.0) D[a] = 1.0; }
             double mx = 0.0;
-            for (int a = 0; a < 4; ++a) { double t = sqrt(A[a * 5]) / D[a]; mx = fmax(mx, t * t); }
+            for (int a = 0; a < 4; ++a) {
+                D[a] = sqrt(A[a * 5]);
+                if (D[a] == 0.0) D[a] = 1.0;
+                const double r = sqrt(A[a * 5]) / D[a];
+                mx = fmax(mx, r * r);
+            }
             mu = 1e-3 * mx;
         } else {
             for (int a = 0; a < 4; ++a) D[a] = fmax(D[a], sqrt(A[a * 5]));
@@ -162,7 +217,20 @@ __global__ void __launch_bounds__(32 * FIT_WARPS) k_gauss_bis(int n_spec, int n,
             if (!chol4(M, rhs, dx)) { mu *= nu; nu *= 2; ++bad; continue; }
             double pt[4];
             for (int a = 0; a < 4; ++a) pt[a] = p[a] + dx[a];
-            double phit = lane_phi(n, x, y, err, pt, lane);
+            // residual sum of squares at pt
+            const double ht = 0.5 * (s2l / pt[3]) * (s2l / pt[3]);
+            double acc = 0.0;
+            for (int i = t; i < n; i += FIT_THREADS) {
+                const double d = x(i) - pt[2];
+                double f = pt[0] + pt[1] * exp(-d * d * ht) - y[i];
+                if (err) f /= err[i];
+                acc += f * f;
+            }
+            for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
+            __syncthreads();
+            if ((t & 31) == 0) sums.part[t >> 5][0] = acc;
+            __syncthreads();
+            const double phit = sums.part[0][0] + sums.part[1][0];
             double jdx = 0.0;   // ||J dx||^2 = dx^T (J^T J) dx
             for (int a = 0; a < 4; ++a)
                 for (int b = 0; b < 4; ++b) jdx += dx[a] * A[a * 4 + b] * dx[b];
@@ -172,8 +240,8 @@ __global__ void __launch_bounds__(32 * FIT_WARPS) k_gauss_bis(int n_spec, int n,
             double rho = (pred > 0 && phit < phi) ? (phi - phit) / pred : -1.0;
             if (rho > 0) {
                 accepted = true;
-                double t = 2 * rho - 1;
-                double fac = 1 - t * t * t;
+                double r = 2 * rho - 1;
+                double fac = 1 - r * r * r;
                 mu *= fmax(fac, 1.0 / 3.0);
                 nu = 2;
                 for (int a = 0; a < 4; ++a) p[a] = pt[a];
@@ -196,72 +264,74 @@ __global__ void __launch_bounds__(32 * FIT_WARPS) k_gauss_bis(int n_spec, int n,
         }
     }
     c = p[0]; k = p[1]; x0 = p[2]; fwhm = p[3];
-    double sigma = gauss_sigma(fwhm);
-    for (int i = lane; i < n; i += 32) {
-        double d = x[i] - x0;
-        model[(long long)s * n + i] = c + k * exp(-d * d / 2 / sigma / sigma);
+    {
+        const double is = s2l / fwhm, h = 0.5 * is * is;
+        for (int i = t; i < n; i += FIT_THREADS) {
+            const double d = x(i) - x0;
+            model[(long long)s * n + i] = c + k * exp(-d * d * h);
+        }
     }
     // bisector, BIS_FIT2.cpp:214-268
-    double *norm = scratch + (long long)s * 4 * n;
+    double *norm = scratch ? scratch + (long long)s * 4 * n : sm_fit;
     double *p0 = norm + n, *p1 = norm + 2 * n, *p2 = norm + 3 * n;
-    double sig_b = fwhm / 2. / pow(2. * log(2.), .5);
-    double v0 = x0 + xin[0];
-    for (int i = lane; i < n; i += 32) norm[i] = -c / k * (1. - y[i] / c);
-    if (lane == 0) { p0[n - 1] = 0.0; p1[n - 1] = 0.0; p2[n - 1] = 0.0; }   // never set by the loop below
-    __syncwarp();
-    for (int i = lane; i < n - 1; i += 32) {
-        double vr = (xin[i] + xin[i + 1]) / 2.;
-        double dd = vr - v0;
-        double ss = sig_b * sig_b;
-        double dC = -dd / ss * exp(-(dd * dd) / 2. / ss);
-        double d2C = ((dd * dd) / ss - 1) / ss * exp(-(dd * dd) / 2. / ss);
-        double d2R = -d2C / (dC * dC * dC);
-        double q2 = d2R / 2.;
-        double a0 = norm[i], a1 = norm[i + 1];
-        double q1 = (xin[i + 1] - xin[i] - q2 * (a1 * a1 - a0 * a0)) / (a1 - a0);
+    const double sig_b = fwhm / 2. / pow(2. * log(2.), .5), ss = sig_b * sig_b, iss = 1.0 / ss;
+    const double v0 = x0 + x00;
+    unsigned long long key = 0ULL;
+    int at = 0;
+    const double nk = -c / k;
+    for (int i = t; i < n; i += FIT_THREADS) {
+        const double v = nk * (1. - y[i] / c);
+        norm[i] = v;
+        const unsigned long long w = v == v ? soap_ord64(v + 0.0) : 0ULL;
+        if (w > key) {
+            key = w;
+            at = i;
+        }
+    }
+    if (t == 0) { p0[n - 1] = 0.0; p1[n - 1] = 0.0; p2[n - 1] = 0.0; }   // never set by the loop below
+    int ind_max = block_argmax(key, at, &s_key, &s_idx);   // (its barriers publish norm)
+    if (ind_max >= n || norm[0] != norm[0]) ind_max = 0;   // nothing is larger than a NaN
+    for (int i = t; i < n - 1; i += FIT_THREADS) {
+        const double vr = (xin[i] + xin[i + 1]) / 2.;
+        const double dd = vr - v0, u = dd * dd * iss;
+        const double e = exp(-0.5 * u);
+        const double dC = -dd * iss * e;
+        const double d2C = (u - 1) * iss * e;
+        const double q2 = -d2C / (dC * dC * dC) / 2.;
+        const double a0 = norm[i], a1 = norm[i + 1];
+        const double q1 = (xin[i + 1] - xin[i] - q2 * (a1 * a1 - a0 * a0)) / (a1 - a0);
         p2[i] = q2;
         p1[i] = q1;
         p0[i] = xin[i] - q1 * a0 - q2 * (a0 * a0);
     }
-    __syncwarp();
-    int ind_max = 0;
-    for (int i = 0; i < n; i++) if (norm[i] > norm[ind_max]) ind_max = i;
+    __syncthreads();
     double *bo = bis_out + (long long)s * FIT_DEPTHS;
-    for (int t = lane; t < FIT_DEPTHS; t += 32) {
-        double dep = (double)(t + 5) / 100;
+    for (int q = t; q < FIT_DEPTHS; q += FIT_THREADS) {
+        const double dep = (double)(q + 5) / 100;
         int i_b = ind_max, i_r = ind_max;
         while ((norm[i_b] > dep) && (i_b > 1)) i_b--;
         while ((norm[i_r + 1] > dep) && (i_r < (n - 2))) i_r++;
         double b = (p0[i_b] + p0[i_r]) + (p1[i_b] + p1[i_r]) * dep + (p2[i_b] + p2[i_r]) * (dep * dep);
         b /= 2.;
-        bo[t] = b;
-        depth_out[(long long)s * FIT_DEPTHS + t] = 1.0 - fabs(k) * dep;
+        bo[q] = b;
+        s_bis[q] = b;
+        depth_out[(long long)s * FIT_DEPTHS + q] = 1.0 - fabs(k) * dep;
     }
-    __syncwarp();
-    if (lane == 0) {
-        // span in the reference's summation order, BIS_FIT2.cpp:256-268
+    __syncthreads();
+    if (t == 0) {
+        // span in the reference's summation order, BIS_FIT2.cpp:256-268: depths 0.1 to 0.4 and
+        // 0.6 to 0.9, the hundredths 10 .. 40 and 60 .. 90
         double top = 0.0, bottom = 0.0;
-        int n1 = 0, n2 = 0;
-        for (int t = 0; t < FIT_DEPTHS; ++t) {
-            double dep = (double)(t + 5) / 100;
-            if ((dep >= 0.1) && (dep <= 0.4)) { n1++; top += bo[t]; }
-            if ((dep >= 0.6) && (dep <= 0.9)) { n2++; bottom += bo[t]; }
-        }
-        top /= n1;
-        bottom /= n2;
+        for (int q = 10; q <= 40; ++q) top += s_bis[q - 5];
+        for (int q = 60; q <= 90; ++q) bottom += s_bis[q - 5];
         double *pp = par + (long long)s * 5;
         pp[0] = c;
         pp[1] = fabs(k);
-        pp[2] = top - bottom;
+        pp[2] = top / 31 - bottom / 31;
         pp[3] = v0;
         pp[4] = fwhm;
         if (iters) iters[s] = status;
     }
-}
-
-__global__ void k_rebase(int n, const double *__restrict__ x, double *xr) {
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n) xr[i] = x[i] - x[0];
 }
 
 extern "C" int soapgb_gauss_bis(soapgb_ctx *ctx, int n_spec, int n, const double *x, const double *y,
@@ -282,8 +352,10 @@ extern "C" int soapgb_gauss_bis(soapgb_ctx *ctx, int n_spec, int n, const double
     int s_dep = ws.add(host ? sizeof(double) * FIT_DEPTHS * n_spec : 0);
     int s_bis = ws.add(host ? sizeof(double) * FIT_DEPTHS * n_spec : 0);
     int s_it = ws.add(host && iters ? sizeof(int) * n_spec : 0);
-    int s_xr = ws.add(sizeof(double) * n);
-    int s_scr = ws.add(sizeof(double) * 4 * (size_t)n * n_spec);
+    // the bisector's arrays: shared memory, or scratch for long CCFs
+    const size_t bis_b = sizeof(double) * 4 * (size_t)n;
+    const bool in_smem = bis_b <= FIT_SMEM_MAX - 4096;
+    int s_scr = ws.add(in_smem ? 0 : bis_b * n_spec);
     int rc = ws.commit();
     if (rc) return rc;
     const double *d_x = (const double *)stage_in(ctx, mem, x, sizeof(double) * n, ws.get<void>(s_x), &rc);
@@ -297,11 +369,8 @@ extern "C" int soapgb_gauss_bis(soapgb_ctx *ctx, int n_spec, int n, const double
     double *d_dep = host ? ws.get<double>(s_dep) : depth;
     double *d_bis = host ? ws.get<double>(s_bis) : bis;
     int *d_it = iters ? (host ? ws.get<int>(s_it) : iters) : nullptr;
-    double *xr = ws.get<double>(s_xr);
-    k_rebase<<<(n + 255) / 256, 256, 0, ctx->stream>>>(n, d_x, xr);
-    SOAP_LAUNCHED(ctx);
-    SOAP_TRACED(ctx, "gauss_bis", k_gauss_bis<<<(n_spec + FIT_WARPS - 1) / FIT_WARPS, 32 * FIT_WARPS, 0, ctx->stream>>>(
-        n_spec, n, d_x, d_y, d_e, xr, d_model, d_par, d_dep, d_bis, d_it, ws.get<double>(s_scr)));
+    SOAP_TRACED(ctx, "gauss_bis", k_gauss_bis<<<n_spec, FIT_THREADS, in_smem ? bis_b : 0, ctx->stream>>>(
+        n_spec, n, d_x, d_y, d_e, d_model, d_par, d_dep, d_bis, d_it, in_smem ? nullptr : ws.get<double>(s_scr)));
     SOAP_LAUNCHED(ctx);
     if (host) {
         SOAP_CUDA(ctx, cudaMemcpyAsync(model, d_model, sizeof(double) * (size_t)n * n_spec, cudaMemcpyDeviceToHost, ctx->stream));
@@ -327,7 +396,7 @@ extern "C" int soapgb_gauss_bis(soapgb_ctx *ctx, int n_spec, int n, const double
 //   G_x0,fwhm = a k e d (d^2 / s^5 - 2 / s^3)
 //   G_fwhm,fwhm = a^2 k e d^2 (d^2 / s^6 - 3 / s^4)   (all c terms vanish).
 // The fitted outputs give c, |k|, v0 = x0 + x[0] and fwhm; the sign of k is that of
-// the model's largest excursion from c.  One warp per spectrum, fixed reduction order.
+// the model's largest excursion from c.  One block per spectrum, fixed reduction order.
 // ---------------------------------------------------------------------------
 // 4x4 solve by Gaussian elimination with partial pivoting; false when singular
 __device__ bool solve4(double *A, double *b, double *z) {
@@ -354,65 +423,69 @@ __device__ bool solve4(double *A, double *b, double *z) {
     return true;
 }
 
-__global__ void __launch_bounds__(32 * FIT_WARPS) k_gauss_fit_adj(int n_spec, int n, const double *__restrict__ x,
-                                                                  const double *__restrict__ yall,
-                                                                  const double *__restrict__ errall,
-                                                                  const double *__restrict__ model,
-                                                                  const double *__restrict__ par,
-                                                                  const double *__restrict__ gpar,
-                                                                  double *__restrict__ grad_y, int *status) {
-    const int lane = threadIdx.x & 31;
-    const int s = blockIdx.x * FIT_WARPS + (threadIdx.x >> 5);
-    if (s >= n_spec) return;
+__global__ void __launch_bounds__(ADJ_THREADS) k_gauss_fit_adj(int n_spec, int n, const double *__restrict__ x,
+                                                               const double *__restrict__ yall,
+                                                               const double *__restrict__ errall,
+                                                               const double *__restrict__ model,
+                                                               const double *__restrict__ par,
+                                                               const double *__restrict__ gpar,
+                                                               double *__restrict__ grad_y,
+                                                               double *__restrict__ scratch, int *status) {
+    extern __shared__ __align__(16) double sm_fit[];
+    __shared__ BlockSums sums;
+    __shared__ unsigned long long s_key;
+    __shared__ int s_idx;
+    const int s = blockIdx.x, tid = threadIdx.x;
     const double *y = yall + (long long)s * n;
     const double *err = errall ? errall + (long long)s * n : nullptr;
     const double *mo = model + (long long)s * n;
     const double *pp = par + (long long)s * 5;
     const double *gp = gpar + (long long)s * 5;
     double *gy = grad_y + (long long)s * n;
+    double *norm = scratch ? scratch + (long long)s * n : sm_fit;
     const double c = pp[0], v0 = pp[3], fwhm = pp[4];
     // sign of k: the model's largest excursion from c (first index at ties)
-    double best = -1.0, sgn = 1.0;
-    int bi = n;
-    for (int i = lane; i < n; i += 32) {
-        const double e = fabs(mo[i] - c);
-        if (e > best) { best = e; bi = i; sgn = (mo[i] - c) >= 0.0 ? 1.0 : -1.0; }
+    unsigned long long key = 0ULL;
+    int at = 0;
+    for (int i = tid; i < n; i += ADJ_THREADS) {
+        const unsigned long long v = (unsigned long long)__double_as_longlong(fabs(mo[i] - c));
+        if (v + 1 > key && v <= 0x7ff0000000000000ULL) {
+            key = v + 1;
+            at = i;
+        }
     }
-    for (int o = 16; o > 0; o >>= 1) {
-        const double ob = __shfl_xor_sync(0xffffffffu, best, o);
-        const int oi = __shfl_xor_sync(0xffffffffu, bi, o);
-        const double os = __shfl_xor_sync(0xffffffffu, sgn, o);
-        if (ob > best || (ob == best && oi < bi)) { best = ob; bi = oi; sgn = os; }
-    }
+    const int top = block_argmax(key, at, &s_key, &s_idx);
+    const double sgn = (top >= n || mo[top] - c >= 0.0) ? 1.0 : -1.0;
     const double k = sgn * pp[1];
     const double a = gauss_sigma(1.0);
-    const double sg = gauss_sigma(fwhm);
-    const double s2 = sg * sg, s3 = s2 * sg, s4 = s2 * s2;
-    double H[10];
+    const double is = 1.0 / gauss_sigma(fwhm), is2 = is * is, is3 = is2 * is, is4 = is2 * is2;
+    double v[16];
 #pragma unroll
-    for (int q = 0; q < 10; ++q) H[q] = 0.0;
-    for (int i = lane; i < n; i += 32) {
-        const double inv = 1.0 / (err ? err[i] : 1.0);
-        const double d = x[i] - v0, d2 = d * d;
-        const double e = exp(-d2 / 2 / s2);
+    for (int q = 0; q < 16; ++q) v[q] = 0.0;
+    for (int i = tid; i < n; i += ADJ_THREADS) {
+        const double inv = err ? 1.0 / err[i] : 1.0;
+        const double d = x[i] - v0, d2 = d * d, u = d2 * is2;
+        const double e = exp(-0.5 * u);
         const double f = (c + k * e - y[i]) * inv;
-        const double G[4] = {1.0, e, k * e * d / s2, k * e * d2 * a / s3};
+        const double G[4] = {1.0, e, k * e * d * is2, k * e * d2 * a * is3};
         double S[10];   // second derivatives, upper triangle row-major
         S[0] = 0.0; S[1] = 0.0; S[2] = 0.0; S[3] = 0.0;
         S[4] = 0.0;
-        S[5] = e * d / s2;
-        S[6] = a * e * d2 / s3;
-        S[7] = k * e * (d2 / s4 - 1.0 / s2);
-        S[8] = a * k * e * d * (d2 / (s4 * sg) - 2.0 / s3);
-        S[9] = a * a * k * e * d2 * (d2 / (s4 * s2) - 3.0 / s4);
+        S[5] = e * d * is2;
+        S[6] = a * e * d2 * is3;
+        S[7] = k * e * is2 * (u - 1.0);
+        S[8] = a * k * e * d * is3 * (u - 2.0);
+        S[9] = a * a * k * e * d2 * is4 * (u - 3.0);
         int t = 0;
 #pragma unroll
         for (int p = 0; p < 4; ++p)
 #pragma unroll
-            for (int q = p; q < 4; ++q, ++t) H[t] += inv * inv * G[p] * G[q] + f * inv * S[t];
+            for (int q = p; q < 4; ++q, ++t) v[t] += inv * inv * G[p] * G[q] + f * inv * S[t];
     }
+    block_sum16(v, sums);
+    double H[10];
 #pragma unroll
-    for (int q = 0; q < 10; ++q) H[q] = warp_sum(H[q]);
+    for (int q = 0; q < 10; ++q) H[q] = sums.tot[q];
     double A[16], b[4] = {gp[0], gp[1] * sgn, gp[3], gp[4]}, z[4] = {0, 0, 0, 0};
     // --- the bisector span (BIS_FIT2.cpp:214-268).  Per depth the forward picks the
     // intervals i_b, i_r where the normalised CCF a_i = (y_i - c) / k crosses it (held fixed
@@ -422,96 +495,90 @@ __global__ void __launch_bounds__(32 * FIT_WARPS) k_gauss_fit_adj(int n_spec, in
     // Gaussian at the interval's middle.  The span is the mean of the bisector over depths
     // 0.1-0.4 minus its mean over 0.6-0.9; its gradient reaches y directly (a_i) and through
     // the fit's parameters (c, k in a_i; v0, sigma in q2_i), the latter added to b.
-    const int wp = threadIdx.x >> 5;
-    __shared__ int sp_ib[FIT_WARPS][FIT_DEPTHS], sp_ir[FIT_WARPS][FIT_DEPTHS];
-    __shared__ double sp_d[FIT_WARPS][FIT_DEPTHS][4];
+    __shared__ int sp_ib[FIT_DEPTHS], sp_ir[FIT_DEPTHS];
+    __shared__ double sp_d[FIT_DEPTHS][4];
     const double gs = gp[2];
-    if (gs != 0.0) {   // uniform for the warp
-        auto nrm = [&](int i) { return -c / k * (1. - y[i] / c); };   // the forward's expression
-        double bv = -1e308;
-        int bix = n;
-        for (int i = lane; i < n; i += 32) {
-            const double v = nrm(i);
-            if (v > bv) { bv = v; bix = i; }
-        }
-        for (int o = 16; o > 0; o >>= 1) {
-            const double ov = __shfl_xor_sync(0xffffffffu, bv, o);
-            const int oi = __shfl_xor_sync(0xffffffffu, bix, o);
-            if (ov > bv || (ov == bv && oi < bix)) { bv = ov; bix = oi; }
-        }
-        const int ind_max = bix;
-        int n1 = 0, n2 = 0;
-        for (int t = 0; t < FIT_DEPTHS; ++t) {
-            const double dep = (double)(t + 5) / 100;
-            if ((dep >= 0.1) && (dep <= 0.4)) n1++;
-            if ((dep >= 0.6) && (dep <= 0.9)) n2++;
-        }
-        const double sig_b = fwhm / 2. / pow(2. * log(2.), .5), ss = sig_b * sig_b;
-        double acc[4] = {0.0, 0.0, 0.0, 0.0};   // d span / d (c, k, v0, ss)
-        for (int t = lane; t < FIT_DEPTHS; t += 32) {
-            const double dep = (double)(t + 5) / 100;
-            double w = 0.0;
-            if ((dep >= 0.1) && (dep <= 0.4)) w += 1.0 / n1;
-            if ((dep >= 0.6) && (dep <= 0.9)) w -= 1.0 / n2;
-            int i_b = ind_max, i_r = ind_max;
-            while ((nrm(i_b) > dep) && (i_b > 1)) i_b--;
-            while ((nrm(i_r + 1) > dep) && (i_r < (n - 2))) i_r++;
-            sp_ib[wp][t] = i_b;
-            sp_ir[wp][t] = i_r;
-            for (int side = 0; side < 2; ++side) {
-                const int i = side ? i_r : i_b;
-                const double a0 = nrm(i), a1 = nrm(i + 1), dx = x[i + 1] - x[i], den = a1 - a0;
-                const double dd = (x[i] + x[i + 1]) / 2. - v0;
-                const double e = exp(-(dd * dd) / 2. / ss);
-                const double dC = -dd / ss * e, d2C = ((dd * dd) / ss - 1) / ss * e;
-                const double q2 = -d2C / (2. * dC * dC * dC);
-                const double d3C = e * dd * (3. - dd * dd / ss) / (ss * ss);
-                const double dCs = dd * e / (ss * ss) * (1. - dd * dd / (2. * ss));
-                const double d2Cs = e * ((-2. * dd * dd / (ss * ss * ss) + 1. / (ss * ss)) +
-                                         (dd * dd / (ss * ss) - 1. / ss) * (dd * dd / (2. * ss * ss)));
-                const double c3 = dC * dC * dC, c4 = c3 * dC;
-                const double q2_dd = -0.5 * (d3C / c3 - 3. * d2C * d2C / c4);
-                const double q2_ss = -0.5 * (d2Cs / c3 - 3. * d2C * dCs / c4);
-                const double h = 0.5 * w;
-                const double pa0 = h * (dx * (dep - a1) / (den * den) - q2 * (dep - a1));
-                const double pa1 = h * (-dx * (dep - a0) / (den * den) - q2 * (dep - a0));
-                const double pq2 = h * (dep - a0) * (dep - a1);
-                sp_d[wp][t][2 * side] = pa0;
-                sp_d[wp][t][2 * side + 1] = pa1;
-                acc[0] += -(pa0 + pa1) / k;
-                acc[1] += -(pa0 * a0 + pa1 * a1) / k;
-                acc[2] += -pq2 * q2_dd;   // dd = vr - v0
-                acc[3] += pq2 * q2_ss;
+    if (gs != 0.0) {   // uniform for the block
+        const double nk = -c / k, ik = 1.0 / k;
+        key = 0ULL;
+        at = 0;
+        for (int i = tid; i < n; i += ADJ_THREADS) {
+            const double w = nk * (1. - y[i] / c);   // the forward's expression
+            norm[i] = w;
+            const unsigned long long o = w == w ? soap_ord64(w + 0.0) : 0ULL;
+            if (o > key) {
+                key = o;
+                at = i;
             }
         }
-        b[0] += gs * warp_sum(acc[0]);
-        b[1] += gs * warp_sum(acc[1]);
-        b[2] += gs * warp_sum(acc[2]);
-        b[3] += gs * warp_sum(acc[3]) * 2. * ss / fwhm;   // ss = (fwhm / 2 sqrt(2 ln 2))^2
+        int ind_max = block_argmax(key, at, &s_key, &s_idx);   // (its barriers publish norm)
+        if (ind_max >= n) ind_max = n - 1;
+        const double sig_b = fwhm / 2. / pow(2. * log(2.), .5), ss = sig_b * sig_b, iss = 1.0 / ss, iss2 = iss * iss;
+#pragma unroll
+        for (int q = 0; q < 16; ++q) v[q] = 0.0;   // first four: d span / d (c, k, v0, ss)
+        for (int t = tid; t < FIT_DEPTHS; t += ADJ_THREADS) {
+            const double dep = (double)(t + 5) / 100;
+            // depths 0.1 to 0.4 and 0.6 to 0.9: 31 each
+            const double w = t >= 5 && t <= 35 ? 1.0 / 31 : t >= 55 && t <= 85 ? -1.0 / 31 : 0.0;
+            int i_b = ind_max, i_r = min(ind_max, n - 2);
+            while ((norm[i_b] > dep) && (i_b > 1)) i_b--;
+            while ((norm[i_r + 1] > dep) && (i_r < (n - 2))) i_r++;
+            sp_ib[t] = i_b;
+            sp_ir[t] = i_r;
+#pragma unroll 1
+            for (int side = 0; side < 2; ++side) {
+                const int i = min(side ? i_r : i_b, n - 2);
+                const double a0 = norm[i], a1 = norm[i + 1], dx = x[i + 1] - x[i], iden = 1.0 / (a1 - a0);
+                const double dd = (x[i] + x[i + 1]) / 2. - v0, u = dd * dd * iss;
+                const double e = exp(-0.5 * u);
+                const double dC = -dd * iss * e, d2C = (u - 1) * iss * e;
+                const double idC = 1.0 / dC, ic3 = idC * idC * idC, ic4 = ic3 * idC;
+                const double q2 = -0.5 * d2C * ic3;
+                const double d3C = e * dd * (3. - u) * iss2;
+                const double dCs = dd * e * iss2 * (1. - 0.5 * u);
+                const double d2Cs = e * iss2 * ((1. - 2. * u) + (u - 1.) * 0.5 * u);
+                const double q2_dd = -0.5 * (d3C * ic3 - 3. * d2C * d2C * ic4);
+                const double q2_ss = -0.5 * (d2Cs * ic3 - 3. * d2C * dCs * ic4);
+                const double h = 0.5 * w, dxi = dx * iden * iden;
+                const double pa0 = h * (dep - a1) * (dxi - q2);
+                const double pa1 = -h * (dep - a0) * (dxi + q2);
+                const double pq2 = h * (dep - a0) * (dep - a1);
+                sp_d[t][2 * side] = pa0;
+                sp_d[t][2 * side + 1] = pa1;
+                v[0] += -(pa0 + pa1) * ik;
+                v[1] += -(pa0 * a0 + pa1 * a1) * ik;
+                v[2] += -pq2 * q2_dd;   // dd = vr - v0
+                v[3] += pq2 * q2_ss;
+            }
+        }
+        block_sum16(v, sums);   // (its barriers publish sp_ib, sp_ir and sp_d)
+        b[0] += gs * sums.tot[0];
+        b[1] += gs * sums.tot[1];
+        b[2] += gs * sums.tot[2];
+        b[3] += gs * sums.tot[3] * 2. * ss / fwhm;   // ss = (fwhm / 2 sqrt(2 ln 2))^2
     }
-    __syncwarp();
     {
         int t = 0;
         for (int p = 0; p < 4; ++p)
             for (int q = p; q < 4; ++q, ++t) { A[p * 4 + q] = H[t]; A[q * 4 + p] = H[t]; }
     }
     if (!solve4(A, b, z)) {
-        if (lane == 0) atomicExch(status, SOAPGB_ST_FIT_SINGULAR);
+        if (tid == 0) atomicExch(status, SOAPGB_ST_FIT_SINGULAR);
         for (int q = 0; q < 4; ++q) z[q] = 0.0;
     }
-    for (int i = lane; i < n; i += 32) {
-        const double inv = 1.0 / (err ? err[i] : 1.0);
+    for (int i = tid; i < n; i += ADJ_THREADS) {
+        const double inv = err ? 1.0 / err[i] : 1.0;
         const double d = x[i] - v0, d2 = d * d;
-        const double e = exp(-d2 / 2 / s2);
-        double g = inv * inv * (z[0] + e * z[1] + (k * e * d / s2) * z[2] + (k * e * d2 * a / s3) * z[3]);
+        const double e = exp(-0.5 * d2 * is2);
+        double g = inv * inv * (z[0] + e * z[1] + (k * e * d * is2) * z[2] + (k * e * d2 * a * is3) * z[3]);
         if (gs != 0.0) {   // the span's direct dependence on y_i (through a_i), depths in order
             double dir = 0.0;
             for (int t = 0; t < FIT_DEPTHS; ++t) {
-                const int ib = sp_ib[wp][t], ir = sp_ir[wp][t];
-                if (ib == i) dir += sp_d[wp][t][0];
-                if (ib + 1 == i) dir += sp_d[wp][t][1];
-                if (ir == i) dir += sp_d[wp][t][2];
-                if (ir + 1 == i) dir += sp_d[wp][t][3];
+                const int ib = sp_ib[t], ir = sp_ir[t];
+                if (ib == i) dir += sp_d[t][0];
+                if (ib + 1 == i) dir += sp_d[t][1];
+                if (ir == i) dir += sp_d[t][2];
+                if (ir + 1 == i) dir += sp_d[t][3];
             }
             g += gs * dir / k;
         }
@@ -533,6 +600,8 @@ extern "C" int soapgb_gauss_fit_adjoint(soapgb_ctx *ctx, int n_spec, int n, cons
     int s_x = ws.add(host ? sizeof(double) * n : 0);
     int s_y = ws.add(host ? sb : 0), s_e = ws.add(host && err ? sb : 0), s_m = ws.add(host ? sb : 0);
     int s_p = ws.add(host ? pb : 0), s_g = ws.add(host ? pb : 0), s_o = ws.add(host ? sb : 0);
+    const bool in_smem = sizeof(double) * (size_t)n <= FIT_SMEM_MAX - 8192;   // the normalised CCF
+    int s_scr = ws.add(in_smem ? 0 : sb);
     int rc = ws.commit();
     if (rc) return rc;
 #define STAGE(dst, src, bytes, slot)                                                  \
@@ -548,8 +617,9 @@ extern "C" int soapgb_gauss_fit_adjoint(soapgb_ctx *ctx, int n_spec, int n, cons
 #undef STAGE
     double *d_o = host ? ws.get<double>(s_o) : grad_y;
     SOAP_TRACED(ctx, "gauss_fit_adjoint",
-                k_gauss_fit_adj<<<(n_spec + FIT_WARPS - 1) / FIT_WARPS, 32 * FIT_WARPS, 0, ctx->stream>>>(
-                    n_spec, n, d_x, d_y, d_e, d_m, d_p, d_g, d_o, ctx->d_status));
+                k_gauss_fit_adj<<<n_spec, ADJ_THREADS, in_smem ? sizeof(double) * n : 0, ctx->stream>>>(
+                    n_spec, n, d_x, d_y, d_e, d_m, d_p, d_g, d_o, in_smem ? nullptr : ws.get<double>(s_scr),
+                    ctx->d_status));
     SOAP_LAUNCHED(ctx);
     if (host) {
         SOAP_CUDA(ctx, cudaMemcpyAsync(grad_y, d_o, sb, cudaMemcpyDeviceToHost, ctx->stream));

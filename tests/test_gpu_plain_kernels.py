@@ -207,3 +207,31 @@ def test_resolution_adjoint_is_the_transposed_window(ctx, n, n_spec, reso):
     gs = ctx.lower_resolution_adjoint(wave, spec, n_eff, sv, g, **kw)[0]
     assert np.isnan(gs[-1][(m >= mid - wid) & (m <= mid + wid - 2)]).all()
     assert not np.isnan(gs[:-1]).any()
+
+
+# fewer and more points than the fit's threads, its bisector arrays in shared memory and in scratch
+@pytest.mark.parametrize("n,n_spec,with_err", [(21, 1, False), (161, 5, True), (4001, 2, False)])
+def test_fit_and_its_adjoint(ctx, n, n_spec, with_err):
+    """The fit against the oracle's (the tolerances of test_gpu_parity: 1e-4 m/s, 1e-9 of the model);
+    its adjoint against a central difference of the fitted velocity along a direction (1e-4 of the
+    gradient's norm, as in test_gpu_ccf_adjoint)."""
+    rng = np.random.default_rng(n)
+    x = np.linspace(-20000.0, 20000.0, n)
+    sig = rng.uniform(3000, 4500, (n_spec, 1))
+    x0 = rng.uniform(-2000, 2000, (n_spec, 1))
+    y = 1.05 - rng.uniform(0.1, 0.4, (n_spec, 1)) * np.exp(-(x - x0) ** 2 / (2 * sig * sig)) + 1e-4 * np.sin(x / 777.0)
+    err = rng.uniform(0.5, 2.0, (n_spec, n)) if with_err else None
+    got = ctx.gauss_bis(x, y, err)
+    for s in range(n_spec):
+        ref = oracle.gauss_bis(x, y[s], None if err is None else err[s])
+        assert got["iters"][s] >= 0 and ref["iters"] >= 0
+        assert np.max(np.abs(got["par"][s, 2:] - ref["par"][2:])) < 1e-4
+        assert np.max(np.abs(got["bis"][s] - ref["bis"])) < 1e-4
+        assert np.max(np.abs(got["model"][s] - ref["model"])) < 1e-9
+    gp = np.zeros((n_spec, 5))
+    gp[:, 3] = 1.0
+    g = ctx.gauss_fit_adjoint(x, y, got["model"], got["par"], gp, err)
+    v = rng.standard_normal(y.shape)
+    h = 1e-4 / np.sqrt(n)
+    d = (ctx.gauss_bis(x, y + h * v, err)["par"][:, 3] - ctx.gauss_bis(x, y - h * v, err)["par"][:, 3]) / (2 * h)
+    assert np.all(np.abs(d - (g * v).sum(1)) <= 1e-4 * np.linalg.norm(g, axis=1) * np.linalg.norm(v, axis=1))
