@@ -286,9 +286,12 @@ extern "C" int soapgb_ccf(soapgb_ctx *ctx, int form, int n_v, const double *vel,
         w_first = wave_trim[0];
         w_last = wave_trim[n_w - 1];
     } else {
-        SOAP_CUDA(ctx, cudaMemcpyAsync(&w_first, wave_trim, sizeof(double), cudaMemcpyDeviceToHost, ctx->stream));
-        SOAP_CUDA(ctx, cudaMemcpyAsync(&w_last, wave_trim + n_w - 1, sizeof(double), cudaMemcpyDeviceToHost, ctx->stream));
+        double w2[2];   // the ends in one copy
+        SOAP_CUDA(ctx, cudaMemcpy2DAsync(w2, sizeof(double), wave_trim, sizeof(double) * (size_t)(n_w - 1), sizeof(double),
+                                         2, cudaMemcpyDeviceToHost, ctx->stream));
         SOAP_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
+        w_first = w2[0];
+        w_last = w2[1];
     }
     if (!(w_last > w_first)) return set_error(ctx, SOAPGB_ERR_ARG, "soapgb_ccf: wavelengths must ascend");
     CcfGeom g;
@@ -468,9 +471,12 @@ extern "C" int soapgb_ccf_adjoint(soapgb_ctx *ctx, int n_v, const double *vel, i
         w_first = wave_trim[0];
         w_last = wave_trim[n_w - 1];
     } else {
-        SOAP_CUDA(ctx, cudaMemcpyAsync(&w_first, wave_trim, sizeof(double), cudaMemcpyDeviceToHost, ctx->stream));
-        SOAP_CUDA(ctx, cudaMemcpyAsync(&w_last, wave_trim + n_w - 1, sizeof(double), cudaMemcpyDeviceToHost, ctx->stream));
+        double w2[2];   // the ends in one copy
+        SOAP_CUDA(ctx, cudaMemcpy2DAsync(w2, sizeof(double), wave_trim, sizeof(double) * (size_t)(n_w - 1), sizeof(double),
+                                         2, cudaMemcpyDeviceToHost, ctx->stream));
         SOAP_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
+        w_first = w2[0];
+        w_last = w2[1];
     }
     if (!(w_last > w_first)) return set_error(ctx, SOAPGB_ERR_ARG, "soapgb_ccf_adjoint: wavelengths must ascend");
     CcfGeom g;
