@@ -81,7 +81,7 @@ struct soapgb_batch {
     char *mem = nullptr;
     size_t bytes = 0;
     double *mu_b = nullptr;
-    char *typed_mem = nullptr;
+    char *typed_mem = nullptr, *quiet_pair = nullptr;
     FirTyped typed{};
     // worker streams: the per-star stages of star s run on worker s % n_work, so that the
     // small launches of different stars overlap; each worker has its own quiet-disk and
@@ -197,10 +197,10 @@ extern "C" int soapgb_batch_create(soapgb_ctx *ctx, const soapgb_batch_desc *d, 
     b->total_phases = d->phase_offsets[d->n_star];
     // sizes
     b->n_work = std::max(1, std::min(4, d->n_star));
-    b->quiet_fp = fir_plan_sizes(b->form, n, n_mu, max_gm, false, 1);
+    b->quiet_fp = fir_plan_sizes(b->form, n, n_mu, max_gm, false, 1, true);
     const size_t res_b = resolution_scratch_bytes(b->form, n, n_eff, (int)std::max(3LL, max_spec));
     size_t total = al256(sizeof(double) * (n_mu > 1 ? n_mu - 1 : 1)) + al256(fir_typed_bytes(b->form, n, n_mu)) +
-                   b->n_work * (al256(b->quiet_fp.bytes) + al256(res_b)) +
+                   al256(fir_quiet_pair_bytes(n, n_mu)) + b->n_work * (al256(b->quiet_fp.bytes) + al256(res_b)) +
                    al256(fir_tile_args_bytes() * d->n_star) + al256(sizeof(int2) * (size_t)std::max(1LL, b->total_phases));
     for (auto &st : b->stars) {
         total += al256(sizeof(double) * st.star.grid) + 4 * al256(sizeof(double) * st.gm) + al256(sizeof(int) * st.gm) +
@@ -221,6 +221,7 @@ extern "C" int soapgb_batch_create(soapgb_ctx *ctx, const soapgb_batch_desc *d, 
         SOAP_CUDA(ctx, cudaMemcpyAsync(b->mu_b, d->mu_boundary, sizeof(double) * (n_mu - 1), cudaMemcpyHostToDevice,
                                        ctx->stream));
     b->typed_mem = take(b.get(), off, fir_typed_bytes(b->form, n, n_mu));
+    b->quiet_pair = take(b.get(), off, fir_quiet_pair_bytes(n, n_mu));
     for (int w = 0; w < b->n_work; ++w) {
         b->quiet_ws.push_back(take(b.get(), off, b->quiet_fp.bytes));
         b->res_ws.push_back(take(b.get(), off, res_b));
@@ -358,6 +359,8 @@ extern "C" int soapgb_batch_run(soapgb_ctx *ctx, soapgb_batch *b, double *lower,
         FirTyped t;
         rc = fir_typed_cubes(ctx, b->form, n, b->cubes, b->typed_mem, &t);
         if (rc) return rc;
+        rc = fir_quiet_pair(ctx, n, b->cubes, b->quiet_pair);
+        if (rc) return rc;
     }
     // fork the workers off the context's stream
     auto fork = [&](int f) -> int {
@@ -375,8 +378,8 @@ extern "C" int soapgb_batch_run(soapgb_ctx *ctx, soapgb_batch *b, double *lower,
     };
     rc = fork(0);
     if (rc) return rc;
-    // per star, on its worker: disk maps, both quiet spectra (one set of lists), geometry
-    // (cell geometry, lists, prefix sums, tile plans)
+    // per star, on its worker: disk maps, geometry (cell geometry, lists, prefix sums, tile
+    // plans), both quiet spectra (one set of lists, of the same cells)
     for (size_t s = 0; s < b->stars.size(); ++s) {
         BatchStar &st = b->stars[s];
         const int w = (int)(s % b->n_work);
@@ -384,12 +387,19 @@ extern "C" int soapgb_batch_run(soapgb_ctx *ctx, soapgb_batch *b, double *lower,
         rc = disk_maps_launch(ctx, &st.star, n_mu, b->mu_b, st.ov, st.sin_incl, st.delta, st.limb, st.mu, st.region,
                               st.lb);
         if (rc) return rc;
+        FirGeoRef geo;
+        if (st.n_run > 0) {
+            st.fa.stage = FIR_STAGE_GEOMETRY;
+            rc = fir_phase(ctx, b->form, st.fa, st.fir, st.fp);
+            if (rc) return rc;
+            geo = fir_phase_geo(b->form, st.fa, st.fir);
+        }
         FirQuietArgs qa;
+        qa.geo = (st.n_run > 0) ? &geo : nullptr;
+        qa.pair = b->quiet_pair;
         qa.n = n;
         qa.n_eff = n_eff;
         qa.wave = b->wave;
-        qa.cube = b->cubes.q_sed;
-        qa.cube2 = b->cubes.q_norm;
         qa.n_mu = n_mu;
         qa.gm = st.gm;
         qa.delta = st.delta;
@@ -400,10 +410,6 @@ extern "C" int soapgb_batch_run(soapgb_ctx *ctx, soapgb_batch *b, double *lower,
         qa.out2 = st.q_norm;
         qa.lambda0 = b->w3[0];
         rc = fir_quiet(ctx, b->form, qa, b->quiet_ws[w], b->quiet_fp);
-        if (rc) return rc;
-        if (st.n_run == 0) continue;
-        st.fa.stage = FIR_STAGE_GEOMETRY;
-        rc = fir_phase(ctx, b->form, st.fa, st.fir, st.fp);
         if (rc) return rc;
     }
     rc = join(0);

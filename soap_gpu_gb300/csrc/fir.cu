@@ -30,6 +30,7 @@
 #include <type_traits>
 
 #include "fir.cuh"
+#include "order.cuh"
 #include "plain64.cuh"
 #include "regions.cuh"
 
@@ -41,7 +42,6 @@ constexpr int FIR_PIX = 4;
 constexpr int FIR_TILE = FIR_THREADS * FIR_PIX;
 constexpr int FIR_WIN = 1152;                    // staged values per cube row (window capacity)
 constexpr int FIR_MCH = FIR_WIN - FIR_TILE - 8;  // shift values per work unit (window + alignment fit)
-constexpr int FIR_EXC = 256;                     // exceptions per batch
 constexpr int FIR_MAX_MU = 256;
 constexpr long long FIR_WAIT_LIMIT = 1LL << 24;  // bounded mbarrier waits
 
@@ -122,14 +122,6 @@ __global__ void k_check_uniform(int n_eff, const double *__restrict__ lam, doubl
     if (fabs(lam[i] - expect) > 1e-6 * step) atomicExch(status, FIR_ST_UNIFORM);
 }
 
-template <typename T>
-__global__ void k_to_type(long long count, const double *__restrict__ a, const double *__restrict__ b, T *out) {
-    long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= count) return;
-    double v = b ? a[i] - b[i] : a[i];
-    out[i] = (T)v;
-}
-
 // FP64 -> FP32 rounded to nearest even on the integer pipes: the 52-bit fraction is cut
 // to 23 bits, rounding up past half and at half to even (a carry into the exponent is
 // the correct next binade, and past the largest exponent gives infinity).  Results
@@ -197,6 +189,33 @@ __global__ void __launch_bounds__(256) k_cube_types32(long long n2, const double
     }
 }
 
+// FP32 copy of a quiet cube, or of two side by side (c1), on the integer pipes (the
+// conversion instruction would occupy the FP64 pipe); paired: the cubes are 16-byte aligned
+__global__ void __launch_bounds__(256) k_quiet_types32(long long count, int paired, const double *__restrict__ c0,
+                                                       const double *__restrict__ c1, float *d) {
+    const long long stride = (long long)gridDim.x * blockDim.x, n2 = count / 2;
+    const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    auto two = [&](const double *c, long long i) {
+        const double2 v =
+            paired ? __ldcs(reinterpret_cast<const double2 *>(c) + i) : make_double2(c[2 * i], c[2 * i + 1]);
+        return make_float2(soap_f64_to_f32(v.x), soap_f64_to_f32(v.y));
+    };
+    for (long long i = t; i < n2; i += stride) {
+        const float2 a = two(c0, i);
+        if (c1) {
+            const float2 b = two(c1, i);
+            reinterpret_cast<float4 *>(d)[i] = make_float4(a.x, b.x, a.y, b.y);
+        } else {
+            reinterpret_cast<float2 *>(d)[i] = a;
+        }
+    }
+    if (t == 0 && (count & 1)) {
+        const long long k = count - 1;
+        if (c1) reinterpret_cast<float2 *>(d)[k] = make_float2(soap_f64_to_f32(c0[k]), soap_f64_to_f32(c1[k]));
+        else d[k] = soap_f64_to_f32(c0[k]);
+    }
+}
+
 // the same interleaved rows of any element type, one pixel per thread (the FP64 form, and
 // cubes whose layout the paired kernel cannot take)
 template <typename T>
@@ -219,8 +238,20 @@ __global__ void k_cube_rows(long long count, const double *__restrict__ qs, cons
 }
 
 // --- cell order ----------------------------------------------------------------
-// pass 1 keys: the slope dlt (order-preserving 64-bit image); pass 2 (stable): mu bin
-// and v == 0, invisible cells last
+// the order's keys: mu bin and v == 0 (invisible cells last), the slope dlt's
+// order-preserving 64-bit image, the cell
+struct FirCellKey {
+    const CellGeo *geo;
+    __device__ __forceinline__ OrderKey operator()(int k) const {
+        const CellGeo &g = geo[k];
+        const unsigned long long bin = (g.L > -998.0) ? (unsigned long long)(g.row * 2 + g.zero_v) : 0x3fffULL;
+        const unsigned long long od = soap_ord64(g.dlt);
+        return OrderKey{(bin << 50) | (od >> 14), ((od & 0x3fffULL) << 32) | (unsigned)k};
+    }
+};
+
+// the same order for grids above ORDER_MAX cells, by two stable radix sorts: pass 1 keys,
+// the slope's image; pass 2, mu bin and v == 0, invisible cells last
 __global__ void k_sort_keys1(long long gm, const CellGeo *__restrict__ geo, unsigned long long *keys, int *vals) {
     long long k = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= gm) return;
@@ -782,6 +813,141 @@ __global__ void __launch_bounds__(256) k_fir_prefix(long long gm, const int *__r
     }
 }
 
+// One list of all visible cells (the quiet disk's), over the whole chip: k_fir_prefix's
+// sums of class 0 in the same order of additions (256 runs of consecutive entries, each
+// summed one by one; the runs' totals scanned), without the facula weights' three, which
+// nothing reads.  The additions of one run are a chain, so its time is the FP64 latency
+// times the run's length; a block per list also issues all 256 runs' sums on one SM, which
+// is what took the time (70,600 cells: 448 us, and 152 us for the ordered list).  Here the
+// list is copied by the whole chip, the constants in list order beside it, and every (32
+// runs, sum) is one warp with an SM partition's FP64 pipe to itself: 47 us for both passes
+// and 6.5 us for the list (31,400 cells: 28 and 6 us against 210 and 72).
+constexpr int FIR_L1_RUNS = 256, FIR_L1_SUMS = 3;
+struct FirList1 {
+    const int *order;
+    const CellGeo *geo;
+    int *list_cell;
+    double *list_dlt, *L, *offir;   // list order
+    int *key;                       // row * 2 + zero_v, list order
+    int *counts;
+    double *run;                    // [2][FIR_L1_SUMS][FIR_L1_RUNS]: inclusive scans per 32 runs, totals
+    double *pre;
+    long long pre_comp;
+    int2 *segs;
+    int *nseg;
+};
+
+// the cells are sorted with the invisible ones last: the list is the order's visible prefix
+__global__ void __launch_bounds__(256) k_fir_list1(int gm, const FirList1 A) {
+    const int r = blockIdx.x * blockDim.x + threadIdx.x;
+    if (r >= gm) return;
+    const int cell = A.order[r], next = (r + 1 < gm) ? A.order[r + 1] : -1;
+    const CellGeo &g = A.geo[cell];
+    if (!(g.L > -998.0)) {
+        if (r == 0) *reinterpret_cast<int4 *>(A.counts) = make_int4(0, 0, 0, 0);
+        return;
+    }
+    A.list_cell[r] = cell;
+    A.list_dlt[r] = g.dlt;
+    A.L[r] = g.L;
+    A.offir[r] = g.offir;
+    A.key[r] = g.row * 2 + g.zero_v;
+    if (next < 0 || !(A.geo[next].L > -998.0)) *reinterpret_cast<int4 *>(A.counts) = make_int4(r + 1, 0, 0, 0);
+}
+
+// the run [a, b)'s sum C continued from s: C 0 of L, 1 of L dlt, 2 of L offir; PUT: the sum
+// before each entry is stored.  Eight entries' loads are in flight ahead of the chain.
+template <int C, bool PUT>
+__device__ __forceinline__ double fir_l1_chain(const FirList1 &A, int a, int b, double s) {
+    constexpr int U = 8;
+    const double *__restrict__ x = A.L, *__restrict__ y = C == 1 ? A.list_dlt : A.offir;
+    double *o = A.pre + C * A.pre_comp;
+    double xv[2][U], yv[2][U];
+    auto load = [&](int h, int q0) {
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            const int q = min(q0 + u, b - 1);
+            xv[h][u] = x[q];
+            yv[h][u] = (C == 0) ? 0.0 : y[q];
+        }
+    };
+    auto add = [&](int h, int q0) {
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            if (q0 + u >= b) break;
+            if (PUT) o[q0 + u] = s;
+            s = (C == 0) ? s + xv[h][u] : fma(xv[h][u], yv[h][u], s);
+        }
+    };
+    if (a >= b) return s;
+    load(0, a);
+    for (int q = a; q < b; q += 2 * U) {
+        load(1, q + U);
+        add(0, q);
+        load(0, q + 2 * U);
+        add(1, q + U);
+    }
+    return s;
+}
+
+// grid (FIR_L1_RUNS / 32, FIR_L1_SUMS [+ 1]) of one warp; PUT: the sums' exclusive prefixes
+// (pre[q] before entry q, the total after the last), else the runs' totals and their scans;
+// the row of blocks past the sums finds the segments of equal keys
+template <int C, bool PUT>
+__device__ __forceinline__ void fir_l1_runs(const FirList1 &A, int cnt) {
+    const int lane = threadIdx.x, run = blockIdx.x * 32 + lane;
+    const int per = (cnt + FIR_L1_RUNS - 1) / FIR_L1_RUNS;
+    const int a = min(cnt, run * per), b = min(cnt, (run + 1) * per);
+    double *inc = A.run + C * FIR_L1_RUNS, *tot = inc + FIR_L1_SUMS * FIR_L1_RUNS;
+    if (!PUT) {
+        const double v = fir_l1_chain<C, false>(A, a, b, 0.0);
+        double i = v;
+        for (int o = 1; o < 32; o <<= 1) {
+            const double t = __shfl_up_sync(0xffffffffu, i, o);
+            if (lane >= o) i += t;
+        }
+        inc[run] = i;
+        tot[run] = v;
+    } else {
+        double off = 0.0, all = 0.0;
+        for (int w = 0; w < FIR_L1_RUNS / 32; ++w) {
+            const double t = inc[32 * w + 31];
+            if (w < (int)blockIdx.x) off += t;
+            all += t;
+        }
+        fir_l1_chain<C, true>(A, a, b, off + inc[run] - tot[run]);
+        if (run == 0) A.pre[C * A.pre_comp + cnt] = all;
+    }
+}
+
+template <bool PUT>
+__global__ void __launch_bounds__(32) k_fir_prefix1(const FirList1 A, int n_key) {
+    const int cnt = A.counts[0], lane = threadIdx.x;
+    if (blockIdx.y == 0) fir_l1_runs<0, PUT>(A, cnt);
+    else if (blockIdx.y == 1) fir_l1_runs<1, PUT>(A, cnt);
+    else if (blockIdx.y == 2) fir_l1_runs<2, PUT>(A, cnt);
+    else if (blockIdx.x == 0) {
+        int ns = 0;
+        for (int k0 = 0; k0 < n_key; k0 += 31) {   // lane's first entry of a key >= k0 + lane
+            int lo = 0, hi = cnt;
+            while (lo < hi) {
+                const int m = (lo + hi) >> 1;
+                if (A.key[m] < k0 + lane) lo = m + 1;
+                else hi = m;
+            }
+            const int end = __shfl_down_sync(0xffffffffu, lo, 1);
+            const bool seg = lane < 31 && k0 + lane < n_key && lo < end;
+            const unsigned m = __ballot_sync(0xffffffffu, seg);
+            if (seg) A.segs[ns + __popc(m & ((1u << lane) - 1))] = make_int2(lo, k0 + lane);
+            ns += __popc(m);
+        }
+        if (lane == 0) {
+            A.nseg[0] = ns;
+            A.nseg[1] = 0;
+        }
+    }
+}
+
 // --- device helpers of the tile kernel -------------------------------------------------
 // per-pixel sums of the FP32 form: compensated (Kahan) when set
 constexpr bool FIR_COMPENSATED = true;
@@ -947,15 +1113,6 @@ struct FirCubes {
     const float2 *fac_sed2;
 };
 
-// cube rows staged for a segment of class cls (window slot q)
-//   spot:   S (q_sed), Qs (q_norm), As (spot_norm), Bs (q_norm - spot_norm)  -- weight L
-//   facula: S (q_sed), Bf (q_norm - fac_norm) -- weight L; Qf (q_norm), Af (fac_norm) -- weight (1+LB) L
-__device__ __forceinline__ int fir_cube_index(int mode, int cls, int q) {
-    if (mode == MODE_QUIET) return 0;
-    if (cls == CLS_SPOT) return q;
-    return (q == 0) ? 0 : (q == 1) ? 5 : (q == 2) ? 1 : 4;
-}
-
 struct FirSeg {
     int start, end;     // list positions
     int key;            // row * 2 + zero_v
@@ -993,23 +1150,52 @@ struct FirExcD {        // directly evaluated cell (reads the cubes in global me
     double temp;
 };
 
+// The quiet disk's records (weight L only): the FP32 form's coefficients twice, as the
+// packed instructions take them; both records are 16-byte loads.
+struct __align__(16) FirGrpQ32 {
+    float a0, a0b, a1, a1b, b, bb;
+    int m, ok;
+    __device__ __forceinline__ FirGrpQ32 &operator=(const FirGrp<float> &g) {
+        a0 = a0b = g.a0;
+        a1 = a1b = g.a1;
+        b = bb = g.b;
+        m = g.m;
+        ok = g.ok;
+        return *this;
+    }
+};
+struct __align__(16) FirExcQ32 {
+    int i0;
+    float phi, dlt, L;
+};
+
+__device__ __forceinline__ void fir_put_exc(FirExcQ32 &d, const FirExcW<float> &x) {
+    d.i0 = x.i0;
+    d.phi = x.phi;
+    d.dlt = x.dlt;
+    d.L = x.L;
+}
+template <typename T>
+__device__ __forceinline__ void fir_put_exc(FirExcW<T> &d, const FirExcW<T> &x) { d = x; }
+
 // Plan of (a batch of) a tile's work units: units, one group per shift value (task),
 // and the wrap cells.  U units, G tasks, E wrap cells at most.
-template <typename T, int U, int G, int E>
+template <typename T, int U, int G, int E, typename GRP = FirGrp<T>, typename EXC = FirExcW<T>>
 struct FirPlanSt {
     static constexpr int NU = U, NG = G, NE = E;
     FirUnit unit[U];
     int ut[U + 1];          // first task of each unit; ut[nb] = ntask
-    FirGrp<T> grp[G];
+    GRP grp[G];
     int wlo[G];             // first list position of each task's wrap cells
     int woff[G + 1];        // exclusive offsets of the tasks' wrap cells; woff[ntask] = etot
-    FirExcW<T> excw[E];
+    EXC excw[E];
     int nunit, nb, ntask, etot, ok;
 };
 
-// the tile kernel's batches, and the plans precomputed per tile by k_fir_plan
-template <typename T>
-using FirTileSt = FirPlanSt<T, 128, (sizeof(T) == 4) ? 512 : 256, (sizeof(T) == 4) ? 512 : 256>;
+// the quiet tile kernel's batches, and the plans precomputed per tile by k_fir_plan
+template <typename T> struct FirTileStT { using type = FirPlanSt<double, 128, 256, 256>; };
+template <> struct FirTileStT<float> { using type = FirPlanSt<float, 128, 512, 512, FirGrpQ32, FirExcQ32>; };
+template <typename T> using FirTileSt = typename FirTileStT<T>::type;
 template <typename T>
 using FirPrePlan = FirPlanSt<T, 32, 128, 128>;
 // one warp per (list, tile): the plan's block barriers are then a single warp's
@@ -1046,23 +1232,23 @@ struct FirListCap {
     static constexpr int N = (sizeof(T) == 4) ? 4096 : 1024;
 };
 
-template <typename T, int NC>
+// the staged element of the quiet disk: a value, or the FP32 form's two cubes side by side
+template <typename T, int NQ> struct FirQuietElT { using type = T; };
+template <> struct FirQuietElT<float, 2> { using type = float2; };
+template <typename T, int NQ> using FirQuietEl = typename FirQuietElT<T, NQ>::type;
+
+// the quiet tile kernel's shared memory, followed by FirSeg seg[] and a short list's slopes
+template <typename T, int NQ>
 struct FirSmem {
-    // staged windows; the direct cells' buffer reuses this space once all copies landed
-    union {
-        T win[2][NC][FIR_WIN];
-        FirExcD<T> excd[FIR_EXC];
-    };
+    FirQuietEl<T, NQ> win[2][FIR_WIN];   // staged windows
     unsigned long long bar[2];
     FirTileSt<T> st;
-    int wsum[FIR_THREADS / 32];
+    int wsum[32];
     int fail;
-    double sdl[FirListCap<T>::N];          // the list's slopes (short lists)
-    // followed by FirSeg seg[] (dynamic, 16-byte aligned)
 };
 
-template <typename T, int NC>
-__host__ __device__ constexpr size_t fir_smem_fixed() { return (sizeof(FirSmem<T, NC>) + 15) & ~size_t(15); }
+template <typename T, int NQ>
+__host__ __device__ constexpr size_t fir_smem_fixed() { return (sizeof(FirSmem<T, NQ>) + 15) & ~size_t(15); }
 
 template <int NT>
 __device__ __forceinline__ int block_excl_scan_int(int v, int *wsum, int &total) {
@@ -1190,12 +1376,10 @@ __device__ int fir_segments(const FirTileArgs &A, int l, int j0, int t_eff, FirS
     return *nunit_sh;
 }
 
-// descriptor of work unit u: its segment, shift values and source window
-// (PHASE: the staged rows are Vec4 elements, 16-byte aligned, so the window starts at
-// its first pixel; QUIET: rows of T, staged from the 16-byte boundary below w0)
-template <typename T, int MODE>
-__device__ __forceinline__ FirUnit fir_describe(int u, const FirSeg *segs, int nsg, int j0, int t_eff, int n,
-                                                int n_eff) {
+// descriptor of work unit u: its segment, shift values and source window (off = 0: the
+// phases' staged rows are Vec4 elements, 16-byte aligned, so the window starts at its first
+// pixel; the quiet kernel finds its own)
+__device__ __forceinline__ FirUnit fir_describe(int u, const FirSeg *segs, int nsg, int j0, int t_eff, int n_eff) {
     int lo = 0, hi = nsg - 1;
     while (lo < hi) {   // last segment with u0 <= u
         int mid = (lo + hi + 1) >> 1;
@@ -1213,9 +1397,7 @@ __device__ __forceinline__ FirUnit fir_describe(int u, const FirSeg *segs, int n
     d.mb = min(g.m_hi, d.ma + FIR_MCH - 1);
     d.w0 = max(0, j0 + d.ma - (d.ma > g.m_lo ? 1 : 0));
     d.w1 = min(n_eff, j0 + t_eff + d.mb + 1);
-    d.off = (MODE == MODE_PHASE || d.w1 <= d.w0)
-                ? 0
-                : (int)(((((long long)(g.key >> 1) * n + d.w0) * (long long)sizeof(T)) & 15) / (long long)sizeof(T));
+    d.off = 0;
     return d;
 }
 
@@ -1232,7 +1414,7 @@ __device__ __forceinline__ void fir_fill_exc(const FirTileArgs &A, int l, int j0
         const int cell = A.list_cell[lbase + st.wlo[a] + (e - st.woff[a])];
         FirExcW<T> x;
         cell_pos<T>(j0, A.geo, A.geo32, cell, x.i0, x.phi, x.dlt, x.L, x.w2);
-        st.excw[e - dst0] = x;
+        fir_put_exc(st.excw[e - dst0], x);
     }
 }
 
@@ -1243,11 +1425,11 @@ template <typename T, int MODE, int NT, typename ST>
 __device__ void fir_plan_batch(const FirTileArgs &A, int l, int j0, int t_eff, const FirSeg *segs, int nsg,
                                int nunit, const double *sl, ST &st, int ub, int *wsum) {
     const int tid = threadIdx.x;
-    const int n = A.n, n_eff = A.n_eff;
+    const int n_eff = A.n_eff;
     const double dj0 = soap_i2d(j0);
     const double iXa = 1.0 / (dj0 + A.los), iXb = 1.0 / (soap_i2d(j0 + t_eff - 1) + A.los);
     const int nbu = min(ST::NU, nunit - ub);
-    for (int t = tid; t < nbu; t += NT) st.unit[t] = fir_describe<T, MODE>(ub + t, segs, nsg, j0, t_eff, n, n_eff);
+    for (int t = tid; t < nbu; t += NT) st.unit[t] = fir_describe(ub + t, segs, nsg, j0, t_eff, n_eff);
     __syncthreads();
     if (tid == 0) {
         int nb = 0, nt = 0;
@@ -1403,80 +1585,115 @@ __global__ void __launch_bounds__(FIR_PLAN_THREADS) k_fir_plan(const FirTileArgs
     }
 }
 
-// QUIET: OutT = double (one spectrum, once per star); PHASE: OutT = T (the FP32 form
-// keeps its deficits in FP32 for the FP32 convolution that consumes them)
-template <typename T, int MODE, typename OutT>
-__global__ void __launch_bounds__(FIR_THREADS) k_fir(const FirTileArgs A) {
-    constexpr int NC = (MODE == MODE_QUIET) ? 1 : 4;
+// Quiet disk: NQ cubes (one, or the FP32 form's SED and normalised cubes interleaved)
+// integrated over one list, FP64 sums out.  A tile's plan -- searches in the list, prefix
+// sums, wrap cells -- and its barriers do not depend on the cube, so both cubes are applied
+// to one plan.  The FP32 form is bound by instruction issue: its sums run in packed pairs
+// (two cubes of a pixel, or two pixels of one cube), a unit whose groups stay inside the
+// grid and a wrap cell whose sources stay inside the window go without tests, and the
+// group's coefficients lie in shared memory twice, ready for the packed instructions.
+// 512 threads share a tile's 1024 pixels (256 in the FP64 form, bound by its pipe): a grid of
+// 303 tiles is two blocks per SM, and eight warps each leave the issue slots half empty.
+// Two cubes, 310,000 pixels, 250 x 250 cells: 260 us against 774 us as two launches with
+// scalar sums; one cube of 300 x 300: 124 against 205 us, 200 x 200 and 100,000: 77 and 100.
+template <typename T, int NQ>
+constexpr int FIR_QUIET_THREADS = (sizeof(T) == 4) ? 512 : 256;
+
+// the quiet sums of a thread's pixels: double, plain; float, packed pairs with their
+// compensation (s, -c of Acc), in Acc's order of operations
+template <typename T, int NQ, int PIX> struct QuietSums;
+template <int PIX> struct QuietSums<double, 1, PIX> {
+    double s[PIX];
+    __device__ __forceinline__ void zero() {
+#pragma unroll
+        for (int q = 0; q < PIX; ++q) s[q] = 0.0;
+    }
+    __device__ __forceinline__ double get(int c, int q) const { return s[q]; }
+};
+template <int NQ, int PIX> struct QuietSums<float, NQ, PIX> {
+    static constexpr int NP = NQ * PIX / 2;   // pairs: NQ = 2, pair q = pixel q; NQ = 1, pixels 2p and 2p + 1
+    float s[NP][2], nc[NP][2];
+    __device__ __forceinline__ void zero() {
+#pragma unroll
+        for (int p = 0; p < NP; ++p) s[p][0] = s[p][1] = nc[p][0] = nc[p][1] = 0.f;
+    }
+    __device__ __forceinline__ double get(int c, int q) const {
+        const int p = NQ == 2 ? q : q / 2, h = NQ == 2 ? c : q % 2;
+        return (double)s[p][h] + (double)nc[p][h];
+    }
+    // pair p: y = the term plus the compensation
+    __device__ __forceinline__ void add(int p, float y0, float y1) {
+        float t0 = s[p][0], t1 = s[p][1];
+        soap_add2(t0, t1, y0, y1);
+        float d0 = t0, d1 = t1;
+        soap_sub2(d0, d1, s[p][0], s[p][1]);
+        soap_sub2(y0, y1, d0, d1);
+        nc[p][0] = y0;
+        nc[p][1] = y1;
+        s[p][0] = t0;
+        s[p][1] = t1;
+    }
+    // one value of pair p
+    __device__ __forceinline__ void add1(int p, int h, float y) {
+        const float t = __fadd_rn(s[p][h], y);
+        nc[p][h] = __fsub_rn(y, __fsub_rn(t, s[p][h]));
+        s[p][h] = t;
+    }
+};
+
+template <typename T, int NQ>
+__global__ void __launch_bounds__(FIR_QUIET_THREADS<T, NQ>) k_fir_quiet(const FirTileArgs A, int stage_slopes) {
+    constexpr int NT = FIR_QUIET_THREADS<T, NQ>, PIX = FIR_TILE / NT;
+    using El = FirQuietEl<T, NQ>;
+    constexpr int PER16 = 16 / (int)sizeof(El);   // elements per 16 bytes
     extern __shared__ __align__(128) unsigned char fir_smem[];
-    FirSmem<T, NC> &sh = *reinterpret_cast<FirSmem<T, NC> *>(fir_smem);
-    FirSeg *segs = reinterpret_cast<FirSeg *>(fir_smem + fir_smem_fixed<T, NC>());
+    FirSmem<T, NQ> &sh = *reinterpret_cast<FirSmem<T, NQ> *>(fir_smem);
+    FirSeg *segs = reinterpret_cast<FirSeg *>(fir_smem + fir_smem_fixed<T, NQ>());
     FirTileSt<T> &st = sh.st;
-    const int l = blockIdx.y;
     const int j0 = blockIdx.x * FIR_TILE;
     const int tid = threadIdx.x;
     const int n = A.n, n_eff = A.n_eff;
-    OutT *out0 = reinterpret_cast<OutT *>(A.out0);
-    OutT *out1 = reinterpret_cast<OutT *>(A.out1);
-    OutT *out2 = reinterpret_cast<OutT *>(A.out2);
+    double *const outs[2] = {reinterpret_cast<double *>(A.out0), reinterpret_cast<double *>(A.out1)};
+    const El *__restrict__ cube = reinterpret_cast<const El *>(A.cubes.c[0]);
     const int t_eff = min(FIR_TILE, n_eff - j0);
     if (t_eff <= 0) {   // whole tile in the zero tail [n_eff, n)
-        for (int q = 0; q < FIR_PIX; ++q) {
-            int j = j0 + tid + q * FIR_THREADS;
-            if (j >= n) continue;
-            long long o = (long long)l * A.out_stride + j;
-            out0[o] = (OutT)0;
-            if constexpr (MODE == MODE_PHASE) { out1[o] = (OutT)0; out2[o] = (OutT)0; }
-        }
+#pragma unroll
+        for (int c = 0; c < NQ; ++c)
+            for (int j = j0 + tid; j < min(n, j0 + FIR_TILE); j += NT) outs[c][j] = 0.0;
         return;
     }
-    const long long lbase = (long long)l * A.gm;
-    const int *cn = A.counts + 4 * l;
     if (tid == 0) {
         mbar_init(&sh.bar[0], 1);
         mbar_init(&sh.bar[1], 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         sh.fail = 0;
     }
-
-    // accumulators: QUIET [0]; PHASE: S, Qs, As, Bs, Qf, Af, Bf
-    constexpr int NACC = (MODE == MODE_QUIET) ? 1 : 7;
-    Acc<T> acc[NACC][FIR_PIX];
-#pragma unroll
-    for (int a = 0; a < NACC; ++a)
-#pragma unroll
-        for (int q = 0; q < FIR_PIX; ++q) acc[a][q].zero();
+    QuietSums<T, NQ, PIX> acc;
+    acc.zero();
 
     constexpr int EXC = FirTileSt<T>::NE;
-    // staging of unit u's rows into buffer u & 1 (thread 0)
+    // staging of unit u's rows into buffer u & 1, from the 16-byte boundary below w0 (thread 0)
     auto issue = [&](int u, const FirUnit &d) {
         const int b = u & 1;
         unsigned bytes = 0;
-        uintptr_t rel = 0;   // 16-byte aligned start, relative to the cube base
+        long long e0 = 0;
         if (d.w1 > d.w0) {
-            const uintptr_t p0 = (uintptr_t)((long long)(d.key >> 1) * n + d.w0) * sizeof(T);
-            const uintptr_t p1 = (uintptr_t)((long long)(d.key >> 1) * n + d.w1) * sizeof(T);
-            rel = p0 & ~uintptr_t(15);
-            bytes = (unsigned)(((p1 + 15) & ~uintptr_t(15)) - rel);
+            const long long row = (long long)(d.key >> 1) * n;
+            e0 = (row + d.w0) & ~(long long)(PER16 - 1);
+            bytes = (unsigned)((((row + d.w1 + PER16 - 1) & ~(long long)(PER16 - 1)) - e0) * (long long)sizeof(El));
         }
         // the buffer was last read through the generic proxy; order those reads before
         // the async-proxy writes
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-        mbar_expect_tx(&sh.bar[b], bytes * NC);
-        if (bytes) {
-#pragma unroll
-            for (int q = 0; q < NC; ++q) {
-                const char *base = reinterpret_cast<const char *>(A.cubes.c[fir_cube_index(MODE, d.cls, q)]);
-                bulk_g2s(&sh.win[b][q][0], base + rel, bytes, &sh.bar[b]);
-            }
-        }
+        mbar_expect_tx(&sh.bar[b], bytes);
+        if (bytes) bulk_g2s(&sh.win[b][0], cube + e0, bytes, &sh.bar[b]);
     };
 
     int u_fail = -1;
     int issued = -1;   // last unit whose copy was issued (thread 0)
     // apply the planned units st.unit[0, nb) (global unit numbers ub + ui)
     auto run_units = [&](int ub) {
-        const int nb = st.nb, ntask = st.ntask;
+        const int nb = st.nb;
         if (tid == 0 && nb > 0 && issued < ub) {
             issue(ub, st.unit[0]);
             issued = ub;
@@ -1488,149 +1705,205 @@ __global__ void __launch_bounds__(FIR_THREADS) k_fir(const FirTileArgs A) {
                 issued = u + 1;
             }
             const FirUnit d = st.unit[ui];
-            const int cls = d.cls, zv = d.key & 1;
+            const int zv = d.key & 1;
             if (!mbar_wait_bounded(&sh.bar[u & 1], (unsigned)((u >> 1) & 1))) atomicExch(&sh.fail, 1);
             __syncthreads();
             if (sh.fail) {
                 u_fail = u;
                 return;
             }
-            const T(*W)[FIR_WIN] = sh.win[u & 1];
-            const int wo = d.off - d.w0;   // staged index of source pixel i: i + wo
+            const El *W = sh.win[u & 1];
+            // staged index of source pixel i: i + wo
+            const int wo = (int)(((long long)(d.key >> 1) * n + d.w0) & (PER16 - 1)) - d.w0;
             const int t_lo = st.ut[ui], t_hi = st.ut[ui + 1];
-            for (int t = t_lo; t < t_hi; ++t) {
-                const FirGrp<T> gr = st.grp[t];
-                if (!gr.ok) continue;
-                const int m = gr.m;
-                // pixels whose owner j + m lies in [0, n_eff - 2] (v == 0: [0, n_eff - 1])
-                const int jlo = max(j0, -m);
-                const int jhi = zv ? j0 + t_eff - 1 : min(j0 + t_eff - 1, n_eff - 2 - m);
-                // the group at the thread's pixels; CHECKED: some pixels of the tile fall
-                // outside [jlo, jhi], else none and no test is needed (same arithmetic)
-                auto group_at = [&](auto checked_c) {
-                    constexpr bool CHECKED = decltype(checked_c)::value;
+            // Pixels whose owner j + m lies in [0, n_eff - 2] (v == 0: [0, n_eff - 1]) take the
+            // group.  CHECKED: for some group of the unit a pixel of the tile does not.
+            auto groups = [&](auto checked_c, auto zv_c) {
+                constexpr bool CHECKED = decltype(checked_c)::value, ZV = decltype(zv_c)::value;
+                for (int t = t_lo; t < t_hi; ++t) {
+                    const auto gr = st.grp[t];
+                    if (!gr.ok) continue;
+                    const int m = gr.m;
+                    const int jlo = max(j0, -m);
+                    const int jhi = ZV ? j0 + t_eff - 1 : min(j0 + t_eff - 1, n_eff - 2 - m);
+                    const int x0 = j0 + tid + m + wo;
+                    if constexpr (sizeof(T) == 8) {
 #pragma unroll
-                    for (int q = 0; q < FIR_PIX; ++q) {
-                        const int dj = tid + q * FIR_THREADS;
-                        const int j = j0 + dj;
-                        if (CHECKED && (j < jlo || j > jhi)) continue;
-                        const int x = j + m + wo;
-                        if (zv) {   // single tap: w == 0
-                            if constexpr (MODE == MODE_QUIET) {
-                                acc[0][q].add(gr.a0 * W[0][x]);
-                            } else if (cls == CLS_SPOT) {
-                                acc[0][q].add(gr.a0 * W[0][x]);
-                                acc[1][q].add(gr.a0 * W[1][x]);
-                                acc[2][q].add(gr.a0 * W[2][x]);
-                                acc[3][q].add(gr.a0 * W[3][x]);
-                            } else {
-                                acc[0][q].add(gr.a0 * W[0][x]);
-                                acc[6][q].add(gr.a0 * W[1][x]);
-                                acc[4][q].add(gr.a0w * W[2][x]);
-                                acc[5][q].add(gr.a0w * W[3][x]);
+                        for (int q = 0; q < PIX; ++q) {
+                            const int dj = tid + q * NT, j = j0 + dj;
+                            if (CHECKED && (j < jlo || j > jhi)) continue;
+                            const int x = x0 + q * NT;
+                            if (ZV) {   // single tap: w == 0
+                                acc.s[q] += gr.a0 * W[x];
+                                continue;
                             }
-                            continue;
+                            const T fdj = (T)dj;
+                            const T c0 = gr.a0 - gr.b * fdj, c1 = gr.a1 + gr.b * fdj;
+                            acc.s[q] += c0 * W[x] + c1 * W[x + 1];
                         }
-                        const T fdj = (T)dj;
-                        const T c0 = gr.a0 - gr.b * fdj, c1 = gr.a1 + gr.b * fdj;
-                        if constexpr (MODE == MODE_QUIET) {
-                            acc[0][q].add(c0 * W[0][x] + c1 * W[0][x + 1]);
-                        } else if (cls == CLS_SPOT) {
-                            acc[0][q].add(c0 * W[0][x] + c1 * W[0][x + 1]);
-                            acc[1][q].add(c0 * W[1][x] + c1 * W[1][x + 1]);
-                            acc[2][q].add(c0 * W[2][x] + c1 * W[2][x + 1]);
-                            acc[3][q].add(c0 * W[3][x] + c1 * W[3][x + 1]);
-                        } else {
-                            const T e0 = gr.a0w - gr.bw * fdj, e1 = gr.a1w + gr.bw * fdj;
-                            acc[0][q].add(c0 * W[0][x] + c1 * W[0][x + 1]);
-                            acc[6][q].add(c0 * W[1][x] + c1 * W[1][x + 1]);
-                            acc[4][q].add(e0 * W[2][x] + e1 * W[2][x + 1]);
-                            acc[5][q].add(e0 * W[3][x] + e1 * W[3][x + 1]);
+                    } else {
+#pragma unroll
+                        for (int p = 0; p < QuietSums<T, NQ, PIX>::NP; ++p) {
+                            // the pair's pixels
+                            const int qa = NQ == 2 ? p : 2 * p, qb = NQ == 2 ? p : 2 * p + 1;
+                            const int ja = j0 + tid + qa * NT, jb = j0 + tid + qb * NT;
+                            const bool oka = !CHECKED || !(ja < jlo || ja > jhi);
+                            const bool okb = !CHECKED || !(jb < jlo || jb > jhi);
+                            float v0a, v0b, v1a = 0.f, v1b = 0.f;
+                            const int xa = oka ? x0 + qa * NT : 0;
+                            if constexpr (NQ == 2) {
+                                const float2 v = W[xa];
+                                v0a = v.x, v0b = v.y;
+                                if (!ZV) {
+                                    const float2 w = W[xa + 1];
+                                    v1a = w.x, v1b = w.y;
+                                }
+                            } else {
+                                const int xb = okb ? x0 + qb * NT : 0;
+                                v0a = W[xa], v0b = W[xb];
+                                if (!ZV) v1a = W[xa + 1], v1b = W[xb + 1];
+                            }
+                            float ya = acc.nc[p][0], yb = acc.nc[p][1];
+                            if (ZV) {   // single tap: w == 0
+                                soap_fma2(ya, yb, gr.a0, gr.a0b, v0a, v0b);
+                            } else {
+                                const float fa = (float)(tid + qa * NT), fb = (float)(tid + qb * NT);
+                                float c0 = gr.a0, c0b = gr.a0b, c1 = gr.a1, c1b = gr.a1b, ta, tb;
+                                soap_fma2(c0, c0b, gr.b, gr.bb, -fa, -fb);
+                                soap_fma2(c1, c1b, gr.b, gr.bb, fa, fb);
+                                soap_mul2(ta, tb, c1, c1b, v1a, v1b);
+                                soap_fma2(ta, tb, c0, c0b, v0a, v0b);
+                                soap_add2(ya, yb, ta, tb);
+                            }
+                            if (!CHECKED) {
+                                acc.add(p, ya, yb);
+                            } else {
+                                if (oka) acc.add1(p, 0, ya);
+                                if (okb) acc.add1(p, 1, yb);
+                            }
                         }
                     }
-                };
-                if (jlo <= j0 && jhi >= j0 + FIR_TILE - 1) group_at(std::integral_constant<bool, false>());
-                else group_at(std::integral_constant<bool, true>());
+                }
+            };
+            using yes = std::integral_constant<bool, true>;
+            using no = std::integral_constant<bool, false>;
+            const bool in_grid = j0 + d.ma >= 0 && t_eff == FIR_TILE && (zv || j0 + FIR_TILE - 1 <= n_eff - 2 - d.mb);
+            if (zv) {
+                if (in_grid) groups(no(), yes());
+                else groups(yes(), yes());
+            } else {
+                if (in_grid) groups(no(), no());
+                else groups(yes(), no());
             }
             // --- wrap cells of the unit (per-cell lerp from the staged rows) ------------
+            // CHECKED: a pixel may lie past n_eff or read a source outside [0, n_eff - 2] or
+            // outside the window; else none can, and the sign of the slope tells at which end
+            // of [0, 1) the weight can leave.
+            auto cell_at = [&](auto checked_c, auto up_c, const auto &xc) {
+                constexpr bool CHECKED = decltype(checked_c)::value, UP = decltype(up_c)::value;
+                auto source = [&](int q, T &wd, int &i) {
+                    const int dj = tid + q * NT;
+                    wd = xc.phi + xc.dlt * (T)dj;
+                    i = xc.i0 + dj;
+                    if ((CHECKED || UP) && wd >= (T)1) { wd -= (T)1; i += 1; }
+                    else if ((CHECKED || !UP) && wd < (T)0) { wd += (T)1; i -= 1; }
+                };
+                // pixel q one by one
+                auto pixels = [&](auto &&put) {
+#pragma unroll
+                    for (int q = 0; q < PIX; ++q) {
+                        if (CHECKED && j0 + tid + q * NT >= n_eff) continue;
+                        T wd;
+                        int i;
+                        source(q, wd, i);
+                        if (CHECKED && (i < 0 || i > n_eff - 2)) continue;
+                        // the per-cell owner can differ by one from the segment's
+                        // classification when t lies within rounding of an integer: such
+                        // pixels read the row in global memory instead of the window
+                        const bool staged = !CHECKED || ((i >= d.w0) && (i + 1 < d.w1));
+                        const El *rowp = staged ? W + (i + wo) : cube + ((long long)(d.key >> 1) * n + i);
+                        put(q, wd, rowp[0], rowp[1]);
+                    }
+                };
+                if constexpr (sizeof(T) == 8) {
+                    pixels([&](int q, T wd, El s0, El s1) { acc.s[q] += xc.L * (s0 + (s1 - s0) * wd); });
+                } else if constexpr (CHECKED) {
+                    pixels([&](int q, T wd, El s0, El s1) {
+                        if constexpr (NQ == 2) {
+                            acc.add1(q, 0, fmaf(xc.L, fmaf(__fsub_rn(s1.x, s0.x), wd, s0.x), acc.nc[q][0]));
+                            acc.add1(q, 1, fmaf(xc.L, fmaf(__fsub_rn(s1.y, s0.y), wd, s0.y), acc.nc[q][1]));
+                        } else {
+                            acc.add1(q / 2, q % 2,
+                                     fmaf(xc.L, fmaf(__fsub_rn(s1, s0), wd, s0), acc.nc[q / 2][q % 2]));
+                        }
+                    });
+                } else {
+#pragma unroll
+                    for (int p = 0; p < QuietSums<T, NQ, PIX>::NP; ++p) {
+                        float wa, wb, s0a, s0b, ga, gb;
+                        int ia;
+                        if constexpr (NQ == 2) {
+                            source(p, wa, ia);
+                            wb = wa;
+                            const float2 s0 = W[ia + wo], s1 = W[ia + wo + 1];
+                            s0a = s0.x, s0b = s0.y, ga = s1.x, gb = s1.y;
+                        } else {
+                            int ib;
+                            source(2 * p, wa, ia);
+                            source(2 * p + 1, wb, ib);
+                            s0a = W[ia + wo], s0b = W[ib + wo], ga = W[ia + wo + 1], gb = W[ib + wo + 1];
+                        }
+                        soap_sub2(ga, gb, s0a, s0b);
+                        soap_fma2(s0a, s0b, ga, gb, wa, wb);
+                        float ya = acc.nc[p][0], yb = acc.nc[p][1];
+                        soap_fma2(ya, yb, xc.L, xc.L, s0a, s0b);
+                        acc.add(p, ya, yb);
+                    }
+                }
+            };
             const int e_lo = st.woff[t_lo], e_hi = st.woff[t_hi];
             for (int cb = e_lo; cb < e_hi; cb += EXC) {
                 const int ce = min(e_hi, cb + EXC);
                 int x0 = cb;   // excw index of entry cb
                 if (e_hi > EXC) {   // not all staged: refill this chunk
                     __syncthreads();
-                    fir_fill_exc<T, FIR_THREADS>(A, l, j0, st, cb, ce, cb);
+                    fir_fill_exc<T, NT>(A, 0, j0, st, cb, ce, cb);
                     __syncthreads();
                     x0 = 0;
                 }
                 for (int e = cb; e < ce; ++e) {
-                    const FirExcW<T> xc = st.excw[x0 + (e - cb)];
-#pragma unroll
-                    for (int q = 0; q < FIR_PIX; ++q) {
-                        const int dj = tid + q * FIR_THREADS;
-                        const int j = j0 + dj;
-                        if (j >= n_eff) continue;
-                        T wd = xc.phi + xc.dlt * (T)dj;
-                        int i = xc.i0 + dj;
-                        if (wd >= (T)1) { wd -= (T)1; i += 1; }
-                        else if (wd < (T)0) { wd += (T)1; i -= 1; }
-                        if (i < 0 || i > n_eff - 2) continue;
-                        const int x = i + wo;
-                        // the per-cell owner can differ by one from the segment's
-                        // classification when t lies within rounding of an integer: such
-                        // pixels read the row in global memory instead of the window
-                        const bool staged = (i >= d.w0) && (i + 1 < d.w1);
-                        auto lv = [&](int c) -> T {
-                            T s0, s1;
-                            if (staged) {
-                                s0 = W[c][x];
-                                s1 = W[c][x + 1];
-                            } else {
-                                const T *rowp = reinterpret_cast<const T *>(A.cubes.c[fir_cube_index(MODE, cls, c)]) +
-                                                (long long)(d.key >> 1) * n;
-                                s0 = rowp[i];
-                                s1 = rowp[i + 1];
-                            }
-                            return s0 + (s1 - s0) * wd;
-                        };
-                        if constexpr (MODE == MODE_QUIET) {
-                            acc[0][q].add(xc.L * lv(0));
-                        } else if (cls == CLS_SPOT) {
-                            acc[0][q].add(xc.L * lv(0));
-                            acc[1][q].add(xc.L * lv(1));
-                            acc[2][q].add(xc.L * lv(2));
-                            acc[3][q].add(xc.L * lv(3));
-                        } else {
-                            acc[0][q].add(xc.L * lv(0));
-                            acc[6][q].add(xc.L * lv(1));
-                            acc[4][q].add(xc.w2 * lv(2));
-                            acc[5][q].add(xc.w2 * lv(3));
-                        }
-                    }
+                    const auto xc = st.excw[x0 + (e - cb)];
+                    // the cell's sources over the tile
+                    const int ilo = xc.i0 - 1, ihi = xc.i0 + FIR_TILE;
+                    const bool inside =
+                        t_eff == FIR_TILE && ilo >= max(0, d.w0) && ihi <= min(n_eff, d.w1) - 2;
+                    if (!inside) cell_at(yes(), yes(), xc);
+                    else if (xc.dlt >= (T)0) cell_at(no(), yes(), xc);
+                    else cell_at(no(), no(), xc);
                 }
             }
             __syncthreads();   // unit's buffer free
         }
     };
 
-    {
-        // --- plan the tile here, batch by batch ------------------------------------------
-        const int nsg = A.nseg[2 * l] + ((MODE == MODE_PHASE) ? A.nseg[2 * l + 1] : 0);
-        const int nunit = fir_segments<MODE, FIR_THREADS>(A, l, j0, t_eff, segs, nsg, &st.nunit);
-        // slopes of a short list in shared memory: the searches then cost no global latency
-        const int n01 = cn[0] + ((MODE == MODE_PHASE) ? cn[1] : 0);
-        const double *sl = A.list_dlt + lbase;
-        if (n01 <= FirListCap<T>::N) {
-            for (int q = tid; q < n01; q += FIR_THREADS) sh.sdl[q] = sl[q];
-            sl = sh.sdl;
-            __syncthreads();
-        }
-        for (int ub = 0; ub < nunit;) {
-            fir_plan_batch<T, MODE, FIR_THREADS>(A, l, j0, t_eff, segs, nsg, nunit, sl, st, ub, sh.wsum);
-            run_units(ub);
-            if (u_fail >= 0) break;
-            ub += st.nb;
-        }
+    // plan the tile, batch by batch
+    const int nsg = A.nseg[0];
+    const int nunit = fir_segments<MODE_QUIET, NT>(A, 0, j0, t_eff, segs, nsg, &st.nunit);
+    // slopes of a short list in shared memory: the searches then cost no global latency
+    const double *sl = A.list_dlt;
+    if (stage_slopes) {
+        double *sdl = reinterpret_cast<double *>(fir_smem + fir_smem_fixed<T, NQ>() +
+                                                 ((sizeof(FirSeg) * (size_t)A.seg_cap + 15) & ~size_t(15)));
+        const int cnt = A.counts[0];
+        for (int q = tid; q < cnt; q += NT) sdl[q] = sl[q];
+        sl = sdl;
+        __syncthreads();
+    }
+    for (int ub = 0; ub < nunit;) {
+        fir_plan_batch<T, MODE_QUIET, NT>(A, 0, j0, t_eff, segs, nsg, nunit, sl, st, ub, sh.wsum);
+        run_units(ub);
+        if (u_fail >= 0) break;
+        ub += st.nb;
     }
     if (u_fail >= 0) {
         // a copy did not land in time: record it, give the copies still in flight (units
@@ -1643,104 +1916,12 @@ __global__ void __launch_bounds__(FIR_THREADS) k_fir(const FirTileArgs A) {
         }
         return;
     }
-
-    // --- directly evaluated cells (class 2: spots of non-integral temperature, solar faculae)
-    if constexpr (MODE == MODE_PHASE) {
-        const int c_start = cn[0] + cn[1], c_cnt = cn[2];
-        for (int b0 = 0; b0 < c_cnt; b0 += FIR_EXC) {
-            const int nb = min(FIR_EXC, c_cnt - b0);
-            if (tid < nb) {
-                const int cell = A.list_cell[lbase + c_start + b0 + tid];
-                FirExcD<T> x;
-                cell_pos<T>(j0, A.geo, A.geo32, cell, x.i0, x.phi, x.dlt, x.L, x.w2);
-                const CellGeo &gg = A.geo[cell];
-                x.row = gg.row;
-                x.zero_v = gg.zero_v;
-                const double2 ax = A.list_aux[lbase + c_start + b0 + tid];
-                x.temp = ax.x;
-                x.kind = bits_is_zero(ax.y) ? 0 : 1;
-                sh.excd[tid] = x;
-            }
-            __syncthreads();
-            for (int e = 0; e < nb; ++e) {
-                const FirExcD<T> xc = sh.excd[e];
-                const long long off = (long long)xc.row * n;
 #pragma unroll
-                for (int q = 0; q < FIR_PIX; ++q) {
-                    const int dj = tid + q * FIR_THREADS;
-                    const int j = j0 + dj;
-                    if (j >= n_eff) continue;
-                    long long i;
-                    T w;
-                    if (xc.zero_v) {
-                        i = j;
-                        w = (T)0;
-                    } else {
-                        T wd = xc.phi + xc.dlt * (T)dj;
-                        i = (long long)xc.i0 + dj;
-                        if (wd >= (T)1) { wd -= (T)1; i += 1; }
-                        else if (wd < (T)0) { wd += (T)1; i -= 1; }
-                        if (i < 0 || i > n_eff - 2) continue;
-                        w = wd;
-                    }
-                    auto val = [&](int ci) -> T {
-                        const T *rowp = reinterpret_cast<const T *>(A.cubes.c[ci]) + off;
-                        if (xc.zero_v) return rowp[i];
-                        return rowp[i] + (rowp[i + 1] - rowp[i]) * w;
-                    };
-                    const T L = xc.L;
-                    acc[0][q].add(L * val(0));                 // S (q_sed)
-                    if (xc.kind == 0) {                        // spot of non-integral temperature
-                        T Lq = (T)((double)L * fir_planck_ratio(A.lam[j], xc.temp, (double)(int)xc.temp));
-                        acc[1][q].add(Lq * val(1));            // Qs (q_norm)
-                        acc[2][q].add(Lq * val(2));            // As (spot_norm)
-                        acc[3][q].add(L * val(3));             // Bs (q_norm - spot_norm)
-                    } else {                                   // facula of the solar variant
-                        acc[6][q].add(L * val(5));             // Bf (q_norm - fac_norm)
-                        T w2 = (T)((double)L * fir_planck_ratio(A.lam[j], xc.temp, (double)A.t_norm_fac));
-                        acc[4][q].add(w2 * val(1));            // Qf (q_norm)
-                        acc[5][q].add(w2 * val(4));            // Af (fac_norm)
-                    }
-                }
-            }
-            __syncthreads();
-        }
-    }
-
-    // --- outputs ----------------------------------------------------------------------
-#pragma unroll
-    for (int q = 0; q < FIR_PIX; ++q) {
-        const int j = j0 + tid + q * FIR_THREADS;
+    for (int q = 0; q < PIX; ++q) {
+        const int j = j0 + tid + q * NT;
         if (j >= n) continue;
-        const long long o = (long long)l * A.out_stride + j;
-        if (j >= n_eff) {
-            out0[o] = (OutT)0;
-            if constexpr (MODE == MODE_PHASE) { out1[o] = (OutT)0; out2[o] = (OutT)0; }
-            continue;
-        }
-        if constexpr (MODE == MODE_QUIET) {
-            out0[o] = (OutT)acc[0][q].get();
-        } else if constexpr (sizeof(T) == 4) {
-            // flux = S - I_s Qs - I_f Qf, tot = S - I_s As - I_f Af in float pairs: the
-            // facula terms nearly cancel S, so no FP32 rounding before the subtraction
-            F2 S{acc[0][q].s, -acc[0][q].c}, Qs{acc[1][q].s, -acc[1][q].c}, As{acc[2][q].s, -acc[2][q].c};
-            F2 Qf{acc[4][q].s, -acc[4][q].c}, Af{acc[5][q].s, -acc[5][q].c};
-            float2 is2 = A.cubes.spot_sed2[j], fs2 = A.cubes.fac_sed2[j];
-            F2 is{is2.x, is2.y}, fs{fs2.x, fs2.y};
-            F2 fl = f2_add(f2_add(S, f2_neg(f2_mul(is, Qs))), f2_neg(f2_mul(fs, Qf)));
-            F2 tt = f2_add(f2_add(S, f2_neg(f2_mul(is, As))), f2_neg(f2_mul(fs, Af)));
-            F2 bc = f2_add(F2{acc[3][q].s, -acc[3][q].c}, F2{acc[6][q].s, -acc[6][q].c});
-            out0[o] = (OutT)(fl.hi + fl.lo);   // flux
-            out1[o] = (OutT)(bc.hi + bc.lo);   // bconv
-            out2[o] = (OutT)(tt.hi + tt.lo);   // tot
-        } else {
-            double S = acc[0][q].get(), Qs = acc[1][q].get(), As = acc[2][q].get(), Bs = acc[3][q].get();
-            double Qf = acc[4][q].get(), Af = acc[5][q].get(), Bf = acc[6][q].get();
-            double is = A.cubes.spot_sed[j], fs = A.cubes.fac_sed[j];
-            out0[o] = (OutT)(S - is * Qs - fs * Qf);   // flux
-            out1[o] = (OutT)(Bs + Bf);                 // bconv
-            out2[o] = (OutT)(S - is * As - fs * Af);   // tot
-        }
+#pragma unroll
+        for (int c = 0; c < NQ; ++c) outs[c][j] = (j >= n_eff) ? 0.0 : acc.get(c, q);
     }
 }
 
@@ -2421,7 +2602,7 @@ namespace {
 struct FirLayout {
     enum {
         GEO, GEO32, CUBE0, SED2A = CUBE0 + 6, SED2B, K1A, K1B, K2A, K2B, VA, VB, SORT_TMP, LCELL, LDLT, LAUX,
-        COUNTS, PRE, SEGS, NSEG, PLAN, NSLOT
+        COUNTS, RUNS, PRE, SEGS, NSEG, PLAN, NSLOT
     };
     size_t off[NSLOT] = {0};
     size_t total = 0;
@@ -2446,7 +2627,8 @@ FirLayout fir_layout(int form, int n, int n_mu, long long gm, int ncube, int n_l
     sz[FirLayout::K1A] = sz[FirLayout::K1B] = sizeof(unsigned long long) * (size_t)gm;
     sz[FirLayout::K2A] = sz[FirLayout::K2B] = sizeof(unsigned) * (size_t)gm;
     sz[FirLayout::VA] = sz[FirLayout::VB] = sizeof(int) * (size_t)gm;
-    sz[FirLayout::SORT_TMP] = soapgb::fir_sort_temp_bytes(gm);
+    sz[FirLayout::SORT_TMP] = (gm > ORDER_MAX) ? soapgb::fir_sort_temp_bytes(gm) : 0;
+    sz[FirLayout::RUNS] = (ncube == 1) ? sizeof(double) * 2 * FIR_L1_SUMS * FIR_L1_RUNS : 0;
     sz[FirLayout::LCELL] = sizeof(int) * (size_t)gm * n_lists;
     sz[FirLayout::LDLT] = sizeof(double) * (size_t)gm * n_lists;
     sz[FirLayout::LAUX] = (ncube == 6) ? sizeof(double2) * (size_t)gm * n_lists : 0;
@@ -2560,6 +2742,28 @@ static int fir_prepare(soapgb_ctx *ctx, const double *wave, int n_eff, double st
     return SOAPGB_OK;
 }
 
+// the cells by (mu bin, v == 0), then slope, then map order, in slot VA (VB: work)
+static int fir_order(soapgb_ctx *ctx, const FirLayout &L, char *ws, long long gm, const CellGeo *geo) {
+    auto *k1a = (unsigned long long *)(ws + L.off[FirLayout::K1A]);
+    auto *k1b = (unsigned long long *)(ws + L.off[FirLayout::K1B]);
+    auto *k2a = (unsigned *)(ws + L.off[FirLayout::K2A]);
+    auto *k2b = (unsigned *)(ws + L.off[FirLayout::K2B]);
+    int *va = (int *)(ws + L.off[FirLayout::VA]);
+    int *vb = (int *)(ws + L.off[FirLayout::VB]);
+    if (gm <= ORDER_MAX) return order_cells(ctx, gm, FirCellKey{geo}, k1a, k1b, (int *)k2a, va);
+    void *tmp = ws + L.off[FirLayout::SORT_TMP];
+    const size_t tmp_bytes = soapgb::fir_sort_temp_bytes(gm);
+    const int g = grid_for(ctx, gm, 256);
+    soapgb::TraceScope ts(ctx, "cell_order");
+    k_sort_keys1<<<g, 256, 0, ctx->stream>>>(gm, geo, k1a, va);
+    SOAP_LAUNCHED(ctx);
+    int rc = soapgb::fir_sort_u64(ctx, gm, k1a, k1b, va, vb, tmp, tmp_bytes);
+    if (rc) return rc;
+    k_sort_keys2<<<g, 256, 0, ctx->stream>>>(gm, geo, vb, k2a);
+    SOAP_LAUNCHED(ctx);
+    return soapgb::fir_sort_u32(ctx, gm, k2a, k2b, vb, va, 14, tmp, tmp_bytes);   // stable: dlt order kept per bin
+}
+
 // velocity-ordered cell lists, prefix sums and segments for n_lists lists
 static int fir_lists(soapgb_ctx *ctx, const FirLayout &L, char *ws, long long gm, int n_lists, const double *temp,
                      const double *bi, int solar, const FirPhaseArgs *boxes = nullptr) {
@@ -2588,30 +2792,11 @@ static int fir_lists(soapgb_ctx *ctx, const FirLayout &L, char *ws, long long gm
         SOAP_LAUNCHED(ctx);
         return SOAPGB_OK;
     }
-    auto *k1a = (unsigned long long *)(ws + L.off[FirLayout::K1A]);
-    auto *k1b = (unsigned long long *)(ws + L.off[FirLayout::K1B]);
-    auto *k2a = (unsigned *)(ws + L.off[FirLayout::K2A]);
-    auto *k2b = (unsigned *)(ws + L.off[FirLayout::K2B]);
     int *va = (int *)(ws + L.off[FirLayout::VA]);
     int *vb = (int *)(ws + L.off[FirLayout::VB]);
-    void *tmp = ws + L.off[FirLayout::SORT_TMP];
-    size_t tmp_bytes = soapgb::fir_sort_temp_bytes(gm);
-    int g = grid_for(ctx, gm, 256);
-    k_sort_keys1<<<g, 256, 0, ctx->stream>>>(gm, geo, k1a, va);
-    SOAP_LAUNCHED(ctx);
-    int rc;
-    {
-        soapgb::TraceScope ts(ctx, "cell_sort");
-        rc = soapgb::fir_sort_u64(ctx, gm, k1a, k1b, va, vb, tmp, tmp_bytes);
-    }
+    int rc = fir_order(ctx, L, ws, gm, geo);
     if (rc) return rc;
-    k_sort_keys2<<<g, 256, 0, ctx->stream>>>(gm, geo, vb, k2a);
-    SOAP_LAUNCHED(ctx);
-    {
-        soapgb::TraceScope ts(ctx, "cell_sort");
-        rc = soapgb::fir_sort_u32(ctx, gm, k2a, k2b, vb, va, 14, tmp, tmp_bytes);   // stable: dlt order kept per bin
-    }
-    if (rc) return rc;
+    const int g = grid_for(ctx, gm, 256);
     int *lcell = (int *)(ws + L.off[FirLayout::LCELL]);
     double *ldlt = (double *)(ws + L.off[FirLayout::LDLT]);
     double2 *laux = (double2 *)(ws + L.off[FirLayout::LAUX]);
@@ -2692,65 +2877,83 @@ static FirTileArgs make_tile_args(soapgb_ctx *ctx, const FirLayout &L, char *ws,
     return A;
 }
 
-template <typename T, int MODE, typename OutT>
+// the phase integration's tiles: plans of every (phase, tile) (stage 1), then the
+// persistent tile kernel over the phases [l0, l1) (stage 4)
+template <typename T>
 static int launch_tiles(soapgb_ctx *ctx, const FirLayout &L, char *ws, int n, int n_eff, const double *lam,
                         double los, const FirCubes &fc, long long gm, int solar,
                         int t_norm_fac, void *o0, void *o1, void *o2, long long out_stride, int n_lists,
-                        int stage = 7, int l0 = 0, int l1 = -1, const FirPhaseArgs *pa = nullptr) {
-    constexpr int NC = (MODE == MODE_QUIET) ? 1 : 4;
-    if (l1 < 0) l1 = n_lists;
+                        int stage, int l0, int l1, const FirPhaseArgs *pa) {
     FirTileArgs A = make_tile_args(ctx, L, ws, n, n_eff, lam, los, fc, gm, solar, t_norm_fac, o0, o1, o2, out_stride,
                                    n_lists);
     const int ntile = (n + FIR_TILE - 1) / FIR_TILE;
-    if constexpr (MODE == MODE_PHASE) {
-        // plans of every (phase, tile) (stage 1), then the persistent tile kernel over the
-        // phases [l0, l1) (stage 4)
-        A.plan = ws + L.off[FirLayout::PLAN];
-        // with run / zero lists: only the listed phases are planned and integrated, the
-        // others zero-filled; [r0, r1) and [z0, z1) are the parts of the lists in [l0, l1)
-        const bool lists = pa && pa->run_list;
-        int r0 = l0, r1 = l1, z0 = 0, z1 = 0;
-        if (lists) {
-            A.run_list = pa->run_list;
-            r0 = (int)(std::lower_bound(pa->run_host, pa->run_host + pa->n_run, l0) - pa->run_host);
-            r1 = (int)(std::lower_bound(pa->run_host, pa->run_host + pa->n_run, l1) - pa->run_host);
-            z0 = (int)(std::lower_bound(pa->zero_host, pa->zero_host + pa->n_zero, l0) - pa->zero_host);
-            z1 = (int)(std::lower_bound(pa->zero_host, pa->zero_host + pa->n_zero, l1) - pa->zero_host);
-        }
-        const int n_plan = lists ? pa->n_run : n_lists;
-        if ((stage & 1) && n_plan > 0) {
-            size_t smem_p = ((sizeof(FirPrePlan<T>) + 15) & ~size_t(15)) + sizeof(FirSeg) * 2 * (size_t)L.seg_cap;
-            SOAP_CUDA(ctx, cudaFuncSetAttribute(k_fir_plan<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_p));
-            SOAP_TRACED(ctx, "fir_plan",
-                        k_fir_plan<T><<<dim3(ntile, n_plan), FIR_PLAN_THREADS, smem_p, ctx->stream>>>(A));
-            SOAP_LAUNCHED(ctx);
-        }
-        if ((stage & 4) && z1 > z0 && pa->zero_fill) {
-            SOAP_TRACED(ctx, "fir_zero",
-                        k_fir_zero<T><<<dim3((n + 255) / 256, z1 - z0), 256, 0, ctx->stream>>>(
-                            n, pa->zero_list + z0, (T *)o0, (T *)o1, (T *)o2, out_stride));
-            SOAP_LAUNCHED(ctx);
-        }
-        if ((stage & 4) && r1 > r0) {
-            const int nrun = ntile * (r1 - r0);
-            size_t smem_t = fir_pp_smem_fixed<T>() + sizeof(FirSeg) * 2 * (size_t)L.seg_cap;
-            auto kern = ctx->fir_compensated ? k_fir_pp<T, true, false> : k_fir_pp<T, false, false>;
-            SOAP_CUDA(ctx, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_t));
-            int per_sm = 0;
-            SOAP_CUDA(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, FIR_THREADS, smem_t));
-            const int nblk = std::max(1, std::min(nrun, std::max(per_sm, 1) * std::max(ctx->num_sms, 1)));
-            SOAP_TRACED(ctx, "fir_tile_phase",
-                        kern<<<nblk, FIR_THREADS, smem_t, ctx->stream>>>(A, ntile, r0, r1 - r0, ntile * n_lists,
-                                                                         nullptr, nullptr, 0));
-            SOAP_LAUNCHED(ctx);
-        }
-        return SOAPGB_OK;
+    A.plan = ws + L.off[FirLayout::PLAN];
+    // with run / zero lists: only the listed phases are planned and integrated, the
+    // others zero-filled; [r0, r1) and [z0, z1) are the parts of the lists in [l0, l1)
+    const bool lists = pa->run_list != nullptr;
+    int r0 = l0, r1 = l1, z0 = 0, z1 = 0;
+    if (lists) {
+        A.run_list = pa->run_list;
+        r0 = (int)(std::lower_bound(pa->run_host, pa->run_host + pa->n_run, l0) - pa->run_host);
+        r1 = (int)(std::lower_bound(pa->run_host, pa->run_host + pa->n_run, l1) - pa->run_host);
+        z0 = (int)(std::lower_bound(pa->zero_host, pa->zero_host + pa->n_zero, l0) - pa->zero_host);
+        z1 = (int)(std::lower_bound(pa->zero_host, pa->zero_host + pa->n_zero, l1) - pa->zero_host);
     }
-    size_t smem = fir_smem_fixed<T, NC>() + sizeof(FirSeg) * (size_t)(MODE == MODE_PHASE ? 2 : 1) * L.seg_cap;
-    SOAP_CUDA(ctx, cudaFuncSetAttribute(k_fir<T, MODE, OutT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    const int n_plan = lists ? pa->n_run : n_lists;
+    if ((stage & 1) && n_plan > 0) {
+        size_t smem_p = ((sizeof(FirPrePlan<T>) + 15) & ~size_t(15)) + sizeof(FirSeg) * 2 * (size_t)L.seg_cap;
+        SOAP_CUDA(ctx, cudaFuncSetAttribute(k_fir_plan<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_p));
+        SOAP_TRACED(ctx, "fir_plan", k_fir_plan<T><<<dim3(ntile, n_plan), FIR_PLAN_THREADS, smem_p, ctx->stream>>>(A));
+        SOAP_LAUNCHED(ctx);
+    }
+    if ((stage & 4) && z1 > z0 && pa->zero_fill) {
+        SOAP_TRACED(ctx, "fir_zero",
+                    k_fir_zero<T><<<dim3((n + 255) / 256, z1 - z0), 256, 0, ctx->stream>>>(
+                        n, pa->zero_list + z0, (T *)o0, (T *)o1, (T *)o2, out_stride));
+        SOAP_LAUNCHED(ctx);
+    }
+    if ((stage & 4) && r1 > r0) {
+        const int nrun = ntile * (r1 - r0);
+        size_t smem_t = fir_pp_smem_fixed<T>() + sizeof(FirSeg) * 2 * (size_t)L.seg_cap;
+        auto kern = ctx->fir_compensated ? k_fir_pp<T, true, false> : k_fir_pp<T, false, false>;
+        SOAP_CUDA(ctx, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_t));
+        int per_sm = 0;
+        SOAP_CUDA(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, FIR_THREADS, smem_t));
+        const int nblk = std::max(1, std::min(nrun, std::max(per_sm, 1) * std::max(ctx->num_sms, 1)));
+        SOAP_TRACED(ctx, "fir_tile_phase",
+                    kern<<<nblk, FIR_THREADS, smem_t, ctx->stream>>>(A, ntile, r0, r1 - r0, ntile * n_lists, nullptr,
+                                                                     nullptr, 0));
+        SOAP_LAUNCHED(ctx);
+    }
+    return SOAPGB_OK;
+}
+
+// FP32 copy of one cube, or of two side by side (c1)
+static int quiet_types(soapgb_ctx *ctx, long long count, const double *c0, const double *c1, void *dst) {
+    auto al16 = [](const void *p) { return ((uintptr_t)p & 15) == 0; };
+    const int paired = al16(c0) && (!c1 || al16(c1));
+    const unsigned g = (unsigned)std::max<long long>(1, (count / 2 + 511) / 512);
+    SOAP_TRACED(ctx, "cube_types", k_quiet_types32<<<g, 256, 0, ctx->stream>>>(count, paired, c0, c1, (float *)dst));
+    SOAP_LAUNCHED(ctx);
+    return SOAPGB_OK;
+}
+
+size_t fir_quiet_pair_bytes(int n, int n_mu) { return align256(sizeof(float2) * (size_t)n * n_mu); }
+
+int fir_quiet_pair(soapgb_ctx *ctx, int n, const soapgb_cubes &c, void *dst) {
+    return quiet_types(ctx, (long long)n * c.n_mu, c.q_sed, c.q_norm, dst);
+}
+
+template <typename T, int NQ>
+static int launch_quiet(soapgb_ctx *ctx, const FirTileArgs &A) {
+    const int stage_slopes = A.gm <= FirListCap<T>::N;
+    const size_t smem = fir_smem_fixed<T, NQ>() + ((sizeof(FirSeg) * (size_t)A.seg_cap + 15) & ~size_t(15)) +
+                        (stage_slopes ? sizeof(double) * (size_t)A.gm : 0);
+    SOAP_CUDA(ctx, cudaFuncSetAttribute(k_fir_quiet<T, NQ>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     // tiles cover [0, n): tiles past n_eff only write the zero tail
-    dim3 g((n + FIR_TILE - 1) / FIR_TILE, n_lists);
-    SOAP_TRACED(ctx, MODE == MODE_QUIET ? "fir_tile_quiet" : "fir_tile_phase", k_fir<T, MODE, OutT><<<g, FIR_THREADS, smem, ctx->stream>>>(A));
+    SOAP_TRACED(ctx, "fir_tile_quiet",
+                k_fir_quiet<T, NQ><<<(A.n + FIR_TILE - 1) / FIR_TILE, FIR_QUIET_THREADS<T, NQ>, smem, ctx->stream>>>(
+                    A, stage_slopes));
     SOAP_LAUNCHED(ctx);
     return SOAPGB_OK;
 }
@@ -2760,39 +2963,63 @@ int fir_quiet(soapgb_ctx *ctx, int form, const FirQuietArgs &a, char *scratch, c
     if (a.n_mu > FIR_MAX_MU)
         return set_error(ctx, SOAPGB_ERR_ARG, "collapsed forms support at most %d mu bins (got %d)", FIR_MAX_MU, a.n_mu);
     const long long gm = a.gm;
-    FirLayout L = fir_layout(form, a.n, a.n_mu, gm, 1, 1);
+    if (a.pair && form != SOAPGB_FAST32) return set_error(ctx, SOAPGB_ERR_ARG, "fir_quiet: paired cubes are FP32");
+    FirLayout L = fir_layout(form, a.n, a.n_mu, gm, 1, 1, a.pair != nullptr);
     char *ws = scratch;
     CellGeo *geo = (CellGeo *)(ws + L.off[FirLayout::GEO]);
     CellGeo32 *geo32 = (CellGeo32 *)(ws + L.off[FirLayout::GEO32]);
     double lambda0 = a.lambda0;
-    int rc = fir_prepare(ctx, a.wave, a.n_eff, a.step, gm, a.delta, a.limb, nullptr, a.region, a.n_mu, geo, geo32,
+    int rc = SOAPGB_OK;
+    if (a.geo) {
+        geo = (CellGeo *)a.geo->geo;
+        geo32 = (CellGeo32 *)a.geo->geo32;
+    } else {
+        rc = fir_prepare(ctx, a.wave, a.n_eff, a.step, gm, a.delta, a.limb, nullptr, a.region, a.n_mu, geo, geo32,
                          &lambda0);
-    if (rc) return rc;
-    rc = fir_lists(ctx, L, ws, gm, 1, nullptr, nullptr, 0);
-    if (rc) return rc;
-    size_t cube_elems = (size_t)a.n * a.n_mu;
-    void *cube = ws + L.off[FirLayout::CUBE0];
-    FirCubes fc{};
-    fc.c[0] = cube;
-    const double los = lambda0 / a.step;
-    // one cube, or two over the same lists (the typed copy is rewritten in stream order)
-    for (int q = 0; q < (a.cube2 ? 2 : 1); ++q) {
-        const double *src = q ? a.cube2 : a.cube;
-        double *out = q ? a.out2 : a.out;
-        if (form == SOAPGB_FAST32) {
-            SOAP_TRACED(ctx, "cube_types", k_to_type<float><<<grid_for(ctx, cube_elems, 256), 256, 0, ctx->stream>>>(cube_elems, src, nullptr, (float *)cube));
-            SOAP_LAUNCHED(ctx);
-            rc = launch_tiles<float, MODE_QUIET, double>(ctx, L, ws, a.n, a.n_eff, a.wave, los, fc, gm, 0, 0, out,
-                                                         nullptr, nullptr, 0, 1);
-        } else {
-            SOAP_TRACED(ctx, "cube_types", k_to_type<double><<<grid_for(ctx, cube_elems, 256), 256, 0, ctx->stream>>>(cube_elems, src, nullptr, (double *)cube));
-            SOAP_LAUNCHED(ctx);
-            rc = launch_tiles<double, MODE_QUIET, double>(ctx, L, ws, a.n, a.n_eff, a.wave, los, fc, gm, 0, 0, out,
-                                                          nullptr, nullptr, 0, 1);
-        }
         if (rc) return rc;
     }
-    return SOAPGB_OK;
+    rc = fir_order(ctx, L, ws, gm, geo);
+    if (rc) return rc;
+    FirList1 l1;
+    l1.order = (const int *)(ws + L.off[FirLayout::VA]);
+    l1.geo = geo;
+    l1.list_cell = (int *)(ws + L.off[FirLayout::LCELL]);
+    l1.list_dlt = (double *)(ws + L.off[FirLayout::LDLT]);
+    l1.L = (double *)(ws + L.off[FirLayout::K1A]);       // the order's work arrays
+    l1.offir = (double *)(ws + L.off[FirLayout::K1B]);
+    l1.key = (int *)(ws + L.off[FirLayout::K2A]);
+    l1.counts = (int *)(ws + L.off[FirLayout::COUNTS]);
+    l1.run = (double *)(ws + L.off[FirLayout::RUNS]);
+    l1.pre = (double *)(ws + L.off[FirLayout::PRE]);
+    l1.pre_comp = L.pre_comp;
+    l1.segs = (int2 *)(ws + L.off[FirLayout::SEGS]);
+    l1.nseg = (int *)(ws + L.off[FirLayout::NSEG]);
+    SOAP_TRACED(ctx, "fir_list1", k_fir_list1<<<(unsigned)((gm + 255) / 256), 256, 0, ctx->stream>>>((int)gm, l1));
+    SOAP_LAUNCHED(ctx);
+    SOAP_TRACED(ctx, "fir_prefix1",
+                k_fir_prefix1<false><<<dim3(FIR_L1_RUNS / 32, FIR_L1_SUMS + 1), 32, 0, ctx->stream>>>(l1, 2 * a.n_mu));
+    SOAP_LAUNCHED(ctx);
+    SOAP_TRACED(ctx, "fir_prefix1",
+                k_fir_prefix1<true><<<dim3(FIR_L1_RUNS / 32, FIR_L1_SUMS), 32, 0, ctx->stream>>>(l1, 0));
+    SOAP_LAUNCHED(ctx);
+    const size_t count = (size_t)a.n * a.n_mu;
+    FirCubes fc{};
+    fc.c[0] = a.pair ? a.pair : ws + L.off[FirLayout::CUBE0];
+    if (!a.pair) {
+        void *c = ws + L.off[FirLayout::CUBE0];
+        if (form == SOAPGB_FAST32) {
+            rc = quiet_types(ctx, (long long)count, a.cube, nullptr, c);
+            if (rc) return rc;
+        } else {   // the staging copies whole 16-byte pieces: an aligned, padded copy
+            SOAP_CUDA(ctx, cudaMemcpyAsync(c, a.cube, sizeof(double) * count, cudaMemcpyDeviceToDevice, ctx->stream));
+        }
+    }
+    FirTileArgs A = make_tile_args(ctx, L, ws, a.n, a.n_eff, a.wave, lambda0 / a.step, fc, gm, 0, 0, a.out, a.out2,
+                                   nullptr, 0, 1);
+    A.geo = geo;
+    A.geo32 = geo32;
+    if (form != SOAPGB_FAST32) return launch_quiet<double, 1>(ctx, A);
+    return a.pair ? launch_quiet<float, 2>(ctx, A) : launch_quiet<float, 1>(ctx, A);
 }
 
 // the typed cubes a phase integration reads: its workspace slots, or the shared copies
@@ -2847,12 +3074,17 @@ int fir_phase(soapgb_ctx *ctx, int form, const FirPhaseArgs &a, char *scratch, c
     const int st = (a.stage & FIR_STAGE_GEOMETRY ? 1 : 0) | (a.stage & FIR_STAGE_RUN ? 4 : 0);
     const int l1 = (a.l1 < 0) ? a.n_phase : a.l1;
     if (form == SOAPGB_FAST32)
-        return launch_tiles<float, MODE_PHASE, float>(ctx, L, ws, a.n, a.n_eff, a.wave, los, fc, a.gm,
+        return launch_tiles<float>(ctx, L, ws, a.n, a.n_eff, a.wave, los, fc, a.gm,
                                                       a.act->solar, t_norm_fac, a.flux, a.bconv, a.tot, a.out_stride,
                                                       a.n_phase, st, a.l0, l1, &a);
-    return launch_tiles<double, MODE_PHASE, double>(ctx, L, ws, a.n, a.n_eff, a.wave, los, fc, a.gm,
+    return launch_tiles<double>(ctx, L, ws, a.n, a.n_eff, a.wave, los, fc, a.gm,
                                                     a.act->solar, t_norm_fac, a.flux, a.bconv, a.tot, a.out_stride,
                                                     a.n_phase, st, a.l0, l1, &a);
+}
+
+FirGeoRef fir_phase_geo(int form, const FirPhaseArgs &a, char *scratch) {
+    const FirLayout L = fir_layout(form, a.n, a.cubes->n_mu, a.gm, 6, a.n_phase, a.typed != nullptr);
+    return FirGeoRef{scratch + L.off[FirLayout::GEO], scratch + L.off[FirLayout::GEO32]};
 }
 
 size_t fir_tile_args_bytes() { return sizeof(FirTileArgs); }

@@ -10,9 +10,9 @@ struct FirPlanSizes {
 
 // workspace of the FAST forms: per-cell geometry for the G*G grid, the velocity order
 // of the cells, per-list cell lists / prefix sums / segments and typed cube copies
-// (one cube for the quiet disk, six for the phase integration)
-// typed_external: the phase integration reads typed cubes shared with other stars
-// (fir_typed_cubes), so the workspace holds none
+// (the quiet disk's cube, or the phase integration's interleaved rows)
+// typed_external: the typed cubes are shared with other stars (fir_typed_cubes,
+// fir_quiet_pair), so the workspace holds none
 FirPlanSizes fir_plan_sizes(int form, int n, int n_mu, long long gm, bool phase, int n_lists,
                             bool typed_external = false);
 
@@ -29,10 +29,19 @@ size_t fir_typed_bytes(int form, int n, int n_mu);
 void fir_typed_layout(int form, int n, int n_mu, char *dst, const soapgb_cubes &c, FirTyped *out);
 int fir_typed_cubes(soapgb_ctx *ctx, int form, int n, const soapgb_cubes &c, char *dst, FirTyped *out);
 
+// q_sed and q_norm side by side in FP32 (float2 per pixel), for the quiet disks of several stars
+size_t fir_quiet_pair_bytes(int n, int n_mu);
+int fir_quiet_pair(soapgb_ctx *ctx, int n, const soapgb_cubes &c, void *dst);
+
+// the per-cell constants in a workspace
+struct FirGeoRef {
+    const void *geo, *geo32;
+};
+
 struct FirQuietArgs {
     int n, n_eff;
     const double *wave;
-    const double *cube;     // n_mu x n (FP64, device)
+    const double *cube = nullptr;   // n_mu x n (FP64, device)
     int n_mu;
     long long gm;           // G*G
     const double *delta, *limb;
@@ -40,9 +49,11 @@ struct FirQuietArgs {
     double step;
     double *out;            // n (tail set to 0)
     double lambda0 = 0.0;   // wave[0] when known on the host (0: read from the device)
-    // optional second cube of the same disk (its cell order, lists and sums shared)
-    const double *cube2 = nullptr;
+    // FP32 form, instead of cube: two cubes side by side (fir_quiet_pair), the second's
+    // sums to out2
+    const void *pair = nullptr;
     double *out2 = nullptr;
+    const FirGeoRef *geo = nullptr;              // the star's cells as its phase geometry wrote them
 };
 
 int fir_quiet(soapgb_ctx *ctx, int form, const FirQuietArgs &a, char *scratch, const FirPlanSizes &plan);
@@ -86,6 +97,9 @@ struct FirPhaseArgs {
 enum { FIR_STAGE_GEOMETRY = 1, FIR_STAGE_CUBES = 2, FIR_STAGE_RUN = 4 };
 
 int fir_phase(soapgb_ctx *ctx, int form, const FirPhaseArgs &a, char *scratch, const FirPlanSizes &plan);
+
+// the cells' constants that a phase geometry stage writes into its workspace
+FirGeoRef fir_phase_geo(int form, const FirPhaseArgs &a, char *scratch);
 
 // Several stars' phase integrations in one persistent launch (FP32 form).  Each star has
 // run its geometry stage (fir_phase with FIR_STAGE_GEOMETRY and run lists) in its own

@@ -3,8 +3,9 @@
 // The collapsed form groups cells by their integer shift at every tile; with the
 // visible cells sorted by (mu bin, v == 0, Doppler slope) the cells sharing a shift
 // form contiguous ranges at every tile, so a tile finds its groups by binary search
-// instead of visiting every cell.  The order comes from two stable radix sorts (CUB,
-// the CUDA toolkit's template library): by slope, then by (mu bin, v == 0).
+// instead of visiting every cell.  For grids above ORDER_MAX cells (order.cuh) the order
+// comes from two stable radix sorts (CUB, the CUDA toolkit's template library): by slope,
+// then by (mu bin, v == 0).
 #include <algorithm>
 
 #include <cub/device/device_radix_sort.cuh>
