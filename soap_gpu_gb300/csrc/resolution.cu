@@ -1114,7 +1114,11 @@ __global__ void __launch_bounds__(FC_THREADS, 3) k_conv32t(int n, int n_eff, con
 // pass 2 of the fused form: exact FP64 extrema of the candidate pixels of the pixel
 // blocks (1024 pixels each) that can hold one.  grid (ceil(nbx / 8), spectra): warp w
 // of a block takes pixel block 8 blockIdx.x + w when its FP32 bounds make it a
-// candidate (most are not, and their warps leave at once).
+// candidate (most are not, and their warps leave at once).  A candidate's time is memory
+// latency -- the FP32 values, then the FP64 base of the pixels that pass, all along a
+// continuum -- so the loads of four pixels of a lane are issued together in both steps:
+// 48 us for 168 spectra of 310,000 pixels against 97 one by one, 14 against 28 for a
+// short spectrum; eight at a time, with a branch per FP64 load, 123 (registers).
 __global__ void __launch_bounds__(256) k_refine64x(int n, int n_eff, int nbx, const float *__restrict__ spec,
                                                    long long spec_stride, const double *__restrict__ ba,
                                                    const double *__restrict__ bb, const double *__restrict__ cba,
@@ -1143,21 +1147,44 @@ __global__ void __launch_bounds__(256) k_refine64x(int n, int n_eff, int nbx, co
     const float *cv = conv + (long long)s * conv_stride;
     unsigned long long mn = ~0ULL, mx = 0ULL;
     const int i_end = min(n, (x + 1) * FC_TILE);
-    for (int i = x * FC_TILE + lane; i < i_end; i += 32) {
-        const float xv = sp[i];
-        if (needA && bs[i] - xv <= mnA + tolA) {
-            const double a = b64[i] - (double)xv;
-            mn = min(mn, soap_ord_enc(a));
-        }
-        if (needC && i < n_eff) {
-            const float cd = cv[i];
-            const float c = cbs[i] + cd;
-            if (c != 0.f && c >= mxC - tolC) {
-                const double cx = c64[i] + (double)cd;
-                if (cx != 0.0) mx = max(mx, soap_ord_enc(cx));
+    constexpr int U = 4;   // pixels per lane whose loads are in flight together
+    // U pixels: their FP32 values p[i], q[i]; those that pass the test, with their FP64 value
+    auto scan = [&](const float *__restrict__ p, const float *__restrict__ q, const double *__restrict__ r, int end,
+                    auto &&test, auto &&put) {
+        for (int i0 = x * FC_TILE + lane; i0 < end; i0 += 32 * U) {
+            float pv[U], qv[U];
+#pragma unroll
+            for (int u = 0; u < U; ++u) {
+                const int i = min(i0 + 32 * u, end - 1);
+                pv[u] = p[i];
+                qv[u] = q[i];
             }
+            unsigned hit = 0;
+#pragma unroll
+            for (int u = 0; u < U; ++u)
+                if (i0 + 32 * u < end && test(pv[u], qv[u])) hit |= 1u << u;
+            if (hit == 0) continue;
+            double rv[U];
+#pragma unroll
+            for (int u = 0; u < U; ++u) rv[u] = ((hit >> u) & 1u) ? r[i0 + 32 * u] : 0.0;
+#pragma unroll
+            for (int u = 0; u < U; ++u)
+                if ((hit >> u) & 1u) put(rv[u], pv[u]);
         }
-    }
+    };
+    if (needA)
+        scan(sp, bs, b64, i_end, [&](float xv, float bv) { return bv - xv <= mnA + tolA; },
+             [&](double b, float xv) { mn = min(mn, soap_ord_enc(b - (double)xv)); });
+    if (needC)
+        scan(cv, cbs, c64, min(i_end, n_eff),
+             [&](float cd, float cb) {
+                 const float c = cb + cd;
+                 return c != 0.f && c >= mxC - tolC;
+             },
+             [&](double cb, float cd) {
+                 const double cx = cb + (double)cd;
+                 if (cx != 0.0) mx = max(mx, soap_ord_enc(cx));
+             });
     for (int o = 16; o > 0; o >>= 1) {
         mn = min(mn, __shfl_xor_sync(0xffffffffu, mn, o));
         mx = max(mx, __shfl_xor_sync(0xffffffffu, mx, o));
