@@ -114,10 +114,17 @@ __global__ void k_cell_geo(long long gm, const double *__restrict__ delta, const
     geo32[k] = h;
 }
 
-// wavelength grid must be uniform for the collapsed form
-__global__ void k_check_uniform(int n_eff, const double *__restrict__ lam, double step, int *status) {
+// wavelength grid must be uniform for the collapsed form; and the tiles' reciprocal
+// positions (two divisions per plan were half of k_fir_plan's FP64 instructions; with the
+// segments' floors on the integer pipes, 29,400 plans take 115 us against 131)
+__global__ void k_check_uniform(int n_eff, const double *__restrict__ lam, double step, double los, double2 *inv,
+                                int *status) {
     int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n_eff) return;
+    if ((long long)i * FIR_TILE < n_eff) {
+        const int j0 = i * FIR_TILE, t_eff = min(FIR_TILE, n_eff - j0);
+        inv[i] = make_double2(1.0 / ((double)j0 + los), 1.0 / ((double)(j0 + t_eff - 1) + los));
+    }
     double expect = lam[0] + (double)i * step;
     if (fabs(lam[i] - expect) > 1e-6 * step) atomicExch(status, FIR_ST_UNIFORM);
 }
@@ -265,6 +272,23 @@ __global__ void k_sort_keys2(long long gm, const CellGeo *__restrict__ geo, cons
     if (k >= gm) return;
     const CellGeo &g = geo[order[k]];
     keys[k] = (g.L > -998.0) ? (unsigned)(g.row * 2 + g.zero_v) : 0x3fffu;
+}
+
+__device__ __forceinline__ bool bits_negative(double v) { return __double2hiint(v) < 0; }
+__device__ __forceinline__ int soap_exp(double v) { return (int)(((unsigned)__double2hiint(v) >> 20) & 0x7ffu); }
+// (int)floor(v), on the integer pipes for |v| < 2^31
+__device__ __forceinline__ int soap_floor_i(double v) {
+    const int e = soap_exp(v) - 1023;
+    if (e >= 31) return (int)floor(v);
+    const unsigned long long u = (unsigned long long)__double_as_longlong(v);
+    const unsigned long long sig = (u & 0xfffffffffffffULL) | 0x10000000000000ULL;
+    unsigned ip = 0;
+    bool frac = (u << 1) != 0;   // |v| < 1: any value but zero
+    if (e >= 0) {
+        ip = (unsigned)(sig >> (52 - e));
+        frac = (sig << (12 + e)) != 0;
+    }
+    return bits_negative(v) ? (int)(0u - ip - (frac ? 1u : 0u)) : (int)ip;
 }
 
 // exact tests on FP64 values with integer instructions (no FP64 pipe)
@@ -557,10 +581,12 @@ __global__ void __launch_bounds__(FIR_BLIST_THREADS)
 
 // Phase lists without maps and without a cell order: one block per phase collects the
 // active cells of its region boxes (as k_fir_blists) and sorts them in shared memory by
-// (class, mu bin key, order-preserving image of the slope, cell index) -- a bitonic
-// network over a power-of-two capacity at least the phase's box cells.  That is the
-// order the two radix sorts of the cell order give (by slope, then stably by mu bin),
-// so the lists are the same as k_fir_blists's, without the G*G sort.
+// (class, mu bin key, order-preserving image of the slope, cell index), in a power-of-two
+// capacity at least the phase's box cells.  The longest phases bound the launch; a bitonic
+// network is 78 barriers for 4096 cells, merging by binary search 12 (55 us against 64 for
+// 100 phases of 300 x 300 cells).  That is the order the radix sorts of the cell order give
+// (by slope, then stably by mu bin), so the lists are the same as k_fir_blists's, without
+// the G*G sort.
 constexpr int FIR_SLIST_THREADS = 1024;
 constexpr int FIR_SLIST_CAP_MAX = 8192;
 
@@ -623,27 +649,47 @@ __global__ void __launch_bounds__(FIR_SLIST_THREADS)
         if (tid < 4) counts[4 * l + tid] = 0;
         return;
     }
-    int np = 1, lnp = 0;
-    while (np < n) np <<= 1, ++lnp;
+    int np = 64;
+    while (np < n) np <<= 1;
     for (int i = n + tid; i < np; i += FIR_SLIST_THREADS) sk[i] = ~0ULL;   // padding sorts last
     __syncthreads();
-    // bitonic network over the np / 2 compare-exchange pairs of each stage: pair m of
-    // stage (k, j) joins i (m with a zero bit inserted at bit log2 j) and i + j
-    const int half = np >> 1;
-    for (int lk = 1; lk <= lnp; ++lk) {
-        for (int lj = lk - 1; lj >= 0; --lj) {
-            const int j = 1 << lj;
-            for (int m = tid; m < half; m += FIR_SLIST_THREADS) {
-                const int i = ((m >> lj) << (lj + 1)) | (m & (j - 1));
-                const int p = i + j;
-                const unsigned long long a = sk[i], b = sk[p];
-                if ((a > b) == (((i >> lk) & 1) == 0)) {
-                    sk[i] = b;
-                    sk[p] = a;
-                }
+    // runs of 64 sorted by a warp each, then merged two by two: a key's place is its place
+    // in its run plus the count of the sibling run's keys below it (the paddings are equal:
+    // the first run's count the second's not at all, the second's the first's all)
+    const int lane = tid & 31, warp = tid >> 5;
+    for (int r = 64 * warp; r < np; r += 2 * FIR_SLIST_THREADS) {
+        unsigned long long k[2] = {sk[r + lane], sk[r + 32 + lane]};
+        order_sort64(k, lane);
+        sk[r + lane] = k[0];
+        sk[r + 32 + lane] = k[1];
+    }
+    __syncthreads();
+    constexpr int PER = FIR_SLIST_CAP_MAX / FIR_SLIST_THREADS;
+    for (int run = 64; run < np; run <<= 1) {
+        unsigned long long k[PER];
+        int to[PER];
+#pragma unroll
+        for (int q = 0; q < PER; ++q) {
+            const int p = tid + q * FIR_SLIST_THREADS;
+            if (p >= np) break;
+            const int s0 = (p & ~(run - 1)) ^ run;
+            const bool second = (p & run) != 0;
+            k[q] = sk[p];
+            int a = s0;
+            for (int w = run >> 1; w > 0; w >>= 1) {
+                const unsigned long long v = sk[a + w - 1];
+                if (v < k[q] || (second && v == k[q])) a += w;
             }
-            __syncthreads();
+            if (sk[a] < k[q] || (second && sk[a] == k[q])) a += 1;
+            to[q] = (p & ~run) + (a - s0);
         }
+        __syncthreads();
+#pragma unroll
+        for (int q = 0; q < PER; ++q) {
+            if (tid + q * FIR_SLIST_THREADS >= np) break;
+            sk[to[q]] = k[q];
+        }
+        __syncthreads();
     }
     // runs of equal (class, bin, top slope bits): order by k2 (the slope's low bits, then
     // the cell); a run is sorted by the thread at its start (runs are short: mostly the
@@ -687,7 +733,7 @@ __global__ void __launch_bounds__(FIR_SLIST_THREADS)
 }
 
 int fir_sorted_box_capacity(long long max_box_cells) {
-    int cap = 32;
+    int cap = 64;
     while (cap < max_box_cells) cap <<= 1;
     return cap <= FIR_SLIST_CAP_MAX ? cap : 0;
 }
@@ -697,10 +743,11 @@ static size_t fir_blists_smem(long long gm) { return sizeof(unsigned) * 3 * (siz
 long long fir_box_lists_max_gm() { return (long long)(FIR_BLIST_SMEM_MAX / (3 * sizeof(unsigned))) * 32; }
 
 // --- prefix sums and segments -------------------------------------------------------
+// exclusive sums over the block's threads; tot, toti: the block's totals, in the last warp
 template <int NV>
 __device__ __forceinline__ void block_scan_excl(double (&v)[NV], int &vi, double (&tot)[NV], int &toti,
-                                                double (*ws)[NV + 1]) {
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nw = blockDim.x >> 5;
+                                                double (*ws)[NV], int *wi) {
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     double inc[NV];
     int inci = vi;
 #pragma unroll
@@ -717,100 +764,110 @@ __device__ __forceinline__ void block_scan_excl(double (&v)[NV], int &vi, double
     if (lane == 31) {
 #pragma unroll
         for (int q = 0; q < NV; ++q) ws[warp][q] = inc[q];
-        ws[warp][NV] = (double)inci;
+        wi[warp] = inci;
     }
     __syncthreads();
     double off[NV];
     int offi = 0;
 #pragma unroll
-    for (int q = 0; q < NV; ++q) off[q] = 0.0, tot[q] = 0.0;
-    toti = 0;
-    for (int w = 0; w < nw; ++w) {
+    for (int q = 0; q < NV; ++q) off[q] = 0.0;
+    for (int w = 0; w < warp; ++w) {
 #pragma unroll
-        for (int q = 0; q < NV; ++q) {
-            if (w < warp) off[q] += ws[w][q];
-            tot[q] += ws[w][q];
-        }
-        int wi = (int)ws[w][NV];
-        if (w < warp) offi += wi;
-        toti += wi;
+        for (int q = 0; q < NV; ++q) off[q] += ws[w][q];
+        offi += wi[w];
     }
-    __syncthreads();
 #pragma unroll
     for (int q = 0; q < NV; ++q) v[q] = off[q] + inc[q] - v[q];
     vi = offi + inci - vi;
+#pragma unroll
+    for (int q = 0; q < NV; ++q) tot[q] = off[q] + ws[warp][q];
+    toti = offi + wi[warp];
 }
 
 // Block (l, c) for classes 0 and 1: exclusive FP64 prefix sums over the class list of
-// L, L dlt, L offir and (1 + LB) L, (1 + LB) L dlt, (1 + LB) L offir (the prefix of
-// the entry at list position q is stored at index q + c, the class total after its
+// L, L dlt, L offir and, for class 1, (1 + LB) L, (1 + LB) L dlt, (1 + LB) L offir (the
+// prefix of the entry at list position q is stored at index q + c, the class total after its
 // last entry), and the list of (mu bin, v == 0) segments:
 // segs[(l*2 + c)*cap + s] = (first position, row * 2 + zero_v), nseg[l*2 + c].
-__global__ void __launch_bounds__(256) k_fir_prefix(long long gm, const int *__restrict__ counts,
-                                                    const int *__restrict__ list_cell,
-                                                    const CellGeo *__restrict__ geo, double *pre, long long pre_stride,
-                                                    long long pre_comp, int2 *segs, int *nseg, int seg_cap,
-                                                    int *status) {
-    const int l = blockIdx.x, c = blockIdx.y, tid = threadIdx.x;
-    const int *cn = counts + 4 * l;
-    const int cs = (c == 0) ? 0 : cn[0];
-    const int cnt = cn[c];
+// The FP64 pipe of an SM bounds a block, so class 0 goes without the sums that only class 1
+// is read for and a warp adds the totals of the warps before it only: 12 us against 19 for
+// 15 phases of 100 x 100 cells, 37 against 50 for 100 phases of 300 x 300.
+template <int NV>
+__device__ __forceinline__ void fir_prefix_class(long long gm, int l, int c, int cs, int cnt,
+                                                 const int *__restrict__ list_cell, const CellGeo *__restrict__ geo,
+                                                 double *pre, long long pre_stride, long long pre_comp, int2 *segs,
+                                                 int *nseg, int seg_cap, int *status, double (*ws)[NV], int *wi) {
+    const int tid = threadIdx.x;
     const long long lbase = (long long)l * gm;
     const long long pbase = (long long)l * pre_stride + c;
-    __shared__ double ws[256 / 32][7];
     const int per = (cnt + blockDim.x - 1) / blockDim.x;
     const int a = cs + min(cnt, tid * per), b = cs + min(cnt, (tid + 1) * per);
     auto key_at = [&](int q) -> int {
         const CellGeo &g = geo[list_cell[lbase + q]];
         return g.row * 2 + g.zero_v;
     };
-    double s[6] = {0, 0, 0, 0, 0, 0};
-    int ns = 0;
-    int prev = (a > cs && a < b) ? key_at(a - 1) : -1;
-    for (int q = a; q < b; ++q) {
-        const CellGeo &g = geo[list_cell[lbase + q]];
+    double s[NV];
+#pragma unroll
+    for (int q = 0; q < NV; ++q) s[q] = 0.0;
+    auto add = [&](const CellGeo &g) {
         s[0] += g.L;
         s[1] += g.L * g.dlt;
         s[2] += g.L * g.offir;
-        s[3] += g.w2;
-        s[4] += g.w2 * g.dlt;
-        s[5] += g.w2 * g.offir;
-        int k = g.row * 2 + g.zero_v;
+        if constexpr (NV == 6) {
+            s[3] += g.w2;
+            s[4] += g.w2 * g.dlt;
+            s[5] += g.w2 * g.offir;
+        }
+    };
+    int ns = 0;
+    const int first = (a > cs && a < b) ? key_at(a - 1) : -1;
+    int prev = first;
+    for (int q = a; q < b; ++q) {
+        const CellGeo &g = geo[list_cell[lbase + q]];
+        add(g);
+        const int k = g.row * 2 + g.zero_v;
         if (q == cs || k != prev) ns++;
         prev = k;
     }
-    double tot[6];
+    double tot[NV];
     int tns;
-    block_scan_excl<6>(s, ns, tot, tns, ws);
-    prev = (a > cs && a < b) ? key_at(a - 1) : -1;
+    block_scan_excl<NV>(s, ns, tot, tns, ws, wi);
+    prev = first;
     for (int q = a; q < b; ++q) {
         const CellGeo &g = geo[list_cell[lbase + q]];
-        long long pi = pbase + q;
-        pre[pi] = s[0];
-        pre[pre_comp + pi] = s[1];
-        pre[2 * pre_comp + pi] = s[2];
-        pre[3 * pre_comp + pi] = s[3];
-        pre[4 * pre_comp + pi] = s[4];
-        pre[5 * pre_comp + pi] = s[5];
-        s[0] += g.L;
-        s[1] += g.L * g.dlt;
-        s[2] += g.L * g.offir;
-        s[3] += g.w2;
-        s[4] += g.w2 * g.dlt;
-        s[5] += g.w2 * g.offir;
-        int k = g.row * 2 + g.zero_v;
+#pragma unroll
+        for (int v = 0; v < NV; ++v) pre[v * pre_comp + pbase + q] = s[v];
+        add(g);
+        const int k = g.row * 2 + g.zero_v;
         if (q == cs || k != prev) {
             if (ns < seg_cap) segs[(long long)(l * 2 + c) * seg_cap + ns] = make_int2(q, k);
             ns++;
         }
         prev = k;
     }
-    if (tid == 0) {
-        long long pi = pbase + cs + cnt;
-        for (int q = 0; q < 6; ++q) pre[q * pre_comp + pi] = tot[q];
+    if (tid == (int)blockDim.x - 1) {
+#pragma unroll
+        for (int v = 0; v < NV; ++v) pre[v * pre_comp + pbase + cs + cnt] = tot[v];
         if (tns > seg_cap) atomicExch(status, FIR_ST_SEGMENTS);
         nseg[l * 2 + c] = min(tns, seg_cap);
     }
+}
+
+__global__ void __launch_bounds__(256) k_fir_prefix(long long gm, const int *__restrict__ counts,
+                                                    const int *__restrict__ list_cell,
+                                                    const CellGeo *__restrict__ geo, double *pre, long long pre_stride,
+                                                    long long pre_comp, int2 *segs, int *nseg, int seg_cap,
+                                                    int *status) {
+    __shared__ double ws[256 / 32][6];
+    __shared__ int wi[256 / 32];
+    const int l = blockIdx.x;
+    const int *cn = counts + 4 * l;
+    if (blockIdx.y == 0)
+        fir_prefix_class<3>(gm, l, 0, 0, cn[0], list_cell, geo, pre, pre_stride, pre_comp, segs, nseg, seg_cap, status,
+                            reinterpret_cast<double(*)[3]>(&ws[0][0]), wi);
+    else
+        fir_prefix_class<6>(gm, l, 1, cn[0], cn[1], list_cell, geo, pre, pre_stride, pre_comp, segs, nseg, seg_cap,
+                            status, ws, wi);
 }
 
 // One list of all visible cells (the quiet disk's), over the whole chip: k_fir_prefix's
@@ -1304,6 +1361,7 @@ struct FirTileArgs {
     int n, n_eff;
     const double *lam;
     double los;                 // lambda0 / step
+    const double2 *inv;         // [tile]: 1 / (j + los) at the tile's first and last pixel
     FirCubes cubes;
     const int *list_cell;       // [l][gm]
     const double *list_dlt;     // [l][gm]
@@ -1338,7 +1396,7 @@ __device__ int fir_segments(const FirTileArgs &A, int l, int j0, int t_eff, FirS
     const int *cn = A.counts + 4 * l;
     const int ns0 = A.nseg[2 * l];
     const int ns1 = nsg - ns0;
-    const double Xa = (double)j0 + A.los, Xb = (double)(j0 + t_eff - 1) + A.los;
+    const double Xa = soap_i2d(j0) + A.los, Xb = soap_i2d(j0 + t_eff - 1) + A.los;   // 0 < Xa <= Xb
     for (int s = tid; s < nsg; s += NT) {
         const int c = (s < ns0) ? 0 : 1;
         const int si = (c == 0) ? s : s - ns0;
@@ -1353,10 +1411,12 @@ __device__ int fir_segments(const FirTileArgs &A, int l, int j0, int t_eff, FirS
         g.cls = c;
         const double d0 = dl[g.start], d1 = dl[g.end - 1];
         // one more shift value on either side covers the cells the searches' thresholds
-        // classify one group away from floor(t)
-        g.m_lo = (int)fmin(floor(d0 * Xa), floor(d0 * Xb)) - 1;
-        g.m_hi = (int)fmax(floor(d1 * Xa), floor(d1 * Xb)) + 1;
-        if (fmax(fabs(d0), fabs(d1)) * (double)(FIR_TILE - 1) >= 1.0) {
+        // classify one group away from floor(t); a slope's sign tells at which end of the
+        // tile its t is least (floor is monotone)
+        g.m_lo = soap_floor_i(d0 * (bits_negative(d0) ? Xb : Xa)) - 1;
+        g.m_hi = soap_floor_i(d1 * (bits_negative(d1) ? Xa : Xb)) + 1;
+        if (max(soap_exp(d0), soap_exp(d1)) >= 1023 - 11 &&   // else below 2^-11: no test on the FP64 pipe
+            fmax(fabs(d0), fabs(d1)) * (double)(FIR_TILE - 1) >= 1.0) {
             atomicExch(A.status, FIR_ST_FAST);   // a weight could wrap twice in one tile
             g.m_hi = g.m_lo;
         }
@@ -1427,7 +1487,8 @@ __device__ void fir_plan_batch(const FirTileArgs &A, int l, int j0, int t_eff, c
     const int tid = threadIdx.x;
     const int n_eff = A.n_eff;
     const double dj0 = soap_i2d(j0);
-    const double iXa = 1.0 / (dj0 + A.los), iXb = 1.0 / (soap_i2d(j0 + t_eff - 1) + A.los);
+    const double2 inv = A.inv[j0 / FIR_TILE];
+    const double iXa = inv.x, iXb = inv.y;
     const int nbu = min(ST::NU, nunit - ub);
     for (int t = tid; t < nbu; t += NT) st.unit[t] = fir_describe(ub + t, segs, nsg, j0, t_eff, n_eff);
     __syncthreads();
@@ -2602,7 +2663,7 @@ namespace {
 struct FirLayout {
     enum {
         GEO, GEO32, CUBE0, SED2A = CUBE0 + 6, SED2B, K1A, K1B, K2A, K2B, VA, VB, SORT_TMP, LCELL, LDLT, LAUX,
-        COUNTS, RUNS, PRE, SEGS, NSEG, PLAN, NSLOT
+        COUNTS, RUNS, INV, PRE, SEGS, NSEG, PLAN, NSLOT
     };
     size_t off[NSLOT] = {0};
     size_t total = 0;
@@ -2639,8 +2700,9 @@ FirLayout fir_layout(int form, int n, int n_mu, long long gm, int ncube, int n_l
     L.seg_cap = 2 * n_mu;
     sz[FirLayout::SEGS] = sizeof(int2) * 2 * (size_t)L.seg_cap * n_lists;
     sz[FirLayout::NSEG] = sizeof(int) * 2 * (size_t)n_lists;
-    // precomputed tile plans of the phase integration
     const size_t ntile = ((size_t)n + FIR_TILE - 1) / FIR_TILE;
+    sz[FirLayout::INV] = sizeof(double2) * ntile;
+    // precomputed tile plans of the phase integration
     if (ncube == 6)
         sz[FirLayout::PLAN] = ntile * n_lists *
                               ((form == SOAPGB_FAST32) ? (size_t)FirPlanSlot<float>::BYTES + sizeof(int)
@@ -2729,12 +2791,13 @@ int fir_typed_cubes(soapgb_ctx *ctx, int form, int n, const soapgb_cubes &c, cha
 
 static int fir_prepare(soapgb_ctx *ctx, const double *wave, int n_eff, double step, long long gm, const double *delta,
                        const double *limb, const double *lb, const int *region, int n_mu, CellGeo *geo,
-                       CellGeo32 *geo32, double *lambda0) {
+                       CellGeo32 *geo32, double2 *inv, double *lambda0) {
     if (!(*lambda0 > 0.0)) {   // not given by the caller: read it from the device
         SOAP_CUDA(ctx, cudaMemcpyAsync(lambda0, wave, sizeof(double), cudaMemcpyDeviceToHost, ctx->stream));
         SOAP_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
     }
-    k_check_uniform<<<grid_for(ctx, n_eff, 256), 256, 0, ctx->stream>>>(n_eff, wave, step, ctx->d_status);
+    k_check_uniform<<<(n_eff + 255) / 256, 256, 0, ctx->stream>>>(n_eff, wave, step, *lambda0 / step, inv,
+                                                                  ctx->d_status);
     SOAP_LAUNCHED(ctx);
     SOAP_TRACED(ctx, "cell_geo", k_cell_geo<<<grid_for(ctx, gm, 256), 256, 0, ctx->stream>>>(gm, delta, limb, lb, region, n_mu, *lambda0, step, geo,
                                                                 geo32, ctx->d_status));
@@ -2847,6 +2910,7 @@ static FirTileArgs make_tile_args(soapgb_ctx *ctx, const FirLayout &L, char *ws,
     A.n_eff = n_eff;
     A.lam = lam;
     A.los = los;
+    A.inv = (const double2 *)(ws + L.off[FirLayout::INV]);
     A.cubes = fc;
     A.list_cell = (const int *)(ws + L.off[FirLayout::LCELL]);
     A.list_dlt = (const double *)(ws + L.off[FirLayout::LDLT]);
@@ -2975,7 +3039,7 @@ int fir_quiet(soapgb_ctx *ctx, int form, const FirQuietArgs &a, char *scratch, c
         geo32 = (CellGeo32 *)a.geo->geo32;
     } else {
         rc = fir_prepare(ctx, a.wave, a.n_eff, a.step, gm, a.delta, a.limb, nullptr, a.region, a.n_mu, geo, geo32,
-                         &lambda0);
+                         (double2 *)(ws + L.off[FirLayout::INV]), &lambda0);
         if (rc) return rc;
     }
     rc = fir_order(ctx, L, ws, gm, geo);
@@ -3018,6 +3082,7 @@ int fir_quiet(soapgb_ctx *ctx, int form, const FirQuietArgs &a, char *scratch, c
                                    nullptr, 0, 1);
     A.geo = geo;
     A.geo32 = geo32;
+    if (a.geo) A.inv = (const double2 *)a.geo->inv;
     if (form != SOAPGB_FAST32) return launch_quiet<double, 1>(ctx, A);
     return a.pair ? launch_quiet<float, 2>(ctx, A) : launch_quiet<float, 1>(ctx, A);
 }
@@ -3053,7 +3118,7 @@ int fir_phase(soapgb_ctx *ctx, int form, const FirPhaseArgs &a, char *scratch, c
     double lambda0 = a.lambda0;
     if (a.stage & FIR_STAGE_GEOMETRY) {
         int rc = fir_prepare(ctx, a.wave, a.n_eff, a.step, a.gm, a.delta, a.limb, a.lb, a.region, n_mu, geo, geo32,
-                             &lambda0);
+                             (double2 *)(ws + L.off[FirLayout::INV]), &lambda0);
         if (rc) return rc;
         if (!a.bi && !a.table) return set_error(ctx, SOAPGB_ERR_ARG, "fir_phase: neither maps nor a region table");
         rc = fir_lists(ctx, L, ws, a.gm, a.n_phase, a.temp, a.bi, a.act->solar, a.bi ? nullptr : &a);
@@ -3084,7 +3149,8 @@ int fir_phase(soapgb_ctx *ctx, int form, const FirPhaseArgs &a, char *scratch, c
 
 FirGeoRef fir_phase_geo(int form, const FirPhaseArgs &a, char *scratch) {
     const FirLayout L = fir_layout(form, a.n, a.cubes->n_mu, a.gm, 6, a.n_phase, a.typed != nullptr);
-    return FirGeoRef{scratch + L.off[FirLayout::GEO], scratch + L.off[FirLayout::GEO32]};
+    return FirGeoRef{scratch + L.off[FirLayout::GEO], scratch + L.off[FirLayout::GEO32],
+                     scratch + L.off[FirLayout::INV]};
 }
 
 size_t fir_tile_args_bytes() { return sizeof(FirTileArgs); }

@@ -33,9 +33,9 @@ int fir_typed_cubes(soapgb_ctx *ctx, int form, int n, const soapgb_cubes &c, cha
 size_t fir_quiet_pair_bytes(int n, int n_mu);
 int fir_quiet_pair(soapgb_ctx *ctx, int n, const soapgb_cubes &c, void *dst);
 
-// the per-cell constants in a workspace
+// the per-cell constants (and the tiles' reciprocal positions) in a workspace
 struct FirGeoRef {
-    const void *geo, *geo32;
+    const void *geo, *geo32, *inv;
 };
 
 struct FirQuietArgs {

@@ -27,7 +27,30 @@ __device__ __forceinline__ bool order_less(unsigned long long ah, unsigned long 
     return ah < bh || (ah == bh && al < bl);
 }
 
-// A warp sorts its 64 keys in registers (bitonic: lane l holds keys l and 32 + l), then runs
+// A warp's 64 keys sorted (bitonic): lane l holds keys l and 32 + l
+__device__ __forceinline__ void order_sort64(unsigned long long (&k)[2], int lane) {
+#pragma unroll
+    for (int lk = 1; lk <= 6; ++lk) {
+#pragma unroll
+        for (int lj = lk - 1; lj >= 0; --lj) {
+            if (lj == 5) {
+                const unsigned long long a = k[0], b = k[1];
+                k[0] = min(a, b);
+                k[1] = max(a, b);
+                continue;
+            }
+            const int j = 1 << lj;
+#pragma unroll
+            for (int q = 0; q < 2; ++q) {
+                const unsigned long long o = __shfl_xor_sync(0xffffffffu, k[q], j);
+                const bool up = (((32 * q + lane) >> lk) & 1) == 0;
+                k[q] = (((lane & j) == 0) == up) ? min(k[q], o) : max(k[q], o);
+            }
+        }
+    }
+}
+
+// A warp sorts its 64 keys in registers (as order_sort64), then runs
 // of 64, 128 ... keys are merged: a key's place is its place in its run plus the count of the
 // sibling run's keys below it, found by binary search.
 template <typename Key>
