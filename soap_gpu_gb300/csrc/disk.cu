@@ -164,6 +164,58 @@ int plain_cells(soapgb_ctx *ctx, long long gm, int n_eff, const double *d_wave, 
 }
 }  // namespace soapgb
 
+// the term of cell c (one owner offset) at the thread's pixel; in: the pixel has an owner, and lanes
+// without one must not send their warp the other way
+__device__ __forceinline__ double quiet_term(const PlainRec &c, const PlainPix &px, const PlainVal &va,
+                                             const unsigned long long *tab, double lj, bool in) {
+    const double ls = pl_shifted(c, px), ls1 = __shfl_down_sync(0xffffffffu, ls, 1);
+    int k;
+    double X, rise;
+    if ((pl_interval(c, lj, ls, ls1, k, X) && px.ok) || !in) rise = pl_rise(c, va, tab[k], k, X);
+    else rise = pl_rise_plain(va.g, lj, ls, ls1);
+    return __dmul_rn(__dadd_rn(va.s0, rise), c.limb);
+}
+
+// the thread's source interval and the row's values there, kept while the cells share both
+struct QuietAt {
+    PlainPix px;
+    PlainVal va;
+    int row = -1, m = 0;
+    __device__ __forceinline__ void move(const PlainRec &c, int n, int n_eff, int j, const double *__restrict__ lam,
+                                         const double *__restrict__ cube) {
+        if (c.row == row && c.m == m) return;
+        row = c.row;
+        m = c.m;
+        const int i = min(max(j + m, 0), n_eff - 1);
+        px.li = lam[i];
+        px.lm = soap_sig(px.li);
+        px.ok = pl_load(va, cube + (long long)row * n, i, min(i + 1, n_eff - 1));
+    }
+};
+
+// a cell without one offset for the tile, or at rest
+__device__ __forceinline__ double quiet_value(const PlainRec &c, const PlainGeo &g, int j, int n, int n_eff,
+                                              const double *__restrict__ lam, const double *__restrict__ cube) {
+    CellShift cs;
+    cs.sq = g.sq;
+    cs.fbeta = g.fbeta;
+    cs.off = g.off;
+    return soap_cell_value(j, n_eff, lam, cube + (long long)c.row * n, c.flags == PL_STILL ? 0.0 : 1.0, c.limb, cs);
+}
+
+// the record of the cell at a position of the list
+__device__ __forceinline__ void quiet_stage(int k, const PlainGeo *__restrict__ geo, const double *__restrict__ delta_m,
+                                            const double *__restrict__ limb_m, const int *__restrict__ region_m,
+                                            int n_mu, int j0, int cnt, double lmid, PlainRec &rec,
+                                            unsigned long long *tab, int *status) {
+    int row = region_m[k];
+    if ((unsigned)row >= (unsigned)n_mu) {   // mu bin outside the cube: report, use bin 0
+        atomicExch(status, 21);
+        row = 0;
+    }
+    pl_stage(geo + k, delta_m[k], limb_m[k], row, j0, cnt, lmid, rec, tab);
+}
+
 // A block takes PL_TILE pixels, a thread one, all cells in order.  Small blocks: 100,000 px
 // are 10.6 blocks per SM.
 __global__ void __launch_bounds__(PL_THREADS) k_quiet_plain64(int n, int n_eff, const double *__restrict__ lam,
@@ -185,58 +237,123 @@ __global__ void __launch_bounds__(PL_THREADS) k_quiet_plain64(int n, int n_eff, 
     const bool mine = j < n_eff && lane != 31;
     const double lj = lam[min(j, n_eff - 1)];
     double sum = 0.0;
-    PlainPix px;
-    PlainVal va;
-    int row_now = -1, m_now = 0;
+    QuietAt at;
     const int n_cells = *n_cells_ptr;
     for (int c0 = 0; c0 < n_cells; c0 += PL_CHUNK) {
         const int nc = min(PL_CHUNK, n_cells - c0);
         __syncthreads();
         if (threadIdx.x < nc) {
             const int k = cells[c0 + threadIdx.x];
-            int row = region_m[k];
-            if ((unsigned)row >= (unsigned)n_mu) {   // mu bin outside the cube: report, use bin 0
-                atomicExch(status, 21);
-                row = 0;
-            }
             s_cell[threadIdx.x] = k;
-            pl_stage(geo + k, delta_m[k], limb_m[k], row, j0, cnt, lmid, s_rec[threadIdx.x], s_tab[threadIdx.x]);
+            quiet_stage(k, geo, delta_m, limb_m, region_m, n_mu, j0, cnt, lmid, s_rec[threadIdx.x], s_tab[threadIdx.x],
+                        status);
         }
         __syncthreads();
         for (int t = 0; t < nc; ++t) {
             const PlainRec c = s_rec[t];
-            const double *row = cube + (long long)c.row * n;
             if (c.flags != PL_CONST) {
-                if (mine) {
-                    const PlainGeo &g = geo[s_cell[t]];
-                    CellShift cs;
-                    cs.sq = g.sq;
-                    cs.fbeta = g.fbeta;
-                    cs.off = g.off;
-                    sum = __dadd_rn(sum, soap_cell_value(j, n_eff, lam, row, c.flags == PL_STILL ? 0.0 : 1.0, c.limb, cs));
-                }
+                if (mine) sum = __dadd_rn(sum, quiet_value(c, geo[s_cell[t]], j, n, n_eff, lam, cube));
                 continue;
             }
-            if (c.row != row_now || c.m != m_now) {
-                row_now = c.row;
-                m_now = c.m;
-                const int i = min(max(j + c.m, 0), n_eff - 1);
-                px.li = lam[i];
-                px.lm = soap_sig(px.li);
-                px.ok = pl_load(va, row, i, min(i + 1, n_eff - 1));
-            }
-            const double ls = pl_shifted(c, px), ls1 = __shfl_down_sync(0xffffffffu, ls, 1);
+            at.move(c, n, n_eff, j, lam, cube);
+            const double ls = pl_shifted(c, at.px), ls1 = __shfl_down_sync(0xffffffffu, ls, 1);
             // lanes without a pixel here must not send their warp the other way
             const bool in = mine && (unsigned)(j + c.m) <= (unsigned)(n_eff - 2);
             int k;
             double X, rise;
-            if ((pl_interval(c, lj, ls, ls1, k, X) && px.ok) || !in) rise = pl_rise(c, va, s_tab[t][k], k, X);
-            else rise = pl_rise_plain(va.g, lj, ls, ls1);
-            const double r = __dadd_rn(sum, __dmul_rn(__dadd_rn(va.s0, rise), c.limb));
+            if ((pl_interval(c, lj, ls, ls1, k, X) && at.px.ok) || !in) rise = pl_rise(c, at.va, s_tab[t][k], k, X);
+            else rise = pl_rise_plain(at.va.g, lj, ls, ls1);
+            const double r = __dadd_rn(sum, __dmul_rn(__dadd_rn(at.va.s0, rise), c.limb));
             if (in) sum = r;
         }
     }
     if (lane != 31 && j < n) out[j] = mine ? sum : 0.0;
+}
+
+// The same sums where the tiles are too few to fill the chip: a cell's term is a chain of some 800
+// cycles, which two warps per tile walk one cell after the other.  Here PQ_WARPS warps share a tile.
+// They compute the terms of a chunk of cells into shared memory, in groups taken from a counter,
+// while one of them adds up the terms of the chunk before, in the cells' order: the additions stay
+// those of the sum above.  100 x 100 cells: 6,000 px 3.38 -> 0.96 ms, 20,000 px 3.64 -> 2.31 ms,
+// 37,600 px 3.78 -> 2.82 ms.  Above four tiles per SM the other kernel's warps fill the pipes
+// (37,800 px: 4.0 ms; 50,000 px 4.2 ms, here 4.1; 100,000 px of 200 x 200 cells 28.0 ms, here 29.9).
+constexpr int PQ_WARPS = 16, PQ_STRIPS = PL_TILE / 31, PQ_CHUNK = 64, PQ_GROUP = 4;
+struct PlainQuietSmem {   // chunks, double buffered
+    double term[2][PQ_STRIPS][PQ_CHUNK][32];
+    unsigned long long tab[2][PQ_CHUNK][PL_TAB];
+    PlainRec rec[2][PQ_CHUNK];
+    int cell[2][PQ_CHUNK];
+    double sum[PQ_STRIPS][32];
+    int next[2][PQ_STRIPS];   // jobs taken in a step, per strip
+};
+
+__global__ void __launch_bounds__(32 * PQ_WARPS, 2) k_quiet_plain64s(
+    int n, int n_eff, const double *__restrict__ lam, const double *__restrict__ cube,
+    const int *__restrict__ n_cells_ptr, const int *__restrict__ cells, const PlainGeo *__restrict__ geo,
+    const double *__restrict__ delta_m, const double *__restrict__ limb_m, const int *__restrict__ region_m, int n_mu,
+    double *__restrict__ out, int *status) {
+    extern __shared__ __align__(16) unsigned char pq_smem[];
+    PlainQuietSmem &sh = *reinterpret_cast<PlainQuietSmem *>(pq_smem);
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, strip = warp % PQ_STRIPS;
+    const int j0 = blockIdx.x * PL_TILE, j = j0 + strip * 31 + lane;
+    const int cnt = max(1, min(PL_TILE, n_eff - j0));
+    const double lmid = lam[min(j0 + cnt / 2, n_eff - 1)];
+    const bool mine = j < n_eff && lane != 31;
+    const double lj = lam[min(j, n_eff - 1)];
+    const int n_cells = *n_cells_ptr, n_chunk = (n_cells + PQ_CHUNK - 1) / PQ_CHUNK;
+    QuietAt at;
+    auto stage = [&](int c) {   // the records of chunk c, by one warp
+        const int b = c & 1;
+        for (int t = lane; t < min(PQ_CHUNK, n_cells - c * PQ_CHUNK); t += 32) {
+            const int k = cells[c * PQ_CHUNK + t];
+            sh.cell[b][t] = k;
+            quiet_stage(k, geo, delta_m, limb_m, region_m, n_mu, j0, cnt, lmid, sh.rec[b][t], sh.tab[b][t], status);
+        }
+    };
+    if (warp < PQ_STRIPS) sh.sum[warp][lane] = 0.0;
+    if (threadIdx.x < PQ_STRIPS) sh.next[0][threadIdx.x] = 0;
+    if (warp == 0) stage(0);
+    // step c: the sum over chunk c - 1, the records of chunk c + 1 (strip 0), the terms of chunk c
+    for (int c = 0; c <= n_chunk; ++c) {
+        __syncthreads();
+        const int b = c & 1;
+        if (threadIdx.x < PQ_STRIPS) sh.next[b ^ 1][threadIdx.x] = 0;
+        const int nt = c < n_chunk ? min(PQ_CHUNK, n_cells - c * PQ_CHUNK) : 0;
+        const int jobs = 2 + (nt + PQ_GROUP - 1) / PQ_GROUP;
+        while (true) {
+            int job = 0;
+            if (lane == 0) job = atomicAdd(&sh.next[b][strip], 1);
+            job = __shfl_sync(0xffffffffu, job, 0);
+            if (job >= jobs) break;
+            if (job == 0) {
+                if (c == 0) continue;
+                const int np = min(PQ_CHUNK, n_cells - (c - 1) * PQ_CHUNK);
+                double sum = sh.sum[strip][lane];
+#pragma unroll 4
+                for (int t = 0; t < np; ++t) sum = __dadd_rn(sum, sh.term[b ^ 1][strip][t][lane]);
+                sh.sum[strip][lane] = sum;
+            } else if (job == 1) {
+                if (strip == 0 && c + 1 < n_chunk) stage(c + 1);
+            } else {
+                const int t0 = (job - 2) * PQ_GROUP, t1 = min(t0 + PQ_GROUP, nt);
+                for (int t = t0; t < t1; ++t) {
+                    const PlainRec r = sh.rec[b][t];
+                    double v = 0.0;   // a pixel without an owner adds zero: the sum's bits stay
+                    if (r.flags != PL_CONST) {
+                        if (mine) v = quiet_value(r, geo[sh.cell[b][t]], j, n, n_eff, lam, cube);
+                    } else {
+                        at.move(r, n, n_eff, j, lam, cube);
+                        const bool in = mine && (unsigned)(j + r.m) <= (unsigned)(n_eff - 2);
+                        const double term = quiet_term(r, at.px, at.va, sh.tab[b][t], lj, in);
+                        if (in) v = term;
+                    }
+                    sh.term[b][strip][t][lane] = v;
+                }
+            }
+        }
+    }
+    __syncthreads();
+    if (warp < PQ_STRIPS && lane != 31 && j < n) out[j] = mine ? sh.sum[strip][lane] : 0.0;
 }
 
 // --------------------------------------------------------------------------
@@ -382,8 +499,18 @@ extern "C" int soapgb_quiet_disk(soapgb_ctx *ctx, int form, int n, int n_eff, co
         PlainGeo *geo = ws.get<PlainGeo>(s_fir);
         rc = plain_cells(ctx, gm, n_eff, d_wave, d_delta, step, geo);
         if (rc) return rc;
-        SOAP_TRACED(ctx, "quiet_plain64", k_quiet_plain64<<<(n + PL_TILE - 1) / PL_TILE, PL_THREADS, 0, ctx->stream>>>(
-            n, n_eff, d_wave, d_cube, d_count, d_cells, geo, d_delta, d_limb, d_region, n_mu, d_out, ctx->d_status));
+        const int ntile = (n + PL_TILE - 1) / PL_TILE;
+        if (ntile <= 4 * ctx->num_sms) {
+            SOAP_CUDA(ctx, cudaFuncSetAttribute(k_quiet_plain64s, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                (int)sizeof(PlainQuietSmem)));
+            SOAP_TRACED(ctx, "quiet_plain64",
+                        k_quiet_plain64s<<<ntile, 32 * PQ_WARPS, sizeof(PlainQuietSmem), ctx->stream>>>(
+                            n, n_eff, d_wave, d_cube, d_count, d_cells, geo, d_delta, d_limb, d_region, n_mu, d_out,
+                            ctx->d_status));
+        } else {
+            SOAP_TRACED(ctx, "quiet_plain64", k_quiet_plain64<<<ntile, PL_THREADS, 0, ctx->stream>>>(
+                n, n_eff, d_wave, d_cube, d_count, d_cells, geo, d_delta, d_limb, d_region, n_mu, d_out, ctx->d_status));
+        }
         SOAP_LAUNCHED(ctx);
     } else {
         FirQuietArgs qa;

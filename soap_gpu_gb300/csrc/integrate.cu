@@ -53,10 +53,17 @@ struct PhaseCell {
     int type;       // 0 spot, 1 facula
     int unit;       // 1: the intensity is the continuum row itself, 0: scale x the row, -1: a Planck ratio
     double scale;   // 1 + LB
+    PlainFactor by; // the limb factor
 };
 
 // The plain form: block (x, p) sums phase p's active cells, in map order, over a tile of
-// pixels (plain64.cuh); three rows per cell.
+// pixels (plain64.cuh); three rows per cell.  INT: the five products of a cell and pixel on the
+// integer pipes (18.4 -> 13 FP64 instructions, 285 -> 440 in all), which pays where the FP64 pipe
+// is the bound: 5 phases of 200 x 200 cells and 100,000 px, 8.2 -> 6.1 ms; 11 phases of 151 x 151
+// and 60,001 px, 7.0 -> 5.2 ms; at 6.4 blocks per SM 0.340 -> 0.317 ms.  With fewer the pipe waits
+// for the chains of the few warps, which the integer products lengthen (5.3 blocks per SM: 0.53 ->
+// 0.59 ms; 2.1: 1.45 -> 1.81 ms).
+template <bool INT>
 __global__ void __launch_bounds__(PL_THREADS) k_phase_plain64(
     int n, int n_eff, const double *__restrict__ lam, const double *__restrict__ q_norm,
     const double *__restrict__ q_sed, const double *__restrict__ spot_norm, const double *__restrict__ fac_norm,
@@ -81,6 +88,7 @@ __global__ void __launch_bounds__(PL_THREADS) k_phase_plain64(
     const bool mine = j < n_eff && lane != 31;
     const int jc = min(j, n_eff - 1);
     const double lj = lam[jc], ssed = spot_sed[jc], fsed = fac_sed[jc];
+    const PlainFactor by_s = pl_factor(ssed), by_f = pl_factor(fsed);
     double fx = 0.0, bc = 0.0, tt = 0.0;
     PlainPix px;
     PlainVal va[3];
@@ -108,6 +116,7 @@ __global__ void __launch_bounds__(PL_THREADS) k_phase_plain64(
                 a.unit = 0;
                 a.scale = __dadd_rn(1.0, lb_m[k]);
             }
+            a.by = pl_factor(limb_m[k]);
             s_cell[threadIdx.x] = a;
             pl_stage(geo + k, delta_m[k], limb_m[k], row, j0, cnt, lmid, s_rec[threadIdx.x], s_tab[threadIdx.x]);
         }
@@ -118,6 +127,8 @@ __global__ void __launch_bounds__(PL_THREADS) k_phase_plain64(
             const long long off = (long long)c.row * n;
             const double *an = (a.type == 0 ? spot_norm : fac_norm) + off;
             double q, s, v;
+            bool fast = false;           // q and v are moderate, or zero where the pixel has no owner
+            bool none = false;           // no owner
             if (c.flags != PL_CONST) {   // the pixel itself, or an owner search per pixel
                 const PlainGeo &g = geo[a.k];
                 CellShift cs;
@@ -156,17 +167,59 @@ __global__ void __launch_bounds__(PL_THREADS) k_phase_plain64(
                     for (int r = 0; r < 3; ++r) x[r] = pl_rise_plain(va[r].g, lj, ls, ls1);
                 }
 #pragma unroll
-                for (int r = 0; r < 3; ++r) x[r] = __dmul_rn(__dadd_rn(va[r].s0, x[r]), c.limb);
-                q = in ? x[0] : 0.0;
-                s = in ? x[1] : 0.0;
-                v = in ? x[2] : 0.0;
+                for (int r = 0; r < 3; ++r) x[r] = __dadd_rn(va[r].s0, x[r]);
+                if constexpr (INT) {
+                    bool plain = a.by.hi == 0 || !(soap_moderate(x[0], PL_SPAN) && soap_moderate(x[1], PL_SPAN) &&
+                                                   soap_moderate(x[2], PL_SPAN));
+                    fast = !plain || !in;
+                    none = !in;
+                    q = pl_mul(x[0], a.by, plain);
+                    s = pl_mul(x[1], a.by, plain);
+                    v = pl_mul(x[2], a.by, plain);
+                    if (plain && in) {
+                        q = pl_mul_plain(x[0], c.limb);
+                        s = pl_mul_plain(x[1], c.limb);
+                        v = pl_mul_plain(x[2], c.limb);
+                    }
+                } else {
+                    q = __dmul_rn(x[0], c.limb);
+                    s = __dmul_rn(x[1], c.limb);
+                    v = __dmul_rn(x[2], c.limb);
+                }
+                q = in ? q : 0.0;
+                s = in ? s : 0.0;
+                v = in ? v : 0.0;
             }
-            double I = a.type == 0 ? ssed : fsed;
-            if (a.unit == 0) I = __dmul_rn(a.scale, I);
-            else if (a.unit < 0) I = soap_intensity(a.type, pt[a.k], lb_m[a.k], lj, ssed, fsed, solar, t_norm_fac);
-            fx = __dsub_rn(__dadd_rn(fx, s), __dmul_rn(I, q));
+            double I = a.type == 0 ? ssed : fsed, iq, iv;
+            if constexpr (INT) {
+                PlainFactor by = a.type == 0 ? by_s : by_f;
+                if (a.unit == 0) {
+                    bool plain = by.hi == 0 || !soap_moderate(a.scale, PL_SPAN);
+                    const double f = I;
+                    I = pl_mul(a.scale, by, plain);
+                    if (plain) I = pl_mul_plain(a.scale, f);
+                    by = pl_factor(I);
+                } else if (a.unit < 0) {
+                    I = soap_intensity(a.type, pt[a.k], lb_m[a.k], lj, ssed, fsed, solar, t_norm_fac);
+                    by = pl_factor(I);
+                }
+                bool plain = !fast || by.hi == 0;
+                iq = pl_mul(q, by, plain);
+                iv = pl_mul(v, by, plain);
+                if (none) iq = iv = 0.0;   // moderate intensity x 0
+                if (plain && !(none && by.hi != 0)) {
+                    iq = pl_mul_plain(I, q);
+                    iv = pl_mul_plain(v, I);
+                }
+            } else {
+                if (a.unit == 0) I = __dmul_rn(a.scale, I);
+                else if (a.unit < 0) I = soap_intensity(a.type, pt[a.k], lb_m[a.k], lj, ssed, fsed, solar, t_norm_fac);
+                iq = __dmul_rn(I, q);
+                iv = __dmul_rn(v, I);
+            }
+            fx = __dsub_rn(__dadd_rn(fx, s), iq);
             bc = __dsub_rn(__dadd_rn(bc, q), v);
-            tt = __dsub_rn(__dadd_rn(tt, s), __dmul_rn(v, I));
+            tt = __dsub_rn(__dadd_rn(tt, s), iv);
         }
     }
     if (lane == 31 || j >= n) return;
@@ -201,7 +254,9 @@ int integrate_device(soapgb_ctx *ctx, int form, int n, int n_eff, const double *
         PlainGeo *geo = (PlainGeo *)fir_scratch;   // PLAIN64 has no plans: its cells' constants stand there
         rc = plain_cells(ctx, gm, n_eff, d_wave, dm.delta, step, geo);
         if (rc) return rc;
-        SOAP_TRACED(ctx, "integrate_plain64", k_phase_plain64<<<dim3((n + PL_TILE - 1) / PL_TILE, n_phase), PL_THREADS, 0, ctx->stream>>>(
+        const dim3 g((n + PL_TILE - 1) / PL_TILE, n_phase);
+        const auto kern = (long long)g.x * g.y >= 6LL * ctx->num_sms ? k_phase_plain64<true> : k_phase_plain64<false>;
+        SOAP_TRACED(ctx, "integrate_plain64", kern<<<g, PL_THREADS, 0, ctx->stream>>>(
             n, n_eff, d_wave, dc.q_norm, dc.q_sed, dc.spot_norm, dc.fac_norm, dc.spot_sed, dc.fac_sed, (int)gm,
             d_cells, d_counts, d_temp, d_bi, geo, dm.delta, dm.limb, dm.lb, dm.region, gm, act->solar,
             act->t_star, act->t_diff_fac, (double *)d_flux, (double *)d_bconv, (double *)d_tot, out_stride, dc.n_mu,

@@ -21,12 +21,16 @@
 //  - the division.  On a grid of constant step l'_{i+1} - l'_i is one of a few neighbouring
 //    integers in units of ulp: the cell's table holds the 64-bit reciprocals of eight of them for
 //    soap_quot_bits;
+//  - in the integration, the products with the limb factor and the intensities: pl_mul, from the
+//    upper half of the significands' product;
 //  - l_j - l'_i.  With X = 2^e + (l_j - l'_i), whose bits are an integer sum, slope x difference is
 //    fma(slope, X, -slope 2^e), rounded once.
 // A cell and pixel takes 4.4 FP64 instructions in the quiet sum (about 60 when every pixel
-// searched its owner, shifted two wavelengths and divided) and 18.4 in the integration, whose pipe
-// bounds both (75 to 80 % busy).  31,417 cells x 100,000 px: 306 -> 28 ms; 5 phases of 200x200 and
-// 100,000 px, three regions: 36 -> 7.5 ms.  One pixel per thread: two took 31 ms and 8.4 ms.
+// searched its owner, shifted two wavelengths and divided) and 13 in the integration.
+// 31,417 cells x 100,000 px: 306 -> 28 ms; 5 phases of 200x200 and 100,000 px, three regions:
+// 36 -> 6.1 ms.  One pixel per thread: two took 31 ms, and 8.4 against 7.5 ms.  The quiet sum's one
+// product stays on the FP64 pipe: with pl_mul 28.6 ms, two cells at a time 28.0 (219 instructions
+// against 147, of which 3.6 against 4.4 on the FP64 pipe: issue and the chain then bound it).
 // What the integers do not cover (another binade, an uneven grid, differences outside the table,
 // non-finite or extreme values) takes the reference's operations.  Every path gives the same bits.
 #pragma once
@@ -62,6 +66,12 @@ enum : int {
     PL_STILL = 2,   // v == 0: the pixel itself
 };
 
+// a factor of many products
+struct PlainFactor {
+    unsigned long long sig;   // significand, leading bit at bit 63
+    int hi;                   // sign and exponent; 0: not normal or not of moderate size
+};
+
 // what a tile needs of a cell
 struct PlainRec {
     double u, limb;
@@ -73,6 +83,35 @@ struct PlainRec {
 };
 
 __device__ __forceinline__ int pl_exp(double v) { return (int)((unsigned)__double2hiint(v) >> 20); }
+
+constexpr int PL_SPAN = 200;   // exponents of a product's factors: products of three stay normal
+
+__device__ __forceinline__ PlainFactor pl_factor(double v) {
+    PlainFactor f;
+    f.sig = soap_sig(v);
+    f.hi = soap_moderate(v, PL_SPAN) ? __double2hiint(v) & 0xfff00000 : 0;
+    return f;
+}
+
+// The bits of a x b (a normal): the upper half of the significands' product holds 53 bits and at
+// least ten to round by.  unsure: those are one half as far as they show, so the reference's
+// operation decides (one product in 2048).
+__device__ __forceinline__ double pl_mul(double a, const PlainFactor &b, bool &unsure) {
+    const int ah = __double2hiint(a);
+    unsigned long long h = __umul64hi(soap_sig(a), b.sig);
+    const int top = (int)(h >> 63);
+    if (!top) h += h;
+    const unsigned low = (unsigned)h & 0x7ffu;
+    unsure = unsure || low == 0x400u;
+    const unsigned long long m = (h >> 11) + (low >> 10);
+    // exponent - 1: the significand's leading bit adds the one
+    const unsigned e = (unsigned)(ah & 0x7ff00000) + (unsigned)(b.hi & 0x7ff00000) - (1024u << 20) + ((unsigned)top << 20);
+    return __longlong_as_double(
+        (long long)(m + ((unsigned long long)(e | ((unsigned)(ah ^ b.hi) & 0x80000000u)) << 32)));
+}
+
+// A call, so that the products of the lanes that need one stay off the others' path.
+static __device__ __noinline__ double pl_mul_plain(double a, double b) { return __dmul_rn(a, b); }
 
 // The table of the binade of l (1 - u) around spacings d sq
 __device__ __forceinline__ void pl_table(double l, double d, double sq, double u, PlainTab &t) {

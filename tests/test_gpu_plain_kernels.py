@@ -235,3 +235,38 @@ def test_fit_and_its_adjoint(ctx, n, n_spec, with_err):
     h = 1e-4 / np.sqrt(n)
     d = (ctx.gauss_bis(x, y + h * v, err)["par"][:, 3] - ctx.gauss_bis(x, y - h * v, err)["par"][:, 3]) / (2 * h)
     assert np.all(np.abs(d - (g * v).sum(1)) <= 1e-4 * np.linalg.norm(g, axis=1) * np.linalg.norm(v, axis=1))
+
+
+@pytest.mark.parametrize("n,n_phase,kind", [(62 * 608, 1, "lines"), (62 * 608 + 1, 2, "flat"), (62 * 66 + 5, 14, "lines"),
+                                            (62 * 66, 14, "wild"), (62 * 66 - 1, 14, "flat")])
+def test_plain_sums_of_many_tiles(ctx, n, n_phase, kind):
+    """As above at the tile counts where the quiet sum goes from 16 warps per tile to two and the
+    integration's products from the FP64 pipe to the integer ones; continuum rows and limb factors with
+    zero, negative, tiny and non-finite values."""
+    rng = np.random.default_rng(n)
+    grid, n_mu, step, n_eff = 8, 3, 0.01, n - 3
+    wave = 4090.0 + step * np.arange(n)   # across a binade
+    maps = dict(_disk(grid, 9.0, 4090.0, n_mu))
+    vis = np.nonzero(maps["limb"] > -998)[0]
+    maps["limb"] = maps["limb"].copy()
+    maps["limb"][vis[[1, 4, 7]]] = 0.0, -0.3, 1e-200
+    cube = [_cube(n, n_mu, rng, kind) for _ in range(4)]
+    sed = [0.3 + 0.1 * np.arange(n) / n, 1.0 + 0.1 * np.arange(n) / n]
+    sed[0][[70, 300]] = 0.0, -0.2
+    sed[1][[71, 301, 500]] = np.nan, np.inf, 1e-100
+    bi = np.full(grid * grid, -9999.0)
+    bi[vis[::2]], bi[vis[1::2]] = 0.0, 1.0
+    temp = np.where(bi == 0.0, 5115.0, np.where(bi == 1.0, 5900.0, -9999.0))
+    from soap_gpu_gb300._lib import Activity
+    names = ("q_norm", "q_sed", "spot_norm", "fac_norm")
+    with np.errstate(all="ignore"):
+        ref = oracle.quiet_disk(wave, cube[0], n_eff, maps, grid, step)
+        got = ctx.quiet_disk("plain64", wave, cube[0], n_eff, maps, grid, step)
+        assert np.array_equal(got, ref, equal_nan=True)
+        out = ctx.phase_integrate("plain64", wave, n_eff, grid, np.tile(temp, (n_phase, 1)), np.tile(bi, (n_phase, 1)),
+                                  maps, dict(zip(names, cube), spot_sed=sed[0], fac_sed=sed[1]), step,
+                                  Activity(5778, 663, 250, 20, 0))
+        want = oracle.phase_integrate(wave, n_eff, grid, temp, bi, maps, *cube, *sed, step)
+    for o, r in zip(out, want):
+        for p in range(n_phase):
+            assert np.array_equal(o[p], r, equal_nan=True)
