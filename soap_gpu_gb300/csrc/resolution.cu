@@ -75,7 +75,7 @@ __device__ __forceinline__ const double *soap_base_for(int s, const double *base
 // PLAIN64 convolution: conv_inst term by term (the reference's operations in its order).
 // ---------------------------------------------------------------------------
 // one pixel of one spectrum over every tap of the reference's window
-__device__ double conv_plain64_pixel(int index, int wid, double step_mult, double step_exp, double norm, double den,
+__device__ __noinline__ double conv_plain64_pixel(int index, int wid, double step_mult, double step_exp, double norm, double den,
                                      const double *__restrict__ sp, const double *__restrict__ bp) {
     double acc = 0.0;
     for (int m = index - wid; m < index + wid - 1; m++) {
@@ -116,12 +116,14 @@ __global__ void __launch_bounds__(256) k_conv_plain64(int n, int n_eff, const do
 // memory for all its spectra.  The spectra's terms step_mult (1 - A) are staged once per block,
 // and the division by s_i sqrt(2 pi) is a soap_quot, so a tap costs two FP64 instructions
 // (product, sum) instead of about 55.
-// Taps with a weight below e^-90 are left out: to the right of the centre they cannot change
-// the rounded sum (below a quarter of its ulp), to the left they change its last bit with a
-// probability of about 1e-17 per pixel (the early partial sums' error is rounded away as the
-// weights grow).  That holds for a block's spectrum whose terms in the whole reference window
-// are finite and within a factor 2^20 of one another (continuum and lines of a disk sum are);
-// another one (NaN, infinities, zeros next to large values) goes through conv_plain64_pixel.
+// Taps with a weight below e^-90 are left out.  That changes no bit of a sum of at least 2^-20 of
+// the window's largest term: to the right of the centre a tap stays below a quarter of the sum's
+// ulp; to the left, what the early partial sums lack is rounded away as the weights grow, but for
+// a chance of about 2^-47 per pixel.  A smaller sum (terms of either sign) is taken over all taps
+// by conv_plain64_pixel, and so are the pixels of a block whose window holds zeros, infinities,
+// NaN or values beyond 2^800.  (The test is per pixel: with one on the block's range of terms, the
+// one block at a spectrum's edge where 1 - A changes its sign took 6.4 ms of a call of 11 phases
+// that takes 0.7 ms otherwise.)
 // Bound by the FP64 pipe: (2 reach + 1) x 2 instructions per pixel and spectrum and
 // (reach + 1) x 20 for the weights per pixel and block.  One spectrum of 310,000 px:
 // 3.28 -> 0.71 ms per call; 10 of 100,000 px: 13.9 -> 0.45 ms.
@@ -193,20 +195,22 @@ __global__ void __launch_bounds__(CP_PIX) k_conv_plain64t(int n, int n_eff, cons
             mn = min(mn, s_mn[w]);
             mx = max(mx, s_mx[w]);
         }
-        // exponents within 2^-800 .. 2^800 and within 2^20 of one another
-        const bool whole = odd_block || mn < (223u << 20) || mx > (1823u << 20) || mx - mn > (20u << 20);
+        // exponents within 2^-800 .. 2^800
+        const bool whole = odd_block || mn < (223u << 20) || mx > (1823u << 20);
         double acc = 0.0;
         if (live) {
-            if (whole) {
-                acc = conv_plain64_pixel(index, wid, step_mult, step_exp, norm, den, sp, bp);
-            } else {
+            bool all_taps = whole;
+            if (!whole) {
                 const double *yc = ys + t + wid;
                 const int lo = min(reach, wid), hi = min(reach, wid - 2);
                 for (int d = lo; d > 0; --d)
                     acc = __dadd_rn(acc, __dmul_rn(soap_quot(yc[-d], by), wt[d * CP_PIX + t]));
                 for (int d = 0; d <= hi; ++d)
                     acc = __dadd_rn(acc, __dmul_rn(soap_quot(yc[d], by), wt[d * CP_PIX + t]));
+                const int ex = (int)(((unsigned)__double2hiint(acc) >> 20) & 0x7ffu);
+                all_taps = ex + (int)((unsigned)__double2hiint(norm) >> 20) - 1023 < (int)(mx >> 20) - 20;
             }
+            if (all_taps) acc = conv_plain64_pixel(index, wid, step_mult, step_exp, norm, den, sp, bp);
         }
         if (index < n_eff) conv[(long long)s * conv_stride + index] = acc;
     }

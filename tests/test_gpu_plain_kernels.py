@@ -270,3 +270,23 @@ def test_plain_sums_of_many_tiles(ctx, n, n_phase, kind):
     for o, r in zip(out, want):
         for p in range(n_phase):
             assert np.array_equal(o[p], r, equal_nan=True)
+
+
+@pytest.mark.parametrize("n,n_spec,top", [(3000, 5, 1e4), (1500, 1, 1e9), (2600, 2, 3.0)])
+def test_plain_convolution_of_small_sums(ctx, n, n_spec, top):
+    """Spectra whose terms 1 - A pass through zero, slowly and steeply, and stretches where they cancel:
+    sums far below their terms."""
+    rng = np.random.default_rng(n)
+    step, sv = 0.01, _sigma_v(115000.0)
+    wave = 5000.0 + step * np.arange(n)
+    n_eff = n // 512 * 512
+    x = np.arange(n)
+    a = 1.0 + top * np.tanh((x - n // 2) / (1.0 + 40.0 * np.arange(n_spec)[:, None]))
+    a[:, n // 4:n // 4 + 60] = 1.0 + 1e-9 * rng.uniform(-1, 1, (n_spec, 60))
+    a[:, n // 3:n // 3 + 200] = 1.0 + top * (1.0 - 2.0 * (x[:200] % 2)) + 1e-7
+    base = 2.0 + top * rng.uniform(0, 1, n)
+    got, mm = ctx.lower_resolution("plain64", wave, base[None, :] - a, n_eff, sv, base=base, step_mult=step, step_exp=step)
+    for s in range(n_spec):
+        ref, _, ext = oracle.lower_resolution(wave, base - (base - a[s]), n_eff, sv, step_mult=step, step_exp=step)
+        assert np.max(np.abs(got[s] - ref)) <= 1e-12 * np.max(np.abs(ref))
+        assert np.allclose(mm[s], ext, rtol=1e-12, atol=0)
