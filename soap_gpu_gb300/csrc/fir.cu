@@ -82,10 +82,27 @@ struct __align__(16) CellGeo32 {
     float4 a, b;
 };
 
+// The wavelength grid must be uniform for the collapsed form; and the tiles' reciprocal
+// positions (two divisions per plan were half of k_fir_plan's FP64 instructions; with the
+// segments' floors on the integer pipes, 29,400 plans take 115 us against 131).
+__device__ __forceinline__ void fir_grid(int i, int n_eff, const double *__restrict__ lam, double step, double los,
+                                         double2 *inv, int *status) {
+    if (i >= n_eff) return;
+    if ((long long)i * FIR_TILE < n_eff) {
+        const int j0 = i * FIR_TILE, t_eff = min(FIR_TILE, n_eff - j0);
+        inv[i] = make_double2(1.0 / ((double)j0 + los), 1.0 / ((double)(j0 + t_eff - 1) + los));
+    }
+    double expect = lam[0] + (double)i * step;
+    if (fabs(lam[i] - expect) > 1e-6 * step) atomicExch(status, FIR_ST_UNIFORM);
+}
+
+// the cells' constants, and fir_grid of the pixels
 __global__ void k_cell_geo(long long gm, const double *__restrict__ delta, const double *__restrict__ limb,
                            const double *__restrict__ lb, const int *__restrict__ region, int n_mu, double lambda0,
-                           double step, CellGeo *geo, CellGeo32 *geo32, int *status) {
+                           double step, int n_eff, const double *__restrict__ lam, double2 *inv, CellGeo *geo,
+                           CellGeo32 *geo32, int *status) {
     long long k = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    if (k < n_eff) fir_grid((int)k, n_eff, lam, step, lambda0 / step, inv, status);
     if (k >= gm) return;
     double d = delta[k];
     CellGeo g;
@@ -112,21 +129,6 @@ __global__ void k_cell_geo(long long gm, const double *__restrict__ delta, const
     h.a = make_float4(dh, (float)(g.dlt - (double)dh), oh, (float)(g.offir - (double)oh));
     h.b = make_float4((float)g.L, (float)g.w2, (float)g.dlt, __int_as_float(g.row | (g.zero_v ? (int)0x80000000 : 0)));
     geo32[k] = h;
-}
-
-// wavelength grid must be uniform for the collapsed form; and the tiles' reciprocal
-// positions (two divisions per plan were half of k_fir_plan's FP64 instructions; with the
-// segments' floors on the integer pipes, 29,400 plans take 115 us against 131)
-__global__ void k_check_uniform(int n_eff, const double *__restrict__ lam, double step, double los, double2 *inv,
-                                int *status) {
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n_eff) return;
-    if ((long long)i * FIR_TILE < n_eff) {
-        const int j0 = i * FIR_TILE, t_eff = min(FIR_TILE, n_eff - j0);
-        inv[i] = make_double2(1.0 / ((double)j0 + los), 1.0 / ((double)(j0 + t_eff - 1) + los));
-    }
-    double expect = lam[0] + (double)i * step;
-    if (fabs(lam[i] - expect) > 1e-6 * step) atomicExch(status, FIR_ST_UNIFORM);
 }
 
 // FP64 -> FP32 rounded to nearest even on the integer pipes: the 52-bit fraction is cut
@@ -177,10 +179,26 @@ __device__ __forceinline__ void cube_rows_store(long long i, double2 a, double2 
     fa[2 * i + 1] = make_float4(qs1, soap_f64_to_f32(b.y - d.y), qn1, soap_f64_to_f32(d.y));
 }
 
+// the continuum rows as float pairs (hi, lo)
+__device__ __forceinline__ void pair_rows_at(int i, const double *__restrict__ a, const double *__restrict__ b,
+                                             float2 *pa, float2 *pb) {
+    float ah = (float)a[i], bh = (float)b[i];
+    pa[i] = make_float2(ah, (float)(a[i] - (double)ah));
+    pb[i] = make_float2(bh, (float)(b[i] - (double)bh));
+}
+__global__ void k_pair_rows(int n, const double *__restrict__ a, const double *__restrict__ b, float2 *pa, float2 *pb) {
+    int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < n) pair_rows_at(i, a, b, pa, pb);
+}
+
 __global__ void __launch_bounds__(256) k_cube_types32(long long n2, const double2 *__restrict__ qs,
                                                       const double2 *__restrict__ qn, const double2 *__restrict__ sn,
-                                                      const double2 *__restrict__ fn, float4 *sp, float4 *fa) {
+                                                      const double2 *__restrict__ fn, float4 *sp, float4 *fa, int n,
+                                                      const double *__restrict__ ssed, const double *__restrict__ fsed,
+                                                      float2 *ssed2, float2 *fsed2) {
     const long long stride = (long long)gridDim.x * blockDim.x;
+    for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride)
+        pair_rows_at((int)i, ssed, fsed, ssed2, fsed2);
     for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n2; i += 2 * stride) {
         const long long j = i + stride;
         const double2 a0 = __ldcs(qs + i), b0 = __ldcs(qn + i), c0 = __ldcs(sn + i), d0 = __ldcs(fn + i);
@@ -2649,14 +2667,6 @@ __global__ void k_fir_zero(int n, const int *__restrict__ zero_list, T *out0, T 
     out2[o] = (T)0;
 }
 
-__global__ void k_pair_rows(int n, const double *__restrict__ a, const double *__restrict__ b, float2 *pa, float2 *pb) {
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    float ah = (float)a[i], bh = (float)b[i];
-    pa[i] = make_float2(ah, (float)(a[i] - (double)ah));
-    pb[i] = make_float2(bh, (float)(b[i] - (double)bh));
-}
-
 namespace {
 
 // workspace layout of the FAST forms
@@ -2750,8 +2760,10 @@ static int typed_cubes_into(soapgb_ctx *ctx, int form, int n, const soapgb_cubes
         SOAP_TRACED(ctx, "cube_types",
                     k_cube_types32<<<nblk, 256, 0, ctx->stream>>>(
                         n2, (const double2 *)c.q_sed, (const double2 *)c.q_norm, (const double2 *)c.spot_norm,
-                        (const double2 *)c.fac_norm, (float4 *)dst[0], (float4 *)dst[1]));
+                        (const double2 *)c.fac_norm, (float4 *)dst[0], (float4 *)dst[1], n, c.spot_sed, c.fac_sed,
+                        sed2a, sed2b));
         SOAP_LAUNCHED(ctx);
+        return SOAPGB_OK;
     } else if (form == SOAPGB_FAST32) {
         SOAP_TRACED(ctx, "cube_types", k_cube_rows<float><<<grid_for(ctx, cube_elems, 256), 256, 0, ctx->stream>>>(
                                            cube_elems, c.q_sed, c.q_norm, c.spot_norm, c.fac_norm,
@@ -2796,11 +2808,10 @@ static int fir_prepare(soapgb_ctx *ctx, const double *wave, int n_eff, double st
         SOAP_CUDA(ctx, cudaMemcpyAsync(lambda0, wave, sizeof(double), cudaMemcpyDeviceToHost, ctx->stream));
         SOAP_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
     }
-    k_check_uniform<<<(n_eff + 255) / 256, 256, 0, ctx->stream>>>(n_eff, wave, step, *lambda0 / step, inv,
-                                                                  ctx->d_status);
-    SOAP_LAUNCHED(ctx);
-    SOAP_TRACED(ctx, "cell_geo", k_cell_geo<<<grid_for(ctx, gm, 256), 256, 0, ctx->stream>>>(gm, delta, limb, lb, region, n_mu, *lambda0, step, geo,
-                                                                geo32, ctx->d_status));
+    const long long threads = std::max<long long>(gm, n_eff);
+    SOAP_TRACED(ctx, "cell_geo", k_cell_geo<<<(unsigned)((threads + 255) / 256), 256, 0, ctx->stream>>>(
+                                     gm, delta, limb, lb, region, n_mu, *lambda0, step, n_eff, wave, inv, geo, geo32,
+                                     ctx->d_status));
     SOAP_LAUNCHED(ctx);
     return SOAPGB_OK;
 }

@@ -274,29 +274,30 @@ static int conv_plain64_launch(soapgb_ctx *ctx, int n, int n_eff, int n_spec, co
 // per-pixel tap parameters of the fast forms: weight scale kq = step_mult / (s sqrt(2 pi)),
 // exponent coefficient cq = step_exp^2 / (2 s^2), significant tap range [dlo, dhi]
 // (dhi < dlo marks a pixel outside the reference's convolution interior)
-template <typename T>
-__global__ void k_conv_params(int n, int n_eff, const double *__restrict__ lam, double ka, double kb, double kr,
-                              int wid, int halo, T *kq, T *cq, int2 *rng) {
+__device__ __forceinline__ void conv_tap_constants(int i, int n, double l, double ka, double kb, double kr, int wid,
+                                                   int halo, double &k, double &c, int2 &rng) {
     // sigma_i = lambda_i (sqrt((1 + b)/(1 - b)) - 1) is proportional to lambda_i, so with
     // ka = step_mult / (s1 sqrt(2 pi)), kb = step_exp^2 / (2 s1^2), kr = sqrt(cut / kb)
     // (s1 = sigma at lambda = 1): kq = ka / lambda, cq = kb / lambda^2, reach = kr lambda
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n_eff) return;
-    bool live = (i > wid) && (i + wid < n - 1);
-    double k = 0.0, c = 0.0;
-    int lo = 0, hi = -1;
-    if (live) {
-        const double l = lam[i];
+    k = c = 0.0;
+    rng = make_int2(0, -1);
+    if ((i > wid) && (i + wid < n - 1)) {
         const double inv = 1.0 / l;
         k = ka * inv;
         c = kb * inv * inv;
         int r = (int)floor(kr * l);
-        lo = max(max(-wid, -r), -halo);
-        hi = min(min(wid - 2, r), halo);
+        rng = make_int2(max(max(-wid, -r), -halo), min(min(wid - 2, r), halo));
     }
+}
+template <typename T>
+__global__ void k_conv_params(int n, int n_eff, const double *__restrict__ lam, double ka, double kb, double kr,
+                              int wid, int halo, T *kq, T *cq, int2 *rng) {
+    int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n_eff) return;
+    double k, c;
+    conv_tap_constants(i, n, lam[i], ka, kb, kr, wid, halo, k, c, rng[i]);
     kq[i] = (T)k;
     cq[i] = (T)c;
-    rng[i] = make_int2(lo, hi);
 }
 
 // ---------------------------------------------------------------------------
@@ -455,18 +456,16 @@ template <int SB>
 __global__ void __launch_bounds__(FC_THREADS) k_conv_base_df(int n, int n_eff, const double *__restrict__ kqa,
                                                              const double *__restrict__ cqa,
                                                              const int2 *__restrict__ rnga,
-                                                             const double *__restrict__ spec, long long spec_stride,
-                                                             int n_spec, int halo, double *__restrict__ conv,
-                                                             long long conv_stride) {
+                                                             const double *__restrict__ base_a,
+                                                             const double *__restrict__ base_b, int halo,
+                                                             double *__restrict__ conv, long long conv_stride) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     float2 *xs = reinterpret_cast<float2 *>(smem_raw);   // staged 1 - base as (hi, lo)
-    const int win = FC_TILE + 2 * halo;
-    const int i0 = blockIdx.x * FC_TILE;
-    const int s0 = blockIdx.y * SB;
-    const int nsb = min(SB, n_spec - s0);
-    for (int q = 0; q < nsb; ++q) {
-        const double *sp = spec + (long long)(s0 + q) * spec_stride;
-        for (int t = threadIdx.x; t < win; t += FC_THREADS) {
+    const int tile = (int)blockDim.x * FC_PIX, win = tile + 2 * halo;
+    const int i0 = blockIdx.x * tile;
+    for (int q = 0; q < SB; ++q) {
+        const double *sp = q ? base_b : base_a;
+        for (int t = threadIdx.x; t < win; t += (int)blockDim.x) {
             const int m = i0 - halo + t;
             const DFloat d = df_of((m >= 0 && m < n) ? 1.0 - sp[m] : 0.0);
             xs[q * win + t] = make_float2(d.hi, d.lo);
@@ -518,18 +517,15 @@ __global__ void __launch_bounds__(FC_THREADS) k_conv_base_df(int n, int n_eff, c
         const int li = e - (i0 - halo);
 #pragma unroll
         for (int q = 0; q < SB; ++q) {
-            if (q < nsb) {
-                const float2 xv = xs[q * win + li];
-                const DFloat x = {xv.x, xv.y};
+            const float2 xv = xs[q * win + li];
+            const DFloat x = {xv.x, xv.y};
 #pragma unroll
-                for (int p = 0; p < FC_PIX; ++p) acc[q][p] = df_add(acc[q][p], df_mul(w[p], x));
-            }
+            for (int p = 0; p < FC_PIX; ++p) acc[q][p] = df_add(acc[q][p], df_mul(w[p], x));
         }
     }
 #pragma unroll
     for (int q = 0; q < SB; ++q) {
-        if (q >= nsb) continue;
-        double *cp = conv + (long long)(s0 + q) * conv_stride;
+        double *cp = conv + (long long)q * conv_stride;
 #pragma unroll
         for (int p = 0; p < FC_PIX; ++p) {
             const int i = ib + p;
@@ -626,80 +622,69 @@ __device__ __forceinline__ float soap_dec32(unsigned u) {
     return __uint_as_float(u);
 }
 
-__global__ void k_base_prep(int n, int n_eff, const double *__restrict__ base, const double *__restrict__ cb,
-                            float *base32, float *cb32) {
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n) base32[i] = (float)base[i];
-    if (i < n_eff) cb32[i] = (float)cb[i];
-}
-
-__global__ void k_mm32_init(int n_spec, double sentinel, unsigned *mm32, unsigned long long *mm64) {
+// the extrema's start values; a zero spectrum's (zero_spec) are its base's, mmz
+__global__ void k_mm32_init(int n_spec, double sentinel, const unsigned char *__restrict__ zero_spec, int b_every,
+                            const unsigned long long *__restrict__ mmz, unsigned *mm32, unsigned long long *mm64) {
     int s = blockIdx.x * blockDim.x + threadIdx.x;
-    if (s < n_spec) {
-        if (mm32) {
-            mm32[4 * s + 0] = 0xffffffffu;             // min A (FP32 key)
-            mm32[4 * s + 1] = 0u;                      // max C (FP32 key)
-            mm32[4 * s + 2] = 0u;                      // max(|base| + |spec|)
-            mm32[4 * s + 3] = 0u;                      // max(|cb| + |conv|)
-        }
-        mm64[2 * s + 0] = ~0ULL;
-        mm64[2 * s + 1] = soap_ord_enc(sentinel);
-    }
+    if (s >= n_spec) return;
+    mm32[4 * s + 0] = 0xffffffffu;             // min A (FP32 key)
+    mm32[4 * s + 1] = 0u;                      // max C (FP32 key)
+    mm32[4 * s + 2] = 0u;                      // max(|base| + |spec|)
+    mm32[4 * s + 3] = 0u;                      // max(|cb| + |conv|)
+    const int q = (b_every > 0 && (s % b_every) == b_every - 1) ? 1 : 0;
+    const bool zero = zero_spec && zero_spec[s];
+    mm64[2 * s + 0] = zero ? mmz[2 * q] : ~0ULL;
+    mm64[2 * s + 1] = zero ? mmz[2 * q + 1] : soap_ord_enc(sentinel);
 }
 
-// per-pixel tap constants of the FP32 convolution: weight(d) = 2^(d^2 c2 + lk) with
-// c2 = -step_exp^2 / (2 s^2) log2(e), lk = log2(step_mult / (s sqrt(2 pi))) (FP64, then
-// rounded once); live = inside the reference's convolution interior; rblk[b] = largest
-// significant reach (weight >= e^-cut of the central one) over block b's pixels
-__global__ void k_conv32_params(int n, int n_eff, const double *__restrict__ lam, double sigma_v, int wid, int halo,
-                                double step_mult, double step_exp, double cut, float *c2, float *lk, int *live,
-                                int *rblk) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    int reach = 0;
-    if (i < n_eff) {
-        bool lv = (i > wid) && (i + wid < n - 1);
-        double a = 0.0, l = -200.0;
-        if (lv) {
-            double sig = soap_delta_lambda(sigma_v, lam[i]);
-            double cq = step_exp * step_exp / (2.0 * sig * sig);
-            a = -cq * 1.4426950408889634;   // log2(e)
-            l = log2(step_mult / (sig * sqrt(2. * SOAP_PI)));
-            reach = min((int)floor(sqrt(cut / cq)) + 1, halo);
-        }
-        c2[i] = (float)a;
-        lk[i] = (float)l;
-        live[i] = lv ? 1 : 0;
+// Set-up of the FP32 form's convolutions, a block per 1024 pixels: the tap constants of the
+// base convolution in FP64 (k_conv_params's) and, from them, those of the spectra in FP32 --
+// weight(d) = 2^(d^2 c2 + lk), c2 = -cq log2(e), lk = log2(kq) (FP32 log2 of the rounded scale:
+// one more rounding of the weights' scale), live = inside the reference's convolution interior,
+// rblk[b] = largest significant reach (weight >= e^-cut of the central one) over the block's
+// pixels --, the bases in FP32, and the start values of the zero spectra's extrema mmz.  One
+// launch: with short spectra a call's time is its launches.
+__global__ void __launch_bounds__(1024) k_conv_setup(int n, int n_eff, const double *__restrict__ lam, double ka,
+                                                     double kb, double kr, int wid, int halo64, int halo, float cut,
+                                                     double *kq, double *cq, int2 *rng, float *c2, float *lk, int *live,
+                                                     int *rblk, const double *__restrict__ base_a,
+                                                     const double *__restrict__ base_b, float *b32a, float *b32b,
+                                                     double sentinel, unsigned long long *mmz) {
+    __shared__ int s_reach;
+    const int i = blockIdx.x * 1024 + threadIdx.x;
+    if (threadIdx.x == 0) s_reach = 0;
+    if (i < 2) {
+        mmz[2 * i] = ~0ULL;
+        mmz[2 * i + 1] = soap_ord_enc(sentinel);
     }
-    // a warp's pixels share one block of 1024: one atomic per warp
-    reach = __reduce_max_sync(0xffffffffu, reach);
-    if ((threadIdx.x & 31) == 0 && reach > 0) atomicMax(&rblk[(blockIdx.x * blockDim.x) / FC_TILE], reach);
-}
-
-// the FP32 tap constants from the FP64 ones of the base convolution (same pixels,
-// same sigma): c2 = -cq log2(e), lk = log2(kq) (FP32 log2 of the rounded scale: one
-// more rounding of the weights' scale), reach from the FP32 cut
-__global__ void k_conv32_derive(int n_eff, const double *__restrict__ kq, const double *__restrict__ cq,
-                                const int2 *__restrict__ rng, int halo, float cut, float *c2, float *lk, int *live,
-                                int *rblk) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    __syncthreads();
     int reach = 0;
+    if (i < n) {
+        b32a[i] = (float)base_a[i];
+        if (base_b) b32b[i] = (float)base_b[i];
+    }
     if (i < n_eff) {
-        const int2 r = rng[i];
+        double k, c;
+        int2 r;
+        conv_tap_constants(i, n, lam[i], ka, kb, kr, wid, halo64, k, c, r);
+        kq[i] = k;
+        cq[i] = c;
+        rng[i] = r;
         const bool lv = r.x <= r.y;
         float a = 0.f, l = -200.f;
         if (lv) {
-            const double c = cq[i];
             a = (float)(-c * 1.4426950408889634);
-            l = log2f((float)kq[i]);
+            l = log2f((float)k);
             reach = min((int)floorf(sqrtf(cut / (float)c)) + 1, halo);
         }
         c2[i] = a;
         lk[i] = l;
         live[i] = lv ? 1 : 0;
     }
-    // a warp's pixels share one block of 1024: one atomic per warp
     reach = __reduce_max_sync(0xffffffffu, reach);
-    if ((threadIdx.x & 31) == 0 && reach > 0) atomicMax(&rblk[(blockIdx.x * blockDim.x) / FC_TILE], reach);
+    if ((threadIdx.x & 31) == 0) atomicMax(&s_reach, reach);
+    __syncthreads();
+    if (threadIdx.x == 0) rblk[blockIdx.x] = s_reach;
 }
 
 __device__ __forceinline__ float soap_ex2(float x) {
@@ -1203,21 +1188,24 @@ __global__ void __launch_bounds__(256) k_refine64x(int n, int n_eff, int nbx, co
 // k_refine64x finds for such a spectrum (its candidates hold the extremes of the base
 // alone): min over [0, n) of base, max over [0, n_eff) of the base convolution where
 // its FP32 and FP64 values are non-zero.  mmz[2 q] / mmz[2 q + 1] for base q, set to
-// (~0, sentinel) by k_mm32_init's rule beforehand.  grid (blocks, bases)
+// (~0, sentinel) by k_conv_setup.  Also the base convolutions' FP32 copies, c32.  grid
+// (blocks, bases)
 __global__ void __launch_bounds__(256) k_zero_extrema(int n, int n_eff, const double *__restrict__ ba,
                                                       const double *__restrict__ bb, const double *__restrict__ cba,
-                                                      const double *__restrict__ cbb, const float *__restrict__ c32a,
-                                                      const float *__restrict__ c32b, unsigned long long *mmz) {
+                                                      const double *__restrict__ cbb, float *c32a, float *c32b,
+                                                      unsigned long long *mmz) {
     const int q = blockIdx.y;
     const double *b64 = q ? bb : ba;
     const double *c64 = q ? cbb : cba;
-    const float *c32 = q ? c32b : c32a;
+    float *c32 = q ? c32b : c32a;
     unsigned long long mn = ~0ULL, mx = 0ULL;
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         mn = min(mn, soap_ord_enc(b64[i] - 0.0));
-        if (i < n_eff && c32[i] != 0.f) {
+        if (i < n_eff) {
             const double cx = c64[i] + 0.0;
-            if (cx != 0.0) mx = max(mx, soap_ord_enc(cx));
+            const float c = (float)c64[i];
+            c32[i] = c;
+            if (c != 0.f && cx != 0.0) mx = max(mx, soap_ord_enc(cx));
         }
     }
     for (int o = 16; o > 0; o >>= 1) {
@@ -1242,16 +1230,6 @@ __global__ void k_zero_rows(int n_eff, int b_every, const float *__restrict__ c3
     const float f = (float)((1.0 - mn) / mx);
     const float c = (q ? c32b : c32a)[i] + 0.f;
     out3[(size_t)t * n_eff + i] = soap_f32_to_f64(fmaf(-c, f, 1.0f));
-}
-
-// extrema of the zero spectra of a chunk from the per-base values
-__global__ void k_zero_mm(int n_spec, const unsigned char *__restrict__ zero_spec, int b_every,
-                          const unsigned long long *__restrict__ mmz, unsigned long long *mm64) {
-    const int s = blockIdx.x * blockDim.x + threadIdx.x;
-    if (s >= n_spec || !zero_spec[s]) return;
-    const int q = (b_every > 0 && (s % b_every) == b_every - 1) ? 1 : 0;
-    mm64[2 * s] = mmz[2 * q];
-    mm64[2 * s + 1] = mmz[2 * q + 1];
 }
 
 // FP64 normalisation constants per spectrum -> FP32 factor
@@ -1329,10 +1307,10 @@ __global__ void __launch_bounds__(256) k_norm32v(int n_eff, const float *__restr
 
 namespace soapgb {
 
-static size_t conv_param_bytes(int n_eff) {
+static size_t conv_param_bytes(int n, int n_eff) {
     // FAST64: kq, cq (double) + ranges (int2); FAST32: c2, lk, live (4 bytes each) + per-block reach
     return 2 * ((sizeof(double) * (size_t)n_eff + 255) & ~size_t(255)) + ((sizeof(int2) * (size_t)n_eff + 255) & ~size_t(255)) +
-           ((sizeof(int) * (size_t)(n_eff / FC_TILE + 2) + 255) & ~size_t(255));
+           ((sizeof(int) * (size_t)(n / FC_TILE + 2) + 255) & ~size_t(255));
 }
 
 size_t resolution_scratch_bytes(int form, int n, int n_eff, int n_spec) {
@@ -1340,7 +1318,7 @@ size_t resolution_scratch_bytes(int form, int n, int n_eff, int n_spec) {
     b += sizeof(unsigned long long) * 2 * n_spec + 256;          // min/max
     b += sizeof(unsigned long long) * 4 + 256 + sizeof(int) * ((size_t)n_spec + 2) + 256;   // zero spectra
     if (form != SOAPGB_PLAIN64)
-        b += 2 * (sizeof(double) * (size_t)n_eff + 256) + 2 * (conv_param_bytes(n_eff) + 256) +
+        b += 2 * (sizeof(double) * (size_t)n_eff + 256) + 2 * (conv_param_bytes(n, n_eff) + 256) +
              2 * sizeof(double) * (size_t)n + 256;   // base convolutions, tap constants, staged bases
     if (form == SOAPGB_FAST32) {
         b += 2 * (sizeof(float) * (size_t)n + 256) + 2 * (sizeof(float) * (size_t)n_eff + 256);   // base32, cb32
@@ -1384,66 +1362,28 @@ static int launch_conv_fast(soapgb_ctx *ctx, int n, int n_eff, const double *lam
     return SOAPGB_OK;
 }
 
-// The base convolution of the FP32 form: FP64 tap constants (k_conv_params), then
-// k_conv_base_df.  Same constants and ranges as launch_conv_fast<double>.
-template <int SB>
-static int launch_conv_base_df(soapgb_ctx *ctx, int n, int n_eff, const double *lam, const double *spec,
-                               long long spec_stride, int n_spec, double sigma_v, int wid, double step_mult,
-                               double step_exp, double cut, double *conv, long long conv_stride, double sig_max,
-                               char *param_scratch) {
+// significant reach of the widest Gaussian at a cut, within the window
+static int conv_halo(double sig_max, double step_exp, double cut, int wid) {
     const double cmin = step_exp * step_exp / (2.0 * sig_max * sig_max);
     const int r = (int)floor(sqrt(cut / cmin)) + 2;
-    int halo = std::min(wid, r);
-    if (halo < 1) halo = 1;
-    const size_t smem = sizeof(float2) * (size_t)SB * (FC_TILE + 2 * halo);
-    if (smem > 200 * 1024) return set_error(ctx, SOAPGB_ERR_ARG, "convolution window too wide (%d px)", halo);
-    if (smem > 48 * 1024)
-        SOAP_CUDA(ctx, cudaFuncSetAttribute(k_conv_base_df<SB>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    double *kq = (double *)param_scratch;
-    double *cq = (double *)(param_scratch + ((sizeof(double) * (size_t)n_eff + 255) & ~size_t(255)));
-    int2 *rng = (int2 *)(param_scratch + 2 * ((sizeof(double) * (size_t)n_eff + 255) & ~size_t(255)));
-    const double s1 = soap_sigma_per_lambda(sigma_v);
-    const double ka = step_mult / (s1 * sqrt(2. * SOAP_PI)), kb = step_exp * step_exp / (2.0 * s1 * s1);
-    const double kr = sqrt(cut / kb);
-    SOAP_TRACED(ctx, "conv_params",
-                k_conv_params<double><<<grid_for(ctx, n_eff, 256), 256, 0, ctx->stream>>>(n, n_eff, lam, ka, kb, kr,
-                                                                                         wid, halo, kq, cq, rng));
-    SOAP_LAUNCHED(ctx);
-    const dim3 g((n_eff + FC_TILE - 1) / FC_TILE, (n_spec + SB - 1) / SB);
-    SOAP_TRACED(ctx, "conv_base", k_conv_base_df<SB><<<g, FC_THREADS, smem, ctx->stream>>>(
-                                      n, n_eff, kq, cq, rng, spec, spec_stride, n_spec, halo, conv, conv_stride));
-    SOAP_LAUNCHED(ctx);
-    return SOAPGB_OK;
+    return std::max(1, std::min(wid, r));
 }
 
-// FP32 tap constants (from the FP64 ones of the base convolution when given) and the
-// reach of every block of 1024 pixels; returns the staging halo
-static int conv32_params(soapgb_ctx *ctx, int n, int n_eff, const double *lam, double sigma_v, int wid,
-                         double step_mult, double step_exp, double cut, double sig_max, char *param_scratch,
-                         const char *params64, int *halo_out) {
-    double cmin = step_exp * step_exp / (2.0 * sig_max * sig_max);
-    int r = (int)floor(sqrt(cut / cmin)) + 2;
-    int halo = std::min(wid, r);
-    if (halo < 1) halo = 1;
-    *halo_out = halo;
-    const size_t pb = (sizeof(float) * (size_t)n_eff + 255) & ~size_t(255);
-    float *c2 = (float *)param_scratch;
-    float *lk = (float *)(param_scratch + pb);
-    int *live = (int *)(param_scratch + 2 * pb);
-    int *rblk = (int *)(param_scratch + 3 * pb);
-    const int nbx = (n + FC_TILE - 1) / FC_TILE;
-    SOAP_CUDA(ctx, cudaMemsetAsync(rblk, 0, sizeof(int) * (size_t)nbx, ctx->stream));
-    if (params64) {   // from the FP64 constants of the base convolution (kq, cq, ranges)
-        const size_t pb64 = (sizeof(double) * (size_t)n_eff + 255) & ~size_t(255);
-        SOAP_TRACED(ctx, "conv_params",
-                    k_conv32_derive<<<grid_for(ctx, n_eff, 256), 256, 0, ctx->stream>>>(
-                        n_eff, (const double *)params64, (const double *)(params64 + pb64),
-                        (const int2 *)(params64 + 2 * pb64), halo, (float)cut, c2, lk, live, rblk));
-    } else {
-        SOAP_TRACED(ctx, "conv_params",
-                    k_conv32_params<<<grid_for(ctx, n_eff, 256), 256, 0, ctx->stream>>>(
-                        n, n_eff, lam, sigma_v, wid, halo, step_mult, step_exp, cut, c2, lk, live, rblk));
-    }
+// The base convolutions of the FP32 form (base_b: or none), conv[0, n_eff) and [n_eff, 2 n_eff).  A
+// block's first taps are FP64 exponentials, a chain of some 30 us on one SM for a tile of 1024 pixels;
+// with fewer such tiles than SMs the tile is 256.
+template <int SB>
+static int launch_conv_base_df(soapgb_ctx *ctx, int n, int n_eff, const double *kq, const double *cq, const int2 *rng,
+                               const double *base_a, const double *base_b, int halo, double *conv) {
+    const int threads = (n_eff + FC_TILE - 1) / FC_TILE < ctx->num_sms ? FC_THREADS / 4 : FC_THREADS;
+    const int tile = threads * FC_PIX;
+    const size_t smem = sizeof(float2) * (size_t)SB * (tile + 2 * halo);
+    if (sizeof(float2) * (size_t)SB * (FC_TILE + 2 * halo) > 200 * 1024)
+        return set_error(ctx, SOAPGB_ERR_ARG, "convolution window too wide (%d px)", halo);
+    if (smem > 48 * 1024)
+        SOAP_CUDA(ctx, cudaFuncSetAttribute(k_conv_base_df<SB>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    SOAP_TRACED(ctx, "conv_base", k_conv_base_df<SB><<<(n_eff + tile - 1) / tile, threads, smem, ctx->stream>>>(
+                                      n, n_eff, kq, cq, rng, base_a, base_b, halo, conv, n_eff));
     SOAP_LAUNCHED(ctx);
     return SOAPGB_OK;
 }
@@ -1531,29 +1471,12 @@ int resolution32_prepare(soapgb_ctx *ctx, int n, int n_eff, int n_spec, const do
     const double lmax = std::max(std::fabs(wave0), std::fabs(wave_last)) * 1.001;
     const double sig_max = -1 * lmax * (1 - sqrt((1 + sigma_v / SOAP_C_LIGHT) / (1 - sigma_v / SOAP_C_LIGHT)));
     if (!(sig_max > 0)) return set_error(ctx, SOAPGB_ERR_ARG, "non-positive instrument sigma");
-    char *pscr = carve(p, conv_param_bytes(n_eff));     // FP64 tap constants of the base convolution
-    char *pscr32 = carve(p, conv_param_bytes(n_eff));   // FP32 tap constants of the spectra's
-    int rc;
-    double *cb_a, *cb_b = nullptr;
-    if (R.base_b) {
-        // both bases in one launch (the FP64 weights are shared): staged as rows of one array
-        double *bb = (double *)carve(p, sizeof(double) * 2 * (size_t)n);
-        double *cb = (double *)carve(p, sizeof(double) * 2 * (size_t)n_eff);
-        SOAP_CUDA(ctx, cudaMemcpyAsync(bb, base_a, sizeof(double) * n, cudaMemcpyDeviceToDevice, ctx->stream));
-        SOAP_CUDA(ctx, cudaMemcpyAsync(bb + n, base_b, sizeof(double) * n, cudaMemcpyDeviceToDevice, ctx->stream));
-        rc = launch_conv_base_df<2>(ctx, n, n_eff, d_wave, bb, n, 2, sigma_v, wid, step_mult, step_exp, 40.0, cb,
-                                    n_eff, sig_max, pscr);
-        if (rc) return rc;
-        cb_a = cb;
-        cb_b = cb + n_eff;
-    } else {
-        cb_a = (double *)carve(p, sizeof(double) * (size_t)n_eff);
-        rc = launch_conv_base_df<1>(ctx, n, n_eff, d_wave, base_a, 0, 1, sigma_v, wid, step_mult, step_exp, 40.0,
-                                    cb_a, 0, sig_max, pscr);
-        if (rc) return rc;
-    }
-    R.cb_a = cb_a;
-    R.cb_b = cb_b;
+    char *pscr = carve(p, conv_param_bytes(n, n_eff));     // FP64 tap constants of the base convolution
+    char *pscr32 = carve(p, conv_param_bytes(n, n_eff));   // FP32 tap constants of the spectra's
+    const int n_base = R.base_b ? 2 : 1;
+    double *cb = (double *)carve(p, sizeof(double) * (size_t)n_base * n_eff);
+    R.cb_a = cb;
+    R.cb_b = R.base_b ? cb + n_eff : nullptr;
     float *b32a = (float *)carve(p, sizeof(float) * (size_t)n);
     float *b32b = (float *)carve(p, sizeof(float) * (size_t)n);
     float *c32a = (float *)carve(p, sizeof(float) * (size_t)n_eff);
@@ -1562,30 +1485,38 @@ int resolution32_prepare(soapgb_ctx *ctx, int n, int n_eff, int n_spec, const do
     R.fac = (float *)carve(p, 4 * (size_t)n_spec);
     R.nbx = (n + FC_TILE - 1) / FC_TILE;   // extrema blocks of 1024 pixels
     R.blk = (float *)carve(p, sizeof(float) * 2 * (size_t)R.nbx * n_spec);
-    k_base_prep<<<grid_for(ctx, n, 256), 256, 0, ctx->stream>>>(n, n_eff, base_a, cb_a, b32a, c32a);
-    SOAP_LAUNCHED(ctx);
-    if (cb_b) {
-        k_base_prep<<<grid_for(ctx, n, 256), 256, 0, ctx->stream>>>(n, n_eff, base_b, cb_b, b32b, c32b);
-        SOAP_LAUNCHED(ctx);
-    }
-    R.b32a = b32a;
-    R.b32b = cb_b ? b32b : b32a;
-    R.c32a = c32a;
-    R.c32b = cb_b ? c32b : c32a;
-    rc = conv32_params(ctx, n, n_eff, d_wave, sigma_v, wid, step_mult, step_exp, 30.0, sig_max, pscr32, pscr,
-                       &R.halo);
-    if (rc) return rc;
-    R.p32 = pscr32;
-    // extrema of the zero spectra, per base
     R.mmz = (unsigned long long *)carve(p, sizeof(unsigned long long) * 4);
     R.blist = (int *)carve(p, sizeof(int) * ((size_t)n_spec + 2));
-    k_mm32_init<<<1, 32, 0, ctx->stream>>>(2, sentinel, nullptr, R.mmz);
-    SOAP_LAUNCHED(ctx);
-    k_zero_extrema<<<dim3(std::max(1, std::min(grid_for(ctx, n, 256), 4 * std::max(ctx->num_sms, 1))), R.base_b ? 2 : 1),
-                     256, 0, ctx->stream>>>(n, n_eff, base_a, R.base_b ? R.base_b : base_a, cb_a, cb_b ? cb_b : cb_a,
-                                            c32a, cb_b ? c32b : c32a, R.mmz);
-    SOAP_LAUNCHED(ctx);
+    R.b32a = b32a;
+    R.b32b = R.base_b ? b32b : b32a;
+    R.c32a = c32a;
+    R.c32b = R.base_b ? c32b : c32a;
+    R.p32 = pscr32;
     R.next = p;
+    // the tap constants and the bases' FP32 copies
+    constexpr double CUT64 = 40.0, CUT32 = 30.0;
+    const int halo64 = conv_halo(sig_max, step_exp, CUT64, wid);
+    R.halo = conv_halo(sig_max, step_exp, CUT32, wid);
+    const size_t pb64 = (sizeof(double) * (size_t)n_eff + 255) & ~size_t(255);
+    const size_t pb32 = (sizeof(float) * (size_t)n_eff + 255) & ~size_t(255);
+    double *kq = (double *)pscr, *cq = (double *)(pscr + pb64);
+    int2 *rng = (int2 *)(pscr + 2 * pb64);
+    const double s1 = soap_sigma_per_lambda(sigma_v);
+    const double ka = step_mult / (s1 * sqrt(2. * SOAP_PI)), kb = step_exp * step_exp / (2.0 * s1 * s1);
+    SOAP_TRACED(ctx, "conv_params",
+                k_conv_setup<<<R.nbx, 1024, 0, ctx->stream>>>(
+                    n, n_eff, d_wave, ka, kb, sqrt(CUT64 / kb), wid, halo64, R.halo, (float)CUT32, kq, cq, rng,
+                    (float *)pscr32, (float *)(pscr32 + pb32), (int *)(pscr32 + 2 * pb32), (int *)(pscr32 + 3 * pb32),
+                    base_a, R.base_b, b32a, b32b, sentinel, R.mmz));
+    SOAP_LAUNCHED(ctx);
+    int rc = R.base_b ? launch_conv_base_df<2>(ctx, n, n_eff, kq, cq, rng, base_a, R.base_b, halo64, cb)
+                      : launch_conv_base_df<1>(ctx, n, n_eff, kq, cq, rng, base_a, nullptr, halo64, cb);
+    if (rc) return rc;
+    // extrema of the zero spectra, per base
+    k_zero_extrema<<<dim3(std::max(1, std::min(grid_for(ctx, n, 256), 4 * std::max(ctx->num_sms, 1))), n_base), 256, 0,
+                     ctx->stream>>>(n, n_eff, base_a, R.base_b ? R.base_b : base_a, R.cb_a, R.base_b ? R.cb_b : R.cb_a,
+                                    c32a, c32b, R.mmz);
+    SOAP_LAUNCHED(ctx);
     return SOAPGB_OK;
 }
 
@@ -1603,11 +1534,11 @@ int resolution32_run(soapgb_ctx *ctx, const Res32 &R, const float *spec32, long 
     unsigned long long *mm = R.mm + 2LL * s0;
     float *fac = R.fac + s0;
     float *blk = R.blk + 2LL * R.nbx * s0;
-    k_mm32_init<<<(ns + 127) / 128, 128, 0, ctx->stream>>>(ns, R.sentinel, mm32, mm);
-    SOAP_LAUNCHED(ctx);
     // spectra known to be zero (both flag copies given): their batches are left out of
     // the convolution and their extrema come from the bases
     const unsigned char *zs = (zero_spec && zero_host) ? zero_spec + s0 : nullptr;
+    k_mm32_init<<<(ns + 127) / 128, 128, 0, ctx->stream>>>(ns, R.sentinel, zs, R.b_every, R.mmz, mm32, mm);
+    SOAP_LAUNCHED(ctx);
     // the non-zero spectra of the chunk (relative indices): only they are convolved, in
     // batches of 8 without zero rows
     const int *blist = nullptr;
@@ -1615,8 +1546,6 @@ int resolution32_run(soapgb_ctx *ctx, const Res32 &R, const float *spec32, long 
     if (zs && blist_pre) {   // the caller uploaded the list with its own small inputs
         blist = blist_pre;
         nlist = nlist_pre;
-        k_zero_mm<<<(ns + 127) / 128, 128, 0, ctx->stream>>>(ns, zs, R.b_every, R.mmz, mm);
-        SOAP_LAUNCHED(ctx);
     } else if (zs) {
         std::vector<int> bl;
         for (int q = 0; q < ns; ++q)
@@ -1625,8 +1554,6 @@ int resolution32_run(soapgb_ctx *ctx, const Res32 &R, const float *spec32, long 
         if (nlist > 0)   // pageable source: staged by the driver before the call returns
             SOAP_CUDA(ctx, cudaMemcpyAsync(R.blist, bl.data(), sizeof(int) * nlist, cudaMemcpyHostToDevice, ctx->stream));
         blist = R.blist;
-        k_zero_mm<<<(ns + 127) / 128, 128, 0, ctx->stream>>>(ns, zs, R.b_every, R.mmz, mm);
-        SOAP_LAUNCHED(ctx);
     }
     int rc = conv32_run(ctx, n, n_eff, R.wid, R.halo, R.p32, sp, spec_stride, ns, R.b32a, R.b32b, R.c32a, R.c32b,
                         R.b_every, conv, mm32, blk, zs, blist, nlist);
@@ -1708,8 +1635,8 @@ int resolution_device(soapgb_ctx *ctx, int form, int n, int n_eff, int n_spec, c
         if (!(sig_max > 0)) return set_error(ctx, SOAPGB_ERR_ARG, "non-positive instrument sigma");
         double cut = (form == SOAPGB_FAST32) ? 30.0 : 40.0;
         int rc;
-        char *pscr = carve(p, conv_param_bytes(n_eff));     // FP64 tap constants of the base convolution
-        char *pscr32 = carve(p, conv_param_bytes(n_eff));   // FP32 tap constants of the spectra's
+        char *pscr = carve(p, conv_param_bytes(n, n_eff));     // FP64 tap constants of the base convolution
+        char *pscr32 = carve(p, conv_param_bytes(n, n_eff));   // FP32 tap constants of the spectra's
         if (base_a && base_b && b_every > 0) {
             // both bases in one launch (the FP64 weights are shared): staged as rows of one array
             double *bb = (double *)carve(p, sizeof(double) * 2 * (size_t)n);
