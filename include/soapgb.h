@@ -236,6 +236,10 @@ int soapgb_ccf(soapgb_ctx *ctx, int form, int n_v, const double *vel, int n_line
                double mask_step, int index_old, int n_spec, const double *spectra,
                int normalise, int mem, double *ccf_out);
 
+/* The normalised CCFs of raw ones (soapgb_ccf with normalise = 0), as soapgb_ccf with
+ * normalise = 1 forms them: raw, ccf_out (n_spec x n_v), may be the same. */
+int soapgb_ccf_normalise(soapgb_ctx *ctx, int n_spec, int n_v, const double *raw, int mem, double *ccf_out);
+
 /* Adjoint of soapgb_ccf in FP64 (the differentiable form; the reference has no
  * counterpart).  Same mask arguments as the forward; g_ccf (n_spec x n_v) is the
  * gradient of a scalar w.r.t. ccf_out.  With `normalise` set, ccf_raw (n_spec x n_v)

@@ -85,6 +85,7 @@ SIGNATURES = [
     ("soapgb_ccf", ctypes.c_int, [_vp, ctypes.c_int, ctypes.c_int, _vp, ctypes.c_int, _vp, _vp, ctypes.c_int, _vp,
                                   ctypes.c_double, ctypes.c_double, ctypes.c_double, ctypes.c_int, ctypes.c_int,
                                   _vp, ctypes.c_int, ctypes.c_int, _vp]),
+    ("soapgb_ccf_normalise", ctypes.c_int, [_vp, ctypes.c_int, ctypes.c_int, _vp, ctypes.c_int, _vp]),
     ("soapgb_ccf_adjoint", ctypes.c_int, [_vp, ctypes.c_int, _vp, ctypes.c_int, _vp, _vp, ctypes.c_int, _vp,
                                           ctypes.c_double, ctypes.c_double, ctypes.c_double, ctypes.c_int,
                                           ctypes.c_int, _vp, ctypes.c_int, _vp, ctypes.c_int, _vp]),

@@ -379,6 +379,31 @@ extern "C" int soapgb_ccf(soapgb_ctx *ctx, int form, int n_v, const double *vel,
     return SOAPGB_OK;
 }
 
+// the normalised CCFs of raw ones (soapgb_ccf with normalise = 0), as soapgb_ccf forms them
+extern "C" int soapgb_ccf_normalise(soapgb_ctx *ctx, int n_spec, int n_v, const double *raw, int mem, double *ccf_out) {
+    if (!ctx) return SOAPGB_ERR_ARG;
+    const int period = (int)((n_v - 1) / 2.), len_app = (int)(period / 2.);
+    if (n_v < 21 || 2 * len_app != period || n_spec < 0 || (n_spec > 0 && (!raw || !ccf_out)))
+        return set_error(ctx, SOAPGB_ERR_ARG, "soapgb_ccf_normalise: bad arguments (n_v = %d)", n_v);
+    if (n_spec == 0) return SOAPGB_OK;
+    SOAP_DEVICE(ctx);
+    const bool host = (mem == SOAPGB_HOST);
+    const size_t bytes = sizeof(double) * (size_t)n_v * n_spec;
+    Workspace ws(ctx);
+    const int s_out = ws.add(host ? bytes : 0);
+    int rc = ws.commit();
+    if (rc) return rc;
+    double *d = host ? ws.get<double>(s_out) : ccf_out;
+    SOAP_CUDA(ctx, cudaMemcpyAsync(d, raw, bytes, host ? cudaMemcpyHostToDevice : cudaMemcpyDeviceToDevice, ctx->stream));
+    k_ccf_normalise<<<(n_spec + 1) / 2, 64, 0, ctx->stream>>>(n_spec, n_v, d);
+    SOAP_LAUNCHED(ctx);
+    if (host) {
+        SOAP_CUDA(ctx, cudaMemcpyAsync(ccf_out, d, bytes, cudaMemcpyDeviceToHost, ctx->stream));
+        SOAP_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
+    }
+    return SOAPGB_OK;
+}
+
 // ---------------------------------------------------------------------------
 // Adjoint of the CCF (the differentiable form; the reference has no gradient path).
 // The raw CCF is linear in the spectra, ccf[s, v] = sum_p M[v, p] spec[s, p], so its

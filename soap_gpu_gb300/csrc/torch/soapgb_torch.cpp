@@ -244,6 +244,17 @@ Tensor ccf(int64_t h, int64_t form, const Tensor &vel, const Tensor &line_wave, 
     return out;
 }
 
+Tensor ccf_normalise(int64_t h, const Tensor &raw) {
+    c10::cuda::CUDAGuard guard(raw.device());
+    soapgb_ctx *ctx = on_stream(h, raw);
+    TORCH_CHECK(raw.dim() == 2, "soapgb: raw is n_spec x n_v");
+    Tensor out = empty64(raw, {raw.size(0), raw.size(1)});
+    check(ctx, soapgb_ccf_normalise(ctx, (int)raw.size(0), (int)raw.size(1), f64(raw, "raw"), SOAPGB_DEVICE,
+                                    out.data_ptr<double>()),
+          "soapgb_ccf_normalise");
+    return out;
+}
+
 Tensor ccf_adjoint(int64_t h, const Tensor &vel, const Tensor &line_wave, const Tensor &line_weight,
                    const Tensor &wave_trim, double step_size, const Tensor &g_ccf,
                    const std::optional<Tensor> &ccf_raw, bool normalise, double wave_extend, double mask_step,
@@ -346,6 +357,7 @@ TORCH_LIBRARY(soapgb, m) {
           "float step_size, Tensor spectra, bool normalise, float wave_extend, float mask_step, int index_old) "
           "-> Tensor",
           ccf);
+    m.def("ccf_normalise(int ctx, Tensor raw) -> Tensor", ccf_normalise);
     m.def("ccf_adjoint(int ctx, Tensor vel, Tensor line_wave, Tensor line_weight, Tensor wave_trim, "
           "float step_size, Tensor g_ccf, Tensor? ccf_raw, bool normalise, float wave_extend, float mask_step, "
           "int index_old) -> Tensor",

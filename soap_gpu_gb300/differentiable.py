@@ -287,7 +287,7 @@ class NormalisedCcf(torch.autograd.Function):
         c = ops(setup.ctx)
         args = (setup.vel, setup.line_wave, setup.line_weight, setup.wave_trim, setup.step, sp)
         raw = c.ccf("plain64", *args, normalise=False, **setup.kwargs())
-        out = c.ccf("plain64", *args, normalise=True, **setup.kwargs())
+        out = c.ccf_normalise(raw)
         fctx.setup, fctx.raw = setup, raw
         return out
 

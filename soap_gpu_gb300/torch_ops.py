@@ -18,7 +18,8 @@ from ._lib import FORMS, Activity
 
 PATH = os.path.join(os.path.dirname(os.path.abspath(__file__)), "lib", "soapgb_torch.so")
 OPS = ("disk_maps", "quiet_disk", "phase_integrate", "phase_integrate_adjoint", "lower_resolution",
-       "lower_resolution_adjoint", "ccf", "ccf_adjoint", "gauss_bis", "gauss_fit_adjoint", "batch_run", "synchronize")
+       "lower_resolution_adjoint", "ccf", "ccf_normalise", "ccf_adjoint", "gauss_bis", "gauss_fit_adjoint",
+       "batch_run", "synchronize")
 _loaded = False
 
 
@@ -118,6 +119,9 @@ class Ops:
                          float(step_size), _t(spectra.reshape(1, -1) if single else spectra), bool(normalise),
                          float(wave_extend), float(mask_step), int(index_old))
         return out[0] if single else out
+
+    def ccf_normalise(self, raw):
+        return self.o.ccf_normalise(self.h, _t(raw))
 
     def ccf_adjoint(self, vel, line_wave, line_weight, wave_trim, step_size, g_ccf, ccf_raw=None, normalise=True,
                     wave_extend=100.0, mask_step=0.005, index_old=20000):

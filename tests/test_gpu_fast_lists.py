@@ -57,3 +57,21 @@ def test_refined_minimum_is_exact(ctx, n):
     _, mm = ctx.lower_resolution("fast32", wave, spec, n // 512 * 512, sigma_v, base=base, step_mult=step,
                                  step_exp=step)
     assert np.array_equal(np.asarray(mm)[:, 0], (base[None, :] - spec).min(1))
+
+
+@pytest.mark.parametrize("n_spec,n_v", [(1, 21), (5, 81), (40, 161)])
+def test_ccf_normalise(ctx, n_spec, n_v):
+    """The normalised CCFs of raw sums are soapgb_ccf's own, bit for bit."""
+    torch = pytest.importorskip("torch")
+    from soap_gpu_gb300.torch_ops import Ops
+    rng = np.random.default_rng(n_v)
+    dev = lambda a: torch.as_tensor(np.ascontiguousarray(a, dtype=np.float64), device="cuda:0")
+    step, n, mask_step = 0.01, 6000, 0.01
+    wave = 5000.0 + step * np.arange(n)
+    lines = np.sort(rng.uniform(5003.0, 5057.0, 40))
+    args = (dev(np.linspace(-20000.0, 20000.0, n_v)), dev(lines), dev(rng.uniform(0.1, 1.0, 40)), dev(wave), step,
+            dev(1.0 - 0.5 * rng.uniform(0, 1, (n_spec, n))))
+    kw = dict(wave_extend=100.0, mask_step=mask_step, index_old=int(100.0 / step))
+    o = Ops(ctx)
+    raw = o.ccf("plain64", *args, normalise=False, **kw)
+    assert torch.equal(o.ccf_normalise(raw), o.ccf("plain64", *args, normalise=True, **kw))
