@@ -116,14 +116,15 @@ __global__ void __launch_bounds__(256) k_conv_plain64(int n, int n_eff, const do
 // memory for all its spectra.  The spectra's terms step_mult (1 - A) are staged once per block,
 // and the division by s_i sqrt(2 pi) is a soap_quot, so a tap costs two FP64 instructions
 // (product, sum) instead of about 55.
-// Taps with a weight below e^-90 are left out.  That changes no bit of a sum of at least 2^-20 of
+// Taps with a weight below e^-90 are left out.  That changes no bit of a sum of at least 2^-32 of
 // the window's largest term: to the right of the centre a tap stays below a quarter of the sum's
-// ulp; to the left, what the early partial sums lack is rounded away as the weights grow, but for
-// a chance of about 2^-47 per pixel.  A smaller sum (terms of either sign) is taken over all taps
-// by conv_plain64_pixel, and so are the pixels of a block whose window holds zeros, infinities,
-// NaN or values beyond 2^800.  (The test is per pixel: with one on the block's range of terms, the
-// one block at a spectrum's edge where 1 - A changes its sign took 6.4 ms of a call of 11 phases
-// that takes 0.7 ms otherwise.)
+// ulp; to the left, what the early partial sums lack (2^-122 of the largest term) is rounded away
+// as the weights grow, but for a chance of 2^-70 per pixel, 2^-38 for a sum at the bound.  A
+// smaller sum (terms of either sign) is taken over all taps by conv_plain64_pixel, and so are the
+// pixels of a block whose window holds zeros, infinities, NaN or values beyond 2^800.  (The test is
+// per pixel: with one on the block's range of terms, the one block at a spectrum's edge where
+// 1 - A changes its sign took 6.4 ms of a call of 11 phases that takes 0.7 ms otherwise; one pixel
+// over all taps takes 0.35 ms, so the bound lies where next to none is.)
 // Bound by the FP64 pipe: (2 reach + 1) x 2 instructions per pixel and spectrum and
 // (reach + 1) x 20 for the weights per pixel and block.  One spectrum of 310,000 px:
 // 3.28 -> 0.71 ms per call; 10 of 100,000 px: 13.9 -> 0.45 ms.
@@ -208,7 +209,7 @@ __global__ void __launch_bounds__(CP_PIX) k_conv_plain64t(int n, int n_eff, cons
                 for (int d = 0; d <= hi; ++d)
                     acc = __dadd_rn(acc, __dmul_rn(soap_quot(yc[d], by), wt[d * CP_PIX + t]));
                 const int ex = (int)(((unsigned)__double2hiint(acc) >> 20) & 0x7ffu);
-                all_taps = ex + (int)((unsigned)__double2hiint(norm) >> 20) - 1023 < (int)(mx >> 20) - 20;
+                all_taps = ex + (int)((unsigned)__double2hiint(norm) >> 20) - 1023 < (int)(mx >> 20) - 32;
             }
             if (all_taps) acc = conv_plain64_pixel(index, wid, step_mult, step_exp, norm, den, sp, bp);
         }
