@@ -27,6 +27,7 @@
 
 #include "internal.cuh"
 #include "fir.cuh"
+#include "order.cuh"
 #include "planck.cuh"
 
 using namespace soapgb;
@@ -101,6 +102,12 @@ __global__ void k_adj_geo(long long gm, const double *__restrict__ lam, const do
     keys[k] = ((unsigned long long)((unsigned)row < (unsigned)n_mu ? row : 0) << 56) | (soap_ord64(g.f) >> 8);
     vals[k] = (int)k;
 }
+
+// the order's keys, the cell last
+struct AdjKey {
+    const unsigned long long *keys;
+    __device__ __forceinline__ OrderKey operator()(int k) const { return OrderKey{keys[k], (unsigned)k}; }
+};
 
 // One block per phase: the active cells in the map's sorted order, class by class, and the
 // first entry of every row.  A thread takes ADJ_LIST_ITEMS consecutive cells at a time.
@@ -844,7 +851,8 @@ extern "C" int soapgb_phase_integrate_adjoint(soapgb_ctx *ctx, int n, int n_eff,
     int s_key[2], s_val[2];
     for (int q = 0; q < 2; ++q) s_key[q] = ws.add(sizeof(unsigned long long) * gm);
     for (int q = 0; q < 2; ++q) s_val[q] = ws.add(sizeof(int) * gm);
-    const size_t sort_b = fir_sort_temp_bytes(gm);
+    const bool ranks = gm <= ORDER_MAX;
+    const size_t sort_b = ranks ? sizeof(unsigned long long) * gm : fir_sort_temp_bytes(gm);
     int s_sort = ws.add(sort_b);
     int s_cell = ws.add(sizeof(int) * pg), s_fb = ws.add(sizeof(double) * pg), s_pre = ws.add(sizeof(AdjPre) * pg);
     int s_noise = ws.add(sizeof(AdjNoise) * pg);
@@ -951,8 +959,12 @@ extern "C" int soapgb_phase_integrate_adjoint(soapgb_ctx *ctx, int n, int n_eff,
                 gm, d_wave, d_delta, d_limb, d_lb, d_region, n_mu, step, ws.get<AdjGeo>(s_geo),
                 ws.get<unsigned long long>(s_key[0]), ws.get<int>(s_val[0]));
             SOAP_LAUNCHED(ctx);
-            rc = fir_sort_u64(ctx, gm, ws.get<unsigned long long>(s_key[0]), ws.get<unsigned long long>(s_key[1]),
-                              ws.get<int>(s_val[0]), ws.get<int>(s_val[1]), ws.get<void>(s_sort), sort_b);
+            rc = ranks ? order_cells(ctx, gm, AdjKey{ws.get<unsigned long long>(s_key[0])},
+                                     ws.get<unsigned long long>(s_key[1]), ws.get<unsigned long long>(s_sort),
+                                     ws.get<int>(s_val[0]), ws.get<int>(s_val[1]))
+                       : fir_sort_u64(ctx, gm, ws.get<unsigned long long>(s_key[0]),
+                                      ws.get<unsigned long long>(s_key[1]), ws.get<int>(s_val[0]),
+                                      ws.get<int>(s_val[1]), ws.get<void>(s_sort), sort_b);
             if (rc) return rc;
             k_adj_lists<<<n_phase, 1024, 0, ctx->stream>>>(gm, n_mu, ws.get<int>(s_val[1]), d_temp, d_bi, A.geo, d_region,
                                                            act->solar, A.t_norm_fac, ws.get<int>(s_cell),
