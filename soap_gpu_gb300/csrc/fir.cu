@@ -809,7 +809,7 @@ __device__ __forceinline__ void block_scan_excl(double (&v)[NV], int &vi, double
 // segs[(l*2 + c)*cap + s] = (first position, row * 2 + zero_v), nseg[l*2 + c].
 // The FP64 pipe of an SM bounds a block, so class 0 goes without the sums that only class 1
 // is read for and a warp adds the totals of the warps before it only: 12 us against 19 for
-// 15 phases of 100 x 100 cells, 37 against 50 for 100 phases of 300 x 300.
+// 25 phases of 100 x 100 cells, 37 against 50 for 100 phases of 300 x 300.
 template <int NV>
 __device__ __forceinline__ void fir_prefix_class(long long gm, int l, int c, int cs, int cnt,
                                                  const int *__restrict__ list_cell, const CellGeo *__restrict__ geo,
