@@ -30,7 +30,8 @@
 // 31,417 cells x 100,000 px: 306 -> 28 ms; 5 phases of 200x200 and 100,000 px, three regions:
 // 36 -> 6.1 ms.  One pixel per thread: two took 31 ms, and 8.4 against 7.5 ms.  The quiet sum's one
 // product stays on the FP64 pipe: with pl_mul 28.6 ms, two cells at a time 28.0 (219 instructions
-// against 147, of which 3.6 against 4.4 on the FP64 pipe: issue and the chain then bound it).
+// against 147, of which 3.6 against 4.4 on the FP64 pipe: issue and the chain then bound it); and the
+// integration's three rises as integer products too took 6.5 ms against 6.1.
 // What the integers do not cover (another binade, an uneven grid, differences outside the table,
 // non-finite or extreme values) takes the reference's operations.  Every path gives the same bits.
 #pragma once
