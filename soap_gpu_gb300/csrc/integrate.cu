@@ -56,6 +56,25 @@ struct PhaseCell {
     PlainFactor by; // the limb factor
 };
 
+// the record of active cell k of temperature T and type b
+__device__ __forceinline__ PhaseCell phase_cell(int k, double T, double b, const double *__restrict__ lb_m,
+                                                const double *__restrict__ limb_m, int solar, int t_norm_fac) {
+    PhaseCell a;
+    a.k = k;
+    a.type = (b == 0.0) ? 0 : 1;
+    a.scale = 1.0;
+    if (a.type == 0) {
+        a.unit = ((double)(int)T == T) ? 1 : -1;
+    } else if (solar) {
+        a.unit = ((double)t_norm_fac == T) ? 1 : -1;
+    } else {
+        a.unit = 0;
+        a.scale = __dadd_rn(1.0, lb_m[k]);
+    }
+    a.by = pl_factor(limb_m[k]);
+    return a;
+}
+
 // The plain form: block (x, p) sums phase p's active cells, in map order, over a tile of
 // pixels (plain64.cuh); three rows per cell.  INT: the five products of a cell and pixel on the
 // integer pipes (18.4 -> 13 FP64 instructions, 285 -> 440 in all), which pays where the FP64 pipe
@@ -103,20 +122,7 @@ __global__ void __launch_bounds__(PL_THREADS) k_phase_plain64(
                 atomicExch(status, 21);
                 row = 0;
             }
-            PhaseCell a;
-            const double T = pt[k];
-            a.k = k;
-            a.type = (pb[k] == 0.0) ? 0 : 1;
-            a.scale = 1.0;
-            if (a.type == 0) {
-                a.unit = ((double)(int)T == T) ? 1 : -1;
-            } else if (solar) {
-                a.unit = ((double)t_norm_fac == T) ? 1 : -1;
-            } else {
-                a.unit = 0;
-                a.scale = __dadd_rn(1.0, lb_m[k]);
-            }
-            a.by = pl_factor(limb_m[k]);
+            const PhaseCell a = phase_cell(k, pt[k], pb[k], lb_m, limb_m, solar, t_norm_fac);
             s_cell[threadIdx.x] = a;
             pl_stage(geo + k, delta_m[k], limb_m[k], row, j0, cnt, lmid, s_rec[threadIdx.x], s_tab[threadIdx.x]);
         }
@@ -229,6 +235,164 @@ __global__ void __launch_bounds__(PL_THREADS) k_phase_plain64(
     tot[o] = mine ? tt : 0.0;
 }
 
+// The same sums where the blocks are too few to fill the chip: a cell's terms are a chain of some
+// 1000 cycles, which a warp per strip of 31 pixels walks one cell after the other.  Here PS_WARPS
+// warps share a tile: they compute the five terms of a chunk's cells into shared memory, cell by
+// cell from a counter, while one of them per strip adds up the chunk before, in the cells' order
+// (as k_quiet_plain64s).  Two blocks fit an SM: up to there one phase of 200 x 200 cells and 6,000 px
+// takes 371 us against 813, 150 x 150 and 18,800 px 295 against 421; above (2.1 blocks per SM, two
+// waves) 1142 against 1145, at 3.2 692 against 649.
+constexpr long long PS_MAX_PER_SM = 2;   // what an SM holds of it
+constexpr int PS_WARPS = 8, PS_STRIPS = PL_TILE / 31, PS_CHUNK = 16;
+struct PlainPhaseSmem {   // chunks, double buffered
+    double term[2][PS_STRIPS][PS_CHUNK][5][32];   // s, I q, q, v, v I
+    unsigned long long tab[2][PS_CHUNK][PL_TAB];
+    PlainRec rec[2][PS_CHUNK];
+    PhaseCell cell[2][PS_CHUNK];
+    double sum[PS_STRIPS][3][32];
+    int next[2][PS_STRIPS];   // jobs taken in a step, per strip
+};
+
+__global__ void __launch_bounds__(32 * PS_WARPS, 2) k_phase_plain64s(
+    int n, int n_eff, const double *__restrict__ lam, const double *__restrict__ q_norm,
+    const double *__restrict__ q_sed, const double *__restrict__ spot_norm, const double *__restrict__ fac_norm,
+    const double *__restrict__ spot_sed, const double *__restrict__ fac_sed, int max_cells,
+    const int *__restrict__ cells, const int *__restrict__ counts, const double *__restrict__ temp,
+    const double *__restrict__ bi, const PlainGeo *__restrict__ geo, const double *__restrict__ delta_m,
+    const double *__restrict__ limb_m, const double *__restrict__ lb_m, const int *__restrict__ region_m,
+    long long gm, int solar, int t_star, int t_diff_fac, double *__restrict__ flux, double *__restrict__ bconv,
+    double *__restrict__ tot, long long out_stride, int n_mu, int *status) {
+    extern __shared__ __align__(16) unsigned char ps_smem[];
+    PlainPhaseSmem &sh = *reinterpret_cast<PlainPhaseSmem *>(ps_smem);
+    const int p = blockIdx.y, lane = threadIdx.x & 31, warp = threadIdx.x >> 5, strip = warp % PS_STRIPS;
+    const int j0 = blockIdx.x * PL_TILE, j = j0 + strip * 31 + lane;
+    const int cnt = max(1, min(PL_TILE, n_eff - j0));
+    const int *pc = cells + (long long)p * max_cells;
+    const int n_cells = counts[p], n_chunk = (n_cells + PS_CHUNK - 1) / PS_CHUNK;
+    const double *pt = temp + (long long)p * gm;
+    const double *pb = bi + (long long)p * gm;
+    const double lmid = lam[min(j0 + cnt / 2, n_eff - 1)];
+    const int t_norm_fac = (int)(t_star + t_diff_fac + 0.9 - 216.8);
+    const bool mine = j < n_eff && lane != 31;
+    const int jc = min(j, n_eff - 1);
+    const double lj = lam[jc], ssed = spot_sed[jc], fsed = fac_sed[jc];
+    PlainPix px;
+    PlainVal va[3];
+    int row_now = -1, m_now = 0, type_now = 0;
+    auto stage = [&](int c) {   // the records of chunk c, by one warp
+        const int b = c & 1, t = lane;
+        if (t >= min(PS_CHUNK, n_cells - c * PS_CHUNK)) return;
+        const int k = pc[c * PS_CHUNK + t];
+        int row = region_m[k];
+        if ((unsigned)row >= (unsigned)n_mu) {   // mu bin outside the cube: report, use bin 0
+            atomicExch(status, 21);
+            row = 0;
+        }
+        sh.cell[b][t] = phase_cell(k, pt[k], pb[k], lb_m, limb_m, solar, t_norm_fac);
+        pl_stage(geo + k, delta_m[k], limb_m[k], row, j0, cnt, lmid, sh.rec[b][t], sh.tab[b][t]);
+    };
+    auto terms = [&](const PlainRec &c, const PhaseCell &a, const unsigned long long *tab, double(*to)[32]) {
+        const long long off = (long long)c.row * n;
+        const double *an = (a.type == 0 ? spot_norm : fac_norm) + off;
+        double q, s, v;
+        if (c.flags != PL_CONST) {   // the pixel itself, or an owner search per pixel
+            const PlainGeo &g = geo[a.k];
+            CellShift cs;
+            cs.sq = g.sq;
+            cs.fbeta = g.fbeta;
+            cs.off = g.off;
+            const double d = c.flags == PL_STILL ? 0.0 : 1.0;
+            CellAt at;
+            at.i = -1;
+            if (d != 0.0) at = soap_cell_at(jc, n_eff, lam, cs);
+            q = soap_lerp_at(at, jc, q_norm + off, d, c.limb);
+            s = soap_lerp_at(at, jc, q_sed + off, d, c.limb);
+            v = soap_lerp_at(at, jc, an, d, c.limb);
+        } else {
+            if (c.row != row_now || c.m != m_now || a.type != type_now) {
+                row_now = c.row;
+                m_now = c.m;
+                type_now = a.type;
+                const int i = min(max(j + c.m, 0), n_eff - 1), i1 = min(i + 1, n_eff - 1);
+                px.li = lam[i];
+                px.lm = soap_sig(px.li);
+                const bool ok0 = pl_load(va[0], q_norm + off, i, i1), ok1 = pl_load(va[1], q_sed + off, i, i1);
+                px.ok = pl_load(va[2], an, i, i1) && ok0 && ok1;
+            }
+            const double ls = pl_shifted(c, px), ls1 = __shfl_down_sync(0xffffffffu, ls, 1);
+            // lanes without a pixel here must not send their warp the other way
+            const bool in = mine && (unsigned)(j + c.m) <= (unsigned)(n_eff - 2);
+            int k;
+            double X, x[3];
+            if ((pl_interval(c, lj, ls, ls1, k, X) && px.ok) || !in) {
+                const unsigned long long rec = tab[k];
+#pragma unroll
+                for (int r = 0; r < 3; ++r) x[r] = pl_rise(c, va[r], rec, k, X);
+            } else {
+#pragma unroll
+                for (int r = 0; r < 3; ++r) x[r] = pl_rise_plain(va[r].g, lj, ls, ls1);
+            }
+#pragma unroll
+            for (int r = 0; r < 3; ++r) x[r] = __dmul_rn(__dadd_rn(va[r].s0, x[r]), c.limb);
+            q = in ? x[0] : 0.0;
+            s = in ? x[1] : 0.0;
+            v = in ? x[2] : 0.0;
+        }
+        double I = a.type == 0 ? ssed : fsed;
+        if (a.unit == 0) I = __dmul_rn(a.scale, I);
+        else if (a.unit < 0) I = soap_intensity(a.type, pt[a.k], lb_m[a.k], lj, ssed, fsed, solar, t_norm_fac);
+        to[0][lane] = s;
+        to[1][lane] = __dmul_rn(I, q);
+        to[2][lane] = q;
+        to[3][lane] = v;
+        to[4][lane] = __dmul_rn(v, I);
+    };
+    if (warp < PS_STRIPS)
+        for (int q = 0; q < 3; ++q) sh.sum[warp][q][lane] = 0.0;
+    if (threadIdx.x < PS_STRIPS) sh.next[0][threadIdx.x] = 0;
+    if (warp == 0) stage(0);
+    // step c: the sums over chunk c - 1, the records of chunk c + 1 (strip 0), the terms of chunk c
+    for (int c = 0; c <= n_chunk; ++c) {
+        __syncthreads();
+        const int b = c & 1;
+        if (threadIdx.x < PS_STRIPS) sh.next[b ^ 1][threadIdx.x] = 0;
+        const int nt = c < n_chunk ? min(PS_CHUNK, n_cells - c * PS_CHUNK) : 0;
+        while (true) {
+            int job = 0;
+            if (lane == 0) job = atomicAdd(&sh.next[b][strip], 1);
+            job = __shfl_sync(0xffffffffu, job, 0);
+            if (job >= nt + 2) break;
+            if (job == 0) {
+                if (c == 0) continue;
+                const int np = min(PS_CHUNK, n_cells - (c - 1) * PS_CHUNK);
+                double fx = sh.sum[strip][0][lane], bc = sh.sum[strip][1][lane], tt = sh.sum[strip][2][lane];
+#pragma unroll 2
+                for (int t = 0; t < np; ++t) {
+                    const double(*x)[32] = sh.term[b ^ 1][strip][t];
+                    fx = __dsub_rn(__dadd_rn(fx, x[0][lane]), x[1][lane]);
+                    bc = __dsub_rn(__dadd_rn(bc, x[2][lane]), x[3][lane]);
+                    tt = __dsub_rn(__dadd_rn(tt, x[0][lane]), x[4][lane]);
+                }
+                sh.sum[strip][0][lane] = fx;
+                sh.sum[strip][1][lane] = bc;
+                sh.sum[strip][2][lane] = tt;
+            } else if (job == 1) {
+                if (strip == 0 && c + 1 < n_chunk) stage(c + 1);
+            } else {
+                const int t = job - 2;
+                const PlainRec r = sh.rec[b][t];
+                terms(r, sh.cell[b][t], sh.tab[b][t], sh.term[b][strip][t]);
+            }
+        }
+    }
+    __syncthreads();
+    if (warp >= PS_STRIPS || lane == 31 || j >= n) return;
+    const long long o = (long long)p * out_stride + j;
+    flux[o] = mine ? sh.sum[strip][0][lane] : 0.0;
+    bconv[o] = mine ? sh.sum[strip][1][lane] : 0.0;
+    tot[o] = mine ? sh.sum[strip][2][lane] : 0.0;
+}
+
 // float -> double copy without FP64 instructions
 __global__ void k_f32_widen(long long count, const float *__restrict__ a, double *__restrict__ out) {
     long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
@@ -255,8 +419,15 @@ int integrate_device(soapgb_ctx *ctx, int form, int n, int n_eff, const double *
         rc = plain_cells(ctx, gm, n_eff, d_wave, dm.delta, step, geo);
         if (rc) return rc;
         const dim3 g((n + PL_TILE - 1) / PL_TILE, n_phase);
-        const auto kern = (long long)g.x * g.y >= 6LL * ctx->num_sms ? k_phase_plain64<true> : k_phase_plain64<false>;
-        SOAP_TRACED(ctx, "integrate_plain64", kern<<<g, PL_THREADS, 0, ctx->stream>>>(
+        const long long blocks = (long long)g.x * g.y;
+        const bool few = blocks <= PS_MAX_PER_SM * ctx->num_sms;
+        const auto kern = few ? k_phase_plain64s
+                              : blocks >= 6LL * ctx->num_sms ? k_phase_plain64<true> : k_phase_plain64<false>;
+        const int threads = few ? 32 * PS_WARPS : PL_THREADS;
+        const size_t smem = few ? sizeof(PlainPhaseSmem) : 0;
+        if (few)
+            SOAP_CUDA(ctx, cudaFuncSetAttribute(k_phase_plain64s, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        SOAP_TRACED(ctx, "integrate_plain64", kern<<<g, threads, smem, ctx->stream>>>(
             n, n_eff, d_wave, dc.q_norm, dc.q_sed, dc.spot_norm, dc.fac_norm, dc.spot_sed, dc.fac_sed, (int)gm,
             d_cells, d_counts, d_temp, d_bi, geo, dm.delta, dm.limb, dm.lb, dm.region, gm, act->solar,
             act->t_star, act->t_diff_fac, (double *)d_flux, (double *)d_bconv, (double *)d_tot, out_stride, dc.n_mu,
