@@ -1887,7 +1887,9 @@ __global__ void __launch_bounds__(256) k_radj_spect(int n, int n_eff, int n_spec
     }
     const bool odd_block = __syncthreads_or(odd ? 1 : 0) != 0;
     const int s1 = min(n_spec, (int)(blockIdx.y + 1) * per);
-    const int down = min(reach, wid - 2), up = min(reach, wid);   // i = m - down .. m + up
+    // i = m - down .. m - 1 and m + first .. m + up: the window m - wid + 2 .. m + wid, which for a
+    // half width of one pixel does not hold m itself
+    const int down = min(reach, wid - 2), first = max(0, 2 - wid), up = min(reach, wid);
     for (int s = blockIdx.y * per; s < s1; ++s) {
         const double f = par[3 * s], dmx = par[3 * s + 2];
         const int imax = idx[2 * s + 1];
@@ -1912,7 +1914,7 @@ __global__ void __launch_bounds__(256) k_radj_spect(int n, int n_eff, int n_spec
             } else {
                 const int x = t + reach;
                 for (int d = down; d > 0; --d) acc = fma(wt[d * win + x - d], gs[x - d], acc);
-                for (int d = 0; d <= up; ++d) acc = fma(wt[d * win + x + d], gs[x + d], acc);
+                for (int d = first; d <= up; ++d) acc = fma(wt[d * win + x + d], gs[x + d], acc);
             }
             const double ga = (m == idx[2 * s] ? par[3 * s + 1] : 0.0) - acc;
             grad_spec[(long long)s * n + m] = has_base ? -ga : ga;

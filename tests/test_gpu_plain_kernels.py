@@ -290,3 +290,49 @@ def test_plain_convolution_of_small_sums(ctx, n, n_spec, top):
         ref, _, ext = oracle.lower_resolution(wave, base - (base - a[s]), n_eff, sv, step_mult=step, step_exp=step)
         assert np.max(np.abs(got[s] - ref)) <= 1e-12 * np.max(np.abs(ref))
         assert np.allclose(mm[s], ext, rtol=1e-12, atol=0)
+
+
+def _transposed_taps(wave, A, conv, mn, mx, g, n_eff, sv, wid, step):
+    """The resolution gradient d out / d A against g over the whole reference window."""
+    n = wave.size
+    b = sv / C
+    sig = -1 * wave[:n_eff] * (1 - np.sqrt((1 + b) / (1 - b)))
+    i = np.arange(n_eff)
+    inside = (i > wid) & (i + wid < n - 1)
+    S = (g * conv).sum()
+    gc = -(1 - mn) / mx * g
+    gc[np.argmax(np.where(conv != 0, conv, -np.inf))] += S * (1 - mn) / mx ** 2
+    ref = np.zeros(n)
+    ref[np.argmin(A)] += S / mx
+    for d in range(-wid, wid - 1):
+        k = np.where(inside, step * np.exp(-d * d * step * step / (2 * sig * sig)) / (sig * np.sqrt(2 * np.pi)), 0)
+        lo, hi = max(0, -d), min(n_eff, n - d)
+        ref[lo + d:hi + d] -= (k * gc)[lo:hi]
+    return ref, max(np.abs(gc).max(), abs(S / mx))
+
+
+# the window is m - i = -wid .. wid - 2: without the central tap for wid = 1, without the upper one for wid = 2
+@pytest.mark.parametrize("wid,window,step", [(1, 0.55, 0.01), (2, 1.1, 0.01), (3, 1.65, 0.01), (1, 50.0, 1.0)])
+def test_resolution_of_narrow_windows(ctx, wid, window, step):
+    """Forward and gradient of half widths of one to three pixels, with a base and without, against the
+    oracle and the transposed taps in numpy (tolerances of the two tests above)."""
+    n, n_eff, n_spec = 1100, 1024, 3
+    rng = np.random.default_rng(wid)
+    wave = 5000.0 + step * np.arange(n)
+    sv = _sigma_v(115000.0)
+    assert oracle.conv_halfwidth(wave, sv, window) == wid
+    a = _spectra("disk", n, n_eff, n_spec, rng)
+    base = a[0] * 1.5
+    g = rng.standard_normal((n_spec, n_eff))
+    kw = dict(window=window, step_mult=step, step_exp=step)
+    for b in (base, None):
+        spec = a if b is None else b[None, :] - a
+        got, mm = ctx.lower_resolution("plain64", wave, spec, n_eff, sv, base=b, **kw)
+        gs = ctx.lower_resolution_adjoint(wave, spec, n_eff, sv, g, base=b, **kw)[0]
+        for s in range(n_spec):
+            A = spec[s] if b is None else b - spec[s]
+            ref, conv, (mn, mx) = oracle.lower_resolution(wave, A, n_eff, sv, **kw)
+            assert np.allclose(mm[s], (mn, mx), rtol=1e-12, atol=0)
+            assert np.max(np.abs(got[s] - ref)) <= 1e-12 * np.max(np.abs(ref))
+            want, scale = _transposed_taps(wave, A, conv, mn, mx, g[s].copy(), n_eff, sv, wid, step)
+            assert np.max(np.abs((gs[s] if b is None else -gs[s]) - want)) <= 1e-11 * scale
