@@ -1881,10 +1881,16 @@ __global__ void __launch_bounds__(256) k_radj_spect(int n, int n_eff, int n_spec
     for (int x = t; x < win; x += T) {
         const int i = ib + x;
         const double k = i >= 0 && i < n_eff ? kq[i] : 0.0, c = k != 0.0 ? cq[i] : 0.0;
-        // the first weight beyond the table must be below the cut
-        if (k != 0.0 && reach < wid) odd |= !((double)(reach + 1) * (double)(reach + 1) * c > CP_CUT);
         for (int d = 0; d <= reach; ++d) wt[d * win + x] = k != 0.0 ? k * exp(-(double)(d * d) * c) : 0.0;
     }
+    // the first weight beyond the table must be below the cut, for every i of the reference's window
+    // (wavelengths need not ascend)
+    if (reach < wid)
+        for (int x = t - (wid - reach); x < win + wid - reach; x += T) {
+            const int i = ib + x;
+            if (i >= 0 && i < n_eff && kq[i] != 0.0)
+                odd |= !((double)(reach + 1) * (double)(reach + 1) * cq[i] > CP_CUT) || !isfinite(kq[i]);
+        }
     const bool odd_block = __syncthreads_or(odd ? 1 : 0) != 0;
     const int s1 = min(n_spec, (int)(blockIdx.y + 1) * per);
     // i = m - down .. m - 1 and m + first .. m + up: the window m - wid + 2 .. m + wid, which for a

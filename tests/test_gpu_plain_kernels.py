@@ -336,3 +336,26 @@ def test_resolution_of_narrow_windows(ctx, wid, window, step):
             assert np.max(np.abs(got[s] - ref)) <= 1e-12 * np.max(np.abs(ref))
             want, scale = _transposed_taps(wave, A, conv, mn, mx, g[s].copy(), n_eff, sv, wid, step)
             assert np.max(np.abs((gs[s] if b is None else -gs[s]) - want)) <= 1e-11 * scale
+
+
+@pytest.mark.parametrize("factor", [2.5, 3.5])
+def test_resolution_of_wavelengths_that_do_not_ascend(ctx, factor):
+    """Pixels in the middle whose Gaussian is wider than at both ends of the grid: their taps reach
+    further than the ends' (tolerances as above)."""
+    n, n_eff, n_spec, step = 1900, 1536, 2, 0.01
+    rng = np.random.default_rng(7)
+    wave = 5000.0 + step * np.arange(n)
+    wave[[700, 701, 900]] *= factor
+    sv = _sigma_v(115000.0)
+    wid = oracle.conv_halfwidth(wave, sv, 50.0)
+    a = _spectra("disk", n, n_eff, n_spec, rng)
+    g = rng.standard_normal((n_spec, n_eff))
+    g[:, [700, 701, 900]] *= 1e6     # their far taps stand out
+    kw = dict(step_mult=step, step_exp=step)
+    got, mm = ctx.lower_resolution("plain64", wave, a, n_eff, sv, **kw)
+    gs = ctx.lower_resolution_adjoint(wave, a, n_eff, sv, g, **kw)[0]
+    for s in range(n_spec):
+        ref, conv, (mn, mx) = oracle.lower_resolution(wave, a[s], n_eff, sv, **kw)
+        assert np.max(np.abs(got[s] - ref)) <= 1e-12 * np.max(np.abs(ref))
+        want, scale = _transposed_taps(wave, a[s], conv, mn, mx, g[s].copy(), n_eff, sv, wid, step)
+        assert np.max(np.abs(gs[s] - want)) <= 1e-11 * scale
