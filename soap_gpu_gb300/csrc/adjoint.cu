@@ -277,8 +277,9 @@ __global__ void k_adj_inv(int n_eff, const double *__restrict__ lam, double *__r
 
 // ---- ranges ----------------------------------------------------------------------------
 // Integer boundaries B of one row of a class at a tile, B0, B0 + 1, ...: entries [lo, hi) may
-// cross B inside the tile; those between hi of B and lo of B + 1 have the offset c = B + 1 (owner
-// o of pixel j = o + c) at every pixel.  A cell's position there is v = f p (source pixels,
+// cross B inside the tile (a fast cell may cross the next ones too: lo of B + 1 then lies below hi of
+// B); those between hi of B and lo of B + 1 have the offset c = B + 1 (owner o of pixel j = o + c) at
+// every pixel.  A cell's position there is v = f p (source pixels,
 // p = o + lambda0 / step) or f p / S (output pixels, p = j + lambda0 / step), ascending in f; the
 // margin eps covers the rounding of the reference's positions.
 struct AdjRange {
@@ -367,6 +368,7 @@ __device__ __forceinline__ void adj_walk(const AdjArgs &A, int p, int c, int b, 
         if (z.x < z.y) still(z.x, z.y);
         return;
     }
+    int done = a;   // entries below it are evaluated
     for (long long first = R.b0;; first += ADJ_NB - 1) {
         const int count = (int)min((long long)ADJ_NB, b1 - first + 1);
         __syncthreads();
@@ -374,9 +376,11 @@ __device__ __forceinline__ void adj_walk(const AdjArgs &A, int p, int c, int b, 
         __syncthreads();
         for (int k = 0; k < count; ++k) {
             if (k + 1 < count && R.hi[k] < R.lo[k + 1]) group((int)(first + k + 1), R.hi[k], R.lo[k + 1]);
-            if (k + 1 < count || first + k == b1)   // a boundary shared by two batches once
-                for (int q = R.lo[k]; q < R.hi[k]; ++q)
+            if (k + 1 < count || first + k == b1) {   // a boundary shared by two batches once
+                for (int q = max(R.lo[k], done); q < R.hi[k]; ++q)
                     if (q < z.x || q >= z.y) single(q);
+                done = max(done, R.hi[k]);
+            }
         }
         if (first + count - 1 >= b1) break;
     }
