@@ -331,7 +331,7 @@ def test_resolution_of_narrow_windows(ctx, wid, window, step):
         gs = ctx.lower_resolution_adjoint(wave, spec, n_eff, sv, g, base=b, **kw)[0]
         for s in range(n_spec):
             A = spec[s] if b is None else b - spec[s]
-            ref, conv, (mn, mx) = oracle.lower_resolution(wave, A, n_eff, sv, **kw)
+            ref, conv, (mn, mx) = oracle.lower_resolution(wave, A, n_eff, sv, window, step, step)
             assert np.allclose(mm[s], (mn, mx), rtol=1e-12, atol=0)
             assert np.max(np.abs(got[s] - ref)) <= 1e-12 * np.max(np.abs(ref))
             want, scale = _transposed_taps(wave, A, conv, mn, mx, g[s].copy(), n_eff, sv, wid, step)
@@ -341,16 +341,18 @@ def test_resolution_of_narrow_windows(ctx, wid, window, step):
 @pytest.mark.parametrize("factor", [2.5, 3.5])
 def test_resolution_of_wavelengths_that_do_not_ascend(ctx, factor):
     """Pixels in the middle whose Gaussian is wider than at both ends of the grid: their taps reach
-    further than the ends' (tolerances as above)."""
+    further than the ends', also into blocks of pixels that the ends' reach from them does not touch
+    (tolerances as above)."""
     n, n_eff, n_spec, step = 1900, 1536, 2, 0.01
+    wide = [700, 740, 741, 1310]
     rng = np.random.default_rng(7)
     wave = 5000.0 + step * np.arange(n)
-    wave[[700, 701, 900]] *= factor
+    wave[wide] *= factor
     sv = _sigma_v(115000.0)
     wid = oracle.conv_halfwidth(wave, sv, 50.0)
     a = _spectra("disk", n, n_eff, n_spec, rng)
     g = rng.standard_normal((n_spec, n_eff))
-    g[:, [700, 701, 900]] *= 1e6     # their far taps stand out
+    g[:, wide] *= 1e6                # their far taps stand out
     kw = dict(step_mult=step, step_exp=step)
     got, mm = ctx.lower_resolution("plain64", wave, a, n_eff, sv, **kw)
     gs = ctx.lower_resolution_adjoint(wave, a, n_eff, sv, g, **kw)[0]
