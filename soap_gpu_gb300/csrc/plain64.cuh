@@ -16,7 +16,8 @@
 //    S[i+1] - S[i] and l_i stay in registers;
 //  - l'_i.  In units of ulp(l), l_i is a 53-bit integer and l_i u a product of two integers with
 //    21 fraction bits kept; it is subtracted rounded to an integer unless its fraction is so near
-//    to one half that the reference's two roundings could go the other way (FP64 then).  l'_{i+1}
+//    to one half that the reference's two roundings could go the other way, or the result lies at
+//    the binade's lower end, below which the reference rounds to half an ulp (FP64 then).  l'_{i+1}
 //    is the next lane's l'_i (a shuffle), a warp's last one serving only for this;
 //  - the division.  On a grid of constant step l'_{i+1} - l'_i is one of a few neighbouring
 //    integers in units of ulp: the cell's table holds the 64-bit reciprocals of eight of them for
@@ -203,7 +204,10 @@ __device__ __forceinline__ double pl_shifted(const PlainRec &c, const PlainPix &
     const long long r = (long long)((v + (1ULL << (PL_FRAC - 1))) >> PL_FRAC);
     const long long b = __double_as_longlong(x.li);
     double ls = __longlong_as_double(__double2hiint(c.u) < 0 ? b + r : b - r);
-    const bool whole = fr > 2u * (unsigned)c.zone && pl_exp(x.li) == c.ex && pl_exp(ls) == c.ex;
+    // inside the binade: at and just above its power of two (2^32 ulp) the reference's difference may
+    // lie below, where it rounds to half an ulp
+    const bool inside = (unsigned)__double2hiint(ls) - ((unsigned)c.ex << 20) - 1u < 0xfffffu;
+    const bool whole = fr > 2u * (unsigned)c.zone && pl_exp(x.li) == c.ex && inside;
     if (!whole) ls = pl_shifted_plain(x.li, c.u);
     return ls;
 }

@@ -361,3 +361,52 @@ def test_resolution_of_wavelengths_that_do_not_ascend(ctx, factor):
         assert np.max(np.abs(got[s] - ref)) <= 1e-12 * np.max(np.abs(ref))
         want, scale = _transposed_taps(wave, a[s], conv, mn, mx, g[s].copy(), n_eff, sv, wid, step)
         assert np.max(np.abs(gs[s] - want)) <= 1e-11 * scale
+
+
+def _power_of_two_hits(rng, count):
+    """(delta, lambda) whose shifted wavelength is 2^12 when l u is rounded to whole ulps of lambda, and
+    half an ulp below in the reference's operations, which round finer there."""
+    hits = []
+    while len(hits) < count:
+        d = -rng.uniform(1.0, 60.0)            # l' below l: the cell's u is positive
+        b = d * 1000. / C
+        u = 1 - np.sqrt((1 + b) / (1 - b))
+        l0 = 4096.0 / (1 - u)
+        for k in range(-3, 4):
+            l = l0 + k * 2.0 ** -40
+            t = int(l * 2 ** 40) * int(u * 2 ** 53)               # l u in units of ulp(l) 2^-53
+            whole = int(l * 2 ** 40) - ((t + (1 << 52)) >> 53)
+            ref = l + (-1.0 * l) * u
+            if whole == 2 ** 52 and ref < 4096.0:
+                hits.append((d, l))
+                break
+    return hits
+
+
+@pytest.mark.parametrize("n", [700, 62 * 608 + 90])
+def test_shifted_wavelengths_at_a_power_of_two(ctx, n):
+    """Sources whose shifted wavelength comes to exactly 2^12: the sums stay the oracle's, bit for bit
+    (the quiet sum and the integration, with few tiles and with many)."""
+    from soap_gpu_gb300._lib import Activity
+    rng = np.random.default_rng(12)
+    step, n_mu, grid, at = 0.01, 2, 2, n // 2
+    names = ("q_norm", "q_sed", "spot_norm", "fac_norm")
+    for d, l in _power_of_two_hits(rng, 6):
+        at -= (at - int(round((l - 4096.0) / step))) % 62 - 5    # early in a tile, whose middle lies above 2^12
+        wave = l + step * (np.arange(n) - at)
+        maps = dict(delta=np.array([d, -999.0, d, -999.0]), limb=np.array([0.9, -999.0, 0.7, -999.0]),
+                    mu=np.array([0.9, -999.0, 0.6, -999.0]), lb=np.array([0.1, -999.0, 0.2, -999.0]),
+                    region=np.array([0, 0, 1, 0], np.int32))
+        cube = [1.0 + 0.5 * rng.uniform(-1, 1, (n_mu, n)) for _ in range(4)]
+        sed = 0.3 + 0.1 * np.arange(n) / n, 1.0 + 0.1 * np.arange(n) / n
+        ref = oracle.quiet_disk(wave, cube[0], n, maps, grid, step)
+        assert np.array_equal(ctx.quiet_disk("plain64", wave, cube[0], n, maps, grid, step), ref)
+        bi = np.array([0.0, -9999.0, 1.0, -9999.0])
+        temp = np.array([5115.0, -9999.0, 5900.0, -9999.0])
+        want = oracle.phase_integrate(wave, n, grid, temp, bi, maps, *cube, *sed, step)
+        for n_phase in (1, 2):
+            out = ctx.phase_integrate("plain64", wave, n, grid, np.tile(temp, (n_phase, 1)), np.tile(bi, (n_phase, 1)),
+                                      maps, dict(zip(names, cube), spot_sed=sed[0], fac_sed=sed[1]), step,
+                                      Activity(5778, 663, 250, 20, 0))
+            for o, r in zip(out, want):
+                assert all(np.array_equal(v, r) for v in o)
