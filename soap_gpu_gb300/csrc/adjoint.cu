@@ -13,12 +13,16 @@
 //   limb and velocity, per cell: the sum over j of (its unit-L values) . h and of their
 //     derivatives in w times dw/ddelta.
 // The spots share I, the faculae's I is (1 + LB) x the row, so for all cells of one row and class
-// that have the same owner offset over a tile of pixels each of these sums needs only the cells'
-// sums of L, L / S and L f / S (and (1 + LB) times them), and the limb gradients of the cells only
-// three sums over the tile's pixels.  Cells of a row sorted by f have their offsets in ascending
-// ranges, so the sums come from prefix sums and a tile finds its ranges by binary search.  Cells
-// whose offset changes inside the tile (|v|/c x tile pixels of them) and cells with a Planck ratio
-// are evaluated one by one.  Every sum runs in a fixed order, without atomics.
+// that have the same owner offset over a tile of pixels each of these sums needs only a few sums over
+// the cells, and the limb gradients of the cells only three sums over the tile's pixels.  With f0 a
+// shift of the range (its first cell's),
+//   sum L w = inv[o] ((l_j - l_o - l_o f0) sum L / S  -  l_o sum (L / S) (f - f0)),
+// in which every term is of the size of a weight: in sums of L f / S itself the offset, up to tens of
+// pixels, cancels, and differences of prefix sums over a row carry the whole row's rounding (1e-13 of
+// a range's weight; summed per tile and centred it is the rounding of single cells, 2e-16).  Cells of
+// a row sorted by f have their offsets in ascending ranges, which a tile finds by binary search.
+// Cells whose offset changes inside the tile (|v|/c x tile pixels of them) and cells with a Planck
+// ratio are evaluated one by one.  Every sum runs in a fixed order, without atomics.
 //
 // A pixel, cell and phase took about 150 FP64 instructions on a pipe that issues two lanes per
 // cycle; a pixel and range of cells takes 20 to 40.
@@ -41,18 +45,31 @@ constexpr int ADJ_FRAC = 21;         // fraction bits of l u
 constexpr int ADJ_CLASS = 3;         // 0 spot, 1 facula, 2 evaluated one by one (Planck ratio, extreme velocity)
 
 struct AdjGeo {
-    double f, off, iS, e;   // S - 1, f lambda0 / step, 1 / S, f / S
+    double f, off, iS, a;   // S - 1, f lambda0 / step, 1 / S, L / S
     double K, L, sig;       // velocity factor, limb, 1 + LB
     double still;           // 1 for v == 0
 };
+// an entry's weights for the sums over a range
+struct AdjEnt {
+    double L, a, sig;       // as AdjGeo
+};
 // for the rounding of the forward's shifted wavelengths (see adj_residue)
 struct AdjNoise {
-    unsigned long long w;   // |1 - S| 2^(53 + ADJ_FRAC), 0 beyond 2^-10
-    float a, as;            // L / S, negative for S > 1, and (1 + LB) times it
+    unsigned long long w;   // |1 - S| 2^(53 + ADJ_FRAC)
+    int a, as;              // L / S, negative for S > 1, and (1 + LB) times it, in units of AdjRow's
 };
-struct AdjPre {
-    double s0, s1, s2;      // sums of L, L / S, L f / S over the row's cells up to this one
-    double t0, t1, t2;      // the same with (1 + LB) L
+// a row of a class
+struct AdjRow {
+    int2 zero;              // its entries with f == 0
+    double s0, t0;          // their sums of L and (1 + LB) L
+    double still0, still1;  // those with v == 0 alone
+    double unit, unit_s;    // of AdjNoise's a, as, times 2^-ADJ_FRAC
+    int even;               // the weights but zero lie within 2^13: 2^-31 of the largest, of half an
+                            // ulp, is then below a weight's rounding
+};
+// sums over a range's cells, f0 its first cell's f: of L, L / S, (L / S) (f - f0), and with (1 + LB) L
+struct AdjSums {
+    double f0, s0, s1, s2, t0, t1, t2;
 };
 
 struct AdjArgs {
@@ -68,10 +85,10 @@ struct AdjArgs {
     // per phase gm entries: the active cells by class, row, f
     const int *cell;
     const double *fb;
-    const AdjPre *pre;
+    const AdjEnt *ent;
     const AdjNoise *noise;
     const int *seg;     // [phase][class][n_mu + 1] first entry of each row
-    const int2 *zero;   // [phase][2][n_mu] the row's entries with f == 0
+    const AdjRow *row;  // [phase][2][n_mu]
     double *acc;        // [Q][phase][gm][2] limb and velocity sums per entry
     double *part;       // [n_mu][2][n] continuum sums per row
     double *d_qn, *d_qs, *d_sn, *d_fn;
@@ -91,9 +108,9 @@ __global__ void k_adj_geo(long long gm, const double *__restrict__ lam, const do
     g.f = cs.fbeta + 0.0;   // +0 for no shift
     g.off = cs.off;
     g.iS = 1.0 / cs.sq;
-    g.e = g.f * g.iS;
     g.K = (1000. / SOAP_C_LIGHT) / (cs.sq * cs.sq * cs.sq * omb * omb);
     g.L = limb_m[k];
+    g.a = g.L * g.iS;
     g.sig = __dadd_rn(1.0, lb_m[k]);
     g.still = d == 0.0 ? 1.0 : 0.0;
     geo[k] = g;
@@ -205,19 +222,25 @@ __global__ void __launch_bounds__(1024) k_adj_lists(long long gm, int n_mu, cons
     }
 }
 
-// inclusive prefix sums of one row of a class (block: row, class, phase) and its entries with f == 0
-__global__ void __launch_bounds__(ADJ_THREADS) k_adj_prefix(long long gm, int n_mu, const int *__restrict__ cell,
-                                                            const double *__restrict__ fb,
-                                                            const int *__restrict__ seg,
-                                                            const AdjGeo *__restrict__ geo, AdjPre *__restrict__ pre,
-                                                            AdjNoise *__restrict__ noise, int2 *__restrict__ zero) {
-    __shared__ double s_tot[6][ADJ_THREADS];
-    const int b = blockIdx.x, c = blockIdx.y, p = blockIdx.z, t = threadIdx.x;
+constexpr double ADJ_W_MAX = 0x1p-10;   // |f| whose residues adj_residue takes
+
+// a row of a class (block: row, class, phase): its entries' weights and AdjRow
+__global__ void __launch_bounds__(ADJ_THREADS) k_adj_entries(long long gm, int n_mu, const int *__restrict__ cell,
+                                                             const double *__restrict__ fb,
+                                                             const int *__restrict__ seg,
+                                                             const AdjGeo *__restrict__ geo, AdjEnt *__restrict__ ent,
+                                                             AdjNoise *__restrict__ noise, AdjRow *__restrict__ row) {
+    __shared__ int2 s_z;
+    __shared__ unsigned long long s_top[2], s_low[2];
+    __shared__ double s_v[ADJ_THREADS / 32][4];
+    const int b = blockIdx.x, c = blockIdx.y, p = blockIdx.z, t = threadIdx.x, lane = t & 31, w = t >> 5;
     const int *sg = seg + ((long long)p * ADJ_CLASS + c) * (n_mu + 1);
     const int a = sg[b], e = sg[b + 1];
     const int *pc = cell + (long long)p * gm;
     const double *pf = fb + (long long)p * gm;
-    AdjPre *pp = pre + (long long)p * gm;
+    AdjEnt *pe = ent + (long long)p * gm;
+    AdjNoise *pn = noise + (long long)p * gm;
+    if (a == e) return;   // (nothing reads its AdjRow)
     if (t < 2) {   // first entry with f >= 0, first with f > 0
         int lo = a, hi = e;
         while (lo < hi) {
@@ -225,47 +248,77 @@ __global__ void __launch_bounds__(ADJ_THREADS) k_adj_prefix(long long gm, int n_
             if (t == 0 ? pf[mid] < 0.0 : pf[mid] <= 0.0) lo = mid + 1;
             else hi = mid;
         }
-        int *z = reinterpret_cast<int *>(zero + ((long long)p * 2 + c) * n_mu + b);
-        z[t] = lo;
+        (t == 0 ? s_z.x : s_z.y) = lo;
+        s_top[t] = 0ULL;
+        s_low[t] = ~0ULL;
     }
-    if (a == e) return;
-    const int per = (e - a + ADJ_THREADS - 1) / ADJ_THREADS, k0 = min(a + t * per, e), k1 = min(k0 + per, e);
-    double v[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
-    auto add = [&](int k) {
+    __syncthreads();
+    // the sums of the entries without a shift, and the largest and smallest finite weights but zero
+    double v[4] = {0.0, 0.0, 0.0, 0.0};
+    unsigned long long top[2] = {0ULL, 0ULL}, low[2] = {~0ULL, ~0ULL};
+    for (int k = a + t; k < e; k += ADJ_THREADS) {
         const AdjGeo &g = geo[pc[k]];
-        const double s = c == 0 ? 1.0 : g.sig, Ls = g.L * s;
+        const double s = c == 0 ? 1.0 : g.sig, x[2] = {fabs(g.a), fabs(g.a * s)};
+        pe[k] = {g.L, g.a, g.sig};
+#pragma unroll
+        for (int q = 0; q < 2; ++q)
+            if (x[q] > 0.0 && x[q] < INFINITY) {
+                top[q] = max(top[q], (unsigned long long)__double_as_longlong(x[q]));
+                low[q] = min(low[q], (unsigned long long)__double_as_longlong(x[q]));
+            }
+        if (k < s_z.x || k >= s_z.y) continue;
         v[0] += g.L;
-        v[1] = fma(g.L, g.iS, v[1]);
-        v[2] = fma(g.L, g.e, v[2]);
-        v[3] += Ls;
-        v[4] = fma(Ls, g.iS, v[4]);
-        v[5] = fma(Ls, g.e, v[5]);
-    };
-    for (int k = k0; k < k1; ++k) add(k);
+        v[1] = fma(g.L, s, v[1]);
+        v[2] = fma(g.still, g.L, v[2]);
+        v[3] = fma(g.still, g.L * s, v[3]);
+    }
 #pragma unroll
-    for (int q = 0; q < 6; ++q) s_tot[q][t] = v[q];
-    __syncthreads();
-    if (t < 6) {   // the threads' totals in order
-        double s = 0.0;
-        for (int k = 0; k < ADJ_THREADS; ++k) {
-            const double x = s_tot[t][k];
-            s_tot[t][k] = s;
-            s += x;
+    for (int q = 0; q < 2; ++q)
+        if (top[q] != 0ULL) {
+            atomicMax(&s_top[q], top[q]);
+            atomicMin(&s_low[q], low[q]);
         }
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+        for (int o = 16; o > 0; o >>= 1) v[q] += __shfl_xor_sync(0xffffffffu, v[q], o);
+        if (lane == 0) s_v[w][q] = v[q];
     }
     __syncthreads();
+    // units that keep the weights below 2^30
+    int ex[2];
 #pragma unroll
-    for (int q = 0; q < 6; ++q) v[q] = s_tot[q][t];
-    for (int k = k0; k < k1; ++k) {
-        add(k);
-        pp[k] = {v[0], v[1], v[2], v[3], v[4], v[5]};
+    for (int q = 0; q < 2; ++q)
+        ex[q] = min(max((int)(s_top[q] >> 52) - 1022, -900), 1023);   // the largest lies below 2^ex
+    if (t == 0) {
+        AdjRow r;
+        double sum[4];
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            sum[q] = s_v[0][q];
+            for (int k = 1; k < ADJ_THREADS / 32; ++k) sum[q] += s_v[k][q];
+        }
+        r.zero = s_z;
+        r.s0 = sum[0];
+        r.t0 = sum[1];
+        r.still0 = sum[2];
+        r.still1 = sum[3];
+        r.unit = scalbn(1.0, ex[0] - 30 - ADJ_FRAC);
+        r.unit_s = scalbn(1.0, ex[1] - 30 - ADJ_FRAC);
+        r.even = 1;
+#pragma unroll
+        for (int q = 0; q < 2; ++q)   // by the exponents
+            if (s_top[q] != 0ULL && (s_low[q] >> 52) + 12 < (s_top[q] >> 52)) r.even = 0;
+        row[((long long)p * 2 + c) * n_mu + b] = r;
+    }
+    for (int k = a + t; k < e; k += ADJ_THREADS) {
         const AdjGeo &g = geo[pc[k]];
-        const double u = fabs(g.f), a = g.f > 0.0 ? -g.L * g.iS : g.L * g.iS;
-        AdjNoise x;
-        x.w = u < 0x1p-10 ? (unsigned long long)__double2ll_rn(u * 0x1p+53) << ADJ_FRAC : 0ULL;
-        x.a = (float)a;
-        x.as = (float)(a * g.sig);
-        noise[(long long)p * gm + k] = x;
+        const double u = fabs(g.f), x = g.f > 0.0 ? -g.a : g.a, y = c == 0 ? x : x * g.sig;
+        const bool in = u < ADJ_W_MAX && u > 0.0;
+        AdjNoise d;
+        d.w = in ? (unsigned long long)__double2ll_rn(u * 0x1p+53) << ADJ_FRAC : 0ULL;
+        d.a = in && fabs(x) < INFINITY ? __double2int_rn(scalbn(x, 30 - ex[0])) : 0;
+        d.as = in && fabs(y) < INFINITY ? __double2int_rn(scalbn(y, 30 - ex[1])) : 0;
+        pn[k] = d;
     }
 }
 
@@ -284,7 +337,8 @@ __global__ void k_adj_inv(int n_eff, const double *__restrict__ lam, double *__r
 // margin eps covers the rounding of the reference's positions.
 struct AdjRange {
     int lo[ADJ_NB], hi[ADJ_NB];
-    long long b0, b1;   // first and last boundary
+    AdjSums sum[ADJ_NB];   // over the entries between boundaries k and k + 1
+    long long b0, b1;      // first and last boundary
 };
 
 template <bool OUT>
@@ -329,24 +383,50 @@ __device__ __forceinline__ void adj_bounds(const double *__restrict__ fb, int a,
     (up ? R.hi : R.lo)[k] = lo;
 }
 
-// sums over the entries [lo, hi) of a row that starts at a
-__device__ __forceinline__ AdjPre adj_sum(const AdjPre *__restrict__ pre, int a, int lo, int hi) {
-    AdjPre s = pre[hi - 1];
-    if (lo > a) {
-        const AdjPre t = pre[lo - 1];
-        s.s0 -= t.s0;
-        s.s1 -= t.s1;
-        s.s2 -= t.s2;
-        s.t0 -= t.t0;
-        s.t1 -= t.t1;
-        s.t2 -= t.t2;
+// sums over the entries [lo, hi) of class c, a warp: every lane's result the same
+__device__ __forceinline__ AdjSums adj_sum(const AdjEnt *__restrict__ ent, const double *__restrict__ fb, int c, int lo,
+                                           int hi) {
+    AdjSums s;
+    s.f0 = fb[lo];
+    s.s0 = s.s1 = s.s2 = s.t0 = s.t1 = s.t2 = 0.0;
+    for (int k = lo + (threadIdx.x & 31); k < hi; k += 32) {
+        const AdjEnt x = ent[k];
+        const double d = fb[k] - s.f0;
+        s.s0 += x.L;
+        s.s1 += x.a;
+        s.s2 = fma(x.a, d, s.s2);
+        if (c == 1) {
+            const double as = x.a * x.sig;
+            s.t0 = fma(x.L, x.sig, s.t0);
+            s.t1 += as;
+            s.t2 = fma(as, d, s.t2);
+        }
+    }
+    for (int o = 16; o > 0; o >>= 1) {
+        s.s0 += __shfl_xor_sync(0xffffffffu, s.s0, o);
+        s.s1 += __shfl_xor_sync(0xffffffffu, s.s1, o);
+        s.s2 += __shfl_xor_sync(0xffffffffu, s.s2, o);
+        if (c == 1) {
+            s.t0 += __shfl_xor_sync(0xffffffffu, s.t0, o);
+            s.t1 += __shfl_xor_sync(0xffffffffu, s.t1, o);
+            s.t2 += __shfl_xor_sync(0xffffffffu, s.t2, o);
+        }
+    }
+    if (c != 1) {
+        s.t0 = s.s0;
+        s.t1 = s.s1;
+        s.t2 = s.s2;
     }
     return s;
 }
 
-// Walks a row of a class over a tile: group(c, lo, hi) for the entries of one offset, still(lo, hi)
-// for those without a shift, single(k) for each of the others.  The calls are uniform over the block.
-template <bool OUT, class G, class Z, class S>
+// l_j - l_o - l_o f, rounded once (l_j - l_o is exact)
+__device__ __forceinline__ double adj_rest(double lj, double lo, double f) { return fma(-lo, f, lj - lo); }
+
+// Walks a row of a class over a tile: group(c, lo, hi, sums) for the entries of one offset (SUMS: with
+// their sums), still(row) for those without a shift, single(k) for each of the others.  The calls are
+// uniform over the block.
+template <bool OUT, bool SUMS, class G, class Z, class S>
 __device__ __forceinline__ void adj_walk(const AdjArgs &A, int p, int c, int b, double pa, double pb, double eps,
                                          AdjRange &R, G group, Z still, S single) {
     const int *sg = A.seg + ((long long)p * ADJ_CLASS + c) * (A.n_mu + 1);
@@ -357,7 +437,8 @@ __device__ __forceinline__ void adj_walk(const AdjArgs &A, int p, int c, int b, 
         for (int k = a; k < e; ++k) single(k);
         return;
     }
-    const int2 z = A.zero[((long long)p * 2 + c) * A.n_mu + b];
+    const AdjRow &row = A.row[((long long)p * 2 + c) * A.n_mu + b];
+    const int2 z = row.zero;
     __syncthreads();
     adj_span<OUT>(fb, a, e, pa, pb, eps, R);
     __syncthreads();
@@ -365,7 +446,7 @@ __device__ __forceinline__ void adj_walk(const AdjArgs &A, int p, int c, int b, 
     if (b1 < R.b0) {
         for (int k = a; k < e; ++k)
             if (k < z.x || k >= z.y) single(k);
-        if (z.x < z.y) still(z.x, z.y);
+        if (z.x < z.y) still(row);
         return;
     }
     int done = a;   // entries below it are evaluated
@@ -374,8 +455,17 @@ __device__ __forceinline__ void adj_walk(const AdjArgs &A, int p, int c, int b, 
         __syncthreads();
         adj_bounds<OUT>(fb, a, e, pa, pb, eps, first, count, R);
         __syncthreads();
+        if constexpr (SUMS) {
+            const AdjEnt *ent = A.ent + (long long)p * A.gm;
+            for (int k = threadIdx.x >> 5; k + 1 < count; k += ADJ_THREADS / 32)
+                if (R.hi[k] < R.lo[k + 1]) {
+                    const AdjSums x = adj_sum(ent, fb, c, R.hi[k], R.lo[k + 1]);
+                    if ((threadIdx.x & 31) == 0) R.sum[k] = x;
+                }
+            __syncthreads();
+        }
         for (int k = 0; k < count; ++k) {
-            if (k + 1 < count && R.hi[k] < R.lo[k + 1]) group((int)(first + k + 1), R.hi[k], R.lo[k + 1]);
+            if (k + 1 < count && R.hi[k] < R.lo[k + 1]) group((int)(first + k + 1), R.hi[k], R.lo[k + 1], R.sum[k]);
             if (k + 1 < count || first + k == b1) {   // a boundary shared by two batches once
                 for (int q = max(R.lo[k], done); q < R.hi[k]; ++q)
                     if (q < z.x || q >= z.y) single(q);
@@ -384,8 +474,13 @@ __device__ __forceinline__ void adj_walk(const AdjArgs &A, int p, int c, int b, 
         }
         if (first + count - 1 >= b1) break;
     }
-    if (z.x < z.y) still(z.x, z.y);
+    if (z.x < z.y) still(row);
 }
+
+__device__ __forceinline__ int adj_exp(double v) { return (int)(((unsigned)__double2hiint(v) >> 20) & 0x7ffu); }
+
+// l'_o as the forward rounds it
+__device__ __forceinline__ double adj_shifted(double lo, double f) { return __dsub_rn(lo, __dmul_rn(lo, -f)); }
 
 __device__ __forceinline__ double adj_intensity(const AdjArgs &A, int p, int c, int k, double lj, double ssed,
                                                 double fsed) {
@@ -397,22 +492,30 @@ __device__ __forceinline__ double adj_intensity(const AdjArgs &A, int p, int c, 
 // The forward's l'_o is l_o - rn(l_o u) rounded to ulp(l_o), u = 1 - S: up to half an ulp, 1e-10 of
 // a pixel, from S l_o.  The row gradients take the weights of that grid, so that they are the
 // transpose of the forward to better than this: the sum over the cells [k0, k1) of L / S times the
-// residue, in ulp(l_o), needs only the fraction bits of the 64-bit product and FP32 sums.  lm:
-// l_o's significand, leading bit at bit 63.
-__device__ __forceinline__ float2 adj_residue(const AdjNoise *__restrict__ x, unsigned long long lm, int k0, int k1) {
+// residue.  The fraction bits of the 64-bit product are integers (|.| <= 2^20; the two products'
+// lower halves are left out, 2^-21 of an ulp on either side), the weights integers of at most 2^30,
+// and the sums exact.  lm: l_o's significand, leading bit at bit 63; TWO: the facula weights too.
+template <bool TWO>
+__device__ __forceinline__ void adj_residue(const AdjNoise *__restrict__ x, unsigned long long lm, int k0, int k1,
+                                            double &r, double &rs) {
+    constexpr int HALF = 1 << (ADJ_FRAC - 1), PART = 4096;   // 2^12 products of at most 2^50
     const unsigned h = (unsigned)(lm >> 32), l = (unsigned)lm;
-    float s = 0.f, t = 0.f;
+    r = rs = 0.0;
+    for (int q = k0; q < k1; q += PART) {
+        long long s = 0, t = 0;
+        const int end = min(k1, q + PART);
 #pragma unroll 4
-    for (int k = k0; k < k1; ++k) {
-        const AdjNoise c = x[k];
-        const unsigned wh = (unsigned)(c.w >> 32), wl = (unsigned)c.w;
-        const unsigned v = h * wh + __umulhi(h, wl) + __umulhi(l, wh) + (1u << (ADJ_FRAC - 1));   // carries: 2^-20 ulp
-        const float fr = __uint_as_float(0x4b000000u | (v & ((1u << ADJ_FRAC) - 1u))) -
-                         (8388608.f + (float)(1 << (ADJ_FRAC - 1)));
-        s = fmaf(c.a, fr, s);
-        t = fmaf(c.as, fr, t);
+        for (int k = q; k < end; ++k) {
+            const AdjNoise c = x[k];
+            const unsigned wh = (unsigned)(c.w >> 32), wl = (unsigned)c.w;
+            const unsigned v = h * wh + __umulhi(h, wl) + __umulhi(l, wh) + (HALF + 1);
+            const int fr = (int)(v & (2u * HALF - 1u)) - HALF;
+            s += (long long)c.a * fr;
+            if (TWO) t += (long long)c.as * fr;
+        }
+        r += (double)s;
+        if (TWO) rs += (double)t;
     }
-    return make_float2(s, t);
 }
 
 // ---- row gradients -----------------------------------------------------------------------
@@ -430,16 +533,16 @@ __global__ void __launch_bounds__(ADJ_THREADS) k_adj_rows(const __grid_constant_
     const double eps = 1.8e-15 * (4.0 * (double)n_eff + 2.0 * ADJ_F_MAX * fabs(ls) + 4.0);
     const bool own = o >= 0 && o <= n_eff - 2;
     const double lo = own ? lam[o] : 0.0, io = own ? A.inv[o] : 0.0, beta = lo * io;
-    const int ex = (int)(((unsigned)__double2hiint(lo) >> 20) & 0x7ffu);
+    const int ex = adj_exp(lo);
     const bool noisy = ex > 200 && ex < 1800;   // a wavelength whose ulp is a normal number
     const unsigned long long lm = ((unsigned long long)__double_as_longlong(lo) << 11) | 0x8000000000000000ULL;
-    const double unit = noisy ? __hiloint2double((ex - 52 - ADJ_FRAC) << 20, 0) * io : 0.0;
+    const double ulp = noisy ? __hiloint2double((ex - 52) << 20, 0) * io : 0.0;
     double L[4] = {0.0, 0.0, 0.0, 0.0}, U[4] = {0.0, 0.0, 0.0, 0.0};   // q_sed, q_norm, spot, facula: lower, upper
     for (int p = 0; p < A.n_phase; ++p) {
         const long long go = (long long)p * A.n;
         const double *gf = A.gF + go, *gb = A.gB + go, *gt = A.gT + go;
-        const AdjPre *pre = A.pre + (long long)p * A.gm;
         const AdjNoise *noise = A.noise + (long long)p * A.gm;
+        const double *fb = A.fb + (long long)p * A.gm;
         const int *cell = A.cell + (long long)p * A.gm;
 #pragma unroll 1
         for (int c = 0; c < ADJ_CLASS; ++c) {
@@ -467,35 +570,40 @@ __global__ void __launch_bounds__(ADJ_THREADS) k_adj_rows(const __grid_constant_
                 }
             };
             auto sed_at = [&](int type, int j) { return BC ? 0.0 : (type == 0 ? A.spot_sed[j] : A.fac_sed[j]); };
-            const int a = A.seg[((long long)p * ADJ_CLASS + c) * (A.n_mu + 1) + b];
-            adj_walk<false>(
+            const AdjRow &row = A.row[((long long)p * 2 + (c < 2 ? c : 0)) * A.n_mu + b];
+            adj_walk<false, true>(
                 A, p, c, b, pa, pb, eps, R,
-                [&](int off, int k0, int k1) {
+                [&](int off, int k0, int k1, const AdjSums &s) {
                     const int j = o + off;
                     if (!own || j < 0 || j >= n_eff) return;
-                    const AdjPre s = adj_sum(pre, a, k0, k1);
-                    const double al = (lam[j] - lo) * io;
-                    const float2 r = adj_residue(noise, lm, k0, k1);
-                    const double w1 = fma(al, s.s1, fma(-beta, s.s2, -unit * (double)r.x)), wl = s.s0 - w1;
-                    double w1s = w1, wls = wl;
-                    if (!BC && c == 1) {
-                        w1s = fma(al, s.t1, fma(-beta, s.t2, -unit * (double)r.y));
-                        wls = s.t0 - w1s;
-                    }
-                    add(j, wl, w1, wls, w1s, sed_at(c, j), c);
-                },
-                [&](int k0, int k1) {   // no shift: pixel j is source j
-                    if (o < 0 || o >= n_eff) return;
-                    AdjPre s = adj_sum(pre, a, k0, k1);
-                    if (o == n_eff - 1) {   // without an interval above it: the cells at rest only
-                        s.s0 = s.t0 = 0.0;
+                    const double lj = lam[j], f1 = fb[k1 - 1];
+                    const bool two = !BC && c == 1;
+                    double w1, w1s;
+                    // l' in l_o's binade for the range's extreme shifts, and |f| below ADJ_W_MAX
+                    if (noisy && row.even && adj_exp(fma(lo, s.f0, lo)) == ex && adj_exp(fma(lo, f1, lo)) == ex &&
+                        fmax(fabs(s.f0), fabs(f1)) < ADJ_W_MAX) {
+                        const double rest = adj_rest(lj, lo, s.f0);
+                        double r, rs;
+                        if (two) adj_residue<true>(noise, lm, k0, k1, r, rs);
+                        else adj_residue<false>(noise, lm, k0, k1, r, rs);
+                        w1 = fma(io, fma(rest, s.s1, -lo * s.s2), -ulp * (row.unit * r));
+                        w1s = two ? fma(io, fma(rest, s.t1, -lo * s.t2), -ulp * (row.unit_s * rs)) : w1;
+                    } else {   // the forward's l' cell by cell
+                        w1 = w1s = 0.0;
                         for (int k = k0; k < k1; ++k) {
                             const AdjGeo &g = A.geo[cell[k]];
-                            s.s0 = fma(g.still, g.L, s.s0);
-                            s.t0 = fma(g.still, g.L * (c == 0 ? 1.0 : g.sig), s.t0);
+                            const double w = g.a * ((lj - adj_shifted(lo, g.f)) * io);
+                            w1 += w;
+                            w1s = fma(w, g.sig, w1s);
                         }
+                        if (!two) w1s = w1;
                     }
-                    add(o, s.s0, 0.0, s.t0, 0.0, sed_at(c, o), c);
+                    add(j, s.s0 - w1, w1, (two ? s.t0 : s.s0) - w1s, w1s, sed_at(c, j), c);
+                },
+                [&](const AdjRow &z) {   // no shift: pixel j is source j
+                    if (o < 0 || o >= n_eff) return;
+                    const bool end = o == n_eff - 1;   // without an interval above it: the cells at rest only
+                    add(o, end ? z.still0 : z.s0, 0.0, end ? z.still1 : z.t0, 0.0, sed_at(c, o), c);
                 },
                 [&](int k) {
                     const AdjGeo &g = A.geo[cell[k]];
@@ -514,7 +622,7 @@ __global__ void __launch_bounds__(ADJ_THREADS) k_adj_rows(const __grid_constant_
                     cs.fbeta = g.f;
                     cs.off = g.off;
                     const long long ja = max(soap_ceil_pos(o, cs), 0LL), jb = min(soap_ceil_pos(o + 1, cs), (long long)n_eff);
-                    const double l1 = __dsub_rn(lo, __dmul_rn(lo, -g.f));   // l'_o
+                    const double l1 = adj_shifted(lo, g.f);
                     for (long long j = ja; j < jb; ++j) {
                         const double w1 = g.L * ((lam[j] - l1) * g.iS * io), wl = g.L - w1;
                         add((int)j, wl, w1, wl * sg, w1 * sg, sed_of((int)j), type);
@@ -550,7 +658,6 @@ __global__ void __launch_bounds__(ADJ_THREADS) k_adj_continuum(const __grid_cons
     for (int p = 0; p < A.n_phase; ++p) {
         const double gf = j < n_eff ? A.gF[(long long)p * A.n + j] : 0.0;
         const double gt = j < n_eff ? A.gT[(long long)p * A.n + j] : 0.0;
-        const AdjPre *pre = A.pre + (long long)p * A.gm;
         const int *cell = A.cell + (long long)p * A.gm;
 #pragma unroll 1
         for (int c = 0; c < ADJ_CLASS; ++c) {
@@ -567,27 +674,16 @@ __global__ void __launch_bounds__(ADJ_THREADS) k_adj_continuum(const __grid_cons
                 if (type == 0) sum[0] += h;
                 else sum[1] += h;
             };
-            const int a = A.seg[((long long)p * ADJ_CLASS + c) * (A.n_mu + 1) + b];
-            adj_walk<true>(
+            adj_walk<true, true>(
                 A, p, c, b, pa, pb, eps, R,
-                [&](int off, int k0, int k1) {
+                [&](int off, int, int, const AdjSums &s) {
                     const int o = j - off;
                     if (j >= n_eff || o < 0 || o > n_eff - 2) return;
-                    const AdjPre s = adj_sum(pre, a, k0, k1);
-                    const double lo = lam[o], io = A.inv[o];
-                    add(o, s.t0, fma((lj - lo) * io, s.t1, -lo * io * s.t2), c);
+                    const double lo = lam[o];
+                    add(o, s.t0, A.inv[o] * fma(adj_rest(lj, lo, s.f0), s.t1, -lo * s.t2), c);
                 },
-                [&](int k0, int k1) {
-                    if (j >= n_eff) return;
-                    double w0 = adj_sum(pre, a, k0, k1).t0;
-                    if (j == n_eff - 1) {
-                        w0 = 0.0;
-                        for (int k = k0; k < k1; ++k) {
-                            const AdjGeo &g = A.geo[cell[k]];
-                            w0 = fma(g.still, g.L * (c == 0 ? 1.0 : g.sig), w0);
-                        }
-                    }
-                    add(j, w0, 0.0, c);
+                [&](const AdjRow &z) {
+                    if (j < n_eff) add(j, j == n_eff - 1 ? z.still1 : z.t0, 0.0, c);
                 },
                 [&](int k) {
                     if (j >= n_eff) return;
@@ -604,7 +700,7 @@ __global__ void __launch_bounds__(ADJ_THREADS) k_adj_continuum(const __grid_cons
                     const long long o = soap_owner(j, n_eff, cs);
                     if (o < 0) return;
                     const double lo = lam[o], io = A.inv[o];
-                    add((int)o, ratio * g.L, ratio * g.L * fma((lj - lo) * io, g.iS, -lo * io * g.e), type);
+                    add((int)o, ratio * g.L, ratio * (g.a * (adj_rest(lj, lo, g.f) * io)), type);
                 });
         }
     }
@@ -630,9 +726,10 @@ __global__ void k_adj_sum_rows(int n, int n_mu, const double *__restrict__ part,
 // ---- limb and velocity ---------------------------------------------------------------------
 // Block: one row of one phase over a share of the pixels, tile by tile.  For each offset's cells
 // the tile gives three sums over its pixels (six for the faculae, whose intensity factor differs
-// from cell to cell): of P, of alpha Q and of beta Q, P and Q the rows' values and differences
-// dotted with h; a cell adds P + (alpha Q) / S - (beta Q) f / S to its limb gradient and
-// -K (alpha Q + beta Q) to its velocity gradient.
+// from cell to cell): of P, of alpha' Q and of beta Q, P and Q the rows' values and differences
+// dotted with h, alpha' = inv[o] (l_j - l_o - l_o f0) with the range's f0; a cell adds
+// P + (alpha' Q - (f - f0) beta Q) / S to its limb gradient and -K (alpha' Q + (1 + f0) beta Q) to its
+// velocity gradient.
 constexpr int ADJ_WARPS = ADJ_THREADS / 32;
 
 template <bool BC>
@@ -690,15 +787,16 @@ __global__ void __launch_bounds__(ADJ_THREADS) k_adj_limb(const __grid_constant_
                 __syncthreads();
                 for (int q = 0; q < nv; ++q) v[q] = s_sum[q];
             };
-            adj_walk<true>(
+            adj_walk<true, false>(
                 A, p, c, b, pa, pb, eps, R,
-                [&](int off, int k0, int k1) {
+                [&](int off, int k0, int k1, const AdjSums &) {
+                    const double f0 = A.fb[(long long)p * A.gm + k0];
                     double v[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
                     const int o = j - off;
                     if (j < n_eff && o >= 0 && o <= n_eff - 2) {
                         double P, Q, Ps, Qsd;
                         dots(j, o, c, sed_at(c, j), false, P, Q, Ps, Qsd);
-                        const double lo = lam[o], io = A.inv[o], al = (lam[j] - lo) * io, be = lo * io;
+                        const double lo = lam[o], io = A.inv[o], al = adj_rest(lam[j], lo, f0) * io, be = lo * io;
                         if (c == 0) {
                             P += Ps;
                             Q += Qsd;
@@ -720,11 +818,12 @@ __global__ void __launch_bounds__(ADJ_THREADS) k_adj_limb(const __grid_constant_
                             g1 = fma(g.sig, v[4], g1);
                             g2 = fma(g.sig, v[5], g2);
                         }
-                        acc[2 * k] += fma(g1, g.iS, fma(-g2, g.e, g0));
-                        acc[2 * k + 1] = fma(-g.K, g1 + g2, acc[2 * k + 1]);
+                        acc[2 * k] += fma(fma(f0 - g.f, g2, g1), g.iS, g0);
+                        acc[2 * k + 1] = fma(-g.K, fma(1.0 + f0, g2, g1), acc[2 * k + 1]);
                     }
                 },
-                [&](int k0, int k1) {
+                [&](const AdjRow &z) {
+                    const int k0 = z.zero.x, k1 = z.zero.y;
                     double v[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
                     double end = 0.0, end_s = 0.0;   // pixel n_eff - 1
                     if (j < n_eff) {
@@ -769,7 +868,7 @@ __global__ void __launch_bounds__(ADJ_THREADS) k_adj_limb(const __grid_constant_
                             double P, Q, Ps, Qsd;
                             dots(j, (int)o, type, I, last, P, Q, Ps, Qsd);
                             const double lo = lam[o], io = last ? 0.0 : A.inv[o];
-                            const double wt = rest ? 0.0 : fma((lj - lo) * io, g.iS, -lo * io * g.e);
+                            const double wt = rest ? 0.0 : adj_rest(lj, lo, g.f) * io * g.iS;
                             const double Qt = fma(s, Qsd, Q);
                             v[0] = fma(wt, Qt, fma(s, Ps, P));
                             v[1] = lj * io * Qt;
@@ -858,10 +957,10 @@ extern "C" int soapgb_phase_integrate_adjoint(soapgb_ctx *ctx, int n, int n_eff,
     const bool ranks = gm <= ORDER_MAX;
     const size_t sort_b = ranks ? sizeof(unsigned long long) * gm : fir_sort_temp_bytes(gm);
     int s_sort = ws.add(sort_b);
-    int s_cell = ws.add(sizeof(int) * pg), s_fb = ws.add(sizeof(double) * pg), s_pre = ws.add(sizeof(AdjPre) * pg);
+    int s_cell = ws.add(sizeof(int) * pg), s_fb = ws.add(sizeof(double) * pg), s_ent = ws.add(sizeof(AdjEnt) * pg);
     int s_noise = ws.add(sizeof(AdjNoise) * pg);
     int s_seg = ws.add(sizeof(int) * ADJ_CLASS * (size_t)(n_mu + 1) * std::max(n_phase, 1));
-    int s_zr = ws.add(sizeof(int2) * 2 * (size_t)n_mu * std::max(n_phase, 1));
+    int s_row = ws.add(sizeof(AdjRow) * 2 * (size_t)n_mu * std::max(n_phase, 1));
     // shares of the pixels in the limb kernel: eight blocks per SM over rows, phases and shares (a
     // phase's regions touch about half of the rows)
     const int tiles = (n_eff + ADJ_THREADS - 1) / ADJ_THREADS;
@@ -947,10 +1046,10 @@ extern "C" int soapgb_phase_integrate_adjoint(soapgb_ctx *ctx, int n, int n_eff,
         A.geo = ws.get<AdjGeo>(s_geo);
         A.cell = ws.get<int>(s_cell);
         A.fb = ws.get<double>(s_fb);
-        A.pre = ws.get<AdjPre>(s_pre);
+        A.ent = ws.get<AdjEnt>(s_ent);
         A.noise = ws.get<AdjNoise>(s_noise);
         A.seg = ws.get<int>(s_seg);
-        A.zero = ws.get<int2>(s_zr);
+        A.row = ws.get<AdjRow>(s_row);
         A.acc = ws.get<double>(s_acc);
         A.part = ws.get<double>(s_part);
         A.d_qn = o_qn;
@@ -974,8 +1073,9 @@ extern "C" int soapgb_phase_integrate_adjoint(soapgb_ctx *ctx, int n, int n_eff,
                                                            act->solar, A.t_norm_fac, ws.get<int>(s_cell),
                                                            ws.get<double>(s_fb), ws.get<int>(s_seg), ctx->d_status);
             SOAP_LAUNCHED(ctx);
-            k_adj_prefix<<<dim3(n_mu, 2, n_phase), ADJ_THREADS, 0, ctx->stream>>>(
-                gm, n_mu, A.cell, A.fb, A.seg, A.geo, ws.get<AdjPre>(s_pre), ws.get<AdjNoise>(s_noise), ws.get<int2>(s_zr));
+            k_adj_entries<<<dim3(n_mu, 2, n_phase), ADJ_THREADS, 0, ctx->stream>>>(
+                gm, n_mu, A.cell, A.fb, A.seg, A.geo, ws.get<AdjEnt>(s_ent), ws.get<AdjNoise>(s_noise),
+                ws.get<AdjRow>(s_row));
             SOAP_LAUNCHED(ctx);
             k_adj_inv<<<grid_for(ctx, n_eff, 256), 256, 0, ctx->stream>>>(n_eff, d_wave, d_inv);
             SOAP_LAUNCHED(ctx);

@@ -114,3 +114,35 @@ def test_cells_that_cross_several_integers_in_a_tile(ctx, vsini):
     ref, mag, _ = _reference(wave, n_eff, bi, maps, x, step, g)
     for k in ref:
         assert np.all(np.abs(got[k] - ref[k]) <= 1e-9 * mag[k] + 1e-300), k
+
+
+# rotators of a few to 400 km/s (beyond 290 km/s the residues of l' are summed cell by cell), a grid
+# across 4096 A, limb factors over twelve orders of magnitude and beyond FP32's range
+@pytest.mark.parametrize("lambda0,vsini,grid,limb", [(5000.0, 60.0, 40, "disk"), (4094.0, 9.0, 24, "disk"),
+                                                     (6000.0, 4.0, 13, "wide"), (5000.0, 400.0, 16, "disk"),
+                                                     (4090.0, 30.0, 20, "huge")])
+def test_entries_carry_the_rounding_of_single_cells(ctx, lambda0, vsini, grid, limb):
+    """Gradients that reach a few output pixels only, so that an entry of the rows is the sum over the
+    cells of one offset.  A cell's term takes at most 16 roundings and the cells' sum one each: (16 +
+    cells) u of the entry's magnitudes.  The limb and velocity gradients sum 6 tiles' pixels in 13
+    steps each, over at most 6 shares: (16 + 13 + 12) u."""
+    rng = np.random.default_rng(grid)
+    n, n_eff, n_mu, step = 1400, 1390, 4, 0.01
+    wave = lambda0 + step * np.arange(n)
+    maps = _maps(grid, vsini, n_mu)
+    vis = maps["limb"] > -998
+    if limb == "wide":
+        maps["limb"] = np.where(vis, maps["limb"] * 10.0 ** rng.uniform(-12, 0, vis.size), maps["limb"])
+    if limb == "huge":
+        maps["limb"] = np.where(vis, maps["limb"] * 1e60, maps["limb"])
+    bi, temp, x = _inputs(rng, n, n_mu, grid, maps)
+    g = np.zeros((3, 2, n))
+    at = np.r_[0, 247, 248, 256, 700, 1023, n_eff - 1, rng.integers(0, n_eff, 8)]
+    g[:, :, at] = rng.standard_normal((3, 2, at.size))
+    got = ctx.phase_integrate_adjoint(wave, n_eff, grid, temp, bi, maps, x, step, Activity(5778, 663, 250, 20, 0), *g)
+    ref, mag, cnt = _reference(wave, n_eff, bi, maps, x, step, g)
+    u = 2.0 ** -53
+    for k in ref:
+        bound = (41 if k in ("limb", "delta") else 16 + cnt[k]) * u * mag[k]
+        bad = np.abs(got[k] - ref[k]) > bound
+        assert not bad.any(), (k, np.argwhere(bad)[:3], float(np.max(np.abs(got[k] - ref[k])[bad] / mag[k][bad]) / u))
