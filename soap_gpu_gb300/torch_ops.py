@@ -121,7 +121,9 @@ class Ops:
         return out[0] if single else out
 
     def ccf_normalise(self, raw):
-        return self.o.ccf_normalise(self.h, _t(raw))
+        single = raw.dim() == 1
+        out = self.o.ccf_normalise(self.h, _t(raw.reshape(1, -1) if single else raw))
+        return out[0] if single else out
 
     def ccf_adjoint(self, vel, line_wave, line_weight, wave_trim, step_size, g_ccf, ccf_raw=None, normalise=True,
                     wave_extend=100.0, mask_step=0.005, index_old=20000):
