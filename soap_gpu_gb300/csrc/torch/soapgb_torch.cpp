@@ -261,6 +261,9 @@ Tensor ccf_adjoint(int64_t h, const Tensor &vel, const Tensor &line_wave, const 
                    int64_t index_old) {
     c10::cuda::CUDAGuard guard(g_ccf.device());
     soapgb_ctx *ctx = on_stream(h, g_ccf);
+    TORCH_CHECK(g_ccf.dim() == 2 && g_ccf.size(1) == vel.numel(), "soapgb: g_ccf is n_spec x n_v");
+    TORCH_CHECK(!normalise || (ccf_raw.has_value() && ccf_raw->sizes() == g_ccf.sizes()),
+                "soapgb: ccf_raw is n_spec x n_v");
     const int n_spec = (int)g_ccf.size(0), n_v = (int)vel.numel(), n_w = (int)wave_trim.numel();
     Tensor out = empty64(g_ccf, {n_spec, n_w});
     check(ctx, soapgb_ccf_adjoint(ctx, n_v, f64(vel, "vel"), (int)line_wave.numel(), f64(line_wave, "line_wave"),

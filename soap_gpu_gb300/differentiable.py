@@ -294,9 +294,13 @@ class NormalisedCcf(torch.autograd.Function):
     @staticmethod
     def backward(fctx, g):
         s = fctx.setup
-        grad = ops(s.ctx).ccf_adjoint(s.vel, s.line_wave, s.line_weight, s.wave_trim, s.step,
-                                 g.to(torch.float64).contiguous(), ccf_raw=fctx.raw, normalise=True, **s.kwargs())
-        return grad, None
+        raw, g = fctx.raw, g.to(torch.float64).contiguous()
+        single = raw.dim() == 1
+        if single:
+            raw, g = raw[None], g[None]
+        grad = ops(s.ctx).ccf_adjoint(s.vel, s.line_wave, s.line_weight, s.wave_trim, s.step, g, ccf_raw=raw,
+                                      normalise=True, **s.kwargs())
+        return (grad[0] if single else grad), None
 
 
 class GaussFit(torch.autograd.Function):

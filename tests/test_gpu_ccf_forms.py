@@ -25,3 +25,21 @@ def test_normalised_ccf_of_one_spectrum(ctx):
         rows = normalised_ccf(sp, cs)
         for s in range(sp.shape[0]):
             assert torch.equal(normalised_ccf(sp[s], cs), rows[s])
+
+
+def test_gradient_of_one_spectrum(ctx):
+    """Its gradient is the row's too, and the operator refuses shapes that its kernels would read past."""
+    from soap_gpu_gb300.differentiable import normalised_ccf
+    from soap_gpu_gb300.torch_ops import ops
+    cs, sp = _spectra(ctx)
+    w = _dev(np.random.default_rng(4).standard_normal((sp.shape[0], cs.vel.numel())))
+    x = sp.clone().requires_grad_(True)
+    (normalised_ccf(x, cs) * w).sum().backward()
+    for s in range(sp.shape[0]):
+        v = sp[s].clone().requires_grad_(True)
+        (normalised_ccf(v, cs) * w[s]).sum().backward()
+        assert torch.equal(v.grad, x.grad[s])
+    args = (cs.vel, cs.line_wave, cs.line_weight, cs.wave_trim, cs.step)
+    for g, raw in ((w[0], w[0]), (w[:, 1:].contiguous(), w[:, 1:].contiguous()), (w, w[:2].contiguous()), (w, None)):
+        with pytest.raises(RuntimeError):
+            ops(ctx).ccf_adjoint(*args, g, ccf_raw=raw, **cs.kwargs())
