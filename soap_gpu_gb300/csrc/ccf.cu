@@ -242,17 +242,19 @@ __device__ __forceinline__ double ccf_apod(int i, int n_v) {
     return 0.0;
 }
 
-// normalise by the max and apodise, run_all_SOAP.py:299-314,369-370; a warp per spectrum
-__global__ void k_ccf_normalise(int n_spec, int n_v, double *ccf) {
+// normalise by the max and apodise, run_all_SOAP.py:299-314,369-370; a warp per spectrum.  raw and
+// ccf may be the same: a value is read before it is written, and the max (its shuffles) before both
+__global__ void k_ccf_normalise(int n_spec, int n_v, const double *raw, double *ccf) {
     const int s = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
     if (s >= n_spec) return;
-    double *c = ccf + (long long)s * n_v;
+    const double *c = raw + (long long)s * n_v;
+    double *o = ccf + (long long)s * n_v;
     double mx = c[0];
     for (int i = lane; i < n_v; i += 32) mx = fmax(mx, c[i]);
-    for (int o = 16; o > 0; o >>= 1) mx = fmax(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+    for (int w = 16; w > 0; w >>= 1) mx = fmax(mx, __shfl_xor_sync(0xffffffffu, mx, w));
     for (int i = lane; i < n_v; i += 32) {
         double v = c[i] / mx;
-        c[i] = 1 - ((-v + 1) * ccf_apod(i, n_v));
+        o[i] = 1 - ((-v + 1) * ccf_apod(i, n_v));
     }
 }
 
@@ -367,7 +369,7 @@ extern "C" int soapgb_ccf(soapgb_ctx *ctx, int form, int n_v, const double *vel,
     }
     SOAP_LAUNCHED(ctx);
     if (normalise) {
-        k_ccf_normalise<<<(n_spec + 1) / 2, 64, 0, ctx->stream>>>(n_spec, n_v, d_out);
+        k_ccf_normalise<<<(n_spec + 1) / 2, 64, 0, ctx->stream>>>(n_spec, n_v, d_out, d_out);
         SOAP_LAUNCHED(ctx);
     }
     rc = check_status(ctx, "soapgb_ccf");
@@ -394,8 +396,8 @@ extern "C" int soapgb_ccf_normalise(soapgb_ctx *ctx, int n_spec, int n_v, const 
     int rc = ws.commit();
     if (rc) return rc;
     double *d = host ? ws.get<double>(s_out) : ccf_out;
-    SOAP_CUDA(ctx, cudaMemcpyAsync(d, raw, bytes, host ? cudaMemcpyHostToDevice : cudaMemcpyDeviceToDevice, ctx->stream));
-    k_ccf_normalise<<<(n_spec + 1) / 2, 64, 0, ctx->stream>>>(n_spec, n_v, d);
+    if (host) SOAP_CUDA(ctx, cudaMemcpyAsync(d, raw, bytes, cudaMemcpyHostToDevice, ctx->stream));
+    k_ccf_normalise<<<(n_spec + 1) / 2, 64, 0, ctx->stream>>>(n_spec, n_v, host ? d : raw, d);
     SOAP_LAUNCHED(ctx);
     if (host) {
         SOAP_CUDA(ctx, cudaMemcpyAsync(ccf_out, d, bytes, cudaMemcpyDeviceToHost, ctx->stream));

@@ -1,4 +1,6 @@
 """Forms of the normalised CCF's call: one spectrum as a vector, in place, long spectra."""
+import ctypes
+
 import numpy as np
 import pytest
 
@@ -43,3 +45,25 @@ def test_gradient_of_one_spectrum(ctx):
     for g, raw in ((w[0], w[0]), (w[:, 1:].contiguous(), w[:, 1:].contiguous()), (w, w[:2].contiguous()), (w, None)):
         with pytest.raises(RuntimeError):
             ops(ctx).ccf_adjoint(*args, g, ccf_raw=raw, **cs.kwargs())
+
+
+def test_normalise_in_place(ctx):
+    """raw and ccf_out the same buffer, on the device and on the host: the values of separate buffers."""
+    from soap_gpu_gb300 import _lib
+    cs, sp = _spectra(ctx, 5)
+    args = (cs.vel, cs.line_wave, cs.line_weight, cs.wave_trim, cs.step, sp)
+    raw = ctx.ccf("plain64", *args, normalise=False, **cs.kwargs())
+    want = ctx.ccf("plain64", *args, normalise=True, **cs.kwargs())
+    lib = _lib.load()
+    n_spec, n_v = raw.shape
+    torch.cuda.synchronize()
+    call = lambda src, mem, dst: lib.soapgb_ccf_normalise(ctx.h, n_spec, n_v, ctypes.c_void_p(src), mem, ctypes.c_void_p(dst))
+    out, same = torch.empty_like(raw), raw.clone()
+    torch.cuda.synchronize()
+    assert call(raw.data_ptr(), _lib.DEVICE, out.data_ptr()) == 0
+    assert call(same.data_ptr(), _lib.DEVICE, same.data_ptr()) == 0
+    ctx.synchronize()
+    assert torch.equal(out, want) and torch.equal(same, want)
+    host = raw.cpu().numpy().copy()
+    assert call(host.ctypes.data, _lib.HOST, host.ctypes.data) == 0
+    assert np.array_equal(host, want.cpu().numpy())
