@@ -258,6 +258,24 @@ __global__ void k_ccf_normalise(int n_spec, int n_v, const double *raw, double *
     }
 }
 
+// the first and the last wavelength of a device grid: one copy where the distance is a pitch that CUDA
+// takes (below 2^31 bytes), else two
+static int grid_ends(soapgb_ctx *ctx, const double *wave, int n, double *first, double *last) {
+    const size_t pitch = sizeof(double) * (size_t)(n - 1);
+    double w2[2];
+    if (pitch <= 0x7fffffffULL) {
+        SOAP_CUDA(ctx, cudaMemcpy2DAsync(w2, sizeof(double), wave, pitch, sizeof(double), 2, cudaMemcpyDeviceToHost,
+                                         ctx->stream));
+    } else {
+        SOAP_CUDA(ctx, cudaMemcpyAsync(w2, wave, sizeof(double), cudaMemcpyDeviceToHost, ctx->stream));
+        SOAP_CUDA(ctx, cudaMemcpyAsync(w2 + 1, wave + n - 1, sizeof(double), cudaMemcpyDeviceToHost, ctx->stream));
+    }
+    SOAP_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
+    *first = w2[0];
+    *last = w2[1];
+    return SOAPGB_OK;
+}
+
 extern "C" int soapgb_ccf(soapgb_ctx *ctx, int form, int n_v, const double *vel, int n_lines,
                           const double *line_wave, const double *line_weight, int n_w, const double *wave_trim,
                           double step_size, double wave_extend, double mask_step, int index_old, int n_spec,
@@ -288,12 +306,8 @@ extern "C" int soapgb_ccf(soapgb_ctx *ctx, int form, int n_v, const double *vel,
         w_first = wave_trim[0];
         w_last = wave_trim[n_w - 1];
     } else {
-        double w2[2];   // the ends in one copy
-        SOAP_CUDA(ctx, cudaMemcpy2DAsync(w2, sizeof(double), wave_trim, sizeof(double) * (size_t)(n_w - 1), sizeof(double),
-                                         2, cudaMemcpyDeviceToHost, ctx->stream));
-        SOAP_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
-        w_first = w2[0];
-        w_last = w2[1];
+        int rc = grid_ends(ctx, wave_trim, n_w, &w_first, &w_last);
+        if (rc) return rc;
     }
     if (!(w_last > w_first)) return set_error(ctx, SOAPGB_ERR_ARG, "soapgb_ccf: wavelengths must ascend");
     CcfGeom g;
@@ -498,12 +512,8 @@ extern "C" int soapgb_ccf_adjoint(soapgb_ctx *ctx, int n_v, const double *vel, i
         w_first = wave_trim[0];
         w_last = wave_trim[n_w - 1];
     } else {
-        double w2[2];   // the ends in one copy
-        SOAP_CUDA(ctx, cudaMemcpy2DAsync(w2, sizeof(double), wave_trim, sizeof(double) * (size_t)(n_w - 1), sizeof(double),
-                                         2, cudaMemcpyDeviceToHost, ctx->stream));
-        SOAP_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
-        w_first = w2[0];
-        w_last = w2[1];
+        int rc = grid_ends(ctx, wave_trim, n_w, &w_first, &w_last);
+        if (rc) return rc;
     }
     if (!(w_last > w_first)) return set_error(ctx, SOAPGB_ERR_ARG, "soapgb_ccf_adjoint: wavelengths must ascend");
     CcfGeom g;

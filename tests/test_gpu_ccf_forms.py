@@ -67,3 +67,20 @@ def test_normalise_in_place(ctx):
     host = raw.cpu().numpy().copy()
     assert call(host.ctypes.data, _lib.HOST, host.ctypes.data) == 0
     assert np.array_equal(host, want.cpu().numpy())
+
+
+def test_grid_longer_than_a_pitch(ctx):
+    """A grid whose ends lie 2^31 bytes apart.  Both lines lie in its first part, which alone gives the
+    same raw CCF and gradient."""
+    n, part, step = (1 << 28) + 2, 1 << 20, 2.0 ** -17
+    wave = torch.arange(n, dtype=torch.float64, device="cuda:0").mul_(step).add_(5000.0)
+    spec = torch.ones((1, n), dtype=torch.float64, device="cuda:0")
+    spec[0, :part] += _dev(0.1 * np.random.default_rng(1).standard_normal(part))
+    lines = (_dev([5001.0, 5005.0]), _dev([0.5, 0.8]))
+    vel, g = _dev([0.0]), _dev([[1.5]])
+    kw = dict(normalise=False, wave_extend=10 * step, mask_step=step, index_old=10)
+    got, want = (ctx.ccf("plain64", vel, *lines, wave[:m], step, spec[:, :m].contiguous(), **kw) for m in (n, part))
+    assert float(want[0, 0]) > 0 and torch.equal(got, want)
+    del spec
+    got, want = (ctx.ccf_adjoint(vel, *lines, wave[:m], step, g, **kw) for m in (n, part))
+    assert torch.equal(got[:, :part], want) and not got[0, part:].any()
