@@ -501,8 +501,7 @@ extern "C" int soapgb_quiet_disk(soapgb_ctx *ctx, int form, int n, int n_eff, co
         if (rc) return rc;
         const int ntile = (n + PL_TILE - 1) / PL_TILE;
         if (ntile <= 4 * ctx->num_sms) {
-            SOAP_CUDA(ctx, cudaFuncSetAttribute(k_quiet_plain64s, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                (int)sizeof(PlainQuietSmem)));
+            SOAP_CUDA(ctx, soap_allow_smem(k_quiet_plain64s, sizeof(PlainQuietSmem)));
             SOAP_TRACED(ctx, "quiet_plain64",
                         k_quiet_plain64s<<<ntile, 32 * PQ_WARPS, sizeof(PlainQuietSmem), ctx->stream>>>(
                             n, n_eff, d_wave, d_cube, d_count, d_cells, geo, d_delta, d_limb, d_region, n_mu, d_out,

@@ -43,6 +43,7 @@ constexpr int FIR_TILE = FIR_THREADS * FIR_PIX;
 constexpr int FIR_WIN = 1152;                    // staged values per cube row (window capacity)
 constexpr int FIR_MCH = FIR_WIN - FIR_TILE - 8;  // shift values per work unit (window + alignment fit)
 constexpr int FIR_MAX_MU = 256;
+constexpr int FIR_SEG_MAX = 2 * FIR_MAX_MU;      // a class's segments at most
 constexpr long long FIR_WAIT_LIMIT = 1LL << 24;  // bounded mbarrier waits
 
 static_assert(FIR_MCH <= FIR_THREADS, "one shift value per thread in a unit");
@@ -2892,7 +2893,7 @@ static int fir_lists(soapgb_ctx *ctx, const FirLayout &L, char *ws, long long gm
         int *counts = (int *)(ws + L.off[FirLayout::COUNTS]);
         const int cap = boxes->box_cap;
         const size_t smem = (size_t)cap * 3 * sizeof(unsigned long long);
-        SOAP_CUDA(ctx, cudaFuncSetAttribute(k_fir_slists, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        SOAP_CUDA(ctx, soap_allow_smem(k_fir_slists, (size_t)FIR_SLIST_CAP_MAX * 3 * sizeof(unsigned long long)));
         const soapgb_activity *act = boxes->act;
         SOAP_TRACED(ctx, "fir_lists",
                     k_fir_slists<<<n_lists, FIR_SLIST_THREADS, smem, ctx->stream>>>(
@@ -2925,7 +2926,7 @@ static int fir_lists(soapgb_ctx *ctx, const FirLayout &L, char *ws, long long gm
         SOAP_TRACED(ctx, "fir_rank", k_fir_rank<<<g, 256, 0, ctx->stream>>>(gm, va, rank));
         SOAP_LAUNCHED(ctx);
         const size_t smem = fir_blists_smem(gm);
-        SOAP_CUDA(ctx, cudaFuncSetAttribute(k_fir_blists, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        SOAP_CUDA(ctx, soap_allow_smem(k_fir_blists, fir_blists_smem(fir_box_lists_max_gm())));
         const soapgb_activity *act = boxes->act;
         SOAP_TRACED(ctx, "fir_lists",
                     k_fir_blists<<<n_lists, FIR_BLIST_THREADS, smem, ctx->stream>>>(
@@ -3018,8 +3019,9 @@ static int launch_tiles(soapgb_ctx *ctx, const FirLayout &L, char *ws, int n, in
     }
     const int n_plan = lists ? pa->n_run : n_lists;
     if ((stage & 1) && n_plan > 0) {
-        size_t smem_p = ((sizeof(FirPrePlan<T>) + 15) & ~size_t(15)) + sizeof(FirSeg) * 2 * (size_t)L.seg_cap;
-        SOAP_CUDA(ctx, cudaFuncSetAttribute(k_fir_plan<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_p));
+        const size_t fixed = (sizeof(FirPrePlan<T>) + 15) & ~size_t(15);
+        size_t smem_p = fixed + sizeof(FirSeg) * 2 * (size_t)L.seg_cap;
+        SOAP_CUDA(ctx, soap_allow_smem(k_fir_plan<T>, fixed + sizeof(FirSeg) * 2 * (size_t)FIR_SEG_MAX));
         SOAP_TRACED(ctx, "fir_plan", k_fir_plan<T><<<dim3(ntile, n_plan), FIR_PLAN_THREADS, smem_p, ctx->stream>>>(A));
         SOAP_LAUNCHED(ctx);
     }
@@ -3033,7 +3035,7 @@ static int launch_tiles(soapgb_ctx *ctx, const FirLayout &L, char *ws, int n, in
         const int nrun = ntile * (r1 - r0);
         size_t smem_t = fir_pp_smem_fixed<T>() + sizeof(FirSeg) * 2 * (size_t)L.seg_cap;
         auto kern = ctx->fir_compensated ? k_fir_pp<T, true, false> : k_fir_pp<T, false, false>;
-        SOAP_CUDA(ctx, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_t));
+        SOAP_CUDA(ctx, soap_allow_smem(kern, fir_pp_smem_fixed<T>() + sizeof(FirSeg) * 2 * (size_t)FIR_SEG_MAX));
         int per_sm = 0;
         SOAP_CUDA(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, FIR_THREADS, smem_t));
         const int nblk = std::max(1, std::min(nrun, std::max(per_sm, 1) * std::max(ctx->num_sms, 1)));
@@ -3064,9 +3066,11 @@ int fir_quiet_pair(soapgb_ctx *ctx, int n, const soapgb_cubes &c, void *dst) {
 template <typename T, int NQ>
 static int launch_quiet(soapgb_ctx *ctx, const FirTileArgs &A) {
     const int stage_slopes = A.gm <= FirListCap<T>::N;
-    const size_t smem = fir_smem_fixed<T, NQ>() + ((sizeof(FirSeg) * (size_t)A.seg_cap + 15) & ~size_t(15)) +
-                        (stage_slopes ? sizeof(double) * (size_t)A.gm : 0);
-    SOAP_CUDA(ctx, cudaFuncSetAttribute(k_fir_quiet<T, NQ>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    auto bytes = [](size_t seg_cap, size_t slopes) {
+        return fir_smem_fixed<T, NQ>() + ((sizeof(FirSeg) * seg_cap + 15) & ~size_t(15)) + sizeof(double) * slopes;
+    };
+    const size_t smem = bytes((size_t)A.seg_cap, stage_slopes ? (size_t)A.gm : 0);
+    SOAP_CUDA(ctx, soap_allow_smem(k_fir_quiet<T, NQ>, bytes(FIR_SEG_MAX, FirListCap<T>::N)));
     // tiles cover [0, n): tiles past n_eff only write the zero tail
     SOAP_TRACED(ctx, "fir_tile_quiet",
                 k_fir_quiet<T, NQ><<<(A.n + FIR_TILE - 1) / FIR_TILE, FIR_QUIET_THREADS<T, NQ>, smem, ctx->stream>>>(
@@ -3234,7 +3238,7 @@ int fir_phase_multi(soapgb_ctx *ctx, int form, const void *star0_args, const voi
     // every star's segments fit the capacity of the cubes' mu bins (seg_cap = 2 n_mu)
     size_t smem_t = fir_pp_smem_fixed<float>() + sizeof(FirSeg) * 2 * (size_t)A0.seg_cap;
     auto kern = ctx->fir_compensated ? k_fir_pp<float, true, true> : k_fir_pp<float, false, true>;
-    SOAP_CUDA(ctx, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_t));
+    SOAP_CUDA(ctx, soap_allow_smem(kern, fir_pp_smem_fixed<float>() + sizeof(FirSeg) * 2 * (size_t)FIR_SEG_MAX));
     int per_sm = 0;
     SOAP_CUDA(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, FIR_THREADS, smem_t));
     per_sm = std::max(per_sm, 1);

@@ -425,8 +425,7 @@ int integrate_device(soapgb_ctx *ctx, int form, int n, int n_eff, const double *
                               : blocks >= 6LL * ctx->num_sms ? k_phase_plain64<true> : k_phase_plain64<false>;
         const int threads = few ? 32 * PS_WARPS : PL_THREADS;
         const size_t smem = few ? sizeof(PlainPhaseSmem) : 0;
-        if (few)
-            SOAP_CUDA(ctx, cudaFuncSetAttribute(k_phase_plain64s, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        if (few) SOAP_CUDA(ctx, soap_allow_smem(k_phase_plain64s, smem));
         SOAP_TRACED(ctx, "integrate_plain64", kern<<<g, threads, smem, ctx->stream>>>(
             n, n_eff, d_wave, dc.q_norm, dc.q_sed, dc.spot_norm, dc.fac_norm, dc.spot_sed, dc.fac_sed, (int)gm,
             d_cells, d_counts, d_temp, d_bi, geo, dm.delta, dm.limb, dm.lb, dm.region, gm, act->solar,

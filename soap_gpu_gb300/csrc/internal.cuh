@@ -248,6 +248,14 @@ __device__ __forceinline__ void soap_fma2(float &x, float &y, float a, float b, 
         : "f"(a), "f"(b), "f"(c), "f"(d));
 }
 
+// The dynamic shared memory that a kernel may be launched with.  The setting belongs to the process:
+// `most` is the most that any call of the kernel needs, not this call's size, so that a thread with
+// another context cannot lower it between a call's setting and its launch.
+template <typename K>
+inline cudaError_t soap_allow_smem(K kernel, size_t most) {
+    return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most);
+}
+
 // Correctly rounded quotients (the bits of __ddiv_rn) on the integer pipes: with the divisor's
 // 64-bit reciprocal at hand, a 64-bit product gives the quotient's significand with 10 bits to
 // spare, which decide the rounding; only a quotient within their error of a rounding boundary (a

@@ -71,6 +71,8 @@ __device__ __forceinline__ const double *soap_base_for(int s, const double *base
     return base_a;
 }
 
+constexpr size_t CONV_SMEM_MAX = 200 * 1024;   // of every convolution kernel's block
+
 // ---------------------------------------------------------------------------
 // PLAIN64 convolution: conv_inst term by term (the reference's operations in its order).
 // ---------------------------------------------------------------------------
@@ -130,7 +132,6 @@ __global__ void __launch_bounds__(256) k_conv_plain64(int n, int n_eff, const do
 // 3.28 -> 0.71 ms per call; 10 of 100,000 px: 13.9 -> 0.45 ms.
 constexpr int CP_PIX = 128;
 constexpr double CP_CUT = 90.0;
-constexpr int CP_SMEM_MAX = 200 * 1024;
 
 __global__ void __launch_bounds__(CP_PIX) k_conv_plain64t(int n, int n_eff, const double *__restrict__ lam,
                                                          const double *__restrict__ spec, long long spec_stride,
@@ -252,7 +253,7 @@ static int conv_plain64_launch(soapgb_ctx *ctx, int n, int n_eff, int n_spec, co
                                double step_exp, double *conv) {
     const int reach = conv_reach(sigma_v, wave0, wave_last, step_exp, wid);
     const size_t smem = sizeof(double) * ((size_t)(reach + 1) * CP_PIX + CP_PIX + 2 * (size_t)wid);
-    if (smem > (size_t)CP_SMEM_MAX) {
+    if (smem > CONV_SMEM_MAX) {
         dim3 g(grid_for(ctx, n_eff, 256), n_spec);
         SOAP_TRACED(ctx, "conv_plain64", k_conv_plain64<<<g, 256, 0, ctx->stream>>>(
             n, n_eff, d_wave, d_spec, spec_stride, base_a, base_b, b_every, sigma_v, wid, step_mult, step_exp, conv,
@@ -260,7 +261,7 @@ static int conv_plain64_launch(soapgb_ctx *ctx, int n, int n_eff, int n_spec, co
         SOAP_LAUNCHED(ctx);
         return SOAPGB_OK;
     }
-    SOAP_CUDA(ctx, cudaFuncSetAttribute(k_conv_plain64t, cudaFuncAttributeMaxDynamicSharedMemorySize, CP_SMEM_MAX));
+    SOAP_CUDA(ctx, soap_allow_smem(k_conv_plain64t, CONV_SMEM_MAX));
     const int bx = (n_eff + CP_PIX - 1) / CP_PIX;
     const int per = conv_per_block(ctx, bx, n_spec, 20LL * (reach + 1), 2LL * (2 * reach + 1));
     const int groups = (n_spec + per - 1) / per;
@@ -1342,10 +1343,8 @@ static int launch_conv_fast(soapgb_ctx *ctx, int n, int n_eff, const double *lam
     int halo = std::min(wid, r);
     if (halo < 1) halo = 1;
     size_t smem = sizeof(T) * (size_t)SB * (FC_TILE + 2 * halo);
-    if (smem > 200 * 1024) return set_error(ctx, SOAPGB_ERR_ARG, "convolution window too wide (%d px)", halo);
-    if (smem > 48 * 1024)
-        SOAP_CUDA(ctx, cudaFuncSetAttribute(k_conv_fast<T, SB, SrcT, OutT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                            (int)smem));
+    if (smem > CONV_SMEM_MAX) return set_error(ctx, SOAPGB_ERR_ARG, "convolution window too wide (%d px)", halo);
+    if (smem > 48 * 1024) SOAP_CUDA(ctx, soap_allow_smem(k_conv_fast<T, SB, SrcT, OutT>, CONV_SMEM_MAX));
     T *kq = (T *)param_scratch;
     T *cq = (T *)(param_scratch + ((sizeof(T) * (size_t)n_eff + 255) & ~size_t(255)));
     int2 *rng = (int2 *)(param_scratch + 2 * ((sizeof(T) * (size_t)n_eff + 255) & ~size_t(255)));
@@ -1379,10 +1378,9 @@ static int launch_conv_base_df(soapgb_ctx *ctx, int n, int n_eff, const double *
     const int threads = (n_eff + FC_TILE - 1) / FC_TILE < ctx->num_sms ? FC_THREADS / 4 : FC_THREADS;
     const int tile = threads * FC_PIX;
     const size_t smem = sizeof(float2) * (size_t)SB * (tile + 2 * halo);
-    if (sizeof(float2) * (size_t)SB * (FC_TILE + 2 * halo) > 200 * 1024)
+    if (sizeof(float2) * (size_t)SB * (FC_TILE + 2 * halo) > CONV_SMEM_MAX)
         return set_error(ctx, SOAPGB_ERR_ARG, "convolution window too wide (%d px)", halo);
-    if (smem > 48 * 1024)
-        SOAP_CUDA(ctx, cudaFuncSetAttribute(k_conv_base_df<SB>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    if (smem > 48 * 1024) SOAP_CUDA(ctx, soap_allow_smem(k_conv_base_df<SB>, CONV_SMEM_MAX));
     SOAP_TRACED(ctx, "conv_base", k_conv_base_df<SB><<<(n_eff + tile - 1) / tile, threads, smem, ctx->stream>>>(
                                       n, n_eff, kq, cq, rng, base_a, base_b, halo, conv, n_eff));
     SOAP_LAUNCHED(ctx);
@@ -1408,8 +1406,8 @@ static int conv32_run(soapgb_ctx *ctx, int n, int n_eff, int wid, int halo, cons
         // TMA staging, double buffered: a block keeps its tile over several spectrum batches
         const int win_t = (FC_TILE + 2 * halo + 12 + 3) & ~3;
         size_t smem_t = sizeof(float) * 2 * (size_t)SB * win_t;
-        if (smem_t > 200 * 1024) return set_error(ctx, SOAPGB_ERR_ARG, "convolution window too wide (%d px)", halo);
-        SOAP_CUDA(ctx, cudaFuncSetAttribute(k_conv32t<SB>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_t));
+        if (smem_t > CONV_SMEM_MAX) return set_error(ctx, SOAPGB_ERR_ARG, "convolution window too wide (%d px)", halo);
+        SOAP_CUDA(ctx, soap_allow_smem(k_conv32t<SB>, CONV_SMEM_MAX));
         const int nwalk = rows ? (nrows + SB - 1) / SB : nbatch;
         if (nwalk == 0) return SOAPGB_OK;   // every spectrum is zero
         int per_sm = 0;
@@ -1428,9 +1426,8 @@ static int conv32_run(soapgb_ctx *ctx, int n, int n_eff, int wid, int halo, cons
     } else {
         const int win = (FC_TILE + 2 * halo + 4 + 3) & ~3;
         size_t smem = sizeof(float) * (size_t)SB * win;
-        if (smem > 200 * 1024) return set_error(ctx, SOAPGB_ERR_ARG, "convolution window too wide (%d px)", halo);
-        if (smem > 48 * 1024)
-            SOAP_CUDA(ctx, cudaFuncSetAttribute(k_conv32x<SB>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        if (smem > CONV_SMEM_MAX) return set_error(ctx, SOAPGB_ERR_ARG, "convolution window too wide (%d px)", halo);
+        if (smem > 48 * 1024) SOAP_CUDA(ctx, soap_allow_smem(k_conv32x<SB>, CONV_SMEM_MAX));
         dim3 g(nbx, nbatch);
         SOAP_TRACED(ctx, "conv32", k_conv32x<SB><<<g, FC_THREADS, smem, ctx->stream>>>(n, n_eff, c2, lk, live, rblk, wid, spec, spec_stride,
                                                            n_spec, halo, b32a, b32b, c32a, c32b, b_every, conv, n_eff,
@@ -2025,9 +2022,9 @@ extern "C" int soapgb_lower_resolution_adjoint(soapgb_ctx *ctx, int n, int n_eff
     // twice), 128 where the reach is long, the general form where neither fits
     const int reach = conv_reach(sigma_v, w01[0], w01[2], step_exp, wid);
     auto smem_of = [&](int T) { return sizeof(double) * (size_t)(reach + 2) * (T + 2 * (size_t)reach); };
-    const int T = smem_of(256) <= (size_t)CP_SMEM_MAX / 2 ? 256 : smem_of(128) <= (size_t)CP_SMEM_MAX ? 128 : 0;
+    const int T = smem_of(256) <= CONV_SMEM_MAX / 2 ? 256 : smem_of(128) <= CONV_SMEM_MAX ? 128 : 0;
     if (T) {
-        SOAP_CUDA(ctx, cudaFuncSetAttribute(k_radj_spect, cudaFuncAttributeMaxDynamicSharedMemorySize, CP_SMEM_MAX));
+        SOAP_CUDA(ctx, soap_allow_smem(k_radj_spect, CONV_SMEM_MAX));
         const int bx = (n + T - 1) / T;
         const int per = conv_per_block(ctx, bx, n_spec, 20LL * (reach + 1) * (T + 2 * reach) / T, 2LL * reach + 1);
         const int groups = (n_spec + per - 1) / per;
