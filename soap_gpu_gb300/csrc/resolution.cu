@@ -76,15 +76,24 @@ constexpr size_t CONV_SMEM_MAX = 200 * 1024;   // of every convolution kernel's 
 // ---------------------------------------------------------------------------
 // PLAIN64 convolution: conv_inst term by term (the reference's operations in its order).
 // ---------------------------------------------------------------------------
+// +0 or -0, on the integer pipes
+__device__ __forceinline__ bool conv_zero(double v) {
+    return (((unsigned)__double2hiint(v) << 1) | (unsigned)__double2loint(v)) == 0u;
+}
+
 // one pixel of one spectrum over every tap of the reference's window
 __device__ __noinline__ double conv_plain64_pixel(int index, int wid, double step_mult, double step_exp, double norm, double den,
                                      const double *__restrict__ sp, const double *__restrict__ bp) {
     double acc = 0.0;
+    // a term of 1 - A = 0 adds a zero where its weight is finite (-d * d stays negative)
+    const bool skip = norm > 0.0 && den > 0.0 && step_exp * step_exp < INFINITY && wid <= 46340;
     for (int m = index - wid; m < index + wid - 1; m++) {
         int d = m - index;
         double a = bp ? __dsub_rn(bp[m], sp[m]) : sp[m];
+        double y = __dmul_rn(step_mult, __dsub_rn(1.0, a));
+        if (skip && conv_zero(y)) continue;
         double e = exp(__ddiv_rn(__dmul_rn(__dmul_rn((double)(-d * d), step_exp), step_exp), den));
-        double t = __dmul_rn(__ddiv_rn(__dmul_rn(__dmul_rn(step_mult, __dsub_rn(1.0, a)), 1.), norm), e);
+        double t = __dmul_rn(__ddiv_rn(__dmul_rn(y, 1.), norm), e);
         acc = __dadd_rn(acc, t);
     }
     return acc;
@@ -123,8 +132,9 @@ __global__ void __launch_bounds__(256) k_conv_plain64(int n, int n_eff, const do
 // ulp; to the left, what the early partial sums lack (2^-122 of the largest term) is rounded away
 // as the weights grow, but for a chance of 2^-70 per pixel, 2^-38 for a sum at the bound.  A
 // smaller sum (terms of either sign) is taken over all taps by conv_plain64_pixel, and so are the
-// pixels of a block whose window holds zeros, infinities, NaN or values beyond 2^800.  (The test is
-// per pixel: with one on the block's range of terms, the one block at a spectrum's edge where
+// pixels of a block whose window holds infinities, NaN or values beyond 2^800.  A term of exactly zero
+// (a continuum of 1) is staged as 2^-790, which the sums of terms above 2^-600 do not hold; a block of
+// such terms alone has sums of zero.  (The test is per pixel: with one on the block's range of terms, the one block at a spectrum's edge where
 // 1 - A changes its sign took 6.4 ms of a call of 11 phases that takes 0.7 ms otherwise; one pixel
 // over all taps takes 0.35 ms, so the bound lies where next to none is.)
 // Bound by the FP64 pipe: (2 reach + 1) x 2 instructions per pixel and spectrum and
@@ -132,6 +142,7 @@ __global__ void __launch_bounds__(256) k_conv_plain64(int n, int n_eff, const do
 // 3.28 -> 0.71 ms per call; 10 of 100,000 px: 13.9 -> 0.45 ms.
 constexpr int CP_PIX = 128;
 constexpr double CP_CUT = 90.0;
+constexpr int CP_ZERO = 1023 - 790;   // exponent of what stands for a term of zero
 
 __global__ void __launch_bounds__(CP_PIX) k_conv_plain64t(int n, int n_eff, const double *__restrict__ lam,
                                                          const double *__restrict__ spec, long long spec_stride,
@@ -172,6 +183,7 @@ __global__ void __launch_bounds__(CP_PIX) k_conv_plain64t(int n, int n_eff, cons
         const double *sp = spec + (long long)s * spec_stride;
         const double *bp = soap_base_for(s, base_a, base_b, b_every);
         unsigned mn = 0xffffffffu, mx = 0u;   // high words of |term| over the window (they order as the values)
+        int none = 0;                         // a term of zero
         __syncthreads();                      // the previous spectrum's terms and extrema are read
         for (int q = t; q < win; q += CP_PIX) {
             const int m = i0 - wid + q;
@@ -179,9 +191,14 @@ __global__ void __launch_bounds__(CP_PIX) k_conv_plain64t(int n, int n_eff, cons
             if (m >= 0 && m < n) {
                 const double a = bp ? __dsub_rn(bp[m], sp[m]) : sp[m];
                 y = __dmul_rn(step_mult, __dsub_rn(1.0, a));
-                const unsigned h = (unsigned)__double2hiint(y) & 0x7fffffffu;
-                mn = min(mn, h);
-                mx = max(mx, h);
+                if (conv_zero(y)) {
+                    y = __hiloint2double(CP_ZERO << 20, 0);
+                    none = 1;
+                } else {
+                    const unsigned h = (unsigned)__double2hiint(y) & 0x7fffffffu;
+                    mn = min(mn, h);
+                    mx = max(mx, h);
+                }
             }
             ys[q] = y;
         }
@@ -191,16 +208,16 @@ __global__ void __launch_bounds__(CP_PIX) k_conv_plain64t(int n, int n_eff, cons
             s_mn[t >> 5] = mn;
             s_mx[t >> 5] = mx;
         }
-        __syncthreads();
+        none = __syncthreads_or(none);
 #pragma unroll
         for (int w = 0; w < CP_PIX / 32; ++w) {
             mn = min(mn, s_mn[w]);
             mx = max(mx, s_mx[w]);
         }
-        // exponents within 2^-800 .. 2^800
-        const bool whole = odd_block || mn < (223u << 20) || mx > (1823u << 20);
+        // exponents within 2^-800 .. 2^800, beside zeros above 2^-600
+        const bool whole = odd_block || mn < (223u << 20) || mx > (1823u << 20) || (none && mx < (423u << 20));
         double acc = 0.0;
-        if (live) {
+        if (live && (odd_block || mn <= mx)) {   // else zeros alone
             bool all_taps = whole;
             if (!whole) {
                 const double *yc = ys + t + wid;

@@ -410,3 +410,31 @@ def test_shifted_wavelengths_at_a_power_of_two(ctx, n):
                                       Activity(5778, 663, 250, 20, 0))
             for o, r in zip(out, want):
                 assert all(np.array_equal(v, r) for v in o)
+
+
+@pytest.mark.parametrize("kind", ["one", "stretch", "lines", "flat", "tiny"])
+def test_plain_convolution_with_terms_of_zero(ctx, kind):
+    """1 - A exactly zero at one pixel, over a stretch longer than a window, between lines, everywhere
+    but at a few pixels, and beside terms of one ulp (tolerance as above; a spectrum of zeros alone
+    keeps the sentinel)."""
+    n, n_eff, step = 3000, 2560, 0.01
+    rng = np.random.default_rng(5)
+    wave, sv, x = 5000.0 + step * np.arange(n), _sigma_v(115000.0), np.arange(n)
+    a = np.tile(1.0 - 0.5 * np.exp(-((x % 97) - 40.0) ** 2 / 18.0) * (1 + 0.1 * rng.uniform(-1, 1, n)), (3, 1))
+    if kind == "one":
+        a[:, [700, 1500]] = 1.0
+    if kind == "stretch":
+        a[:, 900:1400] = 1.0
+    if kind == "lines":
+        a = _spectra("unit", n, n_eff, 3, rng)
+    if kind == "flat":
+        a[:] = 1.0
+        a[0, [640, 1300]], a[1, 2000] = 0.4, 2.0
+    if kind == "tiny":
+        a[:] = 1.0 + 2.0 ** -52 * (x % 3 - 1)
+        a[1, 1000:1300] = 1.0
+    got, mm = ctx.lower_resolution("plain64", wave, a, n_eff, sv, step_mult=step, step_exp=step)
+    for s in range(3):
+        ref, conv, ext = oracle.lower_resolution(wave, a[s], n_eff, sv, step_mult=step, step_exp=step)
+        assert np.allclose(mm[s], ext, rtol=1e-12, atol=0)
+        assert np.max(np.abs(got[s] - ref)) <= 1e-12 * np.max(np.abs(ref))
