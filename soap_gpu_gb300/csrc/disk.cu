@@ -6,6 +6,7 @@
 // spectrum.  Here one launch sums all cells: every thread owns output pixels and
 // gathers, for each cell in iy-major order, the source interval that covers the
 // pixel (the interval-owning form of the scatter; see soap_owner()).
+#include <algorithm>
 #include <cmath>
 #include <vector>
 
@@ -155,10 +156,10 @@ __global__ void __launch_bounds__(64) k_plain_cells(long long gm, int n_eff, con
 }
 
 namespace soapgb {
-int plain_cells(soapgb_ctx *ctx, long long gm, int n_eff, const double *d_wave, const double *d_delta, double step,
-                PlainGeo *geo) {
-    SOAP_TRACED(ctx, "plain_cells", k_plain_cells<<<(unsigned)((gm + 63) / 64), 64, 0, ctx->stream>>>(
-                                        gm, n_eff, d_wave, d_delta, step, geo));
+int plain_cells(soapgb_ctx *ctx, long long k0, long long k1, int n_eff, const double *d_wave, const double *d_delta,
+                double step, PlainGeo *geo) {
+    SOAP_TRACED(ctx, "plain_cells", k_plain_cells<<<(unsigned)((k1 - k0 + 63) / 64), 64, 0, ctx->stream>>>(
+                                        k1 - k0, n_eff, d_wave, d_delta + k0, step, geo));
     SOAP_LAUNCHED(ctx);
     return SOAPGB_OK;
 }
@@ -216,12 +217,12 @@ __device__ __forceinline__ void quiet_stage(int k, const PlainGeo *__restrict__ 
     pl_stage(geo + k, delta_m[k], limb_m[k], row, j0, cnt, lmid, rec, tab);
 }
 
-// A block takes PL_TILE pixels, a thread one, all cells in order.  Small blocks: 100,000 px
-// are 10.6 blocks per SM.
+// A block takes PL_TILE pixels, a thread one, all cells of [k0, k1) in order (geo: of cell k0 on; the
+// sums of the cells before k0 in out).  Small blocks: 100,000 px are 10.6 blocks per SM.
 __global__ void __launch_bounds__(PL_THREADS) k_quiet_plain64(int n, int n_eff, const double *__restrict__ lam,
                                                               const double *__restrict__ cube,
                                                               const int *__restrict__ n_cells_ptr,
-                                                              const int *__restrict__ cells,
+                                                              const int *__restrict__ cells, int k0, int k1,
                                                               const PlainGeo *__restrict__ geo,
                                                               const double *__restrict__ delta_m,
                                                               const double *__restrict__ limb_m,
@@ -236,11 +237,13 @@ __global__ void __launch_bounds__(PL_THREADS) k_quiet_plain64(int n, int n_eff, 
     const double lmid = lam[min(j0 + cnt / 2, n_eff - 1)];
     const bool mine = j < n_eff && lane != 31;
     const double lj = lam[min(j, n_eff - 1)];
-    double sum = 0.0;
+    double sum = k0 > 0 && mine ? out[j] : 0.0;
     QuietAt at;
-    const int n_cells = *n_cells_ptr;
-    for (int c0 = 0; c0 < n_cells; c0 += PL_CHUNK) {
-        const int nc = min(PL_CHUNK, n_cells - c0);
+    int from, to;
+    pl_slab(cells, *n_cells_ptr, k0, k1, from, to);
+    geo -= k0;
+    for (int c0 = from; c0 < to; c0 += PL_CHUNK) {
+        const int nc = min(PL_CHUNK, to - c0);
         __syncthreads();
         if (threadIdx.x < nc) {
             const int k = cells[c0 + threadIdx.x];
@@ -289,7 +292,7 @@ struct PlainQuietSmem {   // chunks, double buffered
 
 __global__ void __launch_bounds__(32 * PQ_WARPS, 2) k_quiet_plain64s(
     int n, int n_eff, const double *__restrict__ lam, const double *__restrict__ cube,
-    const int *__restrict__ n_cells_ptr, const int *__restrict__ cells, const PlainGeo *__restrict__ geo,
+    const int *__restrict__ n_cells_ptr, const int *__restrict__ cells, int k0, int k1, const PlainGeo *__restrict__ geo,
     const double *__restrict__ delta_m, const double *__restrict__ limb_m, const int *__restrict__ region_m, int n_mu,
     double *__restrict__ out, int *status) {
     extern __shared__ __align__(16) unsigned char pq_smem[];
@@ -300,7 +303,11 @@ __global__ void __launch_bounds__(32 * PQ_WARPS, 2) k_quiet_plain64s(
     const double lmid = lam[min(j0 + cnt / 2, n_eff - 1)];
     const bool mine = j < n_eff && lane != 31;
     const double lj = lam[min(j, n_eff - 1)];
-    const int n_cells = *n_cells_ptr, n_chunk = (n_cells + PQ_CHUNK - 1) / PQ_CHUNK;
+    int from, to;
+    pl_slab(cells, *n_cells_ptr, k0, k1, from, to);
+    cells += from;
+    geo -= k0;
+    const int n_cells = to - from, n_chunk = (n_cells + PQ_CHUNK - 1) / PQ_CHUNK;
     QuietAt at;
     auto stage = [&](int c) {   // the records of chunk c, by one warp
         const int b = c & 1;
@@ -310,7 +317,7 @@ __global__ void __launch_bounds__(32 * PQ_WARPS, 2) k_quiet_plain64s(
             quiet_stage(k, geo, delta_m, limb_m, region_m, n_mu, j0, cnt, lmid, sh.rec[b][t], sh.tab[b][t], status);
         }
     };
-    if (warp < PQ_STRIPS) sh.sum[warp][lane] = 0.0;
+    if (warp < PQ_STRIPS) sh.sum[warp][lane] = k0 > 0 && mine ? out[j] : 0.0;
     if (threadIdx.x < PQ_STRIPS) sh.next[0][threadIdx.x] = 0;
     if (warp == 0) stage(0);
     // step c: the sum over chunk c - 1, the records of chunk c + 1 (strip 0), the terms of chunk c
@@ -497,20 +504,25 @@ extern "C" int soapgb_quiet_disk(soapgb_ctx *ctx, int form, int n, int n_eff, co
         rc = compact_cells(ctx, 1, (int)gm, d_limb, -998.0, 1e300, (int)gm, d_cells, d_count);
         if (rc) return rc;
         PlainGeo *geo = ws.get<PlainGeo>(s_fir);
-        rc = plain_cells(ctx, gm, n_eff, d_wave, d_delta, step, geo);
-        if (rc) return rc;
         const int ntile = (n + PL_TILE - 1) / PL_TILE;
-        if (ntile <= 4 * ctx->num_sms) {
-            SOAP_CUDA(ctx, soap_allow_smem(k_quiet_plain64s, sizeof(PlainQuietSmem)));
-            SOAP_TRACED(ctx, "quiet_plain64",
-                        k_quiet_plain64s<<<ntile, 32 * PQ_WARPS, sizeof(PlainQuietSmem), ctx->stream>>>(
-                            n, n_eff, d_wave, d_cube, d_count, d_cells, geo, d_delta, d_limb, d_region, n_mu, d_out,
-                            ctx->d_status));
-        } else {
-            SOAP_TRACED(ctx, "quiet_plain64", k_quiet_plain64<<<ntile, PL_THREADS, 0, ctx->stream>>>(
-                n, n_eff, d_wave, d_cube, d_count, d_cells, geo, d_delta, d_limb, d_region, n_mu, d_out, ctx->d_status));
+        for (long long k0 = 0; k0 < gm; k0 += PL_SLAB) {
+            const long long end = std::min(gm, k0 + PL_SLAB);
+            const int k1 = end < gm ? (int)end : INT_MAX;
+            rc = plain_cells(ctx, k0, end, n_eff, d_wave, d_delta, step, geo);
+            if (rc) return rc;
+            if (ntile <= 4 * ctx->num_sms) {
+                SOAP_CUDA(ctx, soap_allow_smem(k_quiet_plain64s, sizeof(PlainQuietSmem)));
+                SOAP_TRACED(ctx, "quiet_plain64",
+                            k_quiet_plain64s<<<ntile, 32 * PQ_WARPS, sizeof(PlainQuietSmem), ctx->stream>>>(
+                                n, n_eff, d_wave, d_cube, d_count, d_cells, (int)k0, k1, geo, d_delta, d_limb, d_region,
+                                n_mu, d_out, ctx->d_status));
+            } else {
+                SOAP_TRACED(ctx, "quiet_plain64", k_quiet_plain64<<<ntile, PL_THREADS, 0, ctx->stream>>>(
+                    n, n_eff, d_wave, d_cube, d_count, d_cells, (int)k0, k1, geo, d_delta, d_limb, d_region, n_mu, d_out,
+                    ctx->d_status));
+            }
+            SOAP_LAUNCHED(ctx);
         }
-        SOAP_LAUNCHED(ctx);
     } else {
         FirQuietArgs qa;
         qa.n = n;

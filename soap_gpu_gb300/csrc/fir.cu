@@ -2774,7 +2774,7 @@ FirLayout fir_layout(int form, int n, int n_mu, long long gm, int ncube, int n_l
 FirPlanSizes fir_plan_sizes(int form, int n, int n_mu, long long gm, bool phase, int n_lists, bool typed_external) {
     FirPlanSizes p;
     if (form == SOAPGB_PLAIN64) {   // the cells' Doppler constants
-        p.bytes = sizeof(PlainGeo) * (size_t)gm;
+        p.bytes = sizeof(PlainGeo) * (size_t)std::min(gm, PL_SLAB);
         return p;
     }
     p.bytes = fir_layout(form, n, n_mu, gm, phase ? 6 : 1, n_lists > 0 ? n_lists : 1, typed_external).total;

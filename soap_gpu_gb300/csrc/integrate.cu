@@ -6,6 +6,7 @@
 // kernels).  Here one launch covers every phase: block (x, p) owns a pixel range
 // of phase p and gathers all of the phase's active cells, in map order, into
 // register accumulators.
+#include <algorithm>
 #include <cmath>
 
 #include "internal.cuh"
@@ -76,7 +77,8 @@ __device__ __forceinline__ PhaseCell phase_cell(int k, double T, double b, const
 }
 
 // The plain form: block (x, p) sums phase p's active cells, in map order, over a tile of
-// pixels (plain64.cuh); three rows per cell.  INT: the five products of a cell and pixel on the
+// pixels (plain64.cuh); three rows per cell; the cells [k0, k1), geo of cell k0 on, the sums of those
+// before in flux, bconv and tot.  INT: the five products of a cell and pixel on the
 // integer pipes (18.4 -> 13 FP64 instructions, 285 -> 440 in all), which pays where the FP64 pipe
 // is the bound: 5 phases of 200 x 200 cells and 100,000 px, 8.2 -> 6.1 ms; 11 phases of 151 x 151
 // and 60,001 px, 7.0 -> 5.2 ms; at 6.4 blocks per SM 0.340 -> 0.317 ms.  With fewer the pipe waits
@@ -87,7 +89,7 @@ __global__ void __launch_bounds__(PL_THREADS) k_phase_plain64(
     int n, int n_eff, const double *__restrict__ lam, const double *__restrict__ q_norm,
     const double *__restrict__ q_sed, const double *__restrict__ spot_norm, const double *__restrict__ fac_norm,
     const double *__restrict__ spot_sed, const double *__restrict__ fac_sed, int max_cells,
-    const int *__restrict__ cells, const int *__restrict__ counts, const double *__restrict__ temp,
+    const int *__restrict__ cells, const int *__restrict__ counts, int k0, int k1, const double *__restrict__ temp,
     const double *__restrict__ bi, const PlainGeo *__restrict__ geo, const double *__restrict__ delta_m,
     const double *__restrict__ limb_m, const double *__restrict__ lb_m, const int *__restrict__ region_m,
     long long gm, int solar, int t_star, int t_diff_fac, double *__restrict__ flux, double *__restrict__ bconv,
@@ -99,7 +101,9 @@ __global__ void __launch_bounds__(PL_THREADS) k_phase_plain64(
     const int j0 = blockIdx.x * PL_TILE, j = j0 + (threadIdx.x >> 5) * 31 + lane;
     const int cnt = max(1, min(PL_TILE, n_eff - j0));
     const int *pc = cells + (long long)p * max_cells;
-    const int nc_all = counts[p];
+    int from, to;
+    pl_slab(pc, counts[p], k0, k1, from, to);
+    geo -= k0;
     const double *pt = temp + (long long)p * gm;
     const double *pb = bi + (long long)p * gm;
     const double lmid = lam[min(j0 + cnt / 2, n_eff - 1)];
@@ -109,11 +113,17 @@ __global__ void __launch_bounds__(PL_THREADS) k_phase_plain64(
     const double lj = lam[jc], ssed = spot_sed[jc], fsed = fac_sed[jc];
     const PlainFactor by_s = pl_factor(ssed), by_f = pl_factor(fsed);
     double fx = 0.0, bc = 0.0, tt = 0.0;
+    if (k0 > 0 && mine) {
+        const long long o = (long long)p * out_stride + j;
+        fx = flux[o];
+        bc = bconv[o];
+        tt = tot[o];
+    }
     PlainPix px;
     PlainVal va[3];
     int row_now = -1, m_now = 0, type_now = 0;
-    for (int c0 = 0; c0 < nc_all; c0 += PL_CHUNK) {
-        const int nc = min(PL_CHUNK, nc_all - c0);
+    for (int c0 = from; c0 < to; c0 += PL_CHUNK) {
+        const int nc = min(PL_CHUNK, to - c0);
         __syncthreads();
         if (threadIdx.x < nc) {
             const int k = pc[c0 + threadIdx.x];
@@ -257,7 +267,7 @@ __global__ void __launch_bounds__(32 * PS_WARPS, 2) k_phase_plain64s(
     int n, int n_eff, const double *__restrict__ lam, const double *__restrict__ q_norm,
     const double *__restrict__ q_sed, const double *__restrict__ spot_norm, const double *__restrict__ fac_norm,
     const double *__restrict__ spot_sed, const double *__restrict__ fac_sed, int max_cells,
-    const int *__restrict__ cells, const int *__restrict__ counts, const double *__restrict__ temp,
+    const int *__restrict__ cells, const int *__restrict__ counts, int k0, int k1, const double *__restrict__ temp,
     const double *__restrict__ bi, const PlainGeo *__restrict__ geo, const double *__restrict__ delta_m,
     const double *__restrict__ limb_m, const double *__restrict__ lb_m, const int *__restrict__ region_m,
     long long gm, int solar, int t_star, int t_diff_fac, double *__restrict__ flux, double *__restrict__ bconv,
@@ -268,7 +278,11 @@ __global__ void __launch_bounds__(32 * PS_WARPS, 2) k_phase_plain64s(
     const int j0 = blockIdx.x * PL_TILE, j = j0 + strip * 31 + lane;
     const int cnt = max(1, min(PL_TILE, n_eff - j0));
     const int *pc = cells + (long long)p * max_cells;
-    const int n_cells = counts[p], n_chunk = (n_cells + PS_CHUNK - 1) / PS_CHUNK;
+    int from, to;
+    pl_slab(pc, counts[p], k0, k1, from, to);
+    pc += from;
+    geo -= k0;
+    const int n_cells = to - from, n_chunk = (n_cells + PS_CHUNK - 1) / PS_CHUNK;
     const double *pt = temp + (long long)p * gm;
     const double *pb = bi + (long long)p * gm;
     const double lmid = lam[min(j0 + cnt / 2, n_eff - 1)];
@@ -347,8 +361,13 @@ __global__ void __launch_bounds__(32 * PS_WARPS, 2) k_phase_plain64s(
         to[3][lane] = v;
         to[4][lane] = __dmul_rn(v, I);
     };
-    if (warp < PS_STRIPS)
-        for (int q = 0; q < 3; ++q) sh.sum[warp][q][lane] = 0.0;
+    if (warp < PS_STRIPS) {
+        const bool more = k0 > 0 && mine;
+        const long long o = (long long)p * out_stride + j;
+        sh.sum[warp][0][lane] = more ? flux[o] : 0.0;
+        sh.sum[warp][1][lane] = more ? bconv[o] : 0.0;
+        sh.sum[warp][2][lane] = more ? tot[o] : 0.0;
+    }
     if (threadIdx.x < PS_STRIPS) sh.next[0][threadIdx.x] = 0;
     if (warp == 0) stage(0);
     // step c: the sums over chunk c - 1, the records of chunk c + 1 (strip 0), the terms of chunk c
@@ -416,8 +435,6 @@ int integrate_device(soapgb_ctx *ctx, int form, int n, int n_eff, const double *
         int rc = compact_cells(ctx, n_phase, (int)gm, d_bi, -0.5, 1.5, (int)gm, d_cells, d_counts);
         if (rc) return rc;
         PlainGeo *geo = (PlainGeo *)fir_scratch;   // PLAIN64 has no plans: its cells' constants stand there
-        rc = plain_cells(ctx, gm, n_eff, d_wave, dm.delta, step, geo);
-        if (rc) return rc;
         const dim3 g((n + PL_TILE - 1) / PL_TILE, n_phase);
         const long long blocks = (long long)g.x * g.y;
         const bool few = blocks <= PS_MAX_PER_SM * ctx->num_sms;
@@ -426,12 +443,17 @@ int integrate_device(soapgb_ctx *ctx, int form, int n, int n_eff, const double *
         const int threads = few ? 32 * PS_WARPS : PL_THREADS;
         const size_t smem = few ? sizeof(PlainPhaseSmem) : 0;
         if (few) SOAP_CUDA(ctx, soap_allow_smem(k_phase_plain64s, smem));
-        SOAP_TRACED(ctx, "integrate_plain64", kern<<<g, threads, smem, ctx->stream>>>(
-            n, n_eff, d_wave, dc.q_norm, dc.q_sed, dc.spot_norm, dc.fac_norm, dc.spot_sed, dc.fac_sed, (int)gm,
-            d_cells, d_counts, d_temp, d_bi, geo, dm.delta, dm.limb, dm.lb, dm.region, gm, act->solar,
-            act->t_star, act->t_diff_fac, (double *)d_flux, (double *)d_bconv, (double *)d_tot, out_stride, dc.n_mu,
-            ctx->d_status));
-        SOAP_LAUNCHED(ctx);
+        for (long long k0 = 0; k0 < gm; k0 += PL_SLAB) {
+            const long long end = std::min(gm, k0 + PL_SLAB);
+            rc = plain_cells(ctx, k0, end, n_eff, d_wave, dm.delta, step, geo);
+            if (rc) return rc;
+            SOAP_TRACED(ctx, "integrate_plain64", kern<<<g, threads, smem, ctx->stream>>>(
+                n, n_eff, d_wave, dc.q_norm, dc.q_sed, dc.spot_norm, dc.fac_norm, dc.spot_sed, dc.fac_sed, (int)gm,
+                d_cells, d_counts, (int)k0, end < gm ? (int)end : INT_MAX, d_temp, d_bi, geo, dm.delta, dm.limb, dm.lb,
+                dm.region, gm, act->solar, act->t_star, act->t_diff_fac, (double *)d_flux, (double *)d_bconv,
+                (double *)d_tot, out_stride, dc.n_mu, ctx->d_status));
+            SOAP_LAUNCHED(ctx);
+        }
         return SOAPGB_OK;
     }
     FirPhaseArgs a;

@@ -37,6 +37,8 @@
 // non-finite or extreme values) takes the reference's operations.  Every path gives the same bits.
 #pragma once
 
+#include <climits>
+
 #include "internal.cuh"
 
 constexpr int PL_THREADS = 64;                // two warps, each 31 pixels
@@ -44,6 +46,10 @@ constexpr int PL_TILE = PL_THREADS / 32 * 31;
 constexpr int PL_CHUNK = PL_THREADS;          // cells staged at a time, one per thread
 constexpr int PL_TAB = 8;                     // table entries per cell
 constexpr int PL_FRAC = 21;                   // fraction bits of l u
+// Cells whose constants are held at a time (0.94 GB).  A larger map is taken in slabs of as many
+// cells, each adding to what the ones before left: the sums' order stays, and the workspace does not
+// grow with the map's area (90 GB for 20,000 x 20,000 cells).
+constexpr long long PL_SLAB = 1LL << 22;
 
 // the table of one binade of l'
 struct PlainTab {
@@ -53,7 +59,7 @@ struct PlainTab {
     unsigned long long rec[PL_TAB];
 };
 
-// a cell's constants, computed once per call; tables for the first and the last wavelength's binade
+// a cell's constants, computed once per call and slab; tables for the first and the last wavelength's binade
 struct PlainGeo {
     double sq, fbeta, off;   // CellShift
     double u;                // 1 - sq
@@ -67,6 +73,21 @@ enum : int {
     PL_CONST = 1,   // one owner offset m for the tile
     PL_STILL = 2,   // v == 0: the pixel itself
 };
+
+// the cells [k0, k1) of a list in map order as [from, to) of it; k0 = 0 and k1 = INT_MAX: no bound
+__device__ __forceinline__ int pl_first(const int *__restrict__ cells, int n, int k) {
+    int lo = 0, hi = n;
+    while (lo < hi) {
+        const int mid = lo + ((hi - lo) >> 1);
+        if (cells[mid] < k) lo = mid + 1;
+        else hi = mid;
+    }
+    return lo;
+}
+__device__ __forceinline__ void pl_slab(const int *__restrict__ cells, int n, int k0, int k1, int &from, int &to) {
+    from = k0 > 0 ? pl_first(cells, n, k0) : 0;
+    to = k1 != INT_MAX ? pl_first(cells, n, k1) : n;
+}
 
 // a factor of many products
 struct PlainFactor {
@@ -242,7 +263,7 @@ static __device__ __noinline__ double pl_rise_plain(double g, double lj, double 
 }
 
 namespace soapgb {
-// the constants of every cell of the map, geo[gm]
-int plain_cells(soapgb_ctx *ctx, long long gm, int n_eff, const double *d_wave, const double *d_delta, double step,
-                PlainGeo *geo);
+// the constants of the map's cells [k0, k1), geo[k1 - k0]
+int plain_cells(soapgb_ctx *ctx, long long k0, long long k1, int n_eff, const double *d_wave, const double *d_delta,
+                double step, PlainGeo *geo);
 }  // namespace soapgb
