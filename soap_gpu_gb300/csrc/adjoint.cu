@@ -479,9 +479,6 @@ __device__ __forceinline__ void adj_walk(const AdjArgs &A, int p, int c, int b, 
 
 __device__ __forceinline__ int adj_exp(double v) { return (int)(((unsigned)__double2hiint(v) >> 20) & 0x7ffu); }
 
-// l'_o as the forward rounds it
-__device__ __forceinline__ double adj_shifted(double lo, double f) { return __dsub_rn(lo, __dmul_rn(lo, -f)); }
-
 __device__ __forceinline__ double adj_intensity(const AdjArgs &A, int p, int c, int k, double lj, double ssed,
                                                 double fsed) {
     // class 2: the map's temperature and the general ratio; a spot's type is read from the list's class
@@ -489,17 +486,23 @@ __device__ __forceinline__ double adj_intensity(const AdjArgs &A, int p, int c, 
     return soap_intensity(c, T, A.lb[k], lj, ssed, fsed, A.solar, A.t_norm_fac);
 }
 
+// l'_o as the forward rounds it
+__device__ __forceinline__ double adj_shifted(double lo, double f) { return __dsub_rn(lo, __dmul_rn(lo, -f)); }
+
 // The forward's l'_o is l_o - rn(l_o u) rounded to ulp(l_o), u = 1 - S: up to half an ulp, 1e-10 of
 // a pixel, from S l_o.  The row gradients take the weights of that grid, so that they are the
 // transpose of the forward to better than this: the sum over the cells [k0, k1) of L / S times the
-// residue.  The fraction bits of the 64-bit product are integers (|.| <= 2^20; the two products'
+// residue.  The fraction bits of the 64-bit product are integers (about 2^20; the two products'
 // lower halves are left out, 2^-21 of an ulp on either side), the weights integers of at most 2^30,
-// and the sums exact.  lm: l_o's significand, leading bit at bit 63; TWO: the facula weights too.
+// and the sums exact.  Within `zone` of a half, the error of the product and of the reference's rn(l_o
+// u), the whole ulps are the FP64 operations' (one product in 2^19 / zone; without it a pixel in some
+// thousands had a cell's weight wrong by an ulp of l).  lm: l_o's significand, leading bit at bit 63;
+// TWO: the facula weights too.
 template <bool TWO>
-__device__ __forceinline__ void adj_residue(const AdjNoise *__restrict__ x, unsigned long long lm, int k0, int k1,
-                                            double &r, double &rs) {
-    constexpr int HALF = 1 << (ADJ_FRAC - 1), PART = 4096;   // 2^12 products of at most 2^50
-    const unsigned h = (unsigned)(lm >> 32), l = (unsigned)lm;
+__device__ __forceinline__ void adj_residue(const AdjNoise *__restrict__ x, const double *__restrict__ fb, double lo,
+                                            unsigned long long lm, int k0, int k1, int zone, double &r, double &rs) {
+    constexpr int HALF = 1 << (ADJ_FRAC - 1), PART = 4096;   // 2^12 products below 2^51
+    const unsigned h = (unsigned)(lm >> 32), l = (unsigned)lm, add = HALF + 1 + zone;
     r = rs = 0.0;
     for (int q = k0; q < k1; q += PART) {
         long long s = 0, t = 0;
@@ -508,8 +511,14 @@ __device__ __forceinline__ void adj_residue(const AdjNoise *__restrict__ x, unsi
         for (int k = q; k < end; ++k) {
             const AdjNoise c = x[k];
             const unsigned wh = (unsigned)(c.w >> 32), wl = (unsigned)c.w;
-            const unsigned v = h * wh + __umulhi(h, wl) + __umulhi(l, wh) + (HALF + 1);
-            const int fr = (int)(v & (2u * HALF - 1u)) - HALF;
+            const unsigned v = h * wh + __umulhi(h, wl) + __umulhi(l, wh) + add, f = v & (2u * HALF - 1u);
+            int fr = (int)f - (HALF + zone);   // beyond the v >> ADJ_FRAC whole ulps
+            if (f < 2u * (unsigned)zone) {
+                // whole ulps of the FP64 operations beyond those, by their low bits: 0 or -1
+                const long long w = __double_as_longlong(lo) - __double_as_longlong(adj_shifted(lo, fb[k]));
+                const int d = (int)(((unsigned)(w < 0 ? -w : w) - (v >> ADJ_FRAC)) << ADJ_FRAC) >> ADJ_FRAC;
+                fr -= d * (2 * HALF);
+            }
             s += (long long)c.a * fr;
             if (TWO) t += (long long)c.as * fr;
         }
@@ -583,9 +592,10 @@ __global__ void __launch_bounds__(ADJ_THREADS) k_adj_rows(const __grid_constant_
                     if (noisy && row.even && adj_exp(fma(lo, s.f0, lo)) == ex && adj_exp(fma(lo, f1, lo)) == ex &&
                         fmax(fabs(s.f0), fabs(f1)) < ADJ_W_MAX) {
                         const double rest = adj_rest(lj, lo, s.f0);
+                        const int zone = (int)(fmax(fabs(s.f0), fabs(f1)) * (double)(1 << ADJ_FRAC)) + 3;
                         double r, rs;
-                        if (two) adj_residue<true>(noise, lm, k0, k1, r, rs);
-                        else adj_residue<false>(noise, lm, k0, k1, r, rs);
+                        if (two) adj_residue<true>(noise, fb, lo, lm, k0, k1, zone, r, rs);
+                        else adj_residue<false>(noise, fb, lo, lm, k0, k1, zone, r, rs);
                         w1 = fma(io, fma(rest, s.s1, -lo * s.s2), -ulp * (row.unit * r));
                         w1s = two ? fma(io, fma(rest, s.t1, -lo * s.t2), -ulp * (row.unit_s * rs)) : w1;
                     } else {   // the forward's l' cell by cell

@@ -146,3 +146,21 @@ def test_entries_carry_the_rounding_of_single_cells(ctx, lambda0, vsini, grid, l
         bound = (41 if k in ("limb", "delta") else 16 + cnt[k]) * u * mag[k]
         bad = np.abs(got[k] - ref[k]) > bound
         assert not bad.any(), (k, np.argwhere(bad)[:3], float(np.max(np.abs(got[k] - ref[k])[bad] / mag[k][bad]) / u))
+
+
+@pytest.mark.parametrize("lambda0,vsini", [(5000.0, 2.0), (6000.0, 20.0), (4500.0, 200.0)])
+def test_rounding_of_shifted_wavelengths_near_halves(ctx, lambda0, vsini):
+    """The row gradients at every pixel: among some million (cell, pixel) pairs there are shifted
+    wavelengths within 2^-21 of half an ulp, which have to be rounded as the forward rounds them (bound
+    as above)."""
+    rng = np.random.default_rng(3)
+    n, n_eff, n_mu, grid, step = 1400, 1390, 4, 60, 0.01
+    wave = lambda0 + step * np.arange(n)
+    maps = _maps(grid, vsini, n_mu)
+    bi, temp, x = _inputs(rng, n, n_mu, grid, maps, 1)
+    g = rng.standard_normal((3, 1, n))
+    got = ctx.phase_integrate_adjoint(wave, n_eff, grid, temp, bi, maps, x, step, Activity(5778, 663, 250, 20, 0), *g)
+    ref, mag, cnt = _reference(wave, n_eff, bi, maps, x, step, g)
+    for k in ROWS:
+        bad = np.abs(got[k] - ref[k]) > (16 + cnt[k]) * 2.0 ** -53 * mag[k]
+        assert not bad.any(), (k, int(bad.sum()), np.argwhere(bad)[:3])
