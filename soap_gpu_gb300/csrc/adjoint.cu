@@ -42,6 +42,9 @@ constexpr int ADJ_SRC = ADJ_THREADS / 32 * 31;   // source pixels per block of t
 constexpr int ADJ_NB = 64;           // integer boundaries handled at a time
 constexpr double ADJ_F_MAX = 0.01;   // largest |f| of the cells taken in ranges (3000 km/s)
 constexpr int ADJ_FRAC = 21;         // fraction bits of l u
+// Scratch of the lists and of the limb kernel's shares of the pixels: 68 + 16 Q bytes per cell and phase.
+// Phases beyond it are taken in groups, whose gradients add up in the phases' order.
+constexpr size_t ADJ_SCRATCH = 4ULL << 30;
 constexpr int ADJ_CLASS = 3;         // 0 spot, 1 facula, 2 evaluated one by one (Planck ratio, extreme velocity)
 
 struct AdjGeo {
@@ -89,6 +92,7 @@ struct AdjArgs {
     const AdjNoise *noise;
     const int *seg;     // [phase][class][n_mu + 1] first entry of each row
     const AdjRow *row;  // [phase][2][n_mu]
+    int more;           // the outputs hold the sums of the phases before
     double *acc;        // [Q][phase][gm][2] limb and velocity sums per entry
     double *part;       // [n_mu][2][n] continuum sums per row
     double *d_qn, *d_qs, *d_sn, *d_fn;
@@ -645,10 +649,12 @@ __global__ void __launch_bounds__(ADJ_THREADS) k_adj_rows(const __grid_constant_
     if (lane != 0 && o < A.n) {
         const long long at = (long long)b * A.n + o;
         const bool in = o < n_eff;
-        A.d_qs[at] = in ? L[0] : 0.0;
-        A.d_qn[at] = in ? L[1] : 0.0;
-        A.d_sn[at] = in ? L[2] : 0.0;
-        A.d_fn[at] = in ? L[3] : 0.0;
+        double *const out[4] = {A.d_qs, A.d_qn, A.d_sn, A.d_fn};
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            const double v = in ? L[q] : 0.0;
+            out[q][at] = A.more ? out[q][at] + v : v;
+        }
     }
 }
 
@@ -720,11 +726,11 @@ __global__ void __launch_bounds__(ADJ_THREADS) k_adj_continuum(const __grid_cons
     }
 }
 
-__global__ void k_adj_sum_rows(int n, int n_mu, const double *__restrict__ part, double *__restrict__ d_ss,
+__global__ void k_adj_sum_rows(int n, int n_mu, int more, const double *__restrict__ part, double *__restrict__ d_ss,
                                double *__restrict__ d_fs) {
     const int j = blockIdx.x * blockDim.x + threadIdx.x;
     if (j >= n) return;
-    double s = 0.0, f = 0.0;
+    double s = more ? d_ss[j] : 0.0, f = more ? d_fs[j] : 0.0;
     for (int b = 0; b < n_mu; ++b) {
         s += part[((long long)b * 2 + 0) * n + j];
         f += part[((long long)b * 2 + 1) * n + j];
@@ -913,10 +919,10 @@ __global__ void k_adj_limb_cells(const __grid_constant__ AdjArgs A, const double
 }
 
 // grad_limb[k] = sum over phases, in order, of buf[p][k]
-__global__ void k_adj_sum_phases(int n_phase, long long gm, const double *__restrict__ buf, double *out) {
+__global__ void k_adj_sum_phases(int n_phase, long long gm, int more, const double *__restrict__ buf, double *out) {
     const long long k = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= gm) return;
-    double s = 0.0;
+    double s = more ? out[k] : 0.0;
     for (int p = 0; p < n_phase; ++p) s += buf[(long long)p * gm + k];
     out[k] = s;
 }
@@ -959,7 +965,19 @@ extern "C" int soapgb_phase_integrate_adjoint(soapgb_ctx *ctx, int n, int n_eff,
     for (int q = 4; q < 6; ++q) s_o[q] = ws.add(host ? row_b : 0);
     s_o[6] = ws.add(host ? sizeof(double) * gm : 0);
     s_o[7] = ws.add(host ? sizeof(double) * gm : 0);
-    const size_t pg = (size_t)gm * std::max(n_phase, 1);
+    // shares of the pixels in the limb kernel: eight blocks per SM over rows, phases and shares (a
+    // phase's regions touch about half of the rows)
+    const int tiles = (n_eff + ADJ_THREADS - 1) / ADJ_THREADS;
+    auto shares = [&](int phases) {
+        const int by_blocks = std::min({32, tiles, 8 * std::max(ctx->num_sms, 1) / (n_mu * std::max(phases, 1))});
+        const size_t by_scratch = ADJ_SCRATCH / (sizeof(double) * 4 * (size_t)gm * std::max(phases, 1));
+        return std::max(1, (int)std::min<size_t>((size_t)std::max(by_blocks, 1), by_scratch));   // half of it
+    };
+    // phases in a group
+    const size_t per_phase = (sizeof(int) + sizeof(double) + sizeof(AdjEnt) + sizeof(AdjNoise) + 4 * sizeof(double)) * (size_t)gm;
+    const int group = (int)std::min<size_t>({(size_t)std::max(n_phase, 1), std::max<size_t>(1, ADJ_SCRATCH / per_phase), 65535});
+    const int Q = shares(group);
+    const size_t pg = (size_t)gm * group, buf_b = sizeof(double) * pg;
     int s_geo = ws.add(sizeof(AdjGeo) * gm);
     int s_key[2], s_val[2];
     for (int q = 0; q < 2; ++q) s_key[q] = ws.add(sizeof(unsigned long long) * gm);
@@ -969,15 +987,11 @@ extern "C" int soapgb_phase_integrate_adjoint(soapgb_ctx *ctx, int n, int n_eff,
     int s_sort = ws.add(sort_b);
     int s_cell = ws.add(sizeof(int) * pg), s_fb = ws.add(sizeof(double) * pg), s_ent = ws.add(sizeof(AdjEnt) * pg);
     int s_noise = ws.add(sizeof(AdjNoise) * pg);
-    int s_seg = ws.add(sizeof(int) * ADJ_CLASS * (size_t)(n_mu + 1) * std::max(n_phase, 1));
-    int s_row = ws.add(sizeof(AdjRow) * 2 * (size_t)n_mu * std::max(n_phase, 1));
-    // shares of the pixels in the limb kernel: eight blocks per SM over rows, phases and shares (a
-    // phase's regions touch about half of the rows)
-    const int tiles = (n_eff + ADJ_THREADS - 1) / ADJ_THREADS;
-    const int Q = std::max(1, std::min({32, tiles, 8 * std::max(ctx->num_sms, 1) / (n_mu * std::max(n_phase, 1))}));
+    int s_seg = ws.add(sizeof(int) * ADJ_CLASS * (size_t)(n_mu + 1) * group);
+    int s_row = ws.add(sizeof(AdjRow) * 2 * (size_t)n_mu * group);
     int s_acc = ws.add(2 * sizeof(double) * pg * Q);
     int s_part = ws.add(g_flux ? 2 * cube_b : 0);
-    int s_buf = ws.add(map_b), s_bufd = ws.add(map_b);
+    int s_buf = ws.add(buf_b), s_bufd = ws.add(buf_b);
     // no flux or tot gradients: one zero array stands in for both, and the continuum
     // rows, which enter only flux and tot, get no pass
     const bool bconv_only = (g_flux == nullptr);
@@ -1034,7 +1048,6 @@ extern "C" int soapgb_phase_integrate_adjoint(soapgb_ctx *ctx, int n, int n_eff,
         A.n = n;
         A.n_eff = n_eff;
         A.n_mu = n_mu;
-        A.n_phase = n_phase;
         A.Q = Q;
         A.gm = gm;
         A.lam = d_wave;
@@ -1045,14 +1058,10 @@ extern "C" int soapgb_phase_integrate_adjoint(soapgb_ctx *ctx, int n, int n_eff,
         A.fac_norm = d_fn;
         A.spot_sed = d_ss;
         A.fac_sed = d_fs;
-        A.temp = d_temp;
         A.lb = d_lb;
         A.step = step;
         A.solar = act->solar;
         A.t_norm_fac = (int)(act->t_star + act->t_diff_fac + 0.9 - 216.8);
-        A.gF = d_gf;
-        A.gB = d_gb;
-        A.gT = d_gt;
         A.geo = ws.get<AdjGeo>(s_geo);
         A.cell = ws.get<int>(s_cell);
         A.fb = ws.get<double>(s_fb);
@@ -1079,45 +1088,58 @@ extern "C" int soapgb_phase_integrate_adjoint(soapgb_ctx *ctx, int n, int n_eff,
                                       ws.get<unsigned long long>(s_key[1]), ws.get<int>(s_val[0]),
                                       ws.get<int>(s_val[1]), ws.get<void>(s_sort), sort_b);
             if (rc) return rc;
-            k_adj_lists<<<n_phase, 1024, 0, ctx->stream>>>(gm, n_mu, ws.get<int>(s_val[1]), d_temp, d_bi, A.geo, d_region,
-                                                           act->solar, A.t_norm_fac, ws.get<int>(s_cell),
-                                                           ws.get<double>(s_fb), ws.get<int>(s_seg), ctx->d_status);
-            SOAP_LAUNCHED(ctx);
-            k_adj_entries<<<dim3(n_mu, 2, n_phase), ADJ_THREADS, 0, ctx->stream>>>(
-                gm, n_mu, A.cell, A.fb, A.seg, A.geo, ws.get<AdjEnt>(s_ent), ws.get<AdjNoise>(s_noise),
-                ws.get<AdjRow>(s_row));
-            SOAP_LAUNCHED(ctx);
             k_adj_inv<<<grid_for(ctx, n_eff, 256), 256, 0, ctx->stream>>>(n_eff, d_wave, d_inv);
             SOAP_LAUNCHED(ctx);
         }
-        SOAP_TRACED(ctx, "adjoint_rows",
-                    (bconv_only ? k_adj_rows<true> : k_adj_rows<false>)<<<dim3((n + ADJ_SRC - 1) / ADJ_SRC, n_mu),
-                                                                          ADJ_THREADS, 0, ctx->stream>>>(A, d_bi));
-        SOAP_LAUNCHED(ctx);
-        if (bconv_only) {
-            SOAP_CUDA(ctx, cudaMemsetAsync(o_ss, 0, row_b, ctx->stream));
-            SOAP_CUDA(ctx, cudaMemsetAsync(o_fs, 0, row_b, ctx->stream));
-        } else {
-            SOAP_TRACED(ctx, "adjoint_continuum",
-                        k_adj_continuum<<<dim3((n + ADJ_THREADS - 1) / ADJ_THREADS, n_mu), ADJ_THREADS, 0, ctx->stream>>>(
-                            A, d_bi));
+        for (int p0 = 0; p0 < n_phase; p0 += group) {
+            const int ph = std::min(group, n_phase - p0);
+            const double *p_bi = d_bi + (size_t)p0 * gm;
+            A.n_phase = ph;
+            A.more = p0 > 0;
+            A.temp = d_temp + (size_t)p0 * gm;
+            A.gF = d_gf + (size_t)p0 * n;
+            A.gB = d_gb + (size_t)p0 * n;
+            A.gT = d_gt + (size_t)p0 * n;
+            {
+                TraceScope ts(ctx, "adjoint_lists");
+                k_adj_lists<<<ph, 1024, 0, ctx->stream>>>(gm, n_mu, ws.get<int>(s_val[1]), A.temp, p_bi, A.geo, d_region,
+                                                               act->solar, A.t_norm_fac, ws.get<int>(s_cell),
+                                                               ws.get<double>(s_fb), ws.get<int>(s_seg), ctx->d_status);
+                SOAP_LAUNCHED(ctx);
+                k_adj_entries<<<dim3(n_mu, 2, ph), ADJ_THREADS, 0, ctx->stream>>>(
+                    gm, n_mu, A.cell, A.fb, A.seg, A.geo, ws.get<AdjEnt>(s_ent), ws.get<AdjNoise>(s_noise),
+                    ws.get<AdjRow>(s_row));
+                SOAP_LAUNCHED(ctx);
+            }
+            SOAP_TRACED(ctx, "adjoint_rows",
+                        (bconv_only ? k_adj_rows<true> : k_adj_rows<false>)<<<dim3((n + ADJ_SRC - 1) / ADJ_SRC, n_mu),
+                                                                              ADJ_THREADS, 0, ctx->stream>>>(A, p_bi));
             SOAP_LAUNCHED(ctx);
-            k_adj_sum_rows<<<grid_for(ctx, n, 256), 256, 0, ctx->stream>>>(n, n_mu, A.part, o_ss, o_fs);
+            if (bconv_only) {
+                SOAP_CUDA(ctx, cudaMemsetAsync(o_ss, 0, row_b, ctx->stream));
+                SOAP_CUDA(ctx, cudaMemsetAsync(o_fs, 0, row_b, ctx->stream));
+            } else {
+                SOAP_TRACED(ctx, "adjoint_continuum",
+                            k_adj_continuum<<<dim3((n + ADJ_THREADS - 1) / ADJ_THREADS, n_mu), ADJ_THREADS, 0, ctx->stream>>>(
+                                A, p_bi));
+                SOAP_LAUNCHED(ctx);
+                k_adj_sum_rows<<<grid_for(ctx, n, 256), 256, 0, ctx->stream>>>(n, n_mu, A.more, A.part, o_ss, o_fs);
+                SOAP_LAUNCHED(ctx);
+            }
+            SOAP_CUDA(ctx, cudaMemsetAsync(d_buf, 0, buf_b, ctx->stream));
+            SOAP_CUDA(ctx, cudaMemsetAsync(d_bufd, 0, buf_b, ctx->stream));
+            SOAP_CUDA(ctx, cudaMemsetAsync(A.acc, 0, 2 * sizeof(double) * pg * Q, ctx->stream));
+            SOAP_TRACED(ctx, "adjoint_limb",
+                        (bconv_only ? k_adj_limb<true> : k_adj_limb<false>)<<<dim3(n_mu, ph, Q), ADJ_THREADS, 0,
+                                                                              ctx->stream>>>(A, p_bi));
+            SOAP_LAUNCHED(ctx);
+            k_adj_limb_cells<<<dim3((unsigned)((gm + 255) / 256), ph), 256, 0, ctx->stream>>>(A, d_limb, d_buf, d_bufd);
+            SOAP_LAUNCHED(ctx);
+            k_adj_sum_phases<<<grid_for(ctx, gm, 256), 256, 0, ctx->stream>>>(ph, gm, A.more, d_buf, o_lm);
+            SOAP_LAUNCHED(ctx);
+            k_adj_sum_phases<<<grid_for(ctx, gm, 256), 256, 0, ctx->stream>>>(ph, gm, A.more, d_bufd, o_dl);
             SOAP_LAUNCHED(ctx);
         }
-        SOAP_CUDA(ctx, cudaMemsetAsync(d_buf, 0, map_b, ctx->stream));
-        SOAP_CUDA(ctx, cudaMemsetAsync(d_bufd, 0, map_b, ctx->stream));
-        SOAP_CUDA(ctx, cudaMemsetAsync(A.acc, 0, 2 * sizeof(double) * pg * Q, ctx->stream));
-        SOAP_TRACED(ctx, "adjoint_limb",
-                    (bconv_only ? k_adj_limb<true> : k_adj_limb<false>)<<<dim3(n_mu, n_phase, Q), ADJ_THREADS, 0,
-                                                                          ctx->stream>>>(A, d_bi));
-        SOAP_LAUNCHED(ctx);
-        k_adj_limb_cells<<<dim3((unsigned)((gm + 255) / 256), n_phase), 256, 0, ctx->stream>>>(A, d_limb, d_buf, d_bufd);
-        SOAP_LAUNCHED(ctx);
-        k_adj_sum_phases<<<grid_for(ctx, gm, 256), 256, 0, ctx->stream>>>(n_phase, gm, d_buf, o_lm);
-        SOAP_LAUNCHED(ctx);
-        k_adj_sum_phases<<<grid_for(ctx, gm, 256), 256, 0, ctx->stream>>>(n_phase, gm, d_bufd, o_dl);
-        SOAP_LAUNCHED(ctx);
     }
     if (host) {
         SOAP_CUDA(ctx, cudaMemcpyAsync(grad_q_norm, o_qn, cube_b, cudaMemcpyDeviceToHost, ctx->stream));

@@ -164,3 +164,39 @@ def test_rounding_of_shifted_wavelengths_near_halves(ctx, lambda0, vsini):
     for k in ROWS:
         bad = np.abs(got[k] - ref[k]) > (16 + cnt[k]) * 2.0 ** -53 * mag[k]
         assert not bad.any(), (k, int(bad.sum()), np.argwhere(bad)[:3])
+
+
+@pytest.mark.parametrize("grid,n,n_phase,n_mu", [(1500, 200, 30, 1), (3000, 8400, 1, 1)])
+def test_scratch_of_large_maps(grid, n, n_phase, n_mu):
+    """Maps of millions of cells, a few of them active: the phases in groups that fit the scratch, or
+    fewer shares of the pixels, with the gradients of per-cell sums (bounds as above, and one addition
+    per phase); the workspace stays below 5.5 GB (over 6 for all phases and shares at a time)."""
+    torch = pytest.importorskip("torch")
+    from soap_gpu_gb300.api import Context
+    rng = np.random.default_rng(grid)
+    gm, step, n_eff = grid * grid, 0.01, n - 3
+    wave = 5000.0 + step * np.arange(n)
+    at = np.sort(rng.choice(gm, 40, replace=False))
+    maps = dict(delta=np.full(gm, -999.0), limb=np.full(gm, -999.0), lb=np.zeros(gm), region=np.zeros(gm, np.int32))
+    maps["delta"][at], maps["limb"][at] = rng.uniform(-3.0, 3.0, 40), rng.uniform(0.3, 1.0, 40)
+    maps["lb"][at] = rng.uniform(-0.1, 0.2, 40)
+    bi = np.full((n_phase, gm), -9999.0)
+    for p in range(n_phase):
+        on = rng.choice(at, 6, replace=False)
+        bi[p, on[:3]], bi[p, on[3:]] = 0.0, 1.0
+    temp = np.where(bi == 0.0, 5115.0, np.where(bi == 1.0, 5900.0, -9999.0))
+    x = {k: 1.0 + 0.3 * rng.uniform(-1, 1, (n_mu, n)) for k in ROWS}
+    x["spot_sed"], x["fac_sed"] = 0.3 + 0.1 * np.arange(n) / n, 1.0 + 0.1 * np.arange(n) / n
+    g = rng.standard_normal((3, n_phase, n))
+    dev = lambda a: torch.as_tensor(a, device="cuda:0")
+    args = [dev(wave), n_eff, grid, dev(temp), dev(bi), {k: dev(v) for k, v in maps.items()}, {k: dev(v) for k, v in x.items()},
+            step, Activity(5778, 663, 250, 20, 0), *(dev(v) for v in g)]
+    torch.cuda.synchronize()
+    with Context(0) as ctx:
+        free = torch.cuda.mem_get_info()[0]
+        got = {k: v.cpu().numpy() for k, v in ctx.phase_integrate_adjoint(*args).items()}
+        assert free - torch.cuda.mem_get_info()[0] < 5.5e9
+    ref, mag, cnt = _reference(wave, n_eff, bi, maps, x, step, g)
+    for k in ref:
+        bound = (41 + n_phase + (n >> 8) if k in ("limb", "delta") else 16 + n_phase + cnt[k]) * 2.0 ** -53 * mag[k]
+        assert np.all(np.abs(got[k] - ref[k]) <= bound), k
