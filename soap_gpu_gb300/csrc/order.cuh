@@ -153,7 +153,7 @@ static __global__ void __launch_bounds__(ORDER_COUNT_THREADS) k_order_ranks(int 
         const int i = tid + q * ORDER_COUNT_THREADS;
         k[q] = (i < nc) ? hi[cb + i] : 0ULL;
         a[q] = 0;
-        b[q] = nt;
+        b[q] = (i < nc) ? nt : 0;   // nothing to search past the last key
     }
     __syncthreads();
     // the searches of a thread's keys in lock-step, so that their loads overlap
