@@ -499,32 +499,60 @@ __device__ __forceinline__ double adj_shifted(double lo, double f) { return __ds
 // residue.  The fraction bits of the 64-bit product are integers (about 2^20; the two products'
 // lower halves are left out, 2^-21 of an ulp on either side), the weights integers of at most 2^30,
 // and the sums exact.  Within `zone` of a half, the error of the product and of the reference's rn(l_o
-// u), the whole ulps are the FP64 operations' (one product in 2^19 / zone; without it a pixel in some
-// thousands had a cell's weight wrong by an ulp of l).  lm: l_o's significand, leading bit at bit 63;
-// TWO: the facula weights too.
+// u), the whole ulps are the FP64 operations' (without it a pixel in some thousands had a cell's
+// weight wrong by an ulp of l).  lm: l_o's significand, leading bit at bit 63; TWO: the facula
+// weights too.
+constexpr int ADJ_HALF = 1 << (ADJ_FRAC - 1);
+
+// the product's low bits, with half an ulp and the zone added: whole ulps from bit ADJ_FRAC on
+__device__ __forceinline__ unsigned adj_product(const AdjNoise &c, unsigned long long lm, int zone) {
+    const unsigned h = (unsigned)(lm >> 32), l = (unsigned)lm, wh = (unsigned)(c.w >> 32), wl = (unsigned)c.w;
+    return h * wh + __umulhi(h, wl) + __umulhi(l, wh) + (unsigned)(ADJ_HALF + 1 + zone);
+}
+
+// What the cells near a half among [k0, k1) add where the FP64 operations give an ulp less (a call, off
+// the others' path: one in 2^19 / zone cells is near)
+static __device__ __noinline__ longlong2 adj_near_half(const AdjNoise *__restrict__ x, const double *__restrict__ fb,
+                                                       double lo, unsigned long long lm, int k0, int k1, int zone) {
+    longlong2 s = make_longlong2(0, 0);
+    for (int k = k0; k < k1; ++k) {
+        const AdjNoise c = x[k];
+        const unsigned v = adj_product(c, lm, zone);
+        if ((v & (2u * ADJ_HALF - 1u)) >= 2u * (unsigned)zone) continue;
+        const long long w = __double_as_longlong(lo) - __double_as_longlong(adj_shifted(lo, fb[k]));
+        // the difference of the whole ulps, by their low bits: 0 or -1
+        const int d = (int)(((unsigned)(w < 0 ? -w : w) - (v >> ADJ_FRAC)) << ADJ_FRAC) >> ADJ_FRAC;
+        s.x -= (long long)c.a * (d * (2 * ADJ_HALF));
+        s.y -= (long long)c.as * (d * (2 * ADJ_HALF));
+    }
+    return s;
+}
+
 template <bool TWO>
 __device__ __forceinline__ void adj_residue(const AdjNoise *__restrict__ x, const double *__restrict__ fb, double lo,
                                             unsigned long long lm, int k0, int k1, int zone, double &r, double &rs) {
-    constexpr int HALF = 1 << (ADJ_FRAC - 1), PART = 4096;   // 2^12 products below 2^51
-    const unsigned h = (unsigned)(lm >> 32), l = (unsigned)lm, add = HALF + 1 + zone;
+    constexpr int PART = 4096, CHUNK = 32;   // 2^12 products below 2^51
     r = rs = 0.0;
     for (int q = k0; q < k1; q += PART) {
         long long s = 0, t = 0;
         const int end = min(k1, q + PART);
+        for (int c0 = q; c0 < end; c0 += CHUNK) {
+            const int c1 = min(end, c0 + CHUNK);
+            unsigned near = ~0u;
 #pragma unroll 4
-        for (int k = q; k < end; ++k) {
-            const AdjNoise c = x[k];
-            const unsigned wh = (unsigned)(c.w >> 32), wl = (unsigned)c.w;
-            const unsigned v = h * wh + __umulhi(h, wl) + __umulhi(l, wh) + add, f = v & (2u * HALF - 1u);
-            int fr = (int)f - (HALF + zone);   // beyond the v >> ADJ_FRAC whole ulps
-            if (f < 2u * (unsigned)zone) {
-                // whole ulps of the FP64 operations beyond those, by their low bits: 0 or -1
-                const long long w = __double_as_longlong(lo) - __double_as_longlong(adj_shifted(lo, fb[k]));
-                const int d = (int)(((unsigned)(w < 0 ? -w : w) - (v >> ADJ_FRAC)) << ADJ_FRAC) >> ADJ_FRAC;
-                fr -= d * (2 * HALF);
+            for (int k = c0; k < c1; ++k) {
+                const AdjNoise c = x[k];
+                const unsigned f = adj_product(c, lm, zone) & (2u * ADJ_HALF - 1u);
+                const int fr = (int)f - (ADJ_HALF + zone);
+                near = min(near, f);
+                s += (long long)c.a * fr;
+                if (TWO) t += (long long)c.as * fr;
             }
-            s += (long long)c.a * fr;
-            if (TWO) t += (long long)c.as * fr;
+            if (near < 2u * (unsigned)zone) {
+                const longlong2 fix = adj_near_half(x, fb, lo, lm, c0, c1, zone);
+                s += fix.x;
+                if (TWO) t += fix.y;
+            }
         }
         r += (double)s;
         if (TWO) rs += (double)t;
@@ -533,9 +561,12 @@ __device__ __forceinline__ void adj_residue(const AdjNoise *__restrict__ x, cons
 
 // ---- row gradients -----------------------------------------------------------------------
 // Block: ADJ_SRC source pixels of one row, lane l of a warp source o; lane 0 only gives its upper
-// share to lane 1.  BC: the bconv gradient alone (gF = gT = 0).
+// share to lane 1.  BC: the bconv gradient alone (gF = gT = 0).  Bound by the residues' integer
+// instructions and their latency, so four and three blocks per SM although some registers spill (two:
+// 0.65 and 0.58 ms for 100 x 100 cells and 50,000 px, BC, and five phases of 200 x 200 and 100,000
+// px; so 0.53 and 0.48).
 template <bool BC>
-__global__ void __launch_bounds__(ADJ_THREADS) k_adj_rows(const __grid_constant__ AdjArgs A,
+__global__ void __launch_bounds__(ADJ_THREADS, BC ? 4 : 3) k_adj_rows(const __grid_constant__ AdjArgs A,
                                                           const double *__restrict__ bi) {
     __shared__ AdjRange R;
     const int b = blockIdx.y, lane = threadIdx.x & 31, n_eff = A.n_eff;
