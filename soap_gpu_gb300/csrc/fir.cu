@@ -322,7 +322,7 @@ __device__ __forceinline__ bool bits_is_integral(double v) {
 }
 
 // --- per-list cell lists in velocity order ---------------------------------------
-// One block per list (the quiet disk, or one phase): the visible cells in the sorted
+// One block per list (one phase; the quiet disk's: k_fir_list1): the visible cells in the sorted
 // order, split into classes -- 0: spots (integral temperature, Planck ratio exactly 1),
 // 1: faculae, 2: cells evaluated directly (other spots; faculae of the solar
 // variant).  counts[l] = (n0, n1, n2, 0); class c occupies positions
@@ -350,7 +350,6 @@ __device__ __forceinline__ int fir_class_box(const CellGeo &g, int type, int sol
 __device__ __forceinline__ int fir_class(const CellGeo &g, const double *bi, const double *temp, long long idx,
                                          int solar) {
     if (!(g.L > -998.0)) return -1;
-    if (!bi) return CLS_SPOT;
     const double b = bi[idx];
     if (!(b >= -0.5 && b <= 1.5)) return -1;
     return fir_class_tb(g, bits_is_zero(b) ? temp[idx] : 0.0, b, solar);

@@ -4,8 +4,10 @@
 // (wav_sigma, conv_inst, reduceMax/MinIdxOptimizedShared, spec_diff, spec_norm:
 // six launches and four blocking copies per spectrum, every reduction block
 // scanning the whole array).  Here:
-//   PLAIN64  -- conv_inst's arithmetic term by term (one thread per pixel, all
-//               2w-1 taps, the reference's operation order), batched over spectra;
+//   PLAIN64  -- conv_inst's arithmetic term by term in the reference's operation order;
+//               tiles of 128 pixels with the weights once per tile for all spectra, taps
+//               whose weight is below e^-90 left out where that changes no bit of the sum
+//               (k_conv_plain64t), all 2w - 1 taps elsewhere;
 //   FAST64 / FAST32 -- the convolution is linear, so
 //               C = conv(1 - base) + conv(spec);
 //               conv(1 - base) is computed once per base in FP64 and the per-phase
@@ -308,19 +310,14 @@ __device__ __forceinline__ void conv_tap_constants(int i, int n, double l, doubl
         rng = make_int2(max(max(-wid, -r), -halo), min(min(wid - 2, r), halo));
     }
 }
-template <typename T>
 __global__ void k_conv_params(int n, int n_eff, const double *__restrict__ lam, double ka, double kb, double kr,
-                              int wid, int halo, T *kq, T *cq, int2 *rng) {
+                              int wid, int halo, double *kq, double *cq, int2 *rng) {
     int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n_eff) return;
-    double k, c;
-    conv_tap_constants(i, n, lam[i], ka, kb, kr, wid, halo, k, c, rng[i]);
-    kq[i] = (T)k;
-    cq[i] = (T)c;
+    if (i < n_eff) conv_tap_constants(i, n, lam[i], ka, kb, kr, wid, halo, kq[i], cq[i], rng[i]);
 }
 
 // ---------------------------------------------------------------------------
-// FAST convolution of x (no "1 -"): out[i] = sum_d w_i(d) x[i+d], d in the
+// FP64 convolution of the fast forms, of x (no "1 -"): out[i] = sum_d w_i(d) x[i+d], d in the
 // reference window [-wid, wid-2] intersected with the significant taps.  Block =
 // 256 threads x 4 pixels = 1024 pixels; SB spectra per block staged in smem.
 // sign: +1 for conv(x), or the base pass computes conv(1 - base) with x = 1 - base.
@@ -329,43 +326,43 @@ constexpr int FC_THREADS = 256;
 constexpr int FC_PIX = 4;
 constexpr int FC_TILE = FC_THREADS * FC_PIX;
 
-template <typename T, int SB, typename SrcT, typename OutT>
-__global__ void __launch_bounds__(FC_THREADS) k_conv_fast(int n, int n_eff, const T *__restrict__ kqa,
-                                                          const T *__restrict__ cqa, const int2 *__restrict__ rnga,
-                                                          const SrcT *__restrict__ spec, long long spec_stride,
+template <int SB>
+__global__ void __launch_bounds__(FC_THREADS) k_conv_fast(int n, int n_eff, const double *__restrict__ kqa,
+                                                          const double *__restrict__ cqa, const int2 *__restrict__ rnga,
+                                                          const double *__restrict__ spec, long long spec_stride,
                                                           int n_spec, int one_minus, int halo,
-                                                          OutT *__restrict__ conv, long long conv_stride) {
-    extern __shared__ unsigned char smem_raw[];
-    T *xs = reinterpret_cast<T *>(smem_raw);
+                                                          double *__restrict__ conv, long long conv_stride) {
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    double *xs = reinterpret_cast<double *>(smem_raw);
     int win = FC_TILE + 2 * halo;
     int i0 = blockIdx.x * FC_TILE;
     int s0 = blockIdx.y * SB;
     int nsb = min(SB, n_spec - s0);
     // stage [i0 - halo, i0 + FC_TILE + halo) of each spectrum (0 outside [0, n))
     for (int q = 0; q < nsb; ++q) {
-        const SrcT *sp = spec + (long long)(s0 + q) * spec_stride;
+        const double *sp = spec + (long long)(s0 + q) * spec_stride;
         for (int t = threadIdx.x; t < win; t += FC_THREADS) {
             int m = i0 - halo + t;
-            T v = (m >= 0 && m < n) ? (T)sp[m] : (T)0;
-            if (one_minus) v = (m >= 0 && m < n) ? (T)1 - v : (T)0;
+            double v = (m >= 0 && m < n) ? sp[m] : 0.0;
+            if (one_minus) v = (m >= 0 && m < n) ? 1.0 - v : 0.0;
             xs[q * win + t] = v;
         }
     }
     __syncthreads();
     int ib = i0 + threadIdx.x * FC_PIX;   // first pixel of this thread
-    T acc[SB][FC_PIX];
+    double acc[SB][FC_PIX];
 #pragma unroll
     for (int q = 0; q < SB; ++q)
 #pragma unroll
-        for (int p = 0; p < FC_PIX; ++p) acc[q][p] = (T)0;
-    T kq[FC_PIX], cq[FC_PIX];
+        for (int p = 0; p < FC_PIX; ++p) acc[q][p] = 0.0;
+    double kq[FC_PIX], cq[FC_PIX];
     int dlo[FC_PIX], dhi[FC_PIX];
     int elo = 1 << 30, ehi = -(1 << 30);
 #pragma unroll
     for (int p = 0; p < FC_PIX; ++p) {
         int i = ib + p;
-        kq[p] = (T)0;
-        cq[p] = (T)0;
+        kq[p] = 0.0;
+        cq[p] = 0.0;
         dlo[p] = 0;
         dhi[p] = -1;
         if (i < n_eff) {
@@ -380,43 +377,36 @@ __global__ void __launch_bounds__(FC_THREADS) k_conv_fast(int n, int n_eff, cons
             }
         }
     }
-    // FP64: Gaussian weights by the exact-product recurrence exp(-(d+1)^2 c) =
+    // Gaussian weights by the exact-product recurrence exp(-(d+1)^2 c) =
     // exp(-d^2 c) exp(-(2d+1) c), exp(-(2d+3) c) = exp(-(2d+1) c) exp(-2c): three exp per
-    // pixel instead of one per tap (rounding grows by ~1e-16 per tap).  FP32: one
-    // MUFU exp per tap.
-    T wcur[FC_PIX], rcur[FC_PIX], e2[FC_PIX];
-    if constexpr (sizeof(T) == 8) {
+    // pixel instead of one per tap (rounding grows by ~1e-16 per tap).
+    double wcur[FC_PIX], rcur[FC_PIX], e2[FC_PIX];
 #pragma unroll
-        for (int p = 0; p < FC_PIX; ++p) {
-            double c = cq[p], d0 = (double)dlo[p];
-            wcur[p] = kq[p] * exp(-d0 * d0 * c);
-            rcur[p] = exp(-(2.0 * d0 + 1.0) * c);
-            e2[p] = exp(-2.0 * c);
-        }
+    for (int p = 0; p < FC_PIX; ++p) {
+        double c = cq[p], d0 = (double)dlo[p];
+        wcur[p] = kq[p] * exp(-d0 * d0 * c);
+        rcur[p] = exp(-(2.0 * d0 + 1.0) * c);
+        e2[p] = exp(-2.0 * c);
     }
     if (elo <= ehi) {
         for (int e = elo; e <= ehi; ++e) {
-            T w[FC_PIX];
+            double w[FC_PIX];
 #pragma unroll
             for (int p = 0; p < FC_PIX; ++p) {
                 int d = e - (ib + p);
                 if (d >= dlo[p] && d <= dhi[p]) {
-                    if constexpr (sizeof(T) == 4) {
-                        w[p] = kq[p] * __expf(-(T)(d * d) * cq[p]);
-                    } else {
-                        w[p] = wcur[p];
-                        wcur[p] *= rcur[p];
-                        rcur[p] *= e2[p];
-                    }
+                    w[p] = wcur[p];
+                    wcur[p] *= rcur[p];
+                    rcur[p] *= e2[p];
                 } else {
-                    w[p] = (T)0;
+                    w[p] = 0.0;
                 }
             }
             int li = e - (i0 - halo);
 #pragma unroll
             for (int q = 0; q < SB; ++q) {
                 if (q < nsb) {
-                    T xv = xs[q * win + li];
+                    double xv = xs[q * win + li];
 #pragma unroll
                     for (int p = 0; p < FC_PIX; ++p) acc[q][p] += w[p] * xv;
                 }
@@ -426,11 +416,11 @@ __global__ void __launch_bounds__(FC_THREADS) k_conv_fast(int n, int n_eff, cons
 #pragma unroll
     for (int q = 0; q < SB; ++q) {
         if (q >= nsb) continue;
-        OutT *cp = conv + (long long)(s0 + q) * conv_stride;
+        double *cp = conv + (long long)(s0 + q) * conv_stride;
 #pragma unroll
         for (int p = 0; p < FC_PIX; ++p) {
             int i = ib + p;
-            if (i < n_eff) cp[i] = (dlo[p] <= dhi[p]) ? (OutT)acc[q][p] : (OutT)0;
+            if (i < n_eff) cp[i] = (dlo[p] <= dhi[p]) ? acc[q][p] : 0.0;
         }
     }
 }
@@ -1349,31 +1339,31 @@ size_t resolution_scratch_bytes(int form, int n, int n_eff, int n_spec) {
     return b;
 }
 
-template <typename T, int SB, typename SrcT = double, typename OutT = double>
-static int launch_conv_fast(soapgb_ctx *ctx, int n, int n_eff, const double *lam, const SrcT *spec,
+template <int SB>
+static int launch_conv_fast(soapgb_ctx *ctx, int n, int n_eff, const double *lam, const double *spec,
                             long long spec_stride, int n_spec, int one_minus, double sigma_v, int wid,
-                            double step_mult, double step_exp, double cut, OutT *conv, long long conv_stride,
+                            double step_mult, double step_exp, double cut, double *conv, long long conv_stride,
                             double sig_max, char *param_scratch) {
     // halo: the widest significant reach, at the largest sigma (bounded by the window)
     double cmin = step_exp * step_exp / (2.0 * sig_max * sig_max);
     int r = (int)floor(sqrt(cut / cmin)) + 2;
     int halo = std::min(wid, r);
     if (halo < 1) halo = 1;
-    size_t smem = sizeof(T) * (size_t)SB * (FC_TILE + 2 * halo);
+    size_t smem = sizeof(double) * (size_t)SB * (FC_TILE + 2 * halo);
     if (smem > CONV_SMEM_MAX) return set_error(ctx, SOAPGB_ERR_ARG, "convolution window too wide (%d px)", halo);
-    if (smem > 48 * 1024) SOAP_CUDA(ctx, soap_allow_smem(k_conv_fast<T, SB, SrcT, OutT>, CONV_SMEM_MAX));
-    T *kq = (T *)param_scratch;
-    T *cq = (T *)(param_scratch + ((sizeof(T) * (size_t)n_eff + 255) & ~size_t(255)));
-    int2 *rng = (int2 *)(param_scratch + 2 * ((sizeof(T) * (size_t)n_eff + 255) & ~size_t(255)));
+    if (smem > 48 * 1024) SOAP_CUDA(ctx, soap_allow_smem(k_conv_fast<SB>, CONV_SMEM_MAX));
+    double *kq = (double *)param_scratch;
+    double *cq = (double *)(param_scratch + ((sizeof(double) * (size_t)n_eff + 255) & ~size_t(255)));
+    int2 *rng = (int2 *)(param_scratch + 2 * ((sizeof(double) * (size_t)n_eff + 255) & ~size_t(255)));
     const double s1 = soap_sigma_per_lambda(sigma_v);
     const double ka = step_mult / (s1 * sqrt(2. * SOAP_PI)), kb = step_exp * step_exp / (2.0 * s1 * s1);
     const double kr = sqrt(cut / kb);
     SOAP_TRACED(ctx, "conv_params",
-                k_conv_params<T><<<grid_for(ctx, n_eff, 256), 256, 0, ctx->stream>>>(n, n_eff, lam, ka, kb, kr, wid,
+                k_conv_params<<<grid_for(ctx, n_eff, 256), 256, 0, ctx->stream>>>(n, n_eff, lam, ka, kb, kr, wid,
                                                                                     halo, kq, cq, rng));
     SOAP_LAUNCHED(ctx);
     dim3 g((n_eff + FC_TILE - 1) / FC_TILE, (n_spec + SB - 1) / SB);
-    SOAP_TRACED(ctx, "conv64", k_conv_fast<T, SB, SrcT, OutT><<<g, FC_THREADS, smem, ctx->stream>>>(n, n_eff, kq, cq, rng, spec, spec_stride,
+    SOAP_TRACED(ctx, "conv64", k_conv_fast<SB><<<g, FC_THREADS, smem, ctx->stream>>>(n, n_eff, kq, cq, rng, spec, spec_stride,
                                                                         n_spec, one_minus, halo, conv, conv_stride));
     SOAP_LAUNCHED(ctx);
     return SOAPGB_OK;
@@ -1658,19 +1648,19 @@ int resolution_device(soapgb_ctx *ctx, int form, int n, int n_eff, int n_spec, c
             double *cb = (double *)carve(p, sizeof(double) * 2 * (size_t)n_eff);
             SOAP_CUDA(ctx, cudaMemcpyAsync(bb, base_a, sizeof(double) * n, cudaMemcpyDeviceToDevice, ctx->stream));
             SOAP_CUDA(ctx, cudaMemcpyAsync(bb + n, base_b, sizeof(double) * n, cudaMemcpyDeviceToDevice, ctx->stream));
-            rc = launch_conv_fast<double, 2>(ctx, n, n_eff, d_wave, bb, n, 2, 1, sigma_v, wid, step_mult, step_exp,
+            rc = launch_conv_fast<2>(ctx, n, n_eff, d_wave, bb, n, 2, 1, sigma_v, wid, step_mult, step_exp,
                                              40.0, cb, n_eff, sig_max, pscr);
             if (rc) return rc;
             cb_a = cb;
             cb_b = cb + n_eff;
         } else if (base_a) {
             cb_a = (double *)carve(p, sizeof(double) * (size_t)n_eff);
-            rc = launch_conv_fast<double, 1>(ctx, n, n_eff, d_wave, base_a, 0, 1, 1, sigma_v, wid, step_mult,
+            rc = launch_conv_fast<1>(ctx, n, n_eff, d_wave, base_a, 0, 1, 1, sigma_v, wid, step_mult,
                                              step_exp, 40.0, cb_a, 0, sig_max, pscr);
             if (rc) return rc;
         }
         // FAST64, or no base (the whole (1 - A) is convolved): FP64
-        rc = launch_conv_fast<double, 4>(ctx, n, n_eff, d_wave, d_spec, spec_stride, n_spec, base_a ? 0 : 1,
+        rc = launch_conv_fast<4>(ctx, n, n_eff, d_wave, d_spec, spec_stride, n_spec, base_a ? 0 : 1,
                                          sigma_v, wid, step_mult, step_exp, base_a ? cut : 40.0, conv, n_eff,
                                          sig_max, pscr);
         if (rc) return rc;
