@@ -590,27 +590,27 @@ __global__ void __launch_bounds__(ADJ_THREADS, BC ? 4 : 3) k_adj_rows(const __gr
         const int *cell = A.cell + (long long)p * A.gm;
 #pragma unroll 1
         for (int c = 0; c < ADJ_CLASS; ++c) {
-            // shares wl (to o) and w1 (to o + 1) of pixel j; wls, w1s: with the intensity's factor
-            auto add = [&](int j, double wl, double w1, double wls, double w1s, double sed, int type) {
+            // shares wl (to o) and w1 (to o + 1; not without `up`, where a gradient that is not finite
+            // must not reach it) of pixel j; wls, w1s: with the intensity's factor
+            auto add = [&](int j, double wl, double w1, double wls, double w1s, double sed, int type, bool up) {
                 const double B = gb[j];
                 double q = wl * B, u = w1 * B, al = q, au = u;
                 if constexpr (!BC) {
                     const double F = gf[j], T = gt[j], h = F + T, x = sed * F, y = sed * T;
                     L[0] = fma(wl, h, L[0]);
-                    U[0] = fma(w1, h, U[0]);
+                    if (up) U[0] = fma(w1, h, U[0]);
                     q = fma(-wls, x, q);
                     u = fma(-w1s, x, u);
                     al = fma(wls, y, al);
                     au = fma(w1s, y, au);
                 }
                 L[1] += q;
-                U[1] += u;
-                if (type == 0) {
-                    L[2] -= al;
-                    U[2] -= au;
-                } else {
-                    L[3] -= al;
-                    U[3] -= au;
+                if (type == 0) L[2] -= al;
+                else L[3] -= al;
+                if (up) {
+                    U[1] += u;
+                    if (type == 0) U[2] -= au;
+                    else U[3] -= au;
                 }
             };
             auto sed_at = [&](int type, int j) { return BC ? 0.0 : (type == 0 ? A.spot_sed[j] : A.fac_sed[j]); };
@@ -643,12 +643,12 @@ __global__ void __launch_bounds__(ADJ_THREADS, BC ? 4 : 3) k_adj_rows(const __gr
                         }
                         if (!two) w1s = w1;
                     }
-                    add(j, s.s0 - w1, w1, (two ? s.t0 : s.s0) - w1s, w1s, sed_at(c, j), c);
+                    add(j, s.s0 - w1, w1, (two ? s.t0 : s.s0) - w1s, w1s, sed_at(c, j), c, true);
                 },
                 [&](const AdjRow &z) {   // no shift: pixel j is source j
                     if (o < 0 || o >= n_eff) return;
                     const bool end = o == n_eff - 1;   // without an interval above it: the cells at rest only
-                    add(o, end ? z.still0 : z.s0, 0.0, end ? z.still1 : z.t0, 0.0, sed_at(c, o), c);
+                    add(o, end ? z.still0 : z.s0, 0.0, end ? z.still1 : z.t0, 0.0, sed_at(c, o), c, false);
                 },
                 [&](int k) {
                     const AdjGeo &g = A.geo[cell[k]];
@@ -659,7 +659,7 @@ __global__ void __launch_bounds__(ADJ_THREADS, BC ? 4 : 3) k_adj_rows(const __gr
                                                : sed_at(type, j);
                     };
                     if (g.still != 0.0) {
-                        if (o >= 0 && o < n_eff) add(o, g.L, 0.0, g.L * sg, 0.0, sed_of(o), type);
+                        if (o >= 0 && o < n_eff) add(o, g.L, 0.0, g.L * sg, 0.0, sed_of(o), type, false);
                         return;
                     }
                     if (!own) return;
@@ -670,7 +670,7 @@ __global__ void __launch_bounds__(ADJ_THREADS, BC ? 4 : 3) k_adj_rows(const __gr
                     const double l1 = adj_shifted(lo, g.f);
                     for (long long j = ja; j < jb; ++j) {
                         const double w1 = g.L * ((lam[j] - l1) * g.iS * io), wl = g.L - w1;
-                        add((int)j, wl, w1, wl * sg, w1 * sg, sed_of((int)j), type);
+                        add((int)j, wl, w1, wl * sg, w1 * sg, sed_of((int)j), type, true);
                     }
                 });
         }

@@ -200,3 +200,29 @@ def test_scratch_of_large_maps(grid, n, n_phase, n_mu):
     for k in ref:
         bound = (41 + n_phase + (n >> 8) if k in ("limb", "delta") else 16 + n_phase + cnt[k]) * 2.0 ** -53 * mag[k]
         assert np.all(np.abs(got[k] - ref[k]) <= bound), k
+
+
+def test_gradients_that_are_not_finite_stay_at_their_pixels(ctx):
+    """Cells at rest copy their source: a NaN or infinite gradient of pixel j reaches source j of the
+    rows that enter that output and no other, for a row of cells and for one evaluated by itself (Planck
+    ratio)."""
+    n, n_mu, grid, step, at = 700, 2, 4, 0.01, 300
+    wave = 5000.0 + step * np.arange(n)
+    gm = grid * grid
+    maps = dict(delta=np.zeros(gm), limb=np.linspace(0.4, 1.0, gm), lb=np.full(gm, 0.1), region=np.zeros(gm, np.int32))
+    rng = np.random.default_rng(1)
+    x = {k: 1.0 + 0.3 * rng.uniform(-1, 1, (n_mu, n)) for k in ROWS}
+    x["spot_sed"], x["fac_sed"] = 0.3 + 0.1 * np.arange(n) / n, 1.0 + 0.1 * np.arange(n) / n
+    bi = np.tile(np.where(np.arange(gm) < 8, 0.0, 1.0), (1, 1))
+    for t_spot in (5115.0, 5115.5):
+        temp = np.where(bi == 0.0, t_spot, 5900.0)
+        for q, hit in ((0, ("q_sed", "q_norm")), (1, ("q_norm", "spot_norm", "fac_norm")),
+                       (2, ("q_sed", "spot_norm", "fac_norm"))):
+            for bad in (np.nan, np.inf):
+                g = rng.standard_normal((3, 1, n))
+                g[q, 0, at] = bad
+                got = ctx.phase_integrate_adjoint(wave, n, grid, temp, bi, maps, x, step,
+                                                  Activity(5778, 663, 250, 20, 0), *g)
+                for k in ROWS:
+                    bad_at = np.argwhere(~np.isfinite(got[k])).tolist()
+                    assert bad_at == ([[0, at]] if k in hit else []), (k, q, bad_at)
