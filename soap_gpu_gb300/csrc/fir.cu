@@ -2293,9 +2293,11 @@ __global__ void __launch_bounds__(FIR_THREADS, FIR_PP_MINB) k_fir_pp(const FirTi
         if constexpr (sizeof(T) == 4) {
             // Nearly every unit: no group of it leaves the grid at this tile, and no cell is at
             // rest.  No test per group then, and the spot class, whose four rows share one
-            // weight, forms two coefficient pairs per pixel instead of four (with the wrap
-            // cells' single test: 596 us against 613 for 100 phases of 310,000 px, 876
-            // against 914 for a batch's star; the shared-memory loads and their latency stay).
+            // weight, forms two coefficient pairs per pixel instead of four.  With the wrap
+            // cells' single test 591 us against 610 for 100 phases of 310,000 px and two regions
+            // apart, 3.25 ms against 3.35 for six stars of a batch (this branch alone 591 against
+            // 596, 3.25 against 3.28); with the benchmark's two regions one over the other 0.62 ms
+            // either way: the shared-memory loads and their latency stay.
             if (!zv && t_eff == FIR_TILE && j0 + d.ma >= 0 && j0 + FIR_TILE - 1 <= n_eff - 2 - d.mb) {
                 auto all = [&](auto fac_c) {
                     constexpr bool FAC = decltype(fac_c)::value;

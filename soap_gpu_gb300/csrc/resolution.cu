@@ -141,7 +141,8 @@ __global__ void __launch_bounds__(256) k_conv_plain64(int n, int n_eff, const do
 // over all taps takes 0.35 ms, so the bound lies where next to none is.)
 // Bound by the FP64 pipe: (2 reach + 1) x 2 instructions per pixel and spectrum and
 // (reach + 1) x 20 for the weights per pixel and block.  One spectrum of 310,000 px:
-// 3.28 -> 0.71 ms per call; 10 of 100,000 px: 13.9 -> 0.45 ms.
+// 3.28 -> 0.66 ms per call; with a continuum of exactly 1 between lines every 311 px, most of whose
+// sums are taken over all taps, 4.16 -> 1.58 ms; 10 of 100,000 px: 13.9 -> 0.45 ms.
 constexpr int CP_PIX = 128;
 constexpr double CP_CUT = 90.0;
 constexpr int CP_ZERO = 1023 - 790;   // exponent of what stands for a term of zero
