@@ -73,6 +73,7 @@ struct AdjRow {
 // sums over a range's cells, f0 its first cell's f: of L, L / S, (L / S) (f - f0), and with (1 + LB) L
 struct AdjSums {
     double f0, s0, s1, s2, t0, t1, t2;
+    int zone;               // of adj_residue; 0: an |f| beyond ADJ_W_MAX
 };
 
 struct AdjArgs {
@@ -392,6 +393,8 @@ __device__ __forceinline__ AdjSums adj_sum(const AdjEnt *__restrict__ ent, const
                                            int hi) {
     AdjSums s;
     s.f0 = fb[lo];
+    const double u = fmax(fabs(s.f0), fabs(fb[hi - 1]));   // they ascend
+    s.zone = u < ADJ_W_MAX ? (int)(u * (double)(1 << ADJ_FRAC)) + 3 : 0;
     s.s0 = s.s1 = s.s2 = s.t0 = s.t1 = s.t2 = 0.0;
     for (int k = lo + (threadIdx.x & 31); k < hi; k += 32) {
         const AdjEnt x = ent[k];
@@ -562,9 +565,9 @@ __device__ __forceinline__ void adj_residue(const AdjNoise *__restrict__ x, cons
 // ---- row gradients -----------------------------------------------------------------------
 // Block: ADJ_SRC source pixels of one row, lane l of a warp source o; lane 0 only gives its upper
 // share to lane 1.  BC: the bconv gradient alone (gF = gT = 0).  Bound by the residues' integer
-// instructions and their latency, so four and three blocks per SM although some registers spill (two:
-// 0.65 and 0.58 ms for 100 x 100 cells and 50,000 px, BC, and five phases of 200 x 200 and 100,000
-// px; so 0.53 and 0.48).
+// instructions and their latency, so four and three blocks per SM although some registers spill (three
+// and two: 0.49 and 0.56 ms for 100 x 100 cells and 50,000 px, BC, and five phases of 200 x 200 and
+// 100,000 px; so 0.47 and 0.46).
 template <bool BC>
 __global__ void __launch_bounds__(ADJ_THREADS, BC ? 4 : 3) k_adj_rows(const __grid_constant__ AdjArgs A,
                                                           const double *__restrict__ bi) {
@@ -579,6 +582,8 @@ __global__ void __launch_bounds__(ADJ_THREADS, BC ? 4 : 3) k_adj_rows(const __gr
     const double lo = own ? lam[o] : 0.0, io = own ? A.inv[o] : 0.0, beta = lo * io;
     const int ex = adj_exp(lo);
     const bool noisy = ex > 200 && ex < 1800;   // a wavelength whose ulp is a normal number
+    // no shift below ADJ_W_MAX takes l_o out of its binade: 2^-9 of it, 2^11 in the high word, from both ends
+    const bool inner = ((unsigned)__double2hiint(lo) & 0xfffffu) - 2048u < (1u << 20) - 4096u;
     const unsigned long long lm = ((unsigned long long)__double_as_longlong(lo) << 11) | 0x8000000000000000ULL;
     const double ulp = noisy ? __hiloint2double((ex - 52) << 20, 0) * io : 0.0;
     double L[4] = {0.0, 0.0, 0.0, 0.0}, U[4] = {0.0, 0.0, 0.0, 0.0};   // q_sed, q_norm, spot, facula: lower, upper
@@ -620,17 +625,16 @@ __global__ void __launch_bounds__(ADJ_THREADS, BC ? 4 : 3) k_adj_rows(const __gr
                 [&](int off, int k0, int k1, const AdjSums &s) {
                     const int j = o + off;
                     if (!own || j < 0 || j >= n_eff) return;
-                    const double lj = lam[j], f1 = fb[k1 - 1];
+                    const double lj = lam[j];
                     const bool two = !BC && c == 1;
                     double w1, w1s;
-                    // l' in l_o's binade for the range's extreme shifts, and |f| below ADJ_W_MAX
-                    if (noisy && row.even && adj_exp(fma(lo, s.f0, lo)) == ex && adj_exp(fma(lo, f1, lo)) == ex &&
-                        fmax(fabs(s.f0), fabs(f1)) < ADJ_W_MAX) {
+                    // |f| below ADJ_W_MAX, and l' in l_o's binade for the range's extreme shifts
+                    if (noisy && row.even && s.zone != 0 &&
+                        (inner || (adj_exp(fma(lo, s.f0, lo)) == ex && adj_exp(fma(lo, fb[k1 - 1], lo)) == ex))) {
                         const double rest = adj_rest(lj, lo, s.f0);
-                        const int zone = (int)(fmax(fabs(s.f0), fabs(f1)) * (double)(1 << ADJ_FRAC)) + 3;
                         double r, rs;
-                        if (two) adj_residue<true>(noise, fb, lo, lm, k0, k1, zone, r, rs);
-                        else adj_residue<false>(noise, fb, lo, lm, k0, k1, zone, r, rs);
+                        if (two) adj_residue<true>(noise, fb, lo, lm, k0, k1, s.zone, r, rs);
+                        else adj_residue<false>(noise, fb, lo, lm, k0, k1, s.zone, r, rs);
                         w1 = fma(io, fma(rest, s.s1, -lo * s.s2), -ulp * (row.unit * r));
                         w1s = two ? fma(io, fma(rest, s.t1, -lo * s.t2), -ulp * (row.unit_s * rs)) : w1;
                     } else {   // the forward's l' cell by cell
