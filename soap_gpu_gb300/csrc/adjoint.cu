@@ -564,8 +564,9 @@ __device__ __forceinline__ void adj_residue(const AdjNoise *__restrict__ x, cons
 
 // ---- row gradients -----------------------------------------------------------------------
 // Block: ADJ_SRC source pixels of one row, lane l of a warp source o; lane 0 only gives its upper
-// share to lane 1.  BC: the bconv gradient alone (gF = gT = 0).  Bound by the residues' integer
-// instructions and their latency, so four and three blocks per SM although some registers spill (three
+// share to lane 1.  BC: the bconv gradient alone (gF = gT = 0).  Bound by the FP64 pipe (71 % of
+// cycles, some twenty instructions per range and pixel) and the latency of the residues' integer
+// chains, so four and three blocks per SM although some registers spill (three
 // and two: 0.49 and 0.56 ms for 100 x 100 cells and 50,000 px, BC, and five phases of 200 x 200 and
 // 100,000 px; so 0.47 and 0.46).
 template <bool BC>
